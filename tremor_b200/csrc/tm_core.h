@@ -58,7 +58,7 @@ cudaError_t launch_prefix_totals(const float *clean, uint64_t n, const double *c
                                  cudaStream_t s);
 cudaError_t launch_prefix_sums(const float *clean, uint64_t n, const double *centres, double2 *totals,
                                double2 *block_totals, double2 *Q, cudaStream_t s);
-cudaError_t launch_runs(const float *clean, uint64_t n, uint16_t *run, uint16_t *run_tmp, cudaStream_t s);
+cudaError_t launch_runs(const float *clean, const float *raw, uint64_t n, uint16_t *run, uint32_t *first, cudaStream_t s);
 cudaError_t launch_passb_mixed(const uint2 *list, uint32_t items, const float *x, const float *raw, const double2 *P,
                                const double2 *PT, const double *PC, const uint16_t *run, const float *q,
                                const TemplParam *tp, const uint32_t *tkey, uint64_t w0, Candidate *cand,

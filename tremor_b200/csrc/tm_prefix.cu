@@ -12,8 +12,8 @@
 // record, and a block's centre follows a drifting offset.
 //
 // run[i] = number of consecutive samples equal to clean[i] starting at i (capped at
-// 65535): a window is constant, hence not searchable (std 0 in the reference), exactly
-// when run[j] >= m. Constant stretches (gaps filled with zeros, clipped data) are
+// 65535, and 65535 where the raw sample is missing): a window whose first sample is present
+// is constant, hence not searchable (std 0 in the reference), exactly when run[j] >= m. Constant stretches (gaps filled with zeros, clipped data) are
 // recognised without two-pass statistics.
 #include "tm_prefix.cuh"
 
@@ -130,32 +130,95 @@ __global__ void __launch_bounds__(PX_THREADS) k_prefix_apply(const float *__rest
         Q[0] = make_double2(0.0, 0.0);
 }
 
-// run[i]: samples equal to clean[i] from i on, capped. Round 0 looks ahead up to 16
-// samples; each later round doubles the cap by pointer jumping: a run that reaches the
-// cap continues with the (capped) run of the sample cap positions later when that sample
-// has the same value. O(n log cap) in every case, constant stretches included.
-__global__ void k_run_init(const float *__restrict__ clean, uint64_t n, uint16_t *__restrict__ run)
+// run[i]: samples equal to clean[i] from i on, capped at 65535; 65535 too where the raw
+// sample i is missing (a window that starts there is not searched, like a constant one). A
+// run ends at the first j >= i with j = n - 1 or clean[j] != clean[j + 1]: pass 1 finds each
+// chunk's first end, pass 2 scans a chunk's ends backwards, with the first end of the chunks
+// after it as carry (with the cap, at most the next 9 chunks matter). Two reads of the
+// record: 0.16 ms for 2^25 samples, where doubling the look-ahead from 16 samples took 13
+// launches and 0.80 ms.
+constexpr uint32_t kNoEnd = 0xffffffffu; // relative ends are below 2^31
+
+__device__ __forceinline__ uint32_t run_ends(const float *__restrict__ clean, uint64_t n, uint64_t base, uint32_t *ends)
 {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+    // ends[k]: k itself, relative to the thread's 8 samples, if a run ends there, else the next end
+    float v[PX_PER_THREAD + 1];
+#pragma unroll
+    for (int k = 0; k <= PX_PER_THREAD; k++)
+        v[k] = base + k < n ? clean[base + k] : 0.0f;
+    uint32_t next = kNoEnd;
+#pragma unroll
+    for (int k = PX_PER_THREAD - 1; k >= 0; k--)
     {
-        const float v = clean[i];
-        uint32_t len = 1;
-        while (len < 16u && i + len < n && clean[i + len] == v)
-            len++;
-        run[i] = (uint16_t)len;
+        if (base + k < n && (base + k + 1 == n || v[k] != v[k + 1]))
+            next = (uint32_t)k;
+        ends[k] = next;
     }
+    return next;
 }
 
-__global__ void k_run_double(const float *__restrict__ clean, uint64_t n, uint32_t cap,
-                             const uint16_t *__restrict__ in, uint16_t *__restrict__ out)
+__global__ void __launch_bounds__(PX_THREADS) k_run_first(const float *__restrict__ clean, uint64_t n,
+                                                          uint32_t *__restrict__ first)
 {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+    __shared__ uint32_t best;
+    if (threadIdx.x == 0)
+        best = kNoEnd;
+    __syncthreads();
+    uint32_t ends[PX_PER_THREAD];
+    const uint32_t off = threadIdx.x * PX_PER_THREAD;
+    const uint32_t e = run_ends(clean, n, (uint64_t)blockIdx.x * PX_CHUNK + off, ends);
+    const uint32_t m = __reduce_min_sync(0xffffffffu, e == kNoEnd ? kNoEnd : off + e);
+    if ((threadIdx.x & 31) == 0 && m != kNoEnd)
+        atomicMin(&best, m);
+    __syncthreads();
+    if (threadIdx.x == 0)
+        first[blockIdx.x] = best;
+}
+
+__global__ void __launch_bounds__(PX_THREADS) k_run_apply(const float *__restrict__ clean, const float *__restrict__ raw,
+                                                          uint64_t n, const uint32_t *__restrict__ first, uint32_t chunks,
+                                                          uint16_t *__restrict__ run)
+{
+    __shared__ uint32_t warp_first[PX_THREADS / 32], after;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t ends[PX_PER_THREAD];
+    const uint32_t off = threadIdx.x * PX_PER_THREAD;
+    const uint64_t base = (uint64_t)blockIdx.x * PX_CHUNK + off;
+    const uint32_t e = run_ends(clean, n, base, ends);
+    // the first end at or after this thread's samples, within the warp
+    uint32_t scan = e == kNoEnd ? kNoEnd : off + e;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1)
     {
-        uint32_t len = in[i];
-        if (len == cap && i + cap < n && clean[i + cap] == clean[i])
-            len += in[i + cap];
-        out[i] = (uint16_t)min(len, 65535u);
+        const uint32_t o = __shfl_down_sync(0xffffffffu, scan, d);
+        if (lane + d < 32)
+            scan = min(scan, o);
     }
+    if (lane == 0)
+        warp_first[warp] = scan;
+    if (threadIdx.x == 0)
+    {
+        after = kNoEnd;
+        for (uint32_t c = 1; c <= 9 && blockIdx.x + c < chunks && after == kNoEnd; c++)
+            if (first[blockIdx.x + c] != kNoEnd)
+                after = c * PX_CHUNK + first[blockIdx.x + c];
+    }
+    __syncthreads();
+    uint32_t next = __shfl_down_sync(0xffffffffu, scan, 1); // the first end after this thread's samples
+    if (lane == 31)
+        next = kNoEnd;
+    for (int w = warp + 1; w < PX_THREADS / 32 && next == kNoEnd; w++)
+        next = warp_first[w];
+    if (next == kNoEnd)
+        next = after;
+#pragma unroll
+    for (int k = 0; k < PX_PER_THREAD; k++)
+        if (base + k < n)
+        {
+            const uint32_t end = ends[k] != kNoEnd ? off + ends[k] : next;
+            const uint32_t len = end == kNoEnd ? 65535u : min(end - (off + k) + 1u, 65535u);
+            run[base + k] = (uint16_t)(raw[base + k] == kMissing ? 65535u : len);
+        }
 }
 
 uint32_t prefix_chunks(uint64_t n) { return (uint32_t)((n + PX_CHUNK - 1) / PX_CHUNK); }
@@ -181,19 +244,12 @@ cudaError_t launch_prefix_sums(const float *clean, uint64_t n, const double *cen
     return cudaGetLastError();
 }
 
-// run and run_tmp: n uint16 each; the result ends in `run`.
-cudaError_t launch_runs(const float *clean, uint64_t n, uint16_t *run, uint16_t *run_tmp, cudaStream_t s)
+// first: scratch of prefix_chunks(n) entries.
+cudaError_t launch_runs(const float *clean, const float *raw, uint64_t n, uint16_t *run, uint32_t *first, cudaStream_t s)
 {
-    // 16 -> 32 -> ... -> 65536: 12 doublings, an even number, so the result ends in `run`
-    k_run_init<<<1184, 256, 0, s>>>(clean, n, run);
-    uint16_t *a = run, *b = run_tmp;
-    for (uint32_t cap = 16; cap < 65536u; cap *= 2)
-    {
-        k_run_double<<<1184, 256, 0, s>>>(clean, n, cap, a, b);
-        uint16_t *t = a;
-        a = b;
-        b = t;
-    }
+    const uint32_t chunks = prefix_chunks(n);
+    k_run_first<<<chunks, PX_THREADS, 0, s>>>(clean, n, first);
+    k_run_apply<<<chunks, PX_THREADS, 0, s>>>(clean, raw, n, first, chunks, run);
     return cudaGetLastError();
 }
 

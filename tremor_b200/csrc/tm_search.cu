@@ -74,9 +74,9 @@ void ensure_prefix(tm_ctx *ctx, Lane &L)
     ctx->pcen.reserve(sizeof(double) * (blocks + 1));
     TM_CUDA(cudaMemsetAsync(ctx->ptot.p, 0, sizeof(double2) * (blocks + 1), s));
     ctx->run.reserve(sizeof(uint16_t) * n);
-    DevBuf totals, run_tmp;
+    DevBuf totals, run_first;
     totals.reserve(sizeof(double2) * chunks);
-    run_tmp.reserve(sizeof(uint16_t) * n);
+    run_first.reserve(sizeof(uint32_t) * chunks);
     // centres: the mean of each block, from uncentred chunk sums
     TM_CUDA(tmb::launch_prefix_totals(ctx->clean.as<float>(), n, nullptr, totals.as<double2>(), s));
     std::vector<double2> ct(chunks);
@@ -96,11 +96,12 @@ void ensure_prefix(tm_ctx *ctx, Lane &L)
     TM_CUDA(cudaMemcpyAsync(ctx->pcen.p, centres.data(), sizeof(double) * (blocks + 1), cudaMemcpyHostToDevice, s));
     TM_CUDA(tmb::launch_prefix_sums(ctx->clean.as<float>(), n, ctx->pcen.as<double>(), totals.as<double2>(),
                                     ctx->ptot.as<double2>(), ctx->prefix.as<double2>(), s));
-    TM_CUDA(tmb::launch_runs(ctx->clean.as<float>(), n, ctx->run.as<uint16_t>(), run_tmp.as<uint16_t>(), s));
+    TM_CUDA(tmb::launch_runs(ctx->clean.as<float>(), ctx->raw.as<float>(), n, ctx->run.as<uint16_t>(),
+                             run_first.as<uint32_t>(), s));
     TM_CUDA(cudaStreamSynchronize(s));
-    count_launch(L, 4 + 13);
+    count_launch(L, 4 + 2);
     totals.release();
-    run_tmp.release();
+    run_first.release();
     ctx->prefix_ready = true;
 }
 
