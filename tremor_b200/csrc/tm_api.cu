@@ -73,7 +73,10 @@ static void bound_diagnostics_wm(tm_ctx *ctx, int m, const std::vector<int> &idx
     a.n = ctx->n;
     a.col_tile = g.col_tile;
     if (ctx->tiles == TM_TILES_FFT)
+    {
+        prepare_fft(ctx, L, g);
         fft_contract(ctx, L, g, a);
+    }
     else
     {
         TM_CUDA(g.col_tile > 0 ? tmb::launch_scan_wm(a, s) : tmb::launch_scan_umma(a, s));
@@ -165,9 +168,11 @@ int tm_ctx_destroy(tm_ctx *ctx)
         kv.second->flags.release();
     }
     for (DevBuf *b : {&ctx->prefix, &ctx->ptot, &ctx->pcen, &ctx->run, &ctx->raw, &ctx->clean, &ctx->suf,
-                      &ctx->fft2_X, &ctx->fft2_shift, &ctx->fft2_norm, &ctx->fft3_X, &ctx->fft3_shift,
-                      &ctx->fft3_norm, &ctx->fft_roots, &ctx->fft_scratch})
+                      &ctx->fft_roots})
         b->release();
+    for (tm_ctx::FftPieces &f : ctx->fft)
+        for (DevBuf *b : {&f.X, &f.shift, &f.norm})
+            b->release();
     // buffers of batches that outlive the context return to the pool when those batches
     // are destroyed; the driver releases the pool's memory once none is outstanding
     if (ctx->pool)

@@ -268,8 +268,8 @@ struct Lane
     std::vector<std::shared_ptr<PinnedBlock>> pool;
     HostBuf h_split, h_q, h_order, h_slots, h_counters;
     uint32_t cand_cap = 1u << 22, list_cap = 1u << 20;
-    // FFT branch: the template spectra and rows of a launch (both piece lengths)
-    DevBuf fft2_Y, fft3_Y, fft_rows, fft_stats, fft_gmax; // (fft_stats: the correlation kernels' per-block statistics cache; fft_gmax: per row, its length's largest bound coefficients)
+    // FFT branch: the template spectra of a launch
+    DevBuf fft_Y, fft_stats; // (fft_stats: the correlation kernel's per-block statistics cache)
     // instrumentation
     bool profile = false;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr, ev3 = nullptr, ev4 = nullptr;
@@ -293,7 +293,7 @@ struct Lane
         if (stream)
             cudaStreamSynchronize(stream);
         for (DevBuf *b : {&tkey, &bmin_u, &bmin_l, &list, &counters, &cand, &dist, &fp32_qt, &akeys, &avals, &avals64, &sort_tmp,
-                          &segs, &fft2_Y, &fft3_Y, &fft_rows, &fft_stats, &fft_gmax})
+                          &segs, &fft_Y, &fft_stats})
             b->release();
         for (HostBuf *b : {&h_split, &h_q, &h_order, &h_slots, &h_counters})
             b->release();
@@ -342,19 +342,22 @@ struct tm_ctx
     // their block totals and centres, constant runs
     tmh::DevBuf prefix, ptot, pcen, run;
     bool prefix_ready = false;
-    // FFT branch (tm_fftk.cu), built on first use: spectra of pieces of 16384 samples every
-    // 8192 (templates of up to 8192 samples) and of pieces of 32768 every 16384 (longer ones),
-    // their shifts and norms; the twiddle tables; the forward transforms' scratch
-    tmh::DevBuf fft2_X, fft2_shift, fft2_norm, fft3_X, fft3_shift, fft3_norm, fft_roots, fft_scratch;
-    uint32_t fft2_P = 0, fft3_P = 0;
-    bool fft2_ready = false, fft3_ready = false;
+    // FFT branch (tm_fftk.cu): per class of template lengths, built on first use, the spectra
+    // of its pieces, their shifts and norms; the twiddle tables
+    struct FftPieces
+    {
+        tmh::DevBuf X, shift, norm;
+        uint32_t count = 0;
+        bool ready = false;
+    } fft[tmb::kFftClasses];
+    tmh::DevBuf fft_roots;
     std::mutex fft_mu;
     int sms = 148;
     // model: the FFT branch's ms per template per 2^25 samples, for templates of up to 8192
     // samples (the fused kernels) and longer ones, templates of distinct lengths (B200 defaults;
     // tm_autotune measures both)
-    double fft_ms = 0.71;
-    double fft_long_ms = 1.07;
+    double fft_ms = 0.307;
+    double fft_long_ms = 0.63;
     // the context's own memory pool for per-batch buffers (DevBuf::reserve_on); it keeps
     // up to 4 GiB of freed memory for the next batch
     cudaMemPool_t pool = nullptr;
@@ -416,7 +419,16 @@ struct GroupPlan
     // k_scan_umma or, when col_tile > 0, in column tiles of col_tile rows of k_scan_wm
     bool mixed = false;
     int col_tile = 0;
-    bool fft = false; // FFT branch (tm_fft.cu) instead of a contraction kernel
+    bool fft = false; // FFT branch (tm_fftk.cu) instead of a contraction kernel
+    // its launches: rows of one class and number of parts, at [first, first + count) of the
+    // row list
+    struct FftSet
+    {
+        int cls, parts, first, count;
+    };
+    std::vector<FftSet> fft_sets;
+    std::vector<tmb::FftRow> fft_rows;
+    DevBuf d_fft;
     int k_stride = 0;            // row stride of the template arrays
     uint32_t w_max = 0;          // windows of the shortest template
     std::vector<tmb::TileInfo> tiles; // per tile: K blocks
@@ -424,6 +436,7 @@ struct GroupPlan
     void release()
     {
         d_tiles.release();
+        d_fft.release();
         q_hi.release();
         q_lo.release();
         q.release();
@@ -461,6 +474,7 @@ void prepare_group(tm_ctx *ctx, Lane &L, int m, const std::vector<int> &idx, con
                    uint64_t &h2d, int col_tile = 0);
 void prepare_group_mixed(tm_ctx *ctx, Lane &L, const std::vector<int> &idx_in, const tm_request *reqs, GroupPlan &g,
                          uint64_t &h2d, int col_tile = 0);
+void prepare_fft(tm_ctx *ctx, Lane &L, GroupPlan &g);
 int plan_col_tile(const tm_ctx *ctx, const tm_request *reqs, const std::vector<int> &idx, double *cost = nullptr);
 double tile_time(const tm_ctx *ctx, bool mixed, int v, double k);
 void create_batch(tm_ctx *ctx, Lane &L, const tm_request *requests, int count, tm_batch &b, bool serving = false);

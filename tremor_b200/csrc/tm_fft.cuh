@@ -6,31 +6,61 @@
 
 namespace tmb {
 
-// Pieces of kF2L samples every kF2S samples serve templates of up to kF2S samples; pieces of
-// kF3L samples every kF3S serve the longer ones, up to kFftMaxM. Real transforms of length L
-// go through complex ones of L / 2 points.
-constexpr int kF2L = 16384;
-constexpr int kF2S = 8192;
-constexpr int kF2N = kF2L / 2;
-constexpr int kF2H = kF2L / 2 + 1;
-constexpr int kF3L = 32768;
-constexpr int kF3S = 16384;
-constexpr int kF3N = kF3L / 2;
-constexpr int kF3H = kF3L / 2 + 1;
-constexpr int kFftMaxM = kF3S; // longest template of the FFT branch
-
-struct Fft2Args
+// Pieces of 2 n samples, one every `step` (tm_fftk.cu). A template of up to 2 n - step + 1
+// samples has every window of a piece in one transform; a longer one is cut in parts of
+// `step` samples.
+struct FftClass
 {
-    const double2 *X;             // piece spectra, kF2H (or kF3H) bins per piece
+    int n;
+    uint32_t step;
+};
+constexpr int kFftClasses = 4;
+__host__ __device__ constexpr FftClass fft_class(int cls)
+{
+    return cls == 0   ? FftClass{4096, 7168}
+           : cls == 1 ? FftClass{4096, 6144}
+           : cls == 2 ? FftClass{8192, 12288}
+                      : FftClass{8192, 8192};
+}
+// entries of a spectrum: its n + 1 bins in whole 128-byte lines
+__host__ __device__ constexpr int fft_pitch(int n) { return n + 8; }
+constexpr int kFftMaxM = 16384; // longest template of the FFT branch
+constexpr int kFftMaxParts = 2;
+inline int fft_class_of(int m) { return m <= 1025 ? 0 : m <= 2049 ? 1 : m <= 4097 ? 2 : 3; }
+inline int fft_parts(int m, int cls)
+{
+    const int single = 2 * fft_class(cls).n - (int)fft_class(cls).step + 1, step = (int)fft_class(cls).step;
+    return m <= single ? 1 : (m + step - 1) / step;
+}
+
+// One template of a correlation launch. The bound coefficients (a1_main, a2, a5, a6), qs and
+// |s1| are the largest of the launch's templates of its length.
+struct FftRow
+{
+    double inv_m;
+    double sum[kFftMaxParts - 1]; // the sums of its parts after the first
+    float s1, c_lin, a3, thr;
+    float4 c0;
+    float qs, s1_max;
+    int row; // its row in tp
+    int m, mode;
+    uint32_t wcount;
+    int pad[2];
+};
+
+struct FftArgs
+{
+    const double2 *X;             // piece spectra, fft_pitch(n) entries per piece
     const double *shifts, *norms; // per piece: its shift s_p and ||x - s_p||_2
+    uint32_t pieces, step;        // pieces of the record, samples between their starts
     uint32_t p_first, p_count;    // pieces of this launch
-    const double2 *Y;             // template spectra, one per entry of rows
-    const int *rows;              // the launch's template rows (indices into tp)
-    int nrows;
-    const TemplParam *tp;
-    const double2 *roots;         // twiddle tables (fft_roots)
+    const double2 *Y;             // template spectra, one per part and entry of rows
+    const FftRow *rows;           // the launch's templates, equal lengths adjacent
+    int nrows, parts;
+    const double2 *tabs;          // twiddle tables of the correlation kernel
     uint64_t w0;                  // window range start (windows are relative to it)
     uint32_t W;
+    uint64_t n;                   // samples of the record
     PrefixView pv;
     const uint16_t *run;
     const float *raw;
@@ -39,33 +69,22 @@ struct Fft2Args
     Candidate *cand;
     uint32_t *cand_count, cand_cap;
     float *dbg_d, *dbg_e; // diagnostics: d and e of every window, [t][W]; null in searches
-    float4 *stats;        // per block, kFftCache windows' folded statistics of the current piece (a lane's scratch)
-    // per template row t, the largest bound coefficients of the launch's templates of its
-    // length: gmax[2 t] = (a1_main, a2, a5, a6), gmax[2 t + 1] = (qs, |s1|, 0, 0)
-    const float4 *gmax;
+    float4 *stats;        // per block, the folded statistics of a piece's windows (a lane's scratch, kFftStats)
 };
 
-// Work items of one half of a kF3 piece's epilogue (one complex output each, two windows),
-// rounded up; a block's statistics cache holds two windows per item of both halves.
-constexpr int kF3Items = 4104;
-constexpr int kFftCache = 4 * kF3Items;
+// float4s of the statistics scratch per SM: 3 floats per output, two blocks of the shorter
+// transform or one of the longer
+constexpr int kFftStats = 3 * (16384 / 4);
 
-constexpr int kFftRoots = 384; // entries of the twiddle tables
-constexpr int kFftScratchPts = 8192; // complex points of a block's slice of the forward scratch
+constexpr int kFftRoots = 384; // entries of the forward kernel's twiddle tables; the correlation kernels' follow
+constexpr int kFftAllRoots = kFftRoots + (513 + 64 + 128) + (257 + 32 + 64);
 
-uint32_t fft2_pieces(uint64_t n);
-uint32_t fft3_pieces(uint64_t n);
-void fft_roots(double2 *host384);
-cudaError_t launch_fft2_pieces(const float *clean, uint64_t n, const double *centres, uint32_t p0, uint32_t count,
-                               const double2 *roots, double2 *X, double *shifts, double *norms, cudaStream_t s);
-cudaError_t launch_fft2_templates(const float *q, const TemplParam *tp, const int *rows, int nrows,
-                                  const double2 *roots, double2 *Y, cudaStream_t s);
-cudaError_t launch_fft2_corr(const Fft2Args &a, int sms, cudaStream_t s);
-cudaError_t launch_fft3_pieces(const float *clean, uint64_t n, const double *centres, uint32_t p0, uint32_t count,
-                               const double2 *roots, double2 *X, double *shifts, double *norms, double2 *scratch,
-                               int blocks, cudaStream_t s);
-cudaError_t launch_fft3_templates(const float *q, const TemplParam *tp, const int *rows, int nrows,
-                                  const double2 *roots, double2 *Y, double2 *scratch, int blocks, cudaStream_t s);
-cudaError_t launch_fft3_corr(const Fft2Args &a, int sms, cudaStream_t s);
+uint32_t fft_pieces(uint64_t n, int cls);
+void fft_roots(double2 *host); // kFftAllRoots entries
+cudaError_t launch_fft_pieces(const float *clean, uint64_t n, const double *centres, int cls, const double2 *roots,
+                              double2 *X, double *shifts, double *norms, cudaStream_t s);
+cudaError_t launch_fft_templates(const float *q, const TemplParam *tp, const FftRow *rows, int nrows, int cls, int parts,
+                                 const double2 *roots, double2 *Y, cudaStream_t s);
+cudaError_t launch_fft_corr(FftArgs a, int cls, const double2 *roots, int sms, cudaStream_t s);
 
 } // namespace tmb

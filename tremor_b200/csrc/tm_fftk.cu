@@ -6,44 +6,45 @@
 // window and the distance filter with an error bound) has this structure; here neither the
 // product spectrum nor the correlation leaves the SM.
 //
-// Two piece lengths, both with the step half the length (the window j = p S + o,
-// 0 <= o < S, of piece p has its dot product at output o + m - 1 of the circular
-// correlation, which does not wrap for m <= L - S + 1); each piece is shifted by s_p, the
-// centre of the prefix block holding its start, rounded to float:
-//   L = 16384, S = 8192  (kF2*): templates of up to 8192 samples;
-//   L = 32768, S = 16384 (kF3*): templates of up to 16384 samples.
+// Pieces of L samples, one every S; the window j = p S + o, 0 <= o < S, of piece p has its dot
+// product at output o + m - 1 of the circular correlation, which does not wrap for m <= L - S
+// + 1. The work per piece does not depend on S, so the step is as large as the template's
+// length allows (fft_class_of): L = 8192 and S = 7168 or 6144 for templates of up to 1025 or
+// 2049 samples, L = 16384 and S = 12288 up to 4097 samples and 8192 above. Two blocks of the
+// shorter pieces share an SM and overlap; at 2049 samples and above the shorter pieces' wasted
+// outputs cost more than that gains (m = 4096: 0.259 ms per template and 2^25 samples with L =
+// 8192, 0.224 with 16384; m = 1024: 0.181 against 0.212). A template longer than 8192 samples
+// is cut in two parts whose products are added before the one inverse transform (part 1 meets
+// the next piece, whose start is 8192 samples later):
+//     V[k] = X_p[k] Y_0[k] + X_{p+1}[k] Y_1[k],
+// so its cost per window is that of a short template plus a second product. Each piece is
+// shifted by s_p, the centre of the prefix block holding its start, rounded to float (the
+// second part's other shift is corrected by (s_{p+1} - s_p) sum q_1 on the dot product).
 //
 // Real transforms of length L go through complex ones of N = L / 2 points:
 //   forward: z[n] = x[2n] + i x[2n+1], Z = FFT_N(z),
 //            X[k] = (Z[k] + conj Z[N-k]) / 2 - i e^{-2 pi i k / L} (Z[k] - conj Z[N-k]) / 2;
-//   inverse: for a Hermitian spectrum V (V[k] = X[k] Y[k]),
+//   inverse: for a Hermitian spectrum V,
 //            C[k] = (V[k] + conj V[N-k]) + i e^{2 pi i k / L} (V[k] - conj V[N-k]),
 //            c = IFFT_N(C) (unnormalised), out[2n] = Re c[n], out[2n+1] = Im c[n],
-//            and out / L is the circular correlation of x with the reversed template.
-// Every complex transform is built from 8192-point ones, Stockham radix-16, 16, 16 then 2
-// (Govindaraju et al., "High Performance Discrete Fourier Transforms on Graphics
-// Processors", SC 2008): 512 threads, each holding 16 points in registers between a pass's
-// shared-memory read and its write, so every pass works in place; the buffer is padded by
-// one point per 16 so that the first pass's stride-16 writes hit distinct banks. The final
-// radix-2 pass of an inverse is evaluated where its outputs are read (by the distance
-// epilogue). For N = 16384 the forward transform splits z into its even and odd points
-// (Z[k] = E[k] + W^k O[k], Z[k + 8192] = E[k] - W^k O[k], W = e^{-2 pi i / 16384}); the
-// inverse splits C the other way (a[n] = C[n] + C[n + 8192] gives c[2k], b[n] = (C[n] -
-// C[n + 8192]) e^{2 pi i n / 16384} gives c[2k + 1]), two 8192-point passes per piece.
+//            and out / L is the circular correlation of x with the reversed template (the
+//            templates' spectra carry the exact factor 1 / L).
 //
-// Twiddles: e^{2 pi i e / 32768} = R2[e >> 7] R1[e & 127] from tables of 128 and 256 entries
-// computed on the host in extended precision and rounded (error <= 4u with u = 2^-53, the
-// product included); a pass's powers w^r (r = 1..15) by repeated multiplication (error
-// <= 7 r u <= 105u). Error of an output (Higham, Accuracy and Stability of Numerical
-// Algorithms, Thm 24.2, ||fl(FFT x) - FFT x||_2 <= t eta / (1 - t eta) ||FFT x||_2,
-// eta = mu + gamma_4 (sqrt 2 + mu), mu the twiddle error): with mu = 105u, t = log2 L + 2
-// (the complex stages plus the real-transform packing and the even/odd split) and a factor
-// 10 for the radix-16 and packing arithmetic, kappa = 10 t 111u. With X = FFT(x - s_p),
-// Y = FFT(reversed q), ||X||_2 = sqrt(L) ||x - s_p||_2, ||Y||_inf <= ||q||_1 <= sqrt(m)
+// Twiddles of the forward transforms: e^{2 pi i e / 32768} = R2[e >> 7] R1[e & 127] from
+// tables of 128 and 256 entries computed on the host in extended precision and rounded
+// (error <= 4u with u = 2^-53, the product included); a pass's powers w^r (r = 1..15) by
+// repeated multiplication (error <= 7 r u <= 105u). Those of the inverse come from tables of
+// the same precision, their powers and products with 16th roots of unity by at most four
+// multiplications (error <= 40u). Error of an output (Higham, Accuracy and Stability of
+// Numerical Algorithms, Thm 24.2, ||fl(FFT x) - FFT x||_2 <= t eta / (1 - t eta)
+// ||FFT x||_2, eta = mu + gamma_4 (sqrt 2 + mu), mu the twiddle error): with mu = 105u,
+// t = 16 = log2 16384 + 2 (the complex stages plus the real-transform packing) and a factor 10 for
+// the higher-radix and packing arithmetic, kappa = 10 t 111u. With X = FFT(x - s_p), Y =
+// FFT(reversed q), ||X||_2 = sqrt(L) ||x - s_p||_2, ||Y||_inf <= ||q||_1 <= sqrt(m)
 // ||q||_2: ||fl(X) fl(Y) - X Y||_2 <= kappa sqrt(L) ||x - s_p|| ||q|| (sqrt m + sqrt L)
 // (+ rounding), and the inverse adds kappa ||X Y||_2 <= kappa sqrt(L) ||x - s_p|| sqrt(m)
 // ||q||, so every correlation output is within kappa ||x - s_p||_2 ||q||_2 (2 sqrt m +
-// sqrt L) of the exact one.
+// sqrt L) of the exact one; two parts add their bounds.
 #include <cmath>
 
 #include "../../include/tremor_b200.h"
@@ -52,13 +53,11 @@
 
 namespace tmb {
 
-constexpr int kF2T = 512;                        // threads per block
-constexpr int kFPts = 8192;                      // points of the in-shared-memory transforms
-constexpr int kF2Buf = kFPts + kFPts / 16 + 16;  // padded complex entries of the work buffer
-constexpr int kFRoots = 384;                     // twiddle table entries (R1 then R2)
-constexpr double kF2Kappa = 10.0 * 16.0 * 111.0 * 1.1102230246251565e-16;
-constexpr double kF3Kappa = 10.0 * 17.0 * 111.0 * 1.1102230246251565e-16;
-constexpr size_t kF2Smem = sizeof(double2) * (size_t)(kF2Buf + kFRoots);
+// The forward transform's block of N / 16 threads: its work buffer, padded complex entries,
+// and the twiddle tables (R1 then R2).
+template <int N> constexpr int kFBuf = N + N / 16 + 16;
+template <int N> constexpr size_t kFSmem = sizeof(double2) * (size_t)(kFBuf<N> + kFftRoots);
+constexpr double kFftKappa = 10.0 * 16.0 * 111.0 * 1.1102230246251565e-16;
 
 __device__ __forceinline__ int pidx(int i) { return i + (i >> 4); }
 
@@ -68,6 +67,7 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b)
 }
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ double2 cscale(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
 __device__ __forceinline__ double2 conj2(double2 a) { return make_double2(a.x, -a.y); }
 // a * (s i): s = +1 or -1
 template <int S> __device__ __forceinline__ double2 mul_si(double2 a)
@@ -132,15 +132,15 @@ template <int S> __device__ __forceinline__ void dft16(double2 (&v)[16])
         }
 }
 
-// One Stockham radix-16 pass over the padded buffer (N = 8192, 512 threads, in place: every
+// One Stockham radix-16 pass over the padded buffer of N points (N / 16 threads, in place: every
 // thread reads its 16 points, the block synchronises, then every thread writes).
-template <int S> __device__ __forceinline__ void pass16(double2 *buf, const double2 *R, int Ns)
+template <int N, int S> __device__ __forceinline__ void pass16(double2 *buf, const double2 *R, int Ns)
 {
     const int j = threadIdx.x;
     double2 v[16];
 #pragma unroll
     for (int r = 0; r < 16; r++)
-        v[r] = buf[pidx(j + 512 * r)];
+        v[r] = buf[pidx(j + N / 16 * r)];
     __syncthreads();
     const int k = j & (Ns - 1);
     if (Ns > 1)
@@ -163,257 +163,72 @@ template <int S> __device__ __forceinline__ void pass16(double2 *buf, const doub
     __syncthreads();
 }
 
-// The three radix-16 passes of an 8192-point transform; the radix-2 pass is left to the
-// caller (final_out, or the forward kernel's explicit pass).
-template <int S> __device__ __forceinline__ void fft8192_r16(double2 *buf, const double2 *R)
-{
-    pass16<S>(buf, R, 1);
-    pass16<S>(buf, R, 16);
-    pass16<S>(buf, R, 256);
-}
-
-// Output i (0 <= i < 8192) of the final radix-2 pass: c[i] = a + w b, c[i + 4096] = a - w b
-// with a = buf[i mod 4096], b = buf[i mod 4096 + 4096], w = e^{S 2 pi i (i mod 4096) / 8192}.
-template <int S> __device__ __forceinline__ double2 final_out(const double2 *buf, const double2 *R, int i)
-{
-    const int i0 = i & 4095;
-    const double2 a = buf[pidx(i0)], b = cmul(buf[pidx(i0 + 4096)], root<S>(R, 4 * i0));
-    return i < 4096 ? cadd(a, b) : csub(a, b);
-}
-
 __device__ __forceinline__ void load_roots(double2 *R, const double2 *roots)
 {
-    for (int i = threadIdx.x; i < kFRoots; i += blockDim.x)
+    for (int i = threadIdx.x; i < kFftRoots; i += blockDim.x)
         R[i < 128 ? r1_slot(i) : i] = roots[i];
 }
 
-// What the epilogue reads from global memory for one window: its prefix sums at the start
-// and the end, its first sample and its constant run. The epilogues load these for a few
-// windows at once before evaluating any of them, so that the loads overlap (with one block
-// of 512 threads per SM there are too few warps to hide one load's latency at a time).
-struct WinIn
+// Where a spectrum holds bin k (0 <= k <= N). The correlation kernel reads the bins in pairs
+// k, N - k (32 bytes), with Q = N / 8 thread t of Q / 2 the pairs of bins t + Q r, r < 8 (thread
+// 0: Q r, r < 4, and Q / 2 + Q (r - 4), r >= 4): pair (r, t) is at 2 (r Q / 2 + t), bin N / 2
+// after them.
+template <int N> __device__ __forceinline__ int spectrum_slot(int k)
 {
-    double2 qa, qb;
-    float raw;
-    uint32_t run;
-};
-
-__device__ __forceinline__ WinIn load_window(const Fft2Args &a, int m, bool in_range, uint64_t g)
-{
-    WinIn w;
-    if (in_range)
-    {
-        w.qa = a.pv.Q[g];
-        w.qb = a.pv.Q[g + (uint64_t)m];
-        w.raw = a.raw[g];
-        w.run = a.run[g];
-    }
-    else
-    {
-        w.qa = w.qb = make_double2(0.0, 0.0);
-        w.raw = kMissing;
-        w.run = 0;
-    }
-    return w;
+    constexpr int Q = N / 8, T = Q / 2;
+    if (k == N / 2)
+        return N;
+    const int res = k & (Q - 1);
+    const bool second = res == 0 || res == T ? k > N / 2 : res > T; // the pair's first bin is N - k
+    const int f = second ? N - k : k, t = f & (Q - 1);
+    const int r = t == T ? 4 + f / Q : f / Q;
+    return 2 * (T * r + (t == T ? 0 : t)) + (second ? 1 : 0);
 }
 
-// A window's statistics as the epilogue uses them, for one template length: x = mean,
-// y = 1 / std, z and w the two factors of its error term (WindowStats::rel_sd, e_mu);
-// y == 0: the window is not searched (outside the range, first sample missing, constant);
-// y < 0: its statistics are not trusted (it is re-scored exactly whatever its distance).
-// They do not depend on the template: the epilogues fold them (fold_window) and keep them in
-// the block's slice of a global scratch (L2-resident) for the next template of the same
-// length in the same piece.
-// Single-block, well-conditioned windows take the fast path (prefix_stats_fast), the others
-// the full bound.
-__device__ __forceinline__ float4 window_stats4(const Fft2Args &a, int m, double inv_m, bool in_range, uint64_t g,
-                                                const WinIn &w)
+// Forward real FFT of one piece of the record (block b: the piece at (p0 + b) step), or of one
+// part of a template (block b: part b % parts of rows[b / parts], reversed, zero-padded
+// and scaled by 1 / L), into out[b fft_pitch(N) ..] in the order of spectrum_slot. The whole of a template in one part is
+// reversed end to end; a part of a longer one (of `step` samples each) as if it had `step`, so that the
+// outputs of all its parts meet at the same index.
+template <int N>
+__global__ void __launch_bounds__(N / 16) k_fft_forward(const float *__restrict__ clean, uint64_t n,
+                                       const double *__restrict__ centres, uint32_t p0, uint32_t step,
+                                       const float *__restrict__ q, const TemplParam *__restrict__ tp,
+                                       const FftRow *__restrict__ rows, int parts, const double2 *__restrict__ roots,
+                                       double2 *__restrict__ out, double *__restrict__ shifts,
+                                       double *__restrict__ norms)
 {
-    if (!(in_range && w.raw != kMissing && w.run < (uint32_t)min(m, 65535)))
-        return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    const uint64_t b1 = g >> kPrefixBlockLog;
-    if (((g + (uint64_t)m) >> kPrefixBlockLog) == b1)
-    {
-        float mu, iv, emu;
-        if (prefix_stats_fast(w.qa, w.qb, inv_m, (float)inv_m * (1.0f + 1.1920929e-07f), (float)a.pv.C[b1],
-                              block_bounds(a.pv.T[b1].y), mu, iv, emu))
-            return make_float4(mu, iv, kFastRelSd, emu);
-    }
-    WindowStats ws;
-    if (window_prefix_stats(a.pv, w.qa, w.qb, g, m, inv_m, ws) != 0)
-        return make_float4(0.0f, -1.0f, 0.0f, 0.0f);
-    return make_float4(ws.mu, ws.iv, ws.rel_sd, ws.e_mu);
-}
-
-// The folded statistics of a window for the templates of one length in one piece (what the
-// block's cache holds): x = mu - shift, y = 1 / std as in window_stats4 (0: not searched;
-// < 0: statistics not trusted), z = every term of the distance bound that does not depend
-// on the dot product's distance: fast_distance_mixed's bound without its a3 max(d, 0) term,
-// with the largest coefficients c0 = (a1, a2, a5, a6), c1 = (qs, |s1|) of the launch's
-// templates of this length (so it bounds each of them), plus the transform's error
-// 2 e_dot / std.
-__device__ __forceinline__ float4 fold_window(const float4 &st, const float4 &c0, const float4 &c1, int m, float shift,
-                                              float e_dot)
-{
-    if (!(st.y > 0.0f))
-        return make_float4(0.0f, st.y, 0.0f, 0.0f);
-    const float mu = st.x, iv = st.y, ms = mu - shift;
-    const float r = ms * iv, r0 = mu * iv;
-    WindowStats ws;
-    ws.mu = mu;
-    ws.iv = iv;
-    ws.rel_sd = st.z;
-    ws.e_mu = st.w;
-    const float ew = c0.x * sqrtf(1.0f + r * r) + c0.y + c0.z * r0 * r0 + c0.w * (fabsf(mu) + fabsf(shift)) * iv +
-                     stats_error(ws, m, c1.x, c1.y) + 2.0f * e_dot * iv * 1.01f;
-    return make_float4(ms, iv, ew, 0.0f);
-}
-
-// The per-template epilogue of window jr (relative to w0) with folded statistics st and dot
-// product dot: d as fast_distance_mixed, up = d + e and lo = d - e (+inf for windows not
-// searched; lo = -inf when the statistics are not trusted), hit = lo <= the threshold
-// distance.
-__device__ __forceinline__ void corr_eval(const Fft2Args &a, const TemplParam &P, int t, uint32_t jr, const float4 &st,
-                                          double dot, float &up, float &lo, bool &hit)
-{
-    up = inf_f();
-    lo = inf_f();
-    hit = false;
-    if (st.y == 0.0f)
-        return;
-    if (st.y > 0.0f)
-    {
-        const float cross = ((float)dot - st.x * P.s1) * st.y;
-        const float d = P.c_lin - 2.0f * cross;
-        const float e = st.z + P.a3 * fmaxf(d, 0.0f);
-        if (a.dbg_d != nullptr)
-        {
-            a.dbg_d[(size_t)t * a.W + jr] = d;
-            a.dbg_e[(size_t)t * a.W + jr] = e;
-        }
-        up = d + e;
-        lo = d - e;
-        hit = lo <= P.thr_ed;
-    }
-    else
-    {
-        lo = -inf_f();
-        hit = true;
-    }
-}
-
-// kNN bucket minima of a group of J windows per lane (windows jr[j] relative to w0, those
-// with inr[j] in the template's range) whose warp-wide span is under a bucket, so they lie in
-// at most two buckets B and B + 1: per-lane minima first, then one warp reduction per bucket
-// and key, and one atomic per bucket and key (skipped for buckets with no searched window,
-// whose minima stay at +inf's key). Every lane of the warp must call it.
-template <int J>
-__device__ __forceinline__ void bucket_minima(const Fft2Args &a, int t, int lane, const bool (&inr)[J],
-                                              const uint32_t (&jr)[J], const float (&up)[J], const float (&lo)[J])
-{
-    uint32_t bmin = 0xffffffffu;
-#pragma unroll
-    for (int j = 0; j < J; j++)
-        if (inr[j])
-            bmin = min(bmin, jr[j] / (uint32_t)kBucket);
-    const uint32_t B = __reduce_min_sync(0xffffffffu, bmin);
-    if (B == 0xffffffffu)
-        return; // no window of the warp in the range
-    uint32_t uA = 0xffffffffu, lA = 0xffffffffu, uB = 0xffffffffu, lB = 0xffffffffu;
-#pragma unroll
-    for (int j = 0; j < J; j++)
-    {
-        if (!inr[j])
-            continue;
-        const uint32_t ku = float_key(up[j]), kl = float_key(lo[j]);
-        if (jr[j] / (uint32_t)kBucket == B)
-        {
-            uA = min(uA, ku);
-            lA = min(lA, kl);
-        }
-        else
-        {
-            uB = min(uB, ku);
-            lB = min(lB, kl);
-        }
-    }
-    uA = __reduce_min_sync(0xffffffffu, uA);
-    lA = __reduce_min_sync(0xffffffffu, lA);
-    uB = __reduce_min_sync(0xffffffffu, uB);
-    lB = __reduce_min_sync(0xffffffffu, lB);
-    const uint32_t none = float_key(inf_f());
-    if (lane == 0)
-    {
-        if (uA != 0xffffffffu && (uA != none || lA != none))
-        {
-            atomicMin(&a.bmin_u[(size_t)t * a.nb + B], uA);
-            atomicMin(&a.bmin_l[(size_t)t * a.nb + B], lA);
-        }
-        if (uB != 0xffffffffu && (uB != none || lB != none))
-        {
-            atomicMin(&a.bmin_u[(size_t)t * a.nb + B + 1], uB);
-            atomicMin(&a.bmin_l[(size_t)t * a.nb + B + 1], lB);
-        }
-    }
-}
-
-// Threshold candidates of one window per lane: one ballot, one atomic per warp with hits.
-// Entries past the capacity are counted, not written. Every lane of the warp must call it.
-__device__ __forceinline__ void emit_hits(const Fft2Args &a, int t, int lane, bool hit, uint32_t jr)
-{
-    const unsigned b = __ballot_sync(0xffffffffu, hit);
-    if (b == 0u)
-        return;
-    const int leader = __ffs(b) - 1;
-    uint32_t base = 0;
-    if (lane == leader)
-        base = atomicAdd(a.cand_count, (uint32_t)__popc(b));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (hit)
-    {
-        const uint32_t pos = base + (uint32_t)__popc(b & ((1u << lane) - 1u));
-        if (pos < a.cand_cap)
-            a.cand[pos] = Candidate{(uint32_t)t, jr};
-    }
-}
-
-// Forward real FFT of one piece of the record (blockIdx.x < pieces) or one template row
-// (templates: reversed and zero-padded to kF2L), into out[blockIdx.x * kF2H ..].
-__global__ void __launch_bounds__(kF2T, 1) k_fft2_forward(const float *__restrict__ clean, uint64_t n,
-                                                         const double *__restrict__ centres, uint32_t p0,
-                                                         const float *__restrict__ q, const TemplParam *__restrict__ tp,
-                                                         const int *__restrict__ rows, const double2 *__restrict__ roots,
-                                                         double2 *__restrict__ out, double *__restrict__ shifts,
-                                                         double *__restrict__ norms)
-{
+    constexpr int T = N / 16, L = 2 * N;
     extern __shared__ double2 sm2[];
-    double2 *buf = sm2, *R = sm2 + kF2Buf;
-    __shared__ double part[kF2T / 32];
+    double2 *buf = sm2, *R = sm2 + kFBuf<N>;
+    __shared__ double part[T / 32];
     load_roots(R, roots);
     const bool templ = q != nullptr;
     double s = 0.0, sq = 0.0;
     uint64_t start = 0;
     const float *qt = nullptr;
-    int m = 0;
+    int m = 0, top = 0; // the part's samples; its last one's index before the reversal
     if (templ)
     {
-        const TemplParam &p = tp[rows[blockIdx.x]];
-        qt = q + p.q_offset;
-        m = p.m;
+        const TemplParam &p = tp[rows[blockIdx.x / parts].row];
+        const int first = (int)(blockIdx.x % parts) * (int)step;
+        qt = q + p.q_offset + first;
+        m = parts > 1 ? min(p.m - first, (int)step) : p.m;
+        top = parts > 1 ? (int)step - 1 : m - 1;
     }
     else
     {
-        start = (uint64_t)(p0 + blockIdx.x) * kF2S;
+        start = (uint64_t)(p0 + blockIdx.x) * step;
         s = (double)(float)centres[start >> kPrefixBlockLog];
     }
-    for (int i = threadIdx.x; i < kF2N; i += kF2T)
+    for (int i = threadIdx.x; i < N; i += T)
     {
         double a, b;
         if (templ)
         {
-            const int i0 = 2 * i, i1 = 2 * i + 1; // y[i] = q[m - 1 - i]
-            a = i0 < m ? (double)qt[m - 1 - i0] : 0.0;
-            b = i1 < m ? (double)qt[m - 1 - i1] : 0.0;
+            const int i0 = top - 2 * i, i1 = i0 - 1; // y[i] = q[top - i]
+            a = i0 >= 0 && i0 < m ? (double)qt[i0] : 0.0;
+            b = i1 >= 0 && i1 < m ? (double)qt[i1] : 0.0;
         }
         else
         {
@@ -426,34 +241,41 @@ __global__ void __launch_bounds__(kF2T, 1) k_fft2_forward(const float *__restric
         buf[pidx(i)] = make_double2(a, b);
     }
     __syncthreads();
-    fft8192_r16<-1>(buf, R);
-    // the radix-2 pass, in place (each thread owns the pairs (i, i + 4096) it touches)
-    for (int i = threadIdx.x; i < 4096; i += kF2T)
+    // radix 16 three times; for N = 8192 then a radix-2 pass, in place (each thread owns the
+    // pairs (i, i + 4096) it touches)
+    pass16<N, -1>(buf, R, 1);
+    pass16<N, -1>(buf, R, 16);
+    pass16<N, -1>(buf, R, 256);
+    if (N == 8192)
     {
-        const double2 a = buf[pidx(i)], b = cmul(buf[pidx(i + 4096)], root<-1>(R, 4 * i));
-        buf[pidx(i)] = cadd(a, b);
-        buf[pidx(i + 4096)] = csub(a, b);
+        for (int i = threadIdx.x; i < 4096; i += T)
+        {
+            const double2 a = buf[pidx(i)], b = cmul(buf[pidx(i + 4096)], root<-1>(R, 4 * i));
+            buf[pidx(i)] = cadd(a, b);
+            buf[pidx(i + 4096)] = csub(a, b);
+        }
+        __syncthreads();
     }
-    __syncthreads();
-    double2 *o = out + (size_t)blockIdx.x * kF2H;
-    for (int k = threadIdx.x; k <= kF2N / 2; k += kF2T)
+    double2 *o = out + (size_t)blockIdx.x * fft_pitch(N);
+    const double scale = templ ? 1.0 / (double)L : 1.0; // a power of two: exact
+    for (int k = threadIdx.x; k <= N / 2; k += T)
     {
         // X[k] and X[N - k] from Z[k] and Z[N - k] (Z[N] = Z[0])
-        const double2 A = buf[pidx(k)], Bc = conj2(buf[pidx(k == 0 ? 0 : kF2N - k)]);
+        const double2 A = buf[pidx(k)], Bc = conj2(buf[pidx(k == 0 ? 0 : N - k)]);
         const double2 E = make_double2(0.5 * (A.x + Bc.x), 0.5 * (A.y + Bc.y));
         const double2 D = csub(A, Bc);
         const double2 O = make_double2(0.5 * D.y, -0.5 * D.x); // -i (A - B) / 2
-        const double2 w = root<-1>(R, 2 * k);                   // e^{-2 pi i k / L}
-        o[k] = cadd(E, cmul(O, w));
+        const double2 w = root<-1>(R, 32768 / L * k);           // e^{-2 pi i k / L}
+        o[spectrum_slot<N>(k)] = cscale(cadd(E, cmul(O, w)), scale);
         if (k == 0)
-            o[kF2N] = csub(E, O); // twiddle e^{-i pi} = -1
-        else if (k < kF2N / 2)
+            o[spectrum_slot<N>(N)] = cscale(csub(E, O), scale); // twiddle e^{-i pi} = -1
+        else if (k < N / 2)
         {
             const double2 A2 = conj2(Bc), B2c = conj2(A); // Z[N - k], conj Z[k]
             const double2 E2 = make_double2(0.5 * (A2.x + B2c.x), 0.5 * (A2.y + B2c.y));
             const double2 D2 = csub(A2, B2c);
             const double2 O2 = make_double2(0.5 * D2.y, -0.5 * D2.x);
-            o[kF2N - k] = csub(E2, cmul(O2, conj2(w))); // e^{-2 pi i (N - k) / L} = -e^{2 pi i k / L}
+            o[spectrum_slot<N>(N - k)] = cscale(csub(E2, cmul(O2, conj2(w))), scale); // e^{-2 pi i (N - k) / L} = -e^{2 pi i k / L}
         }
     }
     if (!templ)
@@ -466,7 +288,7 @@ __global__ void __launch_bounds__(kF2T, 1) k_fft2_forward(const float *__restric
         if (threadIdx.x == 0)
         {
             double t = 0.0;
-            for (int w = 0; w < kF2T / 32; w++)
+            for (int w = 0; w < T / 32; w++)
                 t += part[w];
             shifts[p0 + blockIdx.x] = s;
             norms[p0 + blockIdx.x] = sqrt(t) * (1.0 + 1e-12); // rounding of the norm itself, generously
@@ -474,509 +296,791 @@ __global__ void __launch_bounds__(kF2T, 1) k_fft2_forward(const float *__restric
     }
 }
 
-// The fused correlation: persistent blocks over pieces; per piece, every template of the
-// launch: C from X[p] Y[t] (the product and the real-transform packing in one step), the
-// radix-16 passes, then one thread per window: its dot product from the final radix-2
-// pass, the distance and bound as the contraction kernels' epilogues (fast_distance_mixed
-// with prefix-sum statistics) plus the FFT's own error, then kNN bucket minima or threshold
-// candidates.
-__global__ void __launch_bounds__(kF2T, 1) k_fft2_corr(const Fft2Args a)
+// ---- the fused correlation ----------------------------------------------------------
+//
+// N / 16 threads hold the N complex points of one inverse transform in registers, 16 each.
+// Pass 1 is radix 8 over the bins b + Q r, Q = N / 8, decimated in frequency (Govindaraju et
+// al., "High Performance Discrete Fourier Transforms on Graphics Processors", SC 2008, for the
+// passes in shared memory): thread t takes the butterflies t and Q - t, whose bins t + Q r and
+// N - t - Q r are each other's partners in the real-transform packing, so the product, the
+// packing and the pass need no exchange (thread 0: butterflies 0 and Q / 2, each its own
+// partner). It leaves eight independent Q-point transforms, outputs n = 8 n1 + g of transform
+// g, and each of those is the work of one warp (N = 4096: passes of radix 8, 8, 8) or two (N =
+// 8192: 16, 8, 8), so that there are two block-wide barriers per transform. The planes are
+// padded by 2 doubles per 16, which puts the quarter warps' accesses in distinct banks. The
+// twiddles are folded into the butterflies, a + w b by four FMAs and a - w b = 2 a - (a + w b)
+// by two.
+//
+// What bounds it (16 templates or more of one length): the load/store unit's data pipe, 73 %
+// busy with N = 4096 and 60 % with 8192 (three exchanges of 16 bytes a point, the spectra and
+// the windows' statistics), the FP64 pipe 35 and 28 %, issue 40 %; templates of distinct lengths
+// also compute their windows' statistics (issue 49 %). Per template and 2^25 samples, in ms
+// (before: FP64 passes of radix 16, 16, 16, 2 with block-wide barriers, steps of 8192 for up to
+// 8192 samples, longer pieces above): m = 1024 0.169 (0.49), 2048 0.170 (0.49), 4096 0.204
+// (0.49), 8192 0.320 (0.49), 16384 0.43 (0.62); with distinct lengths 1000 0.249, 2000 0.274,
+// 4096 0.307 (0.71), 8192 0.432 (0.71), 16000 0.63 (1.07). 32 points per thread and two exchanges
+// (radix 16, 16, 16; 8 warps per SM) took 0.177 at m = 2048 and 0.409 at distinct 4096, also
+// with the epilogue on warps of its own: too few warps to hide the latencies.
+template <int N> struct FftShape
 {
-    extern __shared__ double2 sm2[];
-    __shared__ TemplParam sP;
-    double2 *buf = sm2, *R = sm2 + kF2Buf;
-    load_roots(R, a.roots);
-    const int lane = threadIdx.x & 31;
-    const double inv_l = 1.0 / (double)kF2L;
-    float4 *cache = a.stats + (size_t)blockIdx.x * kFftCache; // this block's statistics cache
-    for (uint32_t pi = blockIdx.x; pi < a.p_count; pi += gridDim.x)
+    static constexpr int T = N / 16;             // threads
+    static constexpr int GT = N / 128;           // of them, those of one transform of N / 8 points
+    static constexpr int Group = N / 8 + N / 64; // doubles of that transform's plane, padding included
+    static constexpr int Ex = 8 * Group;         // doubles of one exchange plane
+    static constexpr int Pitch = fft_pitch(N);   // entries of a spectrum
+    static constexpr int Dot = N / 4 + 4;        // floats of that transform's outputs (the pad: see the epilogue)
+    // the twiddle tables: the packing's roots, then those of the two last radix-8 passes
+    static constexpr int TabB = T + 1, TabC = TabB + 4 * (N == 4096 ? 8 : 16), Tabs = TabC + N / 64;
+    static constexpr size_t Smem =
+        2 * sizeof(double) * Ex + 8 * sizeof(float) * Dot + sizeof(double2) * Tabs + 2 * sizeof(FftRow);
+};
+static_assert(FftShape<8192>::Smem <= 227 * 1024, "shared memory of k_fft_corr");
+static_assert(2 * (FftShape<4096>::Smem + 1024) <= 228 * 1024, "two blocks of k_fft_corr<4096> per SM");
+static_assert(FftShape<8192>::Tabs + FftShape<4096>::Tabs == kFftAllRoots - kFftRoots, "twiddle tables");
+static_assert(sizeof(FftRow) % 16 == 0 && sizeof(FftRow) / 4 <= 32, "one warp copies a row");
+
+// (a, b) -> (a + w b, a - w b), and with i w in place of w
+__device__ __forceinline__ void bfly(double2 &a, double2 &b, double2 w)
+{
+    const double2 s = make_double2(fma(-w.y, b.y, fma(w.x, b.x, a.x)), fma(w.y, b.x, fma(w.x, b.y, a.y)));
+    b = make_double2(fma(2.0, a.x, -s.x), fma(2.0, a.y, -s.y));
+    a = s;
+}
+__device__ __forceinline__ void bfly_i(double2 &a, double2 &b, double2 w)
+{
+    const double2 s = make_double2(fma(-w.y, b.x, fma(-w.x, b.y, a.x)), fma(-w.y, b.y, fma(w.x, b.x, a.y)));
+    b = make_double2(fma(2.0, a.x, -s.x), fma(2.0, a.y, -s.y));
+    a = s;
+}
+__device__ __forceinline__ void bfly1(double2 &a, double2 &b)
+{
+    const double2 s = cadd(a, b);
+    b = csub(a, b);
+    a = s;
+}
+__device__ __forceinline__ void bfly1_i(double2 &a, double2 &b)
+{
+    const double2 s = make_double2(a.x - b.y, a.y + b.x);
+    b = make_double2(a.x + b.y, a.y - b.x);
+    a = s;
+}
+
+constexpr double kH = 0.70710678118654752440, kC16 = 0.92387953251128675613, kS16 = 0.38268343236508977173;
+__device__ __forceinline__ double2 mul_w8(double2 a) // a e^{2 pi i / 8}
+{
+    return make_double2(kH * (a.x - a.y), kH * (a.x + a.y));
+}
+
+// v[a] +- w8 v[b], w8 = e^{2 pi i / 8}, and with i w8
+__device__ __forceinline__ void bfly_w8(double2 &a, double2 &b)
+{
+    const double2 p = make_double2(b.x - b.y, b.x + b.y), s = a;
+    a = make_double2(fma(kH, p.x, s.x), fma(kH, p.y, s.y));
+    b = make_double2(fma(-kH, p.x, s.x), fma(-kH, p.y, s.y));
+}
+__device__ __forceinline__ void bfly_iw8(double2 &a, double2 &b)
+{
+    const double2 p = make_double2(b.x - b.y, b.x + b.y), s = a;
+    a = make_double2(fma(-kH, p.y, s.x), fma(kH, p.x, s.y));
+    b = make_double2(fma(kH, p.y, s.x), fma(-kH, p.x, s.y));
+}
+
+// X[k] = sum_r v[r] e^{2 pi i r k / 8}: X[0..7] left in v[0], v[4], v[2], v[6], v[1], v[5], v[3], v[7]
+__device__ __forceinline__ void radix8_first(double2 (&v)[8])
+{
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+        bfly1(v[r], v[r + 4]);
+    bfly1(v[0], v[2]);
+    bfly1_i(v[4], v[6]);
+    bfly1(v[1], v[3]);
+    bfly1_i(v[5], v[7]);
+    bfly1(v[0], v[1]);
+    bfly1_i(v[2], v[3]);
+    bfly_w8(v[4], v[5]);
+    bfly_iw8(v[6], v[7]);
+}
+// register of output k of a radix-8 butterfly
+__device__ constexpr int out8(int k) { return (k & 3) == 0 ? (k >> 2) : (k & 3) == 2 ? 2 + (k >> 2) : (k & 3) == 1 ? 4 + (k >> 2) : 6 + (k >> 2); }
+
+// the same of v[r] w^r, with w, w^2, w^4 and w e^{2 pi i / 8}
+__device__ __forceinline__ void radix8(double2 (&v)[8], double2 w, double2 w2, double2 w4, double2 w8)
+{
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+        bfly(v[r], v[r + 4], w4);
+    bfly(v[0], v[2], w2);
+    bfly_i(v[4], v[6], w2);
+    bfly(v[1], v[3], w2);
+    bfly_i(v[5], v[7], w2);
+    bfly(v[0], v[1], w);
+    bfly_i(v[2], v[3], w);
+    bfly(v[4], v[5], w8);
+    bfly_i(v[6], v[7], w8);
+}
+
+__device__ __forceinline__ double2 csqr(double2 w) { return make_double2(fma(w.x, w.x, -w.y * w.y), 2.0 * w.x * w.y); }
+
+// X[k] = sum_r v[r] e^{2 pi i r k / 16}: X[k] left in v[out16(k)]
+__device__ __forceinline__ void radix16_first(double2 (&v)[16])
+{
+#pragma unroll
+    for (int r = 0; r < 8; r++)
+        bfly1(v[r], v[r + 8]);
+#pragma unroll
+    for (int r = 0; r < 4; r++)
     {
-        int cached_m = -1; // the length whose statistics of this piece the cache holds
-        const uint32_t p = a.p_first + pi;
-        const double2 *X = a.X + (size_t)p * kF2H;
-        const float shift = (float)a.shifts[p];
-        const double norm = a.norms[p];
-        for (int ti = 0; ti < a.nrows; ti++)
-        {
-            const int t = a.rows[ti];
-            const uint64_t piece_w = (uint64_t)p * kF2S;
-            // windows of this piece in the template's range [w0, w0 + wcount)
-            const uint64_t wcount = a.tp[t].wcount;
-            if (piece_w + kF2S <= a.w0 || piece_w >= a.w0 + wcount)
-                continue;
-            const double2 *Y = a.Y + (size_t)ti * kF2H;
-            __syncthreads(); // the previous template's epilogue has read buf and sP
-            if (threadIdx.x == 0)
-                sP = a.tp[t]; // the template's constants, read by every thread from shared memory
-            const TemplParam &P = sP;
-            // work items k = thread + 512 i (0 <= k <= N / 2), two at a time: their spectrum
-            // loads first, then the products
-            for (int i0 = 0; i0 < 10; i0 += 2)
-            {
-                double2 xk[2], xn[2], yk[2], yn[2];
+        bfly1(v[r], v[r + 4]);
+        bfly1_i(v[r + 8], v[r + 12]);
+    }
 #pragma unroll
-                for (int j = 0; j < 2; j++)
-                {
-                    const int k = (int)threadIdx.x + kF2T * (i0 + j);
-                    if (k <= kF2N / 2)
-                    {
-                        xk[j] = X[k];
-                        xn[j] = X[kF2N - k];
-                        yk[j] = Y[k];
-                        yn[j] = Y[kF2N - k];
-                    }
-                }
+    for (int r = 0; r < 2; r++)
+    {
+        bfly1(v[r], v[r + 2]);
+        bfly1_i(v[r + 4], v[r + 6]);
+        bfly_w8(v[r + 8], v[r + 10]);
+        bfly_iw8(v[r + 12], v[r + 14]);
+    }
+    bfly1(v[0], v[1]);
+    bfly1_i(v[2], v[3]);
+    bfly_w8(v[4], v[5]);
+    bfly_iw8(v[6], v[7]);
+    const double2 wa = make_double2(kC16, kS16), wc = make_double2(kS16, kC16);
+    bfly(v[8], v[9], wa);
+    bfly_i(v[10], v[11], wa);
+    bfly(v[12], v[13], wc);
+    bfly_i(v[14], v[15], wc);
+}
+// register of output k of the radix-16 butterfly: the pair of k mod 8, then k / 8
+__device__ constexpr int out16(int k)
+{
+    constexpr int pair[8] = {0, 4, 2, 6, 1, 5, 3, 7};
+    return 2 * pair[k & 7] + (k >> 3);
+}
+
+// A window's folded statistics for the templates of one length in one piece: 1 / std, mean -
+// shift, and every term of the distance bound that does not depend on the dot product
+// (fast_distance_mixed's bound without a3 max(d, 0), with the largest coefficients c0 = (a1,
+// a2, a5, a6), qs and |s1| of the launch's templates of this length, so it bounds each of
+// them; sqrt(1 + r^2) <= 1 + |r|), plus the transform's error 2 e_dot / std. A window that is
+// not searched has (0, 0, NaN): no comparison accepts its bounds and fminf ignores them; one
+// whose statistics are not trusted has (0, 0, +inf): d - e = -inf, it is re-scored exactly.
+__device__ __forceinline__ void fold_window(float mu, float iv, float rel_sd, float e_mu, float4 c0, float qs, float s1,
+                                            int m, float shift, float e_dot, float &ms, float &ew)
+{
+    ms = mu - shift;
+    const float r = ms * iv, r0 = mu * iv;
+    WindowStats ws;
+    ws.mu = mu;
+    ws.iv = iv;
+    ws.rel_sd = rel_sd;
+    ws.e_mu = e_mu;
+    ew = c0.x * (1.0f + fabsf(r)) + c0.y + c0.z * r0 * r0 + c0.w * (fabsf(mu) + fabsf(shift)) * iv +
+         stats_error(ws, m, qs, s1) + 2.0f * e_dot * iv * 1.01f;
+}
+
+// Statistics by the full bound (two prefix blocks, or ill-conditioned): false when they are
+// not trusted.
+__device__ __forceinline__ bool window_stats_full(const PrefixView &pv, double2 qa, double2 qb, uint64_t g, int m,
+                                                  double inv_m, float4 &out)
+{
+    WindowStats ws;
+    if (window_prefix_stats(pv, qa, qb, g, m, inv_m, ws) != 0)
+        return false;
+    out = make_float4(ws.mu, ws.iv, ws.rel_sd, ws.e_mu);
+    return true;
+}
+
+// The threads that share one of the eight transforms of N / 8 points: a warp (N = 4096) or two
+// (N = 8192, a named barrier).
+template <int N> __device__ __forceinline__ void group_sync(int g)
+{
+    if (N == 4096)
+        __syncwarp();
+    else
+        asm volatile("bar.sync %0, 64;" ::"r"(g + 1) : "memory");
+}
+
+// Candidates: bit j of mask is window j0 + 32 j of template t. Every lane of the warp calls it.
+__device__ __forceinline__ void emit_strided(uint32_t mask, int lane, uint32_t t, uint32_t j0, Candidate *cand,
+                                             uint32_t *count, uint32_t cap)
+{
+    const int c = __popc(mask);
+    int incl = c;
 #pragma unroll
-                for (int j = 0; j < 2; j++)
-                {
-                    const int k = (int)threadIdx.x + kF2T * (i0 + j), kn = kF2N - k;
-                    if (k > kF2N / 2)
-                        continue;
-                    const double2 Vk = cmul(xk[j], yk[j]), Vn = cmul(xn[j], yn[j]);
-                    const double2 w = root<1>(R, 2 * k); // e^{2 pi i k / L}
-                    // C[k] = E + i O with E = Vk + conj Vn, O = w (Vk - conj Vn); C[N - k] = conj E + i conj O
-                    const double2 E = cadd(Vk, conj2(Vn));
-                    const double2 O = cmul(csub(Vk, conj2(Vn)), w);
-                    if (k == 0)
-                        buf[pidx(0)] = cadd(E, mul_si<1>(O)); // C[0] (Vn = V[N], the Nyquist bin)
-                    else
-                    {
-                        buf[pidx(k)] = cadd(E, mul_si<1>(O));
-                        if (k < kF2N / 2)
-                            buf[pidx(kn)] = cadd(conj2(E), mul_si<1>(conj2(O)));
-                    }
-                }
-            }
-            __syncthreads();
-            fft8192_r16<1>(buf, R);
-            // epilogue: work item u = it * 512 + thread takes output i = (base >> 1) + u of the
-            // final pass (base = m - 1), whose real and imaginary parts are the dot products of
-            // windows o = 2 u - odd and 2 u - odd + 1 (odd = base & 1; with odd base, item 0
-            // has only window 0 and item 4096 only window 8191). Window o is in the template's
-            // range when o_lo <= o < o_hi; jr = rel + o is its index relative to w0.
-            const int base = P.m - 1, odd = base & 1, nitems = kF2S / 2 + odd;
-            const int64_t rel = (int64_t)piece_w - (int64_t)a.w0;
-            const int o_lo = (int)(rel < 0 ? -rel : 0);
-            const int o_hi = (int)((int64_t)P.wcount - rel < (int64_t)kF2S ? (int64_t)P.wcount - rel : (int64_t)kF2S);
-            const double sm_ = sqrt((double)P.m);
-            const float e_dot = (float)(kF2Kappa * norm * sm_ * (2.0 * sm_ + sqrt((double)kF2L)) * 1.01);
-            // the windows' folded statistics: computed for the first template of a length in
-            // this piece, then read back from the block's cache (each thread reads what it wrote)
-            const bool cached = P.m == cached_m;
-            const float4 c0 = a.gmax[2 * t], c1 = a.gmax[2 * t + 1];
-            for (int it0 = 0; it0 < 10; it0 += 2)
-            {
-                if (it0 * kF2T + (int)(threadIdx.x & ~31u) >= nitems)
-                    continue; // no item of this warp (uniform across the warp)
-                float4 st[4];
-                bool inr[4], hit[4];
-                uint32_t jr[4];
-                float up[4], lo[4];
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-                {
-                    const int u = (it0 + (j >> 1)) * kF2T + (int)threadIdx.x;
-                    const int o = 2 * u - odd + (j & 1);
-                    inr[j] = u < nitems && o >= o_lo && o < o_hi;
-                    jr[j] = (uint32_t)rel + (uint32_t)o;
-                }
-                if (cached)
-                {
-#pragma unroll
-                    for (int j = 0; j < 4; j++)
-                        st[j] = inr[j] ? cache[2 * ((it0 + (j >> 1)) * kF2T + (int)threadIdx.x) + (j & 1)]
-                                       : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                }
-                else
-                {
-                    WinIn w[4];
-#pragma unroll
-                    for (int j = 0; j < 4; j++)
-                        w[j] = load_window(a, P.m, inr[j], (uint64_t)((int64_t)a.w0 + (int64_t)jr[j]));
-#pragma unroll
-                    for (int j = 0; j < 4; j++)
-                    {
-                        st[j] = fold_window(window_stats4(a, P.m, P.inv_m, inr[j],
-                                                          (uint64_t)((int64_t)a.w0 + (int64_t)jr[j]), w[j]),
-                                            c0, c1, P.m, shift, e_dot);
-                        if (inr[j])
-                            cache[2 * ((it0 + (j >> 1)) * kF2T + (int)threadIdx.x) + (j & 1)] = st[j];
-                    }
-                }
-#pragma unroll
-                for (int j = 0; j < 4; j += 2)
-                {
-                    const int u = (it0 + (j >> 1)) * kF2T + (int)threadIdx.x;
-                    double2 c = make_double2(0.0, 0.0);
-                    if (inr[j] || inr[j + 1])
-                        c = final_out<1>(buf, R, (base >> 1) + u);
-                    corr_eval(a, P, t, jr[j], st[j], c.x * inv_l, up[j], lo[j], hit[j]);
-                    corr_eval(a, P, t, jr[j + 1], st[j + 1], c.y * inv_l, up[j + 1], lo[j + 1], hit[j + 1]);
-                }
-                if (P.mode == TM_MODE_KNN)
-                    bucket_minima<4>(a, t, lane, inr, jr, up, lo); // the group spans 512 x 2 + 64 windows
-                else
-#pragma unroll
-                    for (int j = 0; j < 4; j++)
-                        emit_hits(a, t, lane, hit[j], jr[j]);
-            }
-            cached_m = P.m;
-        }
+    for (int off = 1; off < 32; off <<= 1)
+    {
+        const int v = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off)
+            incl += v;
+    }
+    uint32_t base = 0;
+    if (lane == 31)
+        base = atomicAdd(count, (uint32_t)incl);
+    uint32_t pos = __shfl_sync(0xffffffffu, base, 31) + (uint32_t)(incl - c);
+    for (; mask != 0u; mask &= mask - 1, pos++)
+        if (pos < cap)
+            cand[pos] = Candidate{t, j0 + 32u * (uint32_t)(__ffs(mask) - 1)};
+}
+
+// kNN bucket minima of a warp's windows (key values of d + e and d - e): one atomic per bucket
+// and key, none for a bucket without searched windows. Every lane of the warp calls it.
+__device__ __forceinline__ void bucket_min(const FftArgs &a, int row, uint32_t bucket, float umin, float lmin, int lane)
+{
+    const uint32_t ku = __reduce_min_sync(0xffffffffu, float_key(umin));
+    const uint32_t kl = __reduce_min_sync(0xffffffffu, float_key(lmin));
+    const uint32_t none = float_key(inf_f());
+    if (lane == 0 && (ku != none || kl != none))
+    {
+        atomicMin(&a.bmin_u[(size_t)row * a.nb + bucket], ku);
+        atomicMin(&a.bmin_l[(size_t)row * a.nb + bucket], kl);
     }
 }
 
-// Forward real FFT of length kF3L of pieces (item i: piece p0 + i) or template rows (item i:
-// rows[i], reversed and zero-padded), into out[item * kF3H ..]: persistent blocks, the
-// even-point transform E parked in the block's slice of `scratch` (kFPts points) while the
-// odd-point one O stays in shared memory, then the two combined and unpacked.
-__global__ void __launch_bounds__(kF2T, 1) k_fft3_forward(const float *__restrict__ clean, uint64_t n,
-                                                         const double *__restrict__ centres, uint32_t p0,
-                                                         uint32_t count, const float *__restrict__ q,
-                                                         const TemplParam *__restrict__ tp, const int *__restrict__ rows,
-                                                         const double2 *__restrict__ roots, double2 *__restrict__ out,
-                                                         double *__restrict__ shifts, double *__restrict__ norms,
-                                                         double2 *__restrict__ scratch)
+// Two adjacent bins of a spectrum (32 bytes), X[k] and its partner X[N - k] (spectrum_slot). A
+// block reads them once per item, so they are not kept in L1 (4 % of the kernel's time).
+__device__ __forceinline__ void load_pair(const double2 *p, double2 &x, double2 &xn)
 {
-    extern __shared__ double2 sm2[];
-    double2 *buf = sm2, *R = sm2 + kF2Buf;
-    __shared__ double part[kF2T / 32];
-    load_roots(R, roots);
-    double2 *Es = scratch + (size_t)blockIdx.x * kFPts;
-    const bool templ = q != nullptr;
-    for (uint32_t item = blockIdx.x; item < count; item += gridDim.x)
+    asm("ld.global.nc.L1::no_allocate.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(x.x), "=d"(x.y), "=d"(xn.x), "=d"(xn.y) : "l"(p));
+}
+
+// Persistent blocks over contiguous ranges of the (piece, template) items, template fastest,
+// so that the blocks end together whatever the numbers of pieces and templates are; a block
+// meets a piece's templates in length order, and keeps the folded statistics of the last
+// length in its slice of a global scratch (L2-resident).
+//
+// Per item: product, packing and pass 1; the eight transforms, whose outputs go to shared
+// memory as floats; the epilogue over the item's windows, 128 per warp at a time. A warp goes
+// on to the next item's product while others are in the epilogue.
+template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096 ? 2 : 1) k_fft_corr(const FftArgs a)
+{
+    using C = FftShape<N>;
+    constexpr int T = C::T, L = 2 * N, H = C::Pitch, Q = N / 8;
+    extern __shared__ __align__(16) double csm[];
+    double *re = csm, *im = csm + C::Ex;
+    float *dots = reinterpret_cast<float *>(csm + 2 * C::Ex);
+    double2 *tab = reinterpret_cast<double2 *>(dots + 8 * C::Dot);
+    FftRow *srow = reinterpret_cast<FftRow *>(tab + C::Tabs); // this item's row and the next one's
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const uint64_t total = (uint64_t)a.p_count * (uint32_t)a.nrows;
+    const uint64_t item0 = total * blockIdx.x / gridDim.x;
+    const uint32_t items = (uint32_t)(total * (blockIdx.x + 1) / gridDim.x - item0);
+    uint32_t pi = (uint32_t)(item0 / (uint32_t)a.nrows);
+    int ti = (int)(item0 % (uint32_t)a.nrows), cached_m = -1;
+    auto load_row = [&](int slot, int i) { // by the first threads of warp 0
+        if (t < (int)(sizeof(FftRow) / 4))
+            reinterpret_cast<uint32_t *>(&srow[slot])[t] = reinterpret_cast<const uint32_t *>(a.rows + i)[t];
+    };
+    for (int i = t; i < C::Tabs; i += T)
+        tab[i] = a.tabs[i];
+    load_row(0, ti);
+    __syncthreads();
+    float4 *cache = a.stats + (size_t)blockIdx.x * (3 * (L / 4));
+    const int g = t / C::GT, s = t % C::GT; // this thread's transform of N / 8 points and its place there
+    double *gre = re + g * C::Group, *gim = im + g * C::Group;
+    for (uint32_t item = 0; item < items; item++)
     {
-        double s = 0.0, sq = 0.0;
-        uint64_t start = 0;
-        const float *qt = nullptr;
-        int m = 0;
-        if (templ)
+        const FftRow &P = srow[item & 1];
+        const uint32_t p = a.p_first + pi;
+        const int m = P.m, base = (PARTS ? (int)a.step : m) - 1;
+        const uint64_t piece_w = (uint64_t)p * a.step;
+        // parts of the template that meet samples of the record
+        const int parts = PARTS ? (int)min((uint32_t)a.parts, a.pieces - p) : 1;
+        double add = 0.0;
+        if (PARTS)
+            for (int i = 1; i < parts; i++)
+                add = fma(a.shifts[p + i] - a.shifts[p], P.sum[i - 1], add);
+
+        // ---- product, real-transform packing: C[k] for this thread's bins ----
+        double2 A[8], B[8];
         {
-            const TemplParam &p = tp[rows[item]];
-            qt = q + p.q_offset;
-            m = p.m;
+            const double2 *X = a.X + (size_t)p * H, *Y = a.Y + (size_t)ti * (PARTS ? a.parts : 1) * H;
+            const double2 wA = tab[t], wB = t != 0 ? make_double2(-wA.y, wA.x) : tab[T];
+#pragma unroll
+            for (int r = 0; r < 8; r++)
+            {
+                double2 x, xn, y, yn;
+                load_pair(X + 2 * (r * T + t), x, xn);
+                load_pair(Y + 2 * (r * T + t), y, yn);
+                double2 V = cmul(x, y), Vn = cmul(xn, yn);
+                if (PARTS)
+                    for (int i = 1; i < parts; i++)
+                    {
+                        load_pair(X + i * H + 2 * (r * T + t), x, xn);
+                        load_pair(Y + i * H + 2 * (r * T + t), y, yn);
+                        V = make_double2(fma(x.x, y.x, fma(-x.y, y.y, V.x)), fma(x.x, y.y, fma(x.y, y.x, V.y)));
+                        Vn = make_double2(fma(xn.x, yn.x, fma(-xn.y, yn.y, Vn.x)), fma(xn.x, yn.y, fma(xn.y, yn.x, Vn.y)));
+                    }
+                // w = e^{2 pi i k / L} of the bin k = t + Q r from the thread's root and a 16th root of unity
+                const double2 w0 = r < 4 ? wA : wB;
+                double2 w = w0;
+                if ((r & 3) == 1)
+                    w = make_double2(fma(w0.x, kC16, -w0.y * kS16), fma(w0.x, kS16, w0.y * kC16));
+                if ((r & 3) == 2)
+                    w = mul_w8(w0);
+                if ((r & 3) == 3)
+                    w = make_double2(fma(w0.x, kS16, -w0.y * kC16), fma(w0.x, kC16, w0.y * kS16));
+                // E = V + conj Vn, D = V - conj Vn, C[k] = E + i w D, C[N-k] = conj E + i conj(w D)
+                const double2 E = make_double2(V.x + Vn.x, V.y - Vn.y), D = make_double2(V.x - Vn.x, V.y + Vn.y);
+                const double2 c = make_double2(fma(-w.y, D.x, fma(-w.x, D.y, E.x)), fma(-w.y, D.y, fma(w.x, D.x, E.y)));
+                A[r] = c;
+                B[(8 - r) & 7] = make_double2(fma(2.0, E.x, -c.x), fma(-2.0, E.y, c.y)); // bin -t + Q ((8 - r) & 7)
+            }
+            if (t == 0)
+            {
+                // butterflies 0 (bins Q r, partners within) and Q / 2 (bins Q / 2 + Q r, likewise)
+                double2 V = cmul(X[N], Y[N]); // the slot of bin N / 2
+                if (PARTS)
+                    for (int i = 1; i < parts; i++)
+                        V = cadd(V, cmul(X[i * H + N], Y[i * H + N]));
+                const double2 s4 = A[4], s5 = A[5], s6 = A[6], s7 = A[7];
+                const double2 n1 = B[7], n2 = B[6], n3 = B[5], n4 = B[4], n5 = B[3], n6 = B[2], n7 = B[1];
+                A[4] = make_double2(2.0 * V.x, -2.0 * V.y); // C[N/2] = 2 conj V[N/2]
+                A[5] = n3;
+                A[6] = n2;
+                A[7] = n1;
+                B[0] = s4;
+                B[1] = s5;
+                B[2] = s6;
+                B[3] = s7;
+                B[4] = n7;
+                B[5] = n6;
+                B[6] = n5;
+                B[7] = n4;
+            }
+        }
+
+        // ---- pass 1: output g of butterfly b, times e^{2 pi i b g / N}, is point b of transform g ----
+        radix8_first(A);
+        radix8_first(B);
+        {
+            const int bB = t != 0 ? Q - t : Q / 2;
+            const int eA = t + 2 * (t >> 4), eB = bB + 2 * (bB >> 4);
+            const double2 w1 = csqr(tab[t]), w2 = csqr(w1), w3 = cmul(w2, w1), w4 = csqr(w2);
+            const double2 w[8] = {make_double2(1.0, 0.0), w1, w2, w3, w4, cmul(w4, w1), csqr(w3), cmul(w4, w3)};
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+            {
+                double2 va = A[out8(i)], vb = B[out8(i)];
+                if (i > 0)
+                {
+                    va = cmul(va, w[i]);
+                    vb = cmul(vb, conj2(w[i])); // butterfly -t
+                    if (t == 0)                 // butterfly Q / 2: e^{2 pi i g / 16}
+                    {
+                        constexpr double c[8] = {1.0, kC16, kH, kS16, 0.0, -kS16, -kH, -kC16};
+                        constexpr double n[8] = {0.0, kS16, kH, kC16, 1.0, kC16, kH, kS16};
+                        vb = cmul(vb, make_double2(c[i], n[i]));
+                    }
+                }
+                re[i * C::Group + eA] = va.x;
+                im[i * C::Group + eA] = va.y;
+                re[i * C::Group + eB] = vb.x;
+                im[i * C::Group + eB] = vb.y;
+            }
+        }
+        __syncthreads();
+        load_row((item + 1) & 1, ti + 1 < a.nrows ? ti + 1 : 0); // the last item's epilogue is over: its slot is free
+
+        // ---- transform g: radix 16 (N = 8192) or 8 (N = 4096) with Ns = 1, then 8 and 8 ----
+        constexpr int Ns2 = N == 4096 ? 8 : 16, R8 = Q / 8 + Q / 64; // R8: elements Q / 8 apart, padded
+        const int rd = 2 * s + 2 * (s >> 3); // element r of the butterflies 2 s and 2 s + 1 at rd + R8 r
+        auto read_pairs = [&]() {
+#pragma unroll
+            for (int r = 0; r < 8; r++)
+            {
+                const double2 x = *reinterpret_cast<const double2 *>(gre + rd + R8 * r);
+                const double2 y = *reinterpret_cast<const double2 *>(gim + rd + R8 * r);
+                A[r] = make_double2(x.x, y.x);
+                B[r] = make_double2(x.y, y.y);
+            }
+        };
+        if (N == 8192)
+        {
+            double2 v[16];
+            const int e = s + 2 * (s >> 4);
+#pragma unroll
+            for (int r = 0; r < 16; r++)
+                v[r] = make_double2(gre[e + 72 * r], gim[e + 72 * r]);
+            radix16_first(v);
+            group_sync<N>(g); // the group has read its points
+#pragma unroll
+            for (int r = 0; r < 16; r += 2)
+            {
+                *reinterpret_cast<double2 *>(gre + 18 * s + r) = make_double2(v[out16(r)].x, v[out16(r + 1)].x);
+                *reinterpret_cast<double2 *>(gim + 18 * s + r) = make_double2(v[out16(r)].y, v[out16(r + 1)].y);
+            }
         }
         else
         {
-            start = (uint64_t)(p0 + item) * kF3S;
-            s = (double)(float)centres[start >> kPrefixBlockLog];
-        }
-        for (int half = 0; half < 2; half++)
-        {
-            __syncthreads(); // buf and Es are free (the previous half's or item's readers are done)
-            for (int i = threadIdx.x; i < kFPts; i += kF2T)
+            read_pairs();
+            radix8_first(A);
+            radix8_first(B);
+            group_sync<N>(g);
+#pragma unroll
+            for (int r = 0; r < 8; r += 2)
             {
-                // point 2i + half of z: samples 4i + 2 half and 4i + 2 half + 1
-                const uint64_t t0 = 4 * (uint64_t)i + 2 * (uint64_t)half;
-                double va, vb;
-                if (templ)
+                *reinterpret_cast<double2 *>(gre + 18 * s + r) = make_double2(A[out8(r)].x, A[out8(r + 1)].x);
+                *reinterpret_cast<double2 *>(gim + 18 * s + r) = make_double2(A[out8(r)].y, A[out8(r + 1)].y);
+                *reinterpret_cast<double2 *>(gre + 18 * s + 8 + r) = make_double2(B[out8(r)].x, B[out8(r + 1)].x);
+                *reinterpret_cast<double2 *>(gim + 18 * s + 8 + r) = make_double2(B[out8(r)].y, B[out8(r + 1)].y);
+            }
+        }
+        group_sync<N>(g);
+        read_pairs();
+        {
+            const int k = (2 * s) & (Ns2 - 1);
+            const double2 *w = tab + C::TabB + k;
+            radix8(A, w[0], w[Ns2], w[2 * Ns2], w[3 * Ns2]);
+            radix8(B, w[1], w[Ns2 + 1], w[2 * Ns2 + 1], w[3 * Ns2 + 1]);
+            group_sync<N>(g);
+            const int b = 9 * (2 * s - k) + k;
+#pragma unroll
+            for (int r = 0; r < 8; r++)
+            {
+                const int e = b + Ns2 * r + 2 * (Ns2 * r >> 4);
+                *reinterpret_cast<double2 *>(gre + e) = make_double2(A[out8(r)].x, B[out8(r)].x);
+                *reinterpret_cast<double2 *>(gim + e) = make_double2(A[out8(r)].y, B[out8(r)].y);
+            }
+        }
+        group_sync<N>(g);
+        read_pairs();
+        {
+            const double2 *w = tab + C::TabC + 2 * s;
+            {
+                const double2 w1 = w[0], w2 = csqr(w1);
+                radix8(A, w1, w2, csqr(w2), mul_w8(w1));
+            }
+            {
+                const double2 w1 = w[1], w2 = csqr(w1);
+                radix8(B, w1, w2, csqr(w2), mul_w8(w1));
+            }
+            // outputs n1 = 2 s + (Q / 8) r and the next of transform g: correlation outputs 16 n1 + 2 g (+ 1)
+            float *d = dots + g * C::Dot + 4 * s;
+#pragma unroll
+            for (int r = 0; r < 8; r++)
+            {
+                const double2 x = A[out8(r)], y = B[out8(r)];
+                *reinterpret_cast<float4 *>(d + (Q / 4) * r) =
+                    PARTS ? make_float4((float)(x.x + add), (float)(x.y + add), (float)(y.x + add), (float)(y.y + add))
+                          : make_float4((float)x.x, (float)x.y, (float)y.x, (float)y.y);
+            }
+        }
+        __syncthreads();
+
+        // ---- epilogue: window o of the piece is output i = o + base; a lane's windows are 128 c +
+        // 32 j + lane, j < 4. Output i = 16 n1 + 2 g + h is at dots[g Dot + 2 n1 + h]: the pad puts a
+        // warp's 32 consecutive outputs in distinct banks but for a few. What a chunk needs from
+        // global memory is loaded while the one before is evaluated ----
+        const int64_t rel = (int64_t)piece_w - (int64_t)a.w0; // window o of the piece is rel + o of the range
+        const bool knn = P.mode == TM_MODE_KNN;
+        const float s1 = P.s1, c_lin = P.c_lin, a3 = P.a3, thr = P.thr;
+        const int i0 = base + lane;
+        const float *dl = dots + ((i0 >> 1) & 7) * C::Dot + 2 * (i0 >> 4) + (i0 & 1);
+        auto evaluate = [&](int c, const float (&iv)[4], const float (&ms)[4], const float (&ew)[4]) {
+            const int64_t first = rel + 128 * c; // the warp's first window
+            float d[4], lo[4], umin = inf_f(), lmin = inf_f();
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+            {
+                const float cross = (dl[16 * c + 4 * j] - ms[j] * s1) * iv[j];
+                d[j] = c_lin - 2.0f * cross;
+                const float e = ew[j] + a3 * fmaxf(d[j], 0.0f);
+                lo[j] = d[j] - e;
+                lmin = fminf(lmin, lo[j]);
+                if (a.dbg_d != nullptr && iv[j] > 0.0f)
                 {
-                    va = t0 < (uint64_t)m ? (double)qt[m - 1 - (int)t0] : 0.0;
-                    vb = t0 + 1 < (uint64_t)m ? (double)qt[m - 2 - (int)t0] : 0.0;
+                    a.dbg_d[(size_t)P.row * a.W + (size_t)(first + 32 * j + lane)] = d[j];
+                    a.dbg_e[(size_t)P.row * a.W + (size_t)(first + 32 * j + lane)] = e;
+                }
+                d[j] += e;
+                umin = fminf(umin, d[j]);
+            }
+            if (knn)
+            {
+                // the warp's 128 windows lie in one bucket or in two
+                const uint32_t bk_lo = (uint32_t)((first > 0 ? first : 0) / kBucket);
+                const uint32_t bk_hi = (uint32_t)((first + 127 > 0 ? first + 127 : 0) / kBucket);
+                if (bk_lo == bk_hi)
+                    bucket_min(a, P.row, bk_lo, umin, lmin, lane);
+                else
+                    for (uint32_t bk = bk_lo; bk <= bk_hi; bk++)
+                    {
+                        umin = lmin = inf_f();
+#pragma unroll
+                        for (int j = 0; j < 4; j++)
+                            if ((uint32_t)((uint64_t)(first + 32 * j + lane) / kBucket) == bk)
+                            {
+                                umin = fminf(umin, d[j]);
+                                lmin = fminf(lmin, lo[j]);
+                            }
+                        bucket_min(a, P.row, bk, umin, lmin, lane);
+                    }
+            }
+            else if (__any_sync(0xffffffffu, lmin <= thr))
+            {
+                uint32_t mask = 0;
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    mask |= (lo[j] <= thr ? 1u : 0u) << j;
+                emit_strided(mask, lane, (uint32_t)P.row, (uint32_t)(first + lane), a.cand, a.cand_count, a.cand_cap);
+            }
+        };
+        constexpr int kWarps = T / 32;
+        const int chunks = (int)a.step / 128; // a multiple of the warps
+        int c = warp;
+        if (m == cached_m)
+        {
+            const float4 *cc = cache + lane;
+            float4 x = cc[32 * c], y = cc[L / 4 + 32 * c], z = cc[L / 2 + 32 * c];
+            for (; c < chunks; c += kWarps)
+            {
+                const float iv[4] = {x.x, x.y, x.z, x.w}, ms[4] = {y.x, y.y, y.z, y.w}, ew[4] = {z.x, z.y, z.z, z.w};
+                const int n = c + kWarps < chunks ? c + kWarps : c;
+                x = cc[32 * n];
+                y = cc[L / 4 + 32 * n];
+                z = cc[L / 2 + 32 * n];
+                evaluate(c, iv, ms, ew);
+            }
+        }
+        else
+        {
+            // the next item's template has the same length and meets the same piece
+            const bool keep = item + 1 < items && ti + 1 < a.nrows && srow[(item + 1) & 1].m == m;
+            const float shift = (float)a.shifts[p];
+            const float fm = (float)m, s1m = 2.5f * P.s1_max;
+            // ew = k0 + kr |r| + kq (mu / sd)^2 + (ki + km |mu|) / sd for the fast path's statistics
+            const float kr = P.c0.x, kq = P.c0.z, km = P.c0.w + s1m * 1.3e-7f;
+            const float k0 = P.c0.x + P.c0.y + 1.25f * (4.0f * fm + 2.0f * P.qs) * kFastRelSd;
+            float e_dot;
+            {
+                const double sm = sqrt((double)m), qn = (double)P.qs / sm; // ||q||_2 (the largest of this length)
+                double e = 0.0;
+                for (int i = 0; i < parts; i++)
+                    e += a.norms[p + i];
+                e *= kFftKappa * qn * (2.0 * sm + sqrt((double)L));
+                for (int i = 1; i < parts; i++) // the rounding of the other parts' shift corrections
+                    e += 8.0 * kEps64 * fabs(a.shifts[p + i] - a.shifts[p]) * qn * sm;
+                e_dot = (float)(e * 1.01);
+            }
+            const float ki = P.c0.w * fabsf(shift) + 2.02f * e_dot;
+            // the piece's windows in the template's range; loads for windows outside take the
+            // nearest one inside (an empty range takes the piece's first sample, which exists)
+            const int64_t left = (int64_t)P.wcount - rel;
+            const int o_lo = rel < 0 ? (int)min(-rel, (int64_t)a.step) : 0;
+            const int o_hi = left < (int64_t)a.step ? (int)max(left, (int64_t)0) : (int)a.step;
+            const bool any = o_lo < o_hi;
+            const int w_lo = any ? o_lo : 0, w_hi = any ? o_hi - 1 : 0, len = any ? m : 0;
+            const double2 *Qp = a.pv.Q + piece_w;
+            const uint16_t *rp = a.run + piece_w;
+            const double inv_m = P.inv_m;
+            const float fim = (float)inv_m * (1.0f + 1.1920929e-07f);
+            double2 qa[4], qb[4];
+            uint32_t rn[4];
+            auto load = [&](int n) {
+                const int f = 128 * n; // the warp's first window
+                if (f >= w_lo && f + 127 <= w_hi)
+                {
+                    const double2 *x = Qp + (f + lane);
+                    const double2 *y = x + len;
+                    const uint16_t *z = rp + (f + lane);
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                    {
+                        qa[j] = x[32 * j];
+                        qb[j] = y[32 * j];
+                        rn[j] = z[32 * j];
+                    }
                 }
                 else
                 {
-                    const uint64_t g = start + t0;
-                    va = g < n ? (double)clean[g] - s : 0.0;
-                    vb = g + 1 < n ? (double)clean[g + 1] - s : 0.0;
-                    sq = fma(va, va, sq);
-                    sq = fma(vb, vb, sq);
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                    {
+                        const int w = min(max(f + 32 * j + lane, w_lo), w_hi);
+                        qa[j] = Qp[w];
+                        qb[j] = Qp[w + len];
+                        rn[j] = rp[w];
+                    }
                 }
-                buf[pidx(i)] = make_double2(va, vb);
-            }
-            __syncthreads();
-            fft8192_r16<-1>(buf, R);
-            for (int i = threadIdx.x; i < 4096; i += kF2T)
+            };
+            uint64_t b0 = ~0ull; // the prefix block whose constants follow
+            float cen = 0.0f, kib = 0.0f, va = 0.0f, vb = 0.0f;
+            load(c);
+            for (; c < chunks; c += kWarps)
             {
-                const double2 x0 = buf[pidx(i)], x1 = cmul(buf[pidx(i + 4096)], root<-1>(R, 4 * i));
-                buf[pidx(i)] = cadd(x0, x1);
-                buf[pidx(i + 4096)] = csub(x0, x1);
+                const int f = 128 * c, o = f + lane;
+                // the block of the warp's first window; almost always that of every window's samples too
+                const uint64_t b = (piece_w + (uint64_t)min(max(f, w_lo), w_hi)) >> kPrefixBlockLog;
+                const uint64_t be = (piece_w + (uint64_t)(min(max(f + 127, w_lo), w_hi) + len)) >> kPrefixBlockLog;
+                if (b != b0)
+                {
+                    // prefix_stats_fast's condition is fvar >= va + vb |mu_c| and its e_mu is
+                    // bb.b / m + 1.3e-7 |mu| + 1.9e-7 |c|, all of it folded in kib and km
+                    b0 = b;
+                    cen = (float)a.pv.C[b];
+                    const BlockBounds bb = block_bounds(a.pv.T[b].y);
+                    kib = ki + s1m * (bb.b * fim + 1.9e-7f * fabsf(cen));
+                    va = bb.a * fim * (1.00001f / 0.9e-7f);
+                    vb = 2.0f * bb.b * fim * (1.00001f / 0.9e-7f);
+                }
+                float iv[4], ms[4], ew[4];
+                uint32_t slow = 0;
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                {
+                    const double mu_c = (qb[j].x - qa[j].x) * inv_m;
+                    const double var = fma(-mu_c, mu_c, (qb[j].y - qa[j].y) * inv_m);
+                    const float fvar = (float)var, fmu = (float)mu_c;
+                    const float mu = fmu + cen;
+                    const bool ok = fvar > fmaxf(fmaf(vb, fabsf(fmu), va), fmaxf(1e-6f * fmu * fmu, 2e-22f)) && fvar < 1e36f;
+                    const bool srch = o + 32 * j >= o_lo && o + 32 * j < o_hi && rn[j] < (uint32_t)m;
+                    const float v = rsqrtf(fvar), x = mu - shift, r0 = mu * v;
+                    const float e = fmaf(kr, fabsf(x * v), k0) + fmaf(kq * r0, r0, fmaf(km, fabsf(mu), kib) * v);
+                    iv[j] = srch ? v : 0.0f;
+                    ms[j] = srch ? x : 0.0f;
+                    ew[j] = srch ? e : __int_as_float(0x7fc00000);
+                    slow |= (srch && (!ok || be != b) ? 1u : 0u) << j;
+                }
+                // two prefix blocks, or ill-conditioned: the full bound, one window at a time
+                for (; slow != 0u; slow &= slow - 1)
+                {
+                    const int jj = __ffs(slow) - 1, w = o + 32 * jj;
+                    float4 st;
+                    const bool ok = window_stats_full(a.pv, Qp[w], Qp[w + m], piece_w + (uint64_t)w, m, inv_m, st);
+                    const float v = ok ? st.y : 0.0f;
+                    float x = 0.0f, e = inf_f();
+                    if (ok)
+                        fold_window(st.x, v, st.z, st.w, P.c0, P.qs, P.s1_max, m, shift, e_dot, x, e);
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        if (j == jj)
+                        {
+                            iv[j] = v;
+                            ms[j] = x;
+                            ew[j] = e;
+                        }
+                }
+                load(c + kWarps < chunks ? c + kWarps : c);
+                if (keep)
+                {
+                    float4 *cc = cache + 32 * c + lane;
+                    cc[0] = make_float4(iv[0], iv[1], iv[2], iv[3]);
+                    cc[L / 4] = make_float4(ms[0], ms[1], ms[2], ms[3]);
+                    cc[L / 2] = make_float4(ew[0], ew[1], ew[2], ew[3]);
+                }
+                evaluate(c, iv, ms, ew);
             }
-            __syncthreads();
-            if (half == 0)
-                for (int k = threadIdx.x; k < kFPts; k += kF2T)
-                    Es[k] = buf[pidx(k)];
         }
-        __syncthreads(); // Es written, buf holds O
-        // Z[k] = E[k] + W^k O[k] (k < 8192), Z[k + 8192] = E[k] - W^k O[k], W^k = e^{-2 pi i k / 16384}
-        auto Z = [&](int k) -> double2 {
-            const int k0 = k & (kFPts - 1);
-            const double2 wo = cmul(buf[pidx(k0)], root<-1>(R, 2 * k0));
-            return k < kFPts ? cadd(Es[k0], wo) : csub(Es[k0], wo);
-        };
-        constexpr int N = kF3N;
-        double2 *o = out + (size_t)item * kF3H;
-        for (int k = threadIdx.x; k <= N / 2; k += kF2T)
+        cached_m = m;
+        if (++ti == a.nrows)
         {
-            const double2 A = Z(k), Bc = conj2(Z(k == 0 ? 0 : N - k));
-            const double2 E = make_double2(0.5 * (A.x + Bc.x), 0.5 * (A.y + Bc.y));
-            const double2 D = csub(A, Bc);
-            const double2 O = make_double2(0.5 * D.y, -0.5 * D.x);
-            const double2 w = root<-1>(R, k); // e^{-2 pi i k / 32768}
-            o[k] = cadd(E, cmul(O, w));
-            if (k == 0)
-                o[N] = csub(E, O);
-            else if (k < N / 2)
-            {
-                const double2 A2 = conj2(Bc), B2c = conj2(A);
-                const double2 E2 = make_double2(0.5 * (A2.x + B2c.x), 0.5 * (A2.y + B2c.y));
-                const double2 D2 = csub(A2, B2c);
-                const double2 O2 = make_double2(0.5 * D2.y, -0.5 * D2.x);
-                o[N - k] = csub(E2, cmul(O2, conj2(w)));
-            }
-        }
-        if (!templ)
-        {
-            for (int off = 16; off > 0; off >>= 1)
-                sq += __shfl_down_sync(0xffffffffu, sq, off);
-            if ((threadIdx.x & 31) == 0)
-                part[threadIdx.x >> 5] = sq;
-            __syncthreads();
-            if (threadIdx.x == 0)
-            {
-                double tot = 0.0;
-                for (int w = 0; w < kF2T / 32; w++)
-                    tot += part[w];
-                shifts[p0 + item] = s;
-                norms[p0 + item] = sqrt(tot) * (1.0 + 1e-12);
-            }
+            ti = 0;
+            pi++;
+            cached_m = -1; // the cache holds the last piece's statistics
         }
     }
 }
 
-// The fused correlation for pieces of kF3L samples (templates of up to kF3S samples): per
-// piece and template, two halves h = 0, 1: the product with the template spectrum, the
-// real-transform packing and the even/odd split in one step (h = 0: a[n] = C[n] + C[n + 8192];
-// h = 1: b[n] = (C[n] - C[n + 8192]) e^{2 pi i n / 16384}), the radix-16 passes, then the
-// windows whose output index has c index parity h (out[n0] with (n0 >> 1) & 1 == h, two of
-// every four consecutive windows), each from the final radix-2 pass.
-__global__ void __launch_bounds__(kF2T, 1) k_fft3_corr(const Fft2Args a)
+// The twiddle tables, in extended precision rounded to double: the forward kernel's R1[a] =
+// e^{2 pi i a / 32768} (a < 128) and R2[b] = e^{2 pi i 128 b / 32768} (b < 256), then the
+// correlation kernel's: e^{2 pi i t / L} (t <= 512); w, w^2, w^4 and w e^{2 pi i / 8}, 16 each,
+// of w = e^{2 pi i k / 128} (k < 16); e^{2 pi i b / 1024} (b < 128).
+static double2 root_of(long double num, long double den)
 {
-    extern __shared__ double2 sm2[];
-    __shared__ TemplParam sP;
-    double2 *buf = sm2, *R = sm2 + kF2Buf;
-    load_roots(R, a.roots);
-    const int lane = threadIdx.x & 31;
-    const double inv_l = 1.0 / (double)kF3L;
-    constexpr int N = kF3N;
-    float4 *cache = a.stats + (size_t)blockIdx.x * kFftCache; // this block's statistics cache
-    for (uint32_t pi = blockIdx.x; pi < a.p_count; pi += gridDim.x)
+    const long double a = 6.283185307179586476925286766559005768L * num / den;
+    return make_double2((double)cosl(a), (double)sinl(a));
+}
+
+template <int N> static void corr_tables(double2 *tab)
+{
+    using C = FftShape<N>;
+    constexpr int Ns = N == 4096 ? 8 : 16;
+    for (int i = 0; i <= C::T; i++)
+        tab[i] = root_of(i, 2 * N);
+    for (int k = 0; k < Ns; k++)
     {
-        int cached_m = -1; // the length whose statistics of this piece the cache holds
-        const uint32_t p = a.p_first + pi;
-        const double2 *X = a.X + (size_t)p * kF3H;
-        const float shift = (float)a.shifts[p];
-        const double norm = a.norms[p];
-        for (int ti = 0; ti < a.nrows; ti++)
-        {
-            const int t = a.rows[ti];
-            const uint64_t piece_w = (uint64_t)p * kF3S;
-            const uint64_t wcount = a.tp[t].wcount;
-            if (piece_w + kF3S <= a.w0 || piece_w >= a.w0 + wcount)
-                continue;
-            const double2 *Y = a.Y + (size_t)ti * kF3H;
-            __syncthreads(); // the previous template's epilogue has read sP
-            if (threadIdx.x == 0)
-                sP = a.tp[t]; // the template's constants, read by every thread from shared memory
-            __syncthreads();
-            const TemplParam &P = sP;
-            const double sm_ = sqrt((double)P.m);
-            const float e_dot = (float)(kF3Kappa * norm * sm_ * (2.0 * sm_ + sqrt((double)kF3L)) * 1.01);
-            const int base = P.m - 1;
-            const bool cached = P.m == cached_m; // (each thread reads back only what it wrote)
-            const float4 c0 = a.gmax[2 * t], c1 = a.gmax[2 * t + 1];
-            const int64_t rel = (int64_t)piece_w - (int64_t)a.w0;
-            const int o_lo = (int)(rel < 0 ? -rel : 0);
-            const int o_hi = (int)((int64_t)P.wcount - rel < (int64_t)kF3S ? (int64_t)P.wcount - rel : (int64_t)kF3S);
-            for (int h = 0; h < 2; h++)
-            {
-                __syncthreads(); // the previous half's epilogue has read buf
-                // work items u = thread + 512 i (0 <= u <= 4096): the eight spectrum loads of an
-                // item first, then its products
-                for (int i0 = 0; i0 < 9; i0 += 1)
-                {
-                    double2 v[1][8];
-#pragma unroll
-                    for (int j = 0; j < 1; j++)
-                    {
-                        const int u = (int)threadIdx.x + kF2T * (i0 + j), u2 = u + kFPts;
-                        if (u <= kFPts / 2)
-                        {
-                            v[j][0] = X[u];
-                            v[j][1] = Y[u];
-                            v[j][2] = X[N - u];
-                            v[j][3] = Y[N - u];
-                            v[j][4] = X[u2];
-                            v[j][5] = Y[u2];
-                            v[j][6] = X[N - u2];
-                            v[j][7] = Y[N - u2];
-                        }
-                    }
-#pragma unroll
-                    for (int j = 0; j < 1; j++)
-                    {
-                        const int u = (int)threadIdx.x + kF2T * (i0 + j), u2 = u + kFPts;
-                        if (u > kFPts / 2)
-                            continue;
-                        // C[u], C[N - u] from V[u], V[N - u]; C[u + 8192], C[8192 - u] from V[u + 8192], V[8192 - u]
-                        const double2 V1 = cmul(v[j][0], v[j][1]), V1n = cmul(v[j][2], v[j][3]);
-                        const double2 E1 = cadd(V1, conj2(V1n)), O1 = cmul(csub(V1, conj2(V1n)), root<1>(R, u));
-                        const double2 Cu = cadd(E1, mul_si<1>(O1)), CNu = cadd(conj2(E1), mul_si<1>(conj2(O1)));
-                        const double2 V2 = cmul(v[j][4], v[j][5]), V2n = cmul(v[j][6], v[j][7]);
-                        const double2 E2 = cadd(V2, conj2(V2n)), O2 = cmul(csub(V2, conj2(V2n)), root<1>(R, u2));
-                        const double2 Cv = cadd(E2, mul_si<1>(O2)), C8u = cadd(conj2(E2), mul_si<1>(conj2(O2)));
-                        if (h == 0)
-                        {
-                            buf[pidx(u)] = cadd(Cu, Cv);
-                            if (u > 0 && u < kFPts / 2)
-                                buf[pidx(kFPts - u)] = cadd(C8u, CNu);
-                        }
-                        else
-                        {
-                            buf[pidx(u)] = cmul(csub(Cu, Cv), root<1>(R, 2 * u));
-                            if (u > 0 && u < kFPts / 2)
-                                buf[pidx(kFPts - u)] = cmul(csub(C8u, CNu), root<1>(R, 2 * (kFPts - u)));
-                        }
-                    }
-                }
-                __syncthreads();
-                fft8192_r16<1>(buf, R);
-                // work item u = it * 512 + thread of this half takes output k = (base >> 2) + u of
-                // its transform, c[2 k + h] of the whole one, whose real and imaginary parts are
-                // the dot products of windows o = 4 u - (base & 3) + 2 h and o + 1 (those in
-                // [o_lo, o_hi)); u <= 4096 covers the piece's windows (o_hi <= 16384 keeps u, and
-                // so k <= 8191, in bounds wherever a window is in range).
-                for (int it = 0; it < 9; it++)
-                {
-                    if (it * kF2T + (int)(threadIdx.x & ~31u) >= kF3Items)
-                        continue; // no item of this warp (uniform across the warp)
-                    const int u = it * kF2T + (int)threadIdx.x;
-                    const int o0 = 4 * u - (base & 3) + 2 * h;
-                    float4 st[2];
-                    bool inr[2], hit[2];
-                    uint32_t jr[2];
-                    float up[2], lo[2];
-#pragma unroll
-                    for (int j = 0; j < 2; j++)
-                    {
-                        inr[j] = u < kF3Items && o0 + j >= o_lo && o0 + j < o_hi;
-                        jr[j] = (uint32_t)rel + (uint32_t)(o0 + j);
-                    }
-                    float4 *slot = cache + h * 2 * kF3Items + 2 * u;
-                    if (cached)
-                    {
-#pragma unroll
-                        for (int j = 0; j < 2; j++)
-                            st[j] = inr[j] ? slot[j] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    }
-                    else
-                    {
-                        WinIn w[2];
-#pragma unroll
-                        for (int j = 0; j < 2; j++)
-                            w[j] = load_window(a, P.m, inr[j], (uint64_t)((int64_t)a.w0 + (int64_t)jr[j]));
-#pragma unroll
-                        for (int j = 0; j < 2; j++)
-                        {
-                            st[j] = fold_window(window_stats4(a, P.m, P.inv_m, inr[j],
-                                                              (uint64_t)((int64_t)a.w0 + (int64_t)jr[j]), w[j]),
-                                                c0, c1, P.m, shift, e_dot);
-                            if (inr[j])
-                                slot[j] = st[j];
-                        }
-                    }
-                    double2 c = make_double2(0.0, 0.0);
-                    if (inr[0] || inr[1])
-                        c = final_out<1>(buf, R, (base >> 2) + u);
-                    corr_eval(a, P, t, jr[0], st[0], c.x * inv_l, up[0], lo[0], hit[0]);
-                    corr_eval(a, P, t, jr[1], st[1], c.y * inv_l, up[1], lo[1], hit[1]);
-                    if (P.mode == TM_MODE_KNN)
-                        bucket_minima<2>(a, t, lane, inr, jr, up, lo); // the warp spans 4 x 32 windows
-                    else
-#pragma unroll
-                        for (int j = 0; j < 2; j++)
-                            emit_hits(a, t, lane, hit[j], jr[j]);
-                }
-            }
-            cached_m = P.m;
-        }
+        tab[C::TabB + k] = root_of(k, 8 * Ns);
+        tab[C::TabB + Ns + k] = root_of(2 * k, 8 * Ns);
+        tab[C::TabB + 2 * Ns + k] = root_of(4 * k, 8 * Ns);
+        tab[C::TabB + 3 * Ns + k] = root_of(k + Ns, 8 * Ns);
     }
+    for (int b = 0; b < N / 64; b++)
+        tab[C::TabC + b] = root_of(b, N / 8);
 }
 
-void fft_roots(double2 *host384)
+void fft_roots(double2 *host)
 {
-    // R1[a] = e^{2 pi i a / 32768} (a < 128), R2[b] = e^{2 pi i 128 b / 32768} (b < 256), in
-    // extended precision
-    const long double two_pi = 6.283185307179586476925286766559005768L;
     for (int a = 0; a < 128; a++)
-    {
-        const long double t = two_pi * (long double)a / 32768.0L;
-        host384[a] = make_double2((double)cosl(t), (double)sinl(t));
-    }
+        host[a] = root_of(a, 32768);
     for (int b = 0; b < 256; b++)
-    {
-        const long double t = two_pi * (long double)(128 * b) / 32768.0L;
-        host384[128 + b] = make_double2((double)cosl(t), (double)sinl(t));
-    }
+        host[128 + b] = root_of(128 * b, 32768);
+    corr_tables<8192>(host + kFftRoots);
+    corr_tables<4096>(host + kFftRoots + FftShape<8192>::Tabs);
 }
 
-uint32_t fft2_pieces(uint64_t n) { return (uint32_t)((n + kF2S - 1) / kF2S); }
-uint32_t fft3_pieces(uint64_t n) { return (uint32_t)((n + kF3S - 1) / kF3S); }
+uint32_t fft_pieces(uint64_t n, int cls) { return (uint32_t)((n + fft_class(cls).step - 1) / fft_class(cls).step); }
 
-cudaError_t launch_fft2_pieces(const float *clean, uint64_t n, const double *centres, uint32_t p0, uint32_t count,
-                               const double2 *roots, double2 *X, double *shifts, double *norms, cudaStream_t s)
+template <int N, class... Args> static cudaError_t launch_forward(unsigned blocks, cudaStream_t s, Args... args)
 {
-    cudaFuncSetAttribute(k_fft2_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kF2Smem);
-    if (count > 0)
-        k_fft2_forward<<<count, kF2T, kF2Smem, s>>>(clean, n, centres, p0, nullptr, nullptr, nullptr, roots,
-                                                     X + (size_t)p0 * kF2H, shifts, norms);
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_fft_forward<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFSmem<N>);
+    if (e != cudaSuccess)
+        return e;
+    k_fft_forward<N><<<blocks, N / 16, kFSmem<N>, s>>>(args...);
     return cudaGetLastError();
 }
 
-cudaError_t launch_fft2_templates(const float *q, const TemplParam *tp, const int *rows, int nrows,
-                                  const double2 *roots, double2 *Y, cudaStream_t s)
+cudaError_t launch_fft_pieces(const float *clean, uint64_t n, const double *centres, int cls, const double2 *roots,
+                              double2 *X, double *shifts, double *norms, cudaStream_t s)
 {
-    cudaFuncSetAttribute(k_fft2_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kF2Smem);
-    if (nrows > 0)
-        k_fft2_forward<<<nrows, kF2T, kF2Smem, s>>>(nullptr, 0, nullptr, 0, q, tp, rows, roots, Y, nullptr, nullptr);
+    const FftClass c = fft_class(cls);
+    const float *q = nullptr;
+    const TemplParam *tp = nullptr;
+    const FftRow *rows = nullptr;
+    return c.n == 4096 ? launch_forward<4096>(fft_pieces(n, cls), s, clean, n, centres, 0u, c.step, q, tp, rows, 1, roots, X,
+                                              shifts, norms)
+                       : launch_forward<8192>(fft_pieces(n, cls), s, clean, n, centres, 0u, c.step, q, tp, rows, 1, roots, X,
+                                              shifts, norms);
+}
+
+cudaError_t launch_fft_templates(const float *q, const TemplParam *tp, const FftRow *rows, int nrows, int cls, int parts,
+                                 const double2 *roots, double2 *Y, cudaStream_t s)
+{
+    const FftClass c = fft_class(cls);
+    const float *clean = nullptr;
+    const double *centres = nullptr;
+    double *none = nullptr;
+    const unsigned blocks = (unsigned)(nrows * parts);
+    return c.n == 4096 ? launch_forward<4096>(blocks, s, clean, (uint64_t)0, centres, 0u, c.step, q, tp, rows, parts, roots, Y,
+                                              none, none)
+                       : launch_forward<8192>(blocks, s, clean, (uint64_t)0, centres, 0u, c.step, q, tp, rows, parts, roots, Y,
+                                              none, none);
+}
+
+template <int N, bool PARTS> static cudaError_t launch_corr(FftArgs a, int sms, cudaStream_t s)
+{
+    constexpr size_t smem = FftShape<N>::Smem;
+    auto *kernel = k_fft_corr<N, PARTS>;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess)
+        return e;
+    const uint64_t items = (uint64_t)a.p_count * (uint32_t)a.nrows;
+    const uint64_t most = (uint64_t)sms * (N == 4096 ? 2 : 1);
+    if (items > 0)
+        kernel<<<(unsigned)std::min(items, most), N / 16, smem, s>>>(a);
     return cudaGetLastError();
 }
 
-cudaError_t launch_fft2_corr(const Fft2Args &a, int sms, cudaStream_t s)
+// roots: the tables of fft_roots; a.step and a.tabs are filled in here.
+cudaError_t launch_fft_corr(FftArgs a, int cls, const double2 *roots, int sms, cudaStream_t s)
 {
-    cudaFuncSetAttribute(k_fft2_corr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kF2Smem);
-    if (a.p_count > 0 && a.nrows > 0)
-        k_fft2_corr<<<(unsigned)std::min<uint32_t>(a.p_count, (uint32_t)sms), kF2T, kF2Smem, s>>>(a);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_fft3_pieces(const float *clean, uint64_t n, const double *centres, uint32_t p0, uint32_t count,
-                               const double2 *roots, double2 *X, double *shifts, double *norms, double2 *scratch,
-                               int blocks, cudaStream_t s)
-{
-    cudaFuncSetAttribute(k_fft3_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kF2Smem);
-    if (count > 0)
-        k_fft3_forward<<<(unsigned)std::min<uint32_t>(count, (uint32_t)blocks), kF2T, kF2Smem, s>>>(
-            clean, n, centres, p0, count, nullptr, nullptr, nullptr, roots, X + (size_t)p0 * kF3H, shifts, norms,
-            scratch);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_fft3_templates(const float *q, const TemplParam *tp, const int *rows, int nrows,
-                                  const double2 *roots, double2 *Y, double2 *scratch, int blocks, cudaStream_t s)
-{
-    cudaFuncSetAttribute(k_fft3_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kF2Smem);
-    if (nrows > 0)
-        k_fft3_forward<<<(unsigned)std::min<int>(nrows, blocks), kF2T, kF2Smem, s>>>(
-            nullptr, 0, nullptr, 0, (uint32_t)nrows, q, tp, rows, roots, Y, nullptr, nullptr, scratch);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_fft3_corr(const Fft2Args &a, int sms, cudaStream_t s)
-{
-    cudaFuncSetAttribute(k_fft3_corr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kF2Smem);
-    if (a.p_count > 0 && a.nrows > 0)
-        k_fft3_corr<<<(unsigned)std::min<uint32_t>(a.p_count, (uint32_t)sms), kF2T, kF2Smem, s>>>(a);
-    return cudaGetLastError();
+    const FftClass c = fft_class(cls);
+    a.step = c.step;
+    a.tabs = roots + kFftRoots + (c.n == 4096 ? FftShape<8192>::Tabs : 0);
+    if (c.n == 4096)
+        return a.parts > 1 ? launch_corr<4096, true>(a, sms, s) : launch_corr<4096, false>(a, sms, s);
+    return a.parts > 1 ? launch_corr<8192, true>(a, sms, s) : launch_corr<8192, false>(a, sms, s);
 }
 
 } // namespace tmb

@@ -267,6 +267,67 @@ void prepare_group_mixed(tm_ctx *ctx, Lane &L, const std::vector<int> &idx_in, c
            sizeof(TemplParam) * R + sizeof(tmb::TileInfo) * tiles.size();
 }
 
+// Makes a prepared mixed-length group one of the FFT branch: its rows with windows, sorted by
+// length as they are, in sets of one class and number of parts, and what the correlation
+// kernel needs per row.
+void prepare_fft(tm_ctx *ctx, Lane &L, GroupPlan &g)
+{
+    g.fft = true;
+    g.fft_sets.clear();
+    g.fft_rows.clear();
+    const float *hq = L.h_q.as<float>(); // the templates as prepare_group_mixed left them
+    size_t run = 0;                      // first row of the current length
+    for (int t = 0; t < g.T; t++)
+    {
+        const TemplParam &p = g.htp[static_cast<size_t>(t)];
+        if (g.index[t] < 0 || p.wcount == 0)
+            continue;
+        const int cls = tmb::fft_class_of(p.m), parts = tmb::fft_parts(p.m, cls);
+        const int step = static_cast<int>(tmb::fft_class(cls).step);
+        if (g.fft_sets.empty() || g.fft_sets.back().cls != cls || g.fft_sets.back().parts != parts)
+            g.fft_sets.push_back(GroupPlan::FftSet{cls, parts, static_cast<int>(g.fft_rows.size()), 0});
+        g.fft_sets.back().count++;
+        tmb::FftRow r{};
+        r.inv_m = p.inv_m;
+        if (parts > 1)
+            for (int i = step; i < p.m; i++)
+                r.sum[i / step - 1] += hq[p.q_offset + i];
+        r.s1 = p.s1;
+        r.c_lin = p.c_lin;
+        r.a3 = p.a3;
+        r.thr = p.thr_ed;
+        r.c0 = make_float4(p.a1_main, p.a2, p.a5, p.a6);
+        r.qs = p.qs;
+        r.s1_max = std::fabs(p.s1);
+        r.row = t;
+        r.m = p.m;
+        r.mode = p.mode;
+        r.wcount = p.wcount;
+        if (g.fft_rows.empty() || g.fft_rows[run].m != p.m)
+            run = g.fft_rows.size();
+        g.fft_rows.push_back(r);
+        // the largest coefficients of a length so far, in its first row
+        tmb::FftRow &f = g.fft_rows[run];
+        f.c0 = make_float4(std::max(f.c0.x, r.c0.x), std::max(f.c0.y, r.c0.y), std::max(f.c0.z, r.c0.z),
+                           std::max(f.c0.w, r.c0.w));
+        f.qs = std::max(f.qs, r.qs);
+        f.s1_max = std::max(f.s1_max, r.s1_max);
+    }
+    for (size_t i = 1; i < g.fft_rows.size(); i++) // then in all of them
+        if (g.fft_rows[i].m == g.fft_rows[i - 1].m)
+        {
+            g.fft_rows[i].c0 = g.fft_rows[i - 1].c0;
+            g.fft_rows[i].qs = g.fft_rows[i - 1].qs;
+            g.fft_rows[i].s1_max = g.fft_rows[i - 1].s1_max;
+        }
+    if (g.fft_rows.empty())
+        return;
+    const size_t bytes = sizeof(tmb::FftRow) * g.fft_rows.size();
+    g.d_fft.reserve_on(bytes, L.stream, ctx->pool);
+    TM_CUDA(cudaMemcpyAsync(g.d_fft.p, g.fft_rows.data(), bytes, cudaMemcpyHostToDevice, L.stream));
+    TM_CUDA(cudaStreamSynchronize(L.stream));
+}
+
 // Modelled milliseconds of 128 template rows x 2^25 windows of shape v at K samples:
 // linear between the measured K, proportional to K above the largest, flat below the
 // smallest (epilogue-bound there).
@@ -379,7 +440,7 @@ size_t plan_fft_split(const tm_ctx *ctx, const tm_request *reqs, const std::vect
     for (size_t f = 1; f <= n; f++)
     {
         // the fused kernels take templates of up to 8192 samples; longer ones cost more
-        fft_cost += m[f - 1] <= tmb::kF2S ? ctx->fft_ms : ctx->fft_long_ms;
+        fft_cost += m[f - 1] <= 8192 ? ctx->fft_ms : ctx->fft_long_ms;
         const double c = fft_cost + tensor_cost_sorted(ctx, m.data() + f, n - f);
         if (c < best)
         {
@@ -452,7 +513,7 @@ void create_batch(tm_ctx *ctx, Lane &L, const tm_request *requests, int count, t
         if (specs[gi].kind == 2)
         {
             prepare_group_mixed(ctx, L, idx, requests, g, b.h2d_bytes, 0);
-            g.fft = true;
+            prepare_fft(ctx, L, g);
         }
         else if (specs[gi].kind == 0)
             prepare_group(ctx, L, m, idx, requests, g, b.h2d_bytes,

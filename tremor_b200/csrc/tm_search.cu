@@ -2,7 +2,6 @@
 // resident prefix sums), the contraction kernel or the FFT branch with its bounded
 // epilogue, the kNN bound and FP32 re-pass, exact re-scoring, and the answers assembled on
 // the device and handed to the result in pinned memory.
-#include <unordered_map>
 #include "tm_core.h"
 
 namespace tmh {
@@ -509,165 +508,97 @@ void execute_group(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
 }
 
 // Spectra of the record's pieces for the FFT branch (tm_fftk.cu), their shifts and norms,
-// and the twiddle tables: built once per context and piece length (long = pieces of 32768
-// samples every 16384, else 16384 every 8192), under a lock (serving workers may ask at once).
-static void ensure_fft(tm_ctx *ctx, Lane &L, bool long_pieces)
+// and the twiddle tables: built once per context and class of lengths, under a lock (serving
+// workers may ask at once).
+static tm_ctx::FftPieces &ensure_fft(tm_ctx *ctx, Lane &L, int cls)
 {
+    tm_ctx::FftPieces &f = ctx->fft[cls];
     std::lock_guard<std::mutex> lk(ctx->fft_mu);
-    if (long_pieces ? ctx->fft3_ready : ctx->fft2_ready)
-        return;
+    if (f.ready)
+        return f;
     ensure_prefix(ctx, L);
     cudaStream_t s = L.stream;
     if (ctx->fft_roots.p == nullptr)
     {
-        std::vector<double2> roots(tmb::kFftRoots);
+        std::vector<double2> roots(tmb::kFftAllRoots);
         tmb::fft_roots(roots.data());
-        ctx->fft_roots.reserve(sizeof(double2) * tmb::kFftRoots);
-        TM_CUDA(cudaMemcpyAsync(ctx->fft_roots.p, roots.data(), sizeof(double2) * tmb::kFftRoots,
-                                cudaMemcpyHostToDevice, s));
-        int sms = 0;
-        TM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
-        ctx->sms = sms;
-        ctx->fft_scratch.reserve(sizeof(double2) * static_cast<size_t>(sms) * tmb::kFftScratchPts);
+        DevBuf up;
+        up.reserve(sizeof(double2) * roots.size());
+        TM_CUDA(cudaMemcpy(up.p, roots.data(), sizeof(double2) * roots.size(), cudaMemcpyHostToDevice));
+        std::swap(ctx->fft_roots, up);
+        TM_CUDA(cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->device));
     }
-    const uint32_t B = 16384; // pieces per launch
-    if (!long_pieces)
-    {
-        const uint32_t P = tmb::fft2_pieces(ctx->n);
-        ctx->fft2_X.reserve(sizeof(double2) * static_cast<size_t>(P) * tmb::kF2H);
-        ctx->fft2_shift.reserve(sizeof(double) * P);
-        ctx->fft2_norm.reserve(sizeof(double) * P);
-        for (uint32_t p0 = 0; p0 < P; p0 += B)
-        {
-            TM_CUDA(tmb::launch_fft2_pieces(ctx->clean.as<float>(), ctx->n, ctx->pcen.as<double>(), p0,
-                                            std::min<uint32_t>(B, P - p0), ctx->fft_roots.as<double2>(),
-                                            ctx->fft2_X.as<double2>(), ctx->fft2_shift.as<double>(),
-                                            ctx->fft2_norm.as<double>(), s));
-            count_launch(L);
-        }
-        ctx->fft2_P = P;
-    }
-    else
-    {
-        const uint32_t P = tmb::fft3_pieces(ctx->n);
-        ctx->fft3_X.reserve(sizeof(double2) * static_cast<size_t>(P) * tmb::kF3H);
-        ctx->fft3_shift.reserve(sizeof(double) * P);
-        ctx->fft3_norm.reserve(sizeof(double) * P);
-        for (uint32_t p0 = 0; p0 < P; p0 += B)
-        {
-            TM_CUDA(tmb::launch_fft3_pieces(ctx->clean.as<float>(), ctx->n, ctx->pcen.as<double>(), p0,
-                                            std::min<uint32_t>(B, P - p0), ctx->fft_roots.as<double2>(),
-                                            ctx->fft3_X.as<double2>(), ctx->fft3_shift.as<double>(),
-                                            ctx->fft3_norm.as<double>(), ctx->fft_scratch.as<double2>(), ctx->sms,
-                                            s));
-            count_launch(L);
-        }
-        ctx->fft3_P = P;
-    }
+    const uint32_t P = tmb::fft_pieces(ctx->n, cls);
+    f.X.reserve(sizeof(double2) * static_cast<size_t>(P) * tmb::fft_pitch(tmb::fft_class(cls).n));
+    f.shift.reserve(sizeof(double) * P);
+    f.norm.reserve(sizeof(double) * P);
+    TM_CUDA(tmb::launch_fft_pieces(ctx->clean.as<float>(), ctx->n, ctx->pcen.as<double>(), cls,
+                                   ctx->fft_roots.as<double2>(), f.X.as<double2>(), f.shift.as<double>(),
+                                   f.norm.as<double>(), s));
+    count_launch(L);
     TM_CUDA(cudaStreamSynchronize(s));
-    (long_pieces ? ctx->fft3_ready : ctx->fft2_ready) = true;
+    f.count = P;
+    f.ready = true;
+    return f;
 }
 
-// The FFT branch for the group's rows `rows` (all of up to 8192 samples, or all longer):
-// their spectra, then one persistent launch over the pieces their windows touch.
-static void fft_contract_rows(tm_ctx *ctx, Lane &L, const GroupPlan &g, const tmb::ScanArgs &a,
-                              const std::vector<int> &rows, bool long_pieces)
-{
-    ensure_fft(ctx, L, long_pieces);
-    cudaStream_t s = L.stream;
-    const int nr = static_cast<int>(rows.size());
-    const size_t H = long_pieces ? tmb::kF3H : tmb::kF2H;
-    const uint32_t S = long_pieces ? tmb::kF3S : tmb::kF2S;
-    DevBuf &Y = long_pieces ? L.fft3_Y : L.fft2_Y;
-    Y.reserve(sizeof(double2) * static_cast<size_t>(nr) * H);
-    L.fft_rows.reserve(sizeof(int) * static_cast<size_t>(nr));
-    L.fft_stats.reserve(sizeof(float4) * static_cast<size_t>(ctx->sms) * tmb::kFftCache);
-    TM_CUDA(cudaMemcpyAsync(L.fft_rows.p, rows.data(), sizeof(int) * nr, cudaMemcpyHostToDevice, s));
-    // per row, the largest bound coefficients of the rows of its length (the epilogue's
-    // folded window statistics serve every template of one length in a piece)
-    std::vector<float4> gmax(2 * static_cast<size_t>(g.T), make_float4(0.0f, 0.0f, 0.0f, 0.0f));
-    std::unordered_map<int, std::pair<float4, float4>> by_m;
-    for (int t : rows)
-    {
-        const TemplParam &q = g.htp[static_cast<size_t>(t)];
-        auto it = by_m.emplace(q.m, std::make_pair(make_float4(0.0f, 0.0f, 0.0f, 0.0f),
-                                                   make_float4(0.0f, 0.0f, 0.0f, 0.0f))).first;
-        float4 &c0 = it->second.first, &c1 = it->second.second;
-        c0 = make_float4(std::max(c0.x, q.a1_main), std::max(c0.y, q.a2), std::max(c0.z, q.a5), std::max(c0.w, q.a6));
-        c1 = make_float4(std::max(c1.x, q.qs), std::max(c1.y, std::fabs(q.s1)), 0.0f, 0.0f);
-    }
-    for (int t : rows)
-    {
-        const auto &c = by_m.at(g.htp[static_cast<size_t>(t)].m);
-        gmax[2 * static_cast<size_t>(t)] = c.first;
-        gmax[2 * static_cast<size_t>(t) + 1] = c.second;
-    }
-    L.fft_gmax.reserve(sizeof(float4) * gmax.size());
-    TM_CUDA(cudaMemcpyAsync(L.fft_gmax.p, gmax.data(), sizeof(float4) * gmax.size(), cudaMemcpyHostToDevice, s));
-    if (long_pieces)
-    {
-        // the forward transform's scratch is the context's: one launch at a time
-        std::lock_guard<std::mutex> lk(ctx->fft_mu);
-        TM_CUDA(tmb::launch_fft3_templates(g.q.as<float>(), g.tp.as<TemplParam>(), L.fft_rows.as<int>(), nr,
-                                           ctx->fft_roots.as<double2>(), Y.as<double2>(),
-                                           ctx->fft_scratch.as<double2>(), ctx->sms, s));
-        TM_CUDA(cudaStreamSynchronize(s));
-    }
-    else
-        TM_CUDA(tmb::launch_fft2_templates(g.q.as<float>(), g.tp.as<TemplParam>(), L.fft_rows.as<int>(), nr,
-                                           ctx->fft_roots.as<double2>(), Y.as<double2>(), s));
-    uint64_t wmax = 0;
-    for (int t : rows)
-        wmax = std::max<uint64_t>(wmax, g.htp[static_cast<size_t>(t)].wcount);
-    const uint32_t P = long_pieces ? ctx->fft3_P : ctx->fft2_P;
-    const uint64_t first = a.w0, last = a.w0 + wmax - 1;
-    const uint32_t pa = static_cast<uint32_t>(first / S);
-    const uint32_t pb = std::min<uint32_t>(static_cast<uint32_t>(last / S), P - 1);
-    tmb::Fft2Args f{};
-    f.X = (long_pieces ? ctx->fft3_X : ctx->fft2_X).as<double2>();
-    f.shifts = (long_pieces ? ctx->fft3_shift : ctx->fft2_shift).as<double>();
-    f.norms = (long_pieces ? ctx->fft3_norm : ctx->fft2_norm).as<double>();
-    f.p_first = pa;
-    f.p_count = pb >= pa ? pb - pa + 1 : 0;
-    f.Y = Y.as<double2>();
-    f.rows = L.fft_rows.as<int>();
-    f.nrows = nr;
-    f.tp = g.tp.as<TemplParam>();
-    f.roots = ctx->fft_roots.as<double2>();
-    f.w0 = a.w0;
-    f.W = a.W;
-    f.pv = tmb::PrefixView{a.P, a.PT, a.PC};
-    f.run = a.run;
-    f.raw = a.raw;
-    f.bmin_u = a.bmin_u;
-    f.bmin_l = a.bmin_l;
-    f.nb = a.nb;
-    f.cand = a.cand;
-    f.cand_count = a.cand_count;
-    f.cand_cap = a.cand_cap;
-    f.dbg_d = a.dbg_d;
-    f.dbg_e = a.dbg_e;
-    f.stats = L.fft_stats.as<float4>();
-    f.gmax = L.fft_gmax.as<float4>();
-    TM_CUDA(long_pieces ? tmb::launch_fft3_corr(f, ctx->sms, s) : tmb::launch_fft2_corr(f, ctx->sms, s));
-    count_launch(L, 2);
-}
+// Spectrum entries of one correlation launch's templates: 25 MB, well within L2, where every
+// block reads them once per piece.
+constexpr size_t kFftLaunchBins = 192 * 8200;
 
+// The FFT branch of a group: per set of rows (prepare_fft), their spectra, then persistent
+// launches over the pieces their windows touch.
 void fft_contract(tm_ctx *ctx, Lane &L, const GroupPlan &g, const tmb::ScanArgs &a)
 {
-    // templates of up to 8192 samples: pieces of 16384 samples; longer ones: pieces of 32768
-    std::vector<int> short_rows, long_rows;
-    for (int t = 0; t < g.T; t++)
+    cudaStream_t s = L.stream;
+    for (const GroupPlan::FftSet &set : g.fft_sets)
     {
-        const TemplParam &p = g.htp[t];
-        if (g.index[t] < 0 || p.wcount == 0)
-            continue;
-        (p.m <= tmb::kF2S ? short_rows : long_rows).push_back(t);
+        const tm_ctx::FftPieces &X = ensure_fft(ctx, L, set.cls);
+        const uint32_t step = tmb::fft_class(set.cls).step;
+        const size_t pitch = tmb::fft_pitch(tmb::fft_class(set.cls).n) * static_cast<size_t>(set.parts);
+        const int most = static_cast<int>(kFftLaunchBins / pitch);
+        L.fft_Y.reserve(sizeof(double2) * static_cast<size_t>(std::min(most, set.count)) * pitch);
+        L.fft_stats.reserve(sizeof(float4) * static_cast<size_t>(ctx->sms) * tmb::kFftStats);
+        for (int r0 = 0; r0 < set.count; r0 += most)
+        {
+            const int nr = std::min(most, set.count - r0), first = set.first + r0;
+            tmb::FftArgs f{};
+            f.rows = g.d_fft.as<tmb::FftRow>() + first;
+            f.nrows = nr;
+            f.parts = set.parts;
+            TM_CUDA(tmb::launch_fft_templates(g.q.as<float>(), g.tp.as<TemplParam>(), f.rows, nr, set.cls, set.parts,
+                                              ctx->fft_roots.as<double2>(), L.fft_Y.as<double2>(), s));
+            uint64_t wmax = 0;
+            for (int i = 0; i < nr; i++)
+                wmax = std::max<uint64_t>(wmax, g.fft_rows[static_cast<size_t>(first + i)].wcount);
+            const uint32_t pa = static_cast<uint32_t>(a.w0 / step);
+            const uint32_t pb = std::min<uint32_t>(static_cast<uint32_t>((a.w0 + wmax - 1) / step), X.count - 1);
+            f.X = X.X.as<double2>();
+            f.shifts = X.shift.as<double>();
+            f.norms = X.norm.as<double>();
+            f.pieces = X.count;
+            f.p_first = pa;
+            f.p_count = pb >= pa ? pb - pa + 1 : 0;
+            f.Y = L.fft_Y.as<double2>();
+            f.w0 = a.w0;
+            f.W = a.W;
+            f.n = a.n;
+            f.pv = tmb::PrefixView{a.P, a.PT, a.PC};
+            f.run = a.run;
+            f.raw = a.raw;
+            f.bmin_u = a.bmin_u;
+            f.bmin_l = a.bmin_l;
+            f.nb = a.nb;
+            f.cand = a.cand;
+            f.cand_count = a.cand_count;
+            f.cand_cap = a.cand_cap;
+            f.dbg_d = a.dbg_d;
+            f.dbg_e = a.dbg_e;
+            f.stats = L.fft_stats.as<float4>();
+            TM_CUDA(tmb::launch_fft_corr(f, set.cls, ctx->fft_roots.as<double2>(), ctx->sms, s));
+            count_launch(L, 2);
+        }
     }
-    if (!short_rows.empty())
-        fft_contract_rows(ctx, L, g, a, short_rows, false);
-    if (!long_rows.empty())
-        fft_contract_rows(ctx, L, g, a, long_rows, true);
 }
 
 // Device pipeline for a mixed-length group (tensor-core kernels or the FFT branch).
