@@ -353,9 +353,9 @@ struct tm_ctx
     tmh::DevBuf fft_roots;
     std::mutex fft_mu;
     int sms = 148;
-    // model: the FFT branch's ms per template per 2^25 samples, for templates of up to 8192
-    // samples (the fused kernels) and longer ones, templates of distinct lengths (B200 defaults;
-    // tm_autotune measures both)
+    // model: the FFT branch's ms per template per 2^25 samples, for templates of 4096 samples and
+    // of 16384, of distinct lengths (B200 defaults; tm_autotune measures both); fft_time
+    // scales them to other lengths and to equal ones
     double fft_ms = 0.307;
     double fft_long_ms = 0.63;
     // the context's own memory pool for per-batch buffers (DevBuf::reserve_on); it keeps
@@ -477,6 +477,7 @@ void prepare_group_mixed(tm_ctx *ctx, Lane &L, const std::vector<int> &idx_in, c
 void prepare_fft(tm_ctx *ctx, Lane &L, GroupPlan &g);
 int plan_col_tile(const tm_ctx *ctx, const tm_request *reqs, const std::vector<int> &idx, double *cost = nullptr);
 double tile_time(const tm_ctx *ctx, bool mixed, int v, double k);
+double fft_time(const tm_ctx *ctx, int m, bool shared);
 void create_batch(tm_ctx *ctx, Lane &L, const tm_request *requests, int count, tm_batch &b, bool serving = false);
 
 // tm_serve.cu

@@ -414,13 +414,47 @@ double tensor_cost_sorted(const tm_ctx *ctx, const int *m, size_t n)
     return best;
 }
 
+// Modelled milliseconds of the FFT branch per template of length m per 2^25 samples; shared: a
+// template of the same length precedes it, whose window statistics it takes. The branch's time
+// depends on the length through the pieces' step alone, and within a class little on it; the
+// factors are the classes' times over that of distinct lengths at 4096 (0.304 ms) or 16000
+// (0.63 ms): 0.245, 0.273, 0.304, 0.428 distinct at 1000, 2000, 4096, 8192; 0.167, 0.167,
+// 0.201, 0.315 shared, and 0.43 shared at 16384.
+double fft_time(const tm_ctx *ctx, int m, bool shared)
+{
+    static const double distinct[tmb::kFftClasses] = {0.81, 0.90, 1.0, 1.41};
+    static const double same[tmb::kFftClasses] = {0.55, 0.55, 0.66, 1.04};
+    const int cls = tmb::fft_class_of(m);
+    if (tmb::fft_parts(m, cls) > 1)
+        return ctx->fft_long_ms * (shared ? 0.69 : 1.0);
+    return ctx->fft_ms * (shared ? same[cls] : distinct[cls]);
+}
+
+// Device memory that the FFT branch's resident arrays for these lengths would still take
+// (prefix sums, runs, the classes' spectra).
+static size_t fft_missing_bytes(tm_ctx *ctx, const std::vector<int> &m)
+{
+    std::lock_guard<std::mutex> lk(ctx->fft_mu);
+    size_t need = ctx->prefix_ready ? 0 : 18 * static_cast<size_t>(ctx->n);
+    bool counted[tmb::kFftClasses] = {};
+    for (int len : m)
+    {
+        const int cls = tmb::fft_class_of(len);
+        if (!ctx->fft[cls].ready && !counted[cls])
+            need += sizeof(double2) * static_cast<size_t>(tmb::fft_pieces(ctx->n, cls)) *
+                    tmb::fft_pitch(tmb::fft_class(cls).n);
+        counted[cls] = true;
+    }
+    return need;
+}
+
 // How many of a group's templates (ordered longest first) go to the FFT branch: all of
 // them when it is forced (TM_TILES_FFT); under TM_TILES_AUTO with the automatic kernel,
-// the f minimising f x (the FFT's per-template time) + the tensor cost of the other
+// the f minimising the FFT's time of f templates + the tensor cost of the other
 // templates: the longest templates set a tile's K extent, so moving a few of them to the
 // FFT (whose cost does not grow with the length) can shorten every tile they would have
 // padded. Lengths up to 16384 (the FFT pieces' step); otherwise none.
-size_t plan_fft_split(const tm_ctx *ctx, const tm_request *reqs, const std::vector<int> &sorted_idx)
+size_t plan_fft_split(tm_ctx *ctx, const tm_request *reqs, const std::vector<int> &sorted_idx)
 {
     const size_t n = sorted_idx.size();
     if (n == 0 || ctx->kernel == TM_KERNEL_FP32 || !tmb::umma_supported(0, 0, 0))
@@ -439,8 +473,7 @@ size_t plan_fft_split(const tm_ctx *ctx, const tm_request *reqs, const std::vect
     double best = tensor_cost_sorted(ctx, m.data(), n), fft_cost = 0.0;
     for (size_t f = 1; f <= n; f++)
     {
-        // the fused kernels take templates of up to 8192 samples; longer ones cost more
-        fft_cost += m[f - 1] <= 8192 ? ctx->fft_ms : ctx->fft_long_ms;
+        fft_cost += fft_time(ctx, m[f - 1], f > 1 && m[f - 2] == m[f - 1]);
         const double c = fft_cost + tensor_cost_sorted(ctx, m.data() + f, n - f);
         if (c < best)
         {
@@ -448,6 +481,15 @@ size_t plan_fft_split(const tm_ctx *ctx, const tm_request *reqs, const std::vect
             best_f = f;
         }
     }
+    // a record too large for the branch's arrays beside its other ones is left to the tiles
+    if (best_f > 0)
+        if (const size_t need = fft_missing_bytes(ctx, std::vector<int>(m.begin(), m.begin() + best_f)); need > 0)
+        {
+            size_t free_b = 0, total_b = 0;
+            TM_CUDA(cudaMemGetInfo(&free_b, &total_b));
+            if (need > free_b / 10 * 8)
+                return 0;
+        }
     return best_f;
 }
 
