@@ -41,7 +41,8 @@ static void bound_diagnostics_wm(tm_ctx *ctx, int m, const std::vector<int> &idx
     TM_CUDA(cudaMemsetAsync(dd.p, 0xff, pairs * sizeof(float), s)); // NaN where nothing was written
     TM_CUDA(cudaMemsetAsync(de.p, 0xff, pairs * sizeof(float), s));
     L.cand.reserve(sizeof(Candidate) * 16);
-    const uint32_t nb = static_cast<uint32_t>((W + tmb::kBucket - 1) / tmb::kBucket);
+    const int blog = tmb::bucket_log(static_cast<uint64_t>(g.T), W);
+    const uint32_t nb = tmb::bucket_count(W, blog);
     L.bmin_u.reserve(sizeof(uint32_t) * static_cast<size_t>(g.T) * nb);
     L.bmin_l.reserve(sizeof(uint32_t) * static_cast<size_t>(g.T) * nb);
     tmb::ScanArgs a{};
@@ -54,6 +55,7 @@ static void bound_diagnostics_wm(tm_ctx *ctx, int m, const std::vector<int> &idx
     a.bmin_u = L.bmin_u.as<uint32_t>();
     a.bmin_l = L.bmin_l.as<uint32_t>();
     a.nb = nb;
+    a.bucket_log = blog;
     a.cand = L.cand.as<Candidate>();
     a.cand_count = L.counters.as<uint32_t>();
     a.cand_cap = 0;

@@ -44,13 +44,12 @@ cudaError_t launch_scan_fp32(const ScanArgs &a, cudaStream_t s);
 cudaError_t launch_scan_umma(const ScanArgs &a, cudaStream_t s);
 cudaError_t launch_scan_wm(const ScanArgs &a, cudaStream_t s);
 bool umma_supported(int m, int T, uint64_t W);
-cudaError_t launch_bucket_select(const uint32_t *bmin_u, uint32_t nb, const TemplParam *tp, const int *knn_slots,
-                                 int nk, uint32_t *tkey, cudaStream_t s);
+cudaError_t launch_bucket_select(const uint32_t *bmin_u, uint32_t *sup, uint32_t nb, int blog, const TemplParam *tp,
+                                 const int *knn_slots, int nk, bool super, uint32_t *tkey, cudaStream_t s);
 cudaError_t launch_list_buckets(const uint32_t *bmin_l, uint32_t nb, const int *knn_slots, int nk,
-                                const uint32_t *tkey, uint2 *list, uint32_t *list_count, uint32_t cap, cudaStream_t s);
-cudaError_t launch_passb(const uint2 *list, uint32_t items, const float *x, const float *q, const TemplParam *tp,
-                         const float *mean, const float *inv, const uint32_t *tkey, uint64_t w0, uint32_t W,
-                         Candidate *cand, uint32_t *cand_count, uint32_t cand_cap, cudaStream_t s);
+                                const uint32_t *tkey, uint2 *list, uint32_t *counters, uint32_t cap, cudaStream_t s);
+cudaError_t launch_passb(const uint2 *list, const uint32_t *counters, uint32_t cap, const ScanArgs &c, const uint32_t *tkey,
+                         bool mixed, int sms, cudaStream_t s);
 cudaError_t launch_rescore(const Candidate *cand, uint32_t count, const TemplParam *tp, const float *q,
                            const int *order, const float *raw, uint64_t w0, float *dist, cudaStream_t s);
 uint32_t prefix_chunks(uint64_t n);
@@ -59,10 +58,6 @@ cudaError_t launch_prefix_totals(const float *clean, uint64_t n, const double *c
 cudaError_t launch_prefix_sums(const float *clean, uint64_t n, const double *centres, double2 *totals,
                                double2 *block_totals, double2 *Q, cudaStream_t s);
 cudaError_t launch_runs(const float *clean, const float *raw, uint64_t n, uint16_t *run, uint32_t *first, cudaStream_t s);
-cudaError_t launch_passb_mixed(const uint2 *list, uint32_t items, const float *x, const float *raw, const double2 *P,
-                               const double2 *PT, const double *PC, const uint16_t *run, const float *q,
-                               const TemplParam *tp, const uint32_t *tkey, uint64_t w0, Candidate *cand,
-                               uint32_t *cand_count, uint32_t cand_cap, cudaStream_t s);
 cudaError_t launch_answer_keys(const Candidate *cand, const float *dist, uint32_t count, const TemplParam *tp,
                                unsigned long long *keys, float *vals, uint32_t *kept, cudaStream_t s);
 size_t answer_sort_scratch(uint32_t count, int T);
@@ -262,7 +257,7 @@ namespace tmh {
 struct Lane
 {
     cudaStream_t stream = nullptr;
-    DevBuf tkey, bmin_u, bmin_l, list, counters, cand, dist, fp32_qt; // (fp32_qt: k_scan_fp32's template tiles)
+    DevBuf tkey, bmin_u, bmin_l, bmin_s, list, counters, cand, dist, fp32_qt; // (fp32_qt: k_scan_fp32's template tiles)
     // answer assembly: sort keys and values (double buffers), sort scratch, runs
     DevBuf akeys, avals, avals64, sort_tmp, segs;
     std::vector<std::shared_ptr<PinnedBlock>> pool;
@@ -292,7 +287,7 @@ struct Lane
     {
         if (stream)
             cudaStreamSynchronize(stream);
-        for (DevBuf *b : {&tkey, &bmin_u, &bmin_l, &list, &counters, &cand, &dist, &fp32_qt, &akeys, &avals, &avals64, &sort_tmp,
+        for (DevBuf *b : {&tkey, &bmin_u, &bmin_l, &bmin_s, &list, &counters, &cand, &dist, &fp32_qt, &akeys, &avals, &avals64, &sort_tmp,
                           &segs, &fft_Y, &fft_stats})
             b->release();
         for (HostBuf *b : {&h_split, &h_q, &h_order, &h_slots, &h_counters})

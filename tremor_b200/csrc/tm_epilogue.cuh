@@ -19,7 +19,8 @@ struct ScanArgs
     int T;
     uint32_t *bmin_u;      // [T][nb] bucket minima of d + E (float keys)
     uint32_t *bmin_l;      // [T][nb] bucket minima of d - E
-    uint32_t nb;
+    uint32_t nb;           // buckets per row, of 2^bucket_log windows
+    int bucket_log;
     Candidate *cand;
     uint32_t *cand_count;
     uint32_t cand_cap;

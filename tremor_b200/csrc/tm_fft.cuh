@@ -66,6 +66,7 @@ struct FftArgs
     const float *raw;
     uint32_t *bmin_u, *bmin_l;
     uint32_t nb;
+    int bucket_log;
     Candidate *cand;
     uint32_t *cand_count, cand_cap;
     float *dbg_d, *dbg_e; // diagnostics: d and e of every window, [t][W]; null in searches

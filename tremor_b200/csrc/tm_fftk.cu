@@ -799,8 +799,8 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
             if (knn)
             {
                 // the warp's 128 windows lie in one bucket or in two
-                const uint32_t bk_lo = (uint32_t)((first > 0 ? first : 0) / kBucket);
-                const uint32_t bk_hi = (uint32_t)((first + 127 > 0 ? first + 127 : 0) / kBucket);
+                const uint32_t bk_lo = (uint32_t)((first > 0 ? first : 0) >> a.bucket_log);
+                const uint32_t bk_hi = (uint32_t)((first + 127 > 0 ? first + 127 : 0) >> a.bucket_log);
                 if (bk_lo == bk_hi)
                     bucket_min(a, P.row, bk_lo, umin, lmin, lane);
                 else
@@ -809,7 +809,7 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
                         umin = lmin = inf_f();
 #pragma unroll
                         for (int j = 0; j < 4; j++)
-                            if ((uint32_t)((uint64_t)(first + 32 * j + lane) / kBucket) == bk)
+                            if ((uint32_t)((uint64_t)(first + 32 * j + lane) >> a.bucket_log) == bk)
                             {
                                 umin = fminf(umin, d[j]);
                                 lmin = fminf(lmin, lo[j]);

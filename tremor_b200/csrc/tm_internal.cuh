@@ -9,7 +9,24 @@ namespace tmb {
 constexpr float kMissing = -100000.0f; // ZnormSearch.hpp:21
 constexpr float kFltMax = 3.402823466e+38f;
 constexpr int kZnormBlock = 32;      // ZnormSearch.hpp:65
-constexpr int kBucket = 2048;        // windows per kNN bound bucket
+// Windows per kNN bound bucket: 2^8, or as many (up to 2^11) as keep a group's minima, 8 bytes
+// per template and bucket, within 2 GiB. Small buckets bound the k-th distance more tightly and
+// leave the re-pass fewer windows; each contraction kernel's tile or chunk is at most 2^8
+// windows, so none of them does more work for a smaller bucket.
+constexpr int kBucketLogMin = 8, kBucketLogMax = 11;
+inline int bucket_log(uint64_t templates, uint64_t windows)
+{
+    int b = kBucketLogMin;
+    while (b < kBucketLogMax && 8 * templates * ((windows >> b) + 4) > (2ull << 30))
+        b++;
+    return b;
+}
+// Buckets of a row of minima, rounded up so that rows start at 16-byte boundaries (the padding
+// stays empty).
+inline uint32_t bucket_count(uint64_t windows, int log)
+{
+    return (uint32_t)(((windows + (1ull << log) - 1) >> log) + 3) & ~3u;
+}
 constexpr int kStagePad = 16384 + 512; // zero samples after the waveform (template padding)
 
 // per-window flags (one byte per window and length)

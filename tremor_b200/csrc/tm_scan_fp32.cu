@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(F_THREADS, 2) k_scan_fp32(ScanArgs a)
         mu[w] = j < a.W ? a.mean[j] : 0.0f;
         iv[w] = j < a.W ? a.inv[j] : 0.0f;
     }
-    const uint32_t bucket = tile_j / kBucket;
+    const uint32_t bucket = tile_j >> a.bucket_log;
 #pragma unroll
     for (int tt = 0; tt < 8; tt++)
     {

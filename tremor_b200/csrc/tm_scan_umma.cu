@@ -811,7 +811,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             stage_flush(sm.stage[ew], staged, lane, a.cand, a.cand_count, a.cand_cap);
             if (valid && p.mode == 1 && (umin <= kFltMax || lmin == -inf_f()))
             {
-                const size_t at = (size_t)t * a.nb + j0 / kBucket;
+                const size_t at = (size_t)t * a.nb + (j0 >> a.bucket_log);
                 atomicMin(&a.bmin_u[at], float_key(umin));
                 atomicMin(&a.bmin_l[at], float_key(lmin));
             }
@@ -1150,7 +1150,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             const float jcf = MIXED && in ? (float)a.PC[jb] : 0.0f;
             const BlockBounds jbb = block_bounds(MIXED && in ? a.PT[jb].y : 0.0);
             const float shift = wm_shift<MIXED>(a, j0);
-            const size_t bucket = j0 / kBucket;
+            const size_t bucket = (j0 >> a.bucket_log);
             if (!mbar_wait_warp(&sm.acc_full[buf], (tc >> 1) & 1, sm.abort, wa.err, 26))
                 goto done;
             tc_fence_after();

@@ -348,6 +348,52 @@ void rescore_and_answer(tm_ctx *ctx, Lane &L, const GroupPlan &g, uint32_t ncand
         L.phase_ms[5] += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
 }
 
+// kNN bound, bucket list and FP32 re-pass after a group's contraction (a: its arguments), then
+// the counters: the group's candidates, whether the contraction gave up waiting. One wait for
+// the device; a list that did not fit is made again, larger.
+static uint32_t collect_candidates(tm_ctx *ctx, Lane &L, const GroupPlan &g, const tmb::ScanArgs &a, bool mixed)
+{
+    cudaStream_t s = L.stream;
+    uint32_t *hc = L.h_counters.as<uint32_t>(), *counters = L.counters.as<uint32_t>();
+    if (g.nk > 0)
+    {
+        bool super = false;
+        for (int t = 0; t < g.T; t++)
+            super = super || (g.mode[t] == TM_MODE_KNN && g.merge[t] > (1 << a.bucket_log));
+        if (super)
+            L.bmin_s.reserve(sizeof(uint32_t) * static_cast<size_t>(g.nk) * a.nb);
+        TM_CUDA(tmb::launch_bucket_select(a.bmin_u, L.bmin_s.as<uint32_t>(), a.nb, a.bucket_log, a.tp, g.slots.as<int>(), g.nk,
+                                          super, L.tkey.as<uint32_t>(), s));
+        count_launch(L, super ? 2 : 1);
+    }
+    for (int attempt = 0; attempt < 3; attempt++)
+    {
+        if (g.nk > 0)
+        {
+            L.list.reserve(sizeof(uint2) * static_cast<size_t>(L.list_cap));
+            TM_CUDA(tmb::launch_list_buckets(a.bmin_l, a.nb, g.slots.as<int>(), g.nk, L.tkey.as<uint32_t>(), L.list.as<uint2>(),
+                                             counters, L.list_cap, s));
+            TM_CUDA(tmb::launch_passb(L.list.as<uint2>(), counters, L.list_cap, a, L.tkey.as<uint32_t>(), mixed, ctx->sms, s));
+            count_launch(L, 2);
+        }
+        if (L.profile)
+            TM_CUDA(cudaEventRecord(L.ev2, s));
+        TM_CUDA(cudaMemcpyAsync(hc, counters, 3 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+        TM_CUDA(cudaStreamSynchronize(s));
+        if (L.profile)
+            add_span(L, 1, L.ev1, L.ev2);
+        if (hc[2] != 0)
+            throw Failure{TM_ERR_TIMEOUT, "contraction kernel gave up waiting (code " + std::to_string(hc[2]) + ")"};
+        if (g.nk == 0 || hc[1] <= L.list_cap)
+            return hc[0];
+        // back to the contraction's candidates, and a longer list
+        L.list_cap = hc[1] + hc[1] / 2;
+        TM_CUDA(cudaMemcpyAsync(counters, counters + 5, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
+        TM_CUDA(cudaMemsetAsync(counters + 1, 0, sizeof(uint32_t), s));
+    }
+    throw Failure{TM_ERR_NO_MEMORY, "bucket list overflow"};
+}
+
 // Device pipeline and selection for one prepared group; writes answers[index].
 void execute_group(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
 {
@@ -378,7 +424,8 @@ void execute_group(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
     }
     L.tkey.reserve(sizeof(uint32_t) * T);
 
-    const uint32_t nb = static_cast<uint32_t>((W + tmb::kBucket - 1) / tmb::kBucket);
+    const int blog = tmb::bucket_log(static_cast<uint64_t>(T), W);
+    const uint32_t nb = tmb::bucket_count(W, blog);
     if (nk > 0)
     {
         L.bmin_u.reserve(sizeof(uint32_t) * static_cast<size_t>(T) * nb);
@@ -386,7 +433,6 @@ void execute_group(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
     }
     L.counters.reserve(8 * sizeof(uint32_t));
     L.h_counters.reserve(8 * sizeof(uint32_t));
-    uint32_t *hc = L.h_counters.as<uint32_t>();
 
     uint32_t ncand = 0;
     for (int attempt = 0; attempt < 3; attempt++)
@@ -399,7 +445,6 @@ void execute_group(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
         }
         TM_CUDA(cudaMemsetAsync(L.counters.p, 0, 4 * sizeof(uint32_t), s));
         uint32_t *d_cand_count = L.counters.as<uint32_t>();
-        uint32_t *d_list_count = d_cand_count + 1;
 
         tmb::ScanArgs a{};
         a.x = ctx->clean.as<float>();
@@ -414,6 +459,7 @@ void execute_group(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
         a.bmin_u = L.bmin_u.as<uint32_t>();
         a.bmin_l = L.bmin_l.as<uint32_t>();
         a.nb = nb;
+        a.bucket_log = blog;
         a.cand = L.cand.as<Candidate>();
         a.cand_count = d_cand_count;
         a.cand_cap = L.cand_cap;
@@ -450,43 +496,7 @@ void execute_group(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
         }
 
         // 3. kNN bound, bucket list, FP32 re-pass
-        if (nk > 0)
-        {
-            TM_CUDA(tmb::launch_bucket_select(L.bmin_u.as<uint32_t>(), nb, g.tp.as<TemplParam>(),
-                                              g.slots.as<int>(), nk, L.tkey.as<uint32_t>(), s));
-            for (int la = 0; la < 3; la++)
-            {
-                L.list.reserve(sizeof(uint2) * static_cast<size_t>(L.list_cap));
-                TM_CUDA(cudaMemsetAsync(d_list_count, 0, sizeof(uint32_t), s));
-                TM_CUDA(tmb::launch_list_buckets(L.bmin_l.as<uint32_t>(), nb, g.slots.as<int>(), nk,
-                                                 L.tkey.as<uint32_t>(), L.list.as<uint2>(), d_list_count,
-                                                 L.list_cap, s));
-                TM_CUDA(cudaMemcpyAsync(hc + 1, d_list_count, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-                TM_CUDA(cudaStreamSynchronize(s));
-                count_launch(L, 2);
-                if (hc[1] <= L.list_cap)
-                    break;
-                L.list_cap = hc[1] + hc[1] / 2;
-            }
-            if (hc[1] > L.list_cap)
-                throw Failure{TM_ERR_NO_MEMORY, "bucket list overflow"};
-            TM_CUDA(tmb::launch_passb(L.list.as<uint2>(), hc[1], ctx->clean.as<float>(), g.q.as<float>(),
-                                      g.tp.as<TemplParam>(), ls.mean.as<float>(), ls.inv.as<float>(),
-                                      L.tkey.as<uint32_t>(), w0, static_cast<uint32_t>(W),
-                                      L.cand.as<Candidate>(), d_cand_count, L.cand_cap, s));
-            if (hc[1] > 0)
-                count_launch(L);
-        }
-        if (L.profile)
-            TM_CUDA(cudaEventRecord(L.ev2, s));
-        TM_CUDA(cudaMemcpyAsync(hc, d_cand_count, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-        TM_CUDA(cudaMemcpyAsync(hc + 2, d_cand_count + 2, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-        TM_CUDA(cudaStreamSynchronize(s));
-        if (L.profile)
-            add_span(L, 1, L.ev1, L.ev2);
-        if (hc[2] != 0)
-            throw Failure{TM_ERR_TIMEOUT, "contraction kernel gave up waiting (code " + std::to_string(hc[2]) + ")"};
-        ncand = hc[0];
+        ncand = collect_candidates(ctx, L, g, a, false);
         if (ncand <= L.cand_cap)
             break;
         L.cand_cap = ncand + ncand / 2;
@@ -589,6 +599,7 @@ void fft_contract(tm_ctx *ctx, Lane &L, const GroupPlan &g, const tmb::ScanArgs 
             f.bmin_u = a.bmin_u;
             f.bmin_l = a.bmin_l;
             f.nb = a.nb;
+            f.bucket_log = a.bucket_log;
             f.cand = a.cand;
             f.cand_count = a.cand_count;
             f.cand_cap = a.cand_cap;
@@ -622,7 +633,8 @@ void execute_group_mixed(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
         throw Failure{TM_ERR_ARGUMENT, "more than 2^32 - 1 windows in one range; split the range"};
     cudaStream_t s = L.stream;
     L.tkey.reserve(sizeof(uint32_t) * T);
-    const uint32_t nb = static_cast<uint32_t>((W + tmb::kBucket - 1) / tmb::kBucket);
+    const int blog = tmb::bucket_log(static_cast<uint64_t>(T), W);
+    const uint32_t nb = tmb::bucket_count(W, blog);
     if (nk > 0)
     {
         L.bmin_u.reserve(sizeof(uint32_t) * static_cast<size_t>(T) * nb);
@@ -630,7 +642,6 @@ void execute_group_mixed(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
     }
     L.counters.reserve(8 * sizeof(uint32_t));
     L.h_counters.reserve(8 * sizeof(uint32_t));
-    uint32_t *hc = L.h_counters.as<uint32_t>();
     double flops = 0.0;
     for (int t = 0; t < T; t++)
         flops += 2.0 * g.htp[t].m * static_cast<double>(g.htp[t].wcount);
@@ -646,7 +657,6 @@ void execute_group_mixed(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
         }
         TM_CUDA(cudaMemsetAsync(L.counters.p, 0, 4 * sizeof(uint32_t), s));
         uint32_t *d_cand_count = L.counters.as<uint32_t>();
-        uint32_t *d_list_count = d_cand_count + 1;
         tmb::ScanArgs a{};
         a.x = ctx->clean.as<float>();
         a.q = g.q.as<float>();
@@ -658,6 +668,7 @@ void execute_group_mixed(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
         a.bmin_u = L.bmin_u.as<uint32_t>();
         a.bmin_l = L.bmin_l.as<uint32_t>();
         a.nb = nb;
+        a.bucket_log = blog;
         a.cand = L.cand.as<Candidate>();
         a.cand_count = d_cand_count;
         a.cand_cap = L.cand_cap;
@@ -695,45 +706,7 @@ void execute_group_mixed(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
             L.phase_ms[0] += ms;
             L.prof_flops += flops;
         }
-        if (nk > 0)
-        {
-            TM_CUDA(tmb::launch_bucket_select(L.bmin_u.as<uint32_t>(), nb, g.tp.as<TemplParam>(),
-                                              g.slots.as<int>(), nk, L.tkey.as<uint32_t>(), s));
-            for (int la = 0; la < 3; la++)
-            {
-                L.list.reserve(sizeof(uint2) * static_cast<size_t>(L.list_cap));
-                TM_CUDA(cudaMemsetAsync(d_list_count, 0, sizeof(uint32_t), s));
-                TM_CUDA(tmb::launch_list_buckets(L.bmin_l.as<uint32_t>(), nb, g.slots.as<int>(), nk,
-                                                 L.tkey.as<uint32_t>(), L.list.as<uint2>(), d_list_count,
-                                                 L.list_cap, s));
-                TM_CUDA(cudaMemcpyAsync(hc + 1, d_list_count, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-                TM_CUDA(cudaStreamSynchronize(s));
-                count_launch(L, 2);
-                if (hc[1] <= L.list_cap)
-                    break;
-                L.list_cap = hc[1] + hc[1] / 2;
-            }
-            if (hc[1] > L.list_cap)
-                throw Failure{TM_ERR_NO_MEMORY, "bucket list overflow"};
-            TM_CUDA(tmb::launch_passb_mixed(L.list.as<uint2>(), hc[1], ctx->clean.as<float>(),
-                                            ctx->raw.as<float>(), ctx->prefix.as<double2>(), ctx->ptot.as<double2>(),
-                                            ctx->pcen.as<double>(), ctx->run.as<uint16_t>(), g.q.as<float>(),
-                                            g.tp.as<TemplParam>(),
-                                            L.tkey.as<uint32_t>(), w0, L.cand.as<Candidate>(), d_cand_count,
-                                            L.cand_cap, s));
-            if (hc[1] > 0)
-                count_launch(L);
-        }
-        if (L.profile)
-            TM_CUDA(cudaEventRecord(L.ev2, s));
-        TM_CUDA(cudaMemcpyAsync(hc, d_cand_count, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-        TM_CUDA(cudaMemcpyAsync(hc + 2, d_cand_count + 2, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-        TM_CUDA(cudaStreamSynchronize(s));
-        if (L.profile)
-            add_span(L, 1, L.ev1, L.ev2);
-        if (hc[2] != 0)
-            throw Failure{TM_ERR_TIMEOUT, "contraction kernel gave up waiting (code " + std::to_string(hc[2]) + ")"};
-        ncand = hc[0];
+        ncand = collect_candidates(ctx, L, g, a, true);
         if (ncand <= L.cand_cap)
             break;
         L.cand_cap = ncand + ncand / 2;

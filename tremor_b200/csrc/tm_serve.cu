@@ -59,7 +59,7 @@ static uint64_t serve_bytes(const tm_ctx *ctx, const tm_request &r)
 {
     const uint64_t W = ctx->n - static_cast<uint64_t>(r.m) + 1;
     const uint64_t row = 10ull * 16384 + sizeof(TemplParam);
-    const uint64_t cands = r.mode == TM_MODE_KNN ? std::min<uint64_t>(W, (2ull * r.k) * tmb::kBucket / 4)
+    const uint64_t cands = r.mode == TM_MODE_KNN ? std::min<uint64_t>(W, (2ull * r.k) * 512)
                                                  : std::max<uint64_t>(W / 512, 1024);
     return row + 48ull * cands;
 }
