@@ -33,7 +33,7 @@ static void bound_diagnostics_wm(tm_ctx *ctx, int m, const std::vector<int> &idx
         g.htp[t].thr_ed = -FLT_MAX; // emit nothing
     TM_CUDA(cudaMemcpyAsync(g.tp.p, g.htp.data(), sizeof(TemplParam) * g.T, cudaMemcpyHostToDevice, s));
     const size_t pairs = W * static_cast<size_t>(count);
-    DevBuf dd, de, dc, dx;
+    DevBuf dd, de, dc, dx, todo;
     dd.reserve(pairs * sizeof(float));
     de.reserve(pairs * sizeof(float));
     L.counters.reserve(8 * sizeof(uint32_t));
@@ -95,9 +95,11 @@ static void bound_diagnostics_wm(tm_ctx *ctx, int m, const std::vector<int> &idx
         dc.reserve(pairs * sizeof(Candidate));
         dx.reserve(pairs * sizeof(float));
         TM_CUDA(cudaMemcpyAsync(dc.p, all.data(), pairs * sizeof(Candidate), cudaMemcpyHostToDevice, s));
+        todo.reserve(pairs * sizeof(uint32_t));
         TM_CUDA(tmb::launch_rescore(dc.as<Candidate>(), static_cast<uint32_t>(pairs), g.tp.as<TemplParam>(),
-                                    g.q.as<float>(), g.order.as<int>(), ctx->raw.as<float>(), ctx->range_first,
-                                    dx.as<float>(), s));
+                                    g.q.as<float>(), g.order.as<int>(), ctx->raw.as<float>(),
+                                    tmb::PrefixView{a.P, a.PT, a.PC}, nullptr, ctx->range_first, dx.as<float>(),
+                                    todo.as<uint32_t>(), L.counters.as<uint32_t>() + 6, s));
         count_launch(L);
         TM_CUDA(cudaMemcpyAsync(exact, dx.p, pairs * sizeof(float), cudaMemcpyDeviceToHost, s));
     }
@@ -618,7 +620,7 @@ int tm_bound_diagnostics(tm_ctx *ctx, const float *queries, int count, int m, fl
         DevBuf dd, de, dc;
         dd.reserve(pairs * sizeof(float));
         de.reserve(pairs * sizeof(float));
-        ctx->main.counters.reserve(4 * sizeof(uint32_t));
+        ctx->main.counters.reserve(8 * sizeof(uint32_t));
         TM_CUDA(cudaMemsetAsync(ctx->main.counters.p, 0, 4 * sizeof(uint32_t), s));
         TM_CUDA(cudaMemsetAsync(dd.p, 0xff, pairs * sizeof(float), s)); // NaN where nothing was written
         TM_CUDA(cudaMemsetAsync(de.p, 0xff, pairs * sizeof(float), s));
@@ -660,16 +662,18 @@ int tm_bound_diagnostics(tm_ctx *ctx, const float *queries, int count, int m, fl
                 for (uint64_t j = 0; j < W; j++)
                     all[static_cast<size_t>(t) * W + j] = Candidate{static_cast<uint32_t>(t), static_cast<uint32_t>(j)};
             dc.reserve(pairs * sizeof(Candidate));
-            DevBuf dx;
+            DevBuf dx, todo;
             dx.reserve(pairs * sizeof(float));
+            todo.reserve(pairs * sizeof(uint32_t));
             TM_CUDA(cudaMemcpyAsync(dc.p, all.data(), pairs * sizeof(Candidate), cudaMemcpyHostToDevice, s));
             TM_CUDA(tmb::launch_rescore(dc.as<Candidate>(), static_cast<uint32_t>(pairs), g.tp.as<TemplParam>(),
-                                        g.q.as<float>(), g.order.as<int>(), ctx->raw.as<float>(), ls.w0, dx.as<float>(),
-                                        s));
+                                        g.q.as<float>(), g.order.as<int>(), ctx->raw.as<float>(), tmb::PrefixView{}, ls.mean.as<float>(), ls.w0,
+                                        dx.as<float>(), todo.as<uint32_t>(), ctx->main.counters.as<uint32_t>() + 6, s));
             count_launch(ctx->main);
             TM_CUDA(cudaMemcpyAsync(exact, dx.p, pairs * sizeof(float), cudaMemcpyDeviceToHost, s));
             TM_CUDA(cudaStreamSynchronize(s));
             dx.release();
+            todo.release();
         }
         uint32_t err = 0;
         TM_CUDA(cudaMemcpyAsync(&err, ctx->main.counters.as<uint32_t>() + 2, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));

@@ -84,4 +84,75 @@ __device__ __forceinline__ float replica_distance(const float *__restrict__ q, c
     return dist;
 }
 
+// replica_distance by the 16 lanes of a half warp (`lane` 0..15 of them, `half` their mask):
+// lane l < 8 is acc0[l], lane 8 + l acc1[l], so a step's 16 samples are one coalesced load and
+// every accumulator takes its terms in the same order. All lanes return the distance.
+__device__ __forceinline__ float replica_distance16(const float *__restrict__ q, const int *__restrict__ order,
+                                                    const float *__restrict__ raw, uint64_t g, int m, float mean,
+                                                    float stddev, int lane, unsigned half)
+{
+    if (stddev <= 1e-12f)
+        return kFltMax;
+    const float *x = raw + g + lane;
+    const float *ql = q + lane;
+    const float inv = __fdiv_rn(1.0f, stddev);
+    const int blocks = m / kZnormBlock;
+    float acc = 0.0f;
+    auto step = [&](float r, float t) {
+        const float d = __fmaf_rn(-__fsub_rn(clean32(r), mean), inv, t);
+        acc = __fmaf_rn(d, d, acc);
+    };
+    // 16 block offsets per load, one load ahead; 8 blocks' samples in flight
+    int ahead = lane < blocks ? order[lane] : 0;
+    for (int b0 = 0; b0 < blocks; b0 += 16)
+    {
+        const int now = ahead;
+        if (b0 + 16 + lane < blocks)
+            ahead = order[b0 + 16 + lane];
+        const int n = min(16, blocks - b0);
+        int b = 0;
+        for (; b + 8 <= n; b += 8)
+        {
+            float r[16], t[16];
+#pragma unroll
+            for (int k = 0; k < 8; k++)
+            {
+                const int off = __shfl_sync(half, now, b + k, 16);
+                r[2 * k] = x[off];
+                r[2 * k + 1] = x[off + 16];
+                t[2 * k] = ql[off];
+                t[2 * k + 1] = ql[off + 16];
+            }
+#pragma unroll
+            for (int k = 0; k < 16; k++)
+                step(r[k], t[k]);
+        }
+        for (; b < n; b++)
+        {
+            const int off = __shfl_sync(half, now, b, 16);
+            const float r0 = x[off], r1 = x[off + 16], t0 = ql[off], t1 = ql[off + 16];
+            step(r0, t0);
+            step(r1, t1);
+        }
+    }
+    // hsum256's order: acc0 + acc1, then l + (l + 4), then (s0 + s2) + (s1 + s3)
+    float v = __fadd_rn(acc, __shfl_xor_sync(half, acc, 8));
+    v = __fadd_rn(v, __shfl_xor_sync(half, v, 4));
+    v = __fadd_rn(v, __shfl_xor_sync(half, v, 2));
+    float dist = __fadd_rn(v, __shfl_xor_sync(half, v, 1));
+    for (int i = blocks * kZnormBlock; i < m; i += 16) // the m % 32 tail, one term after the other
+    {
+        const int n = min(16, m - i);
+        float d = 0.0f;
+        if (lane < n)
+            d = __fmaf_rn(-__fsub_rn(clean32(x[i]), mean), inv, ql[i]);
+        for (int k = 0; k < n; k++)
+        {
+            const float e = __shfl_sync(half, d, k, 16);
+            dist = __fmaf_rn(e, e, dist);
+        }
+    }
+    return dist;
+}
+
 } // namespace tmb

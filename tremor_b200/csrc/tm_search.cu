@@ -231,11 +231,11 @@ void add_span(Lane &L, int phase, cudaEvent_t a, cudaEvent_t b)
     L.phase_ms[phase] += ms;
 }
 
-// Exact re-scoring of a group's ncand candidates, answer order and kNN selection on the
+// Exact re-scoring of a group's ncand candidates (pv: prefix sums of mixed groups, mean: window means of the others), answer order and kNN selection on the
 // device, one copy to a pinned block that the result keeps, canonical answers.
 template <class Degenerate>
-void rescore_and_answer(tm_ctx *ctx, Lane &L, const GroupPlan &g, uint32_t ncand, uint64_t w0, tm_result &res,
-                        Degenerate degenerate_windows)
+void rescore_and_answer(tm_ctx *ctx, Lane &L, const GroupPlan &g, uint32_t ncand, const tmb::PrefixView &pv,
+                        const float *mean, uint64_t w0, tm_result &res, Degenerate degenerate_windows)
 {
     cudaStream_t s = L.stream;
     const int T = g.T, nk = g.nk;
@@ -257,9 +257,10 @@ void rescore_and_answer(tm_ctx *ctx, Lane &L, const GroupPlan &g, uint32_t ncand
     if (L.profile)
         TM_CUDA(cudaEventRecord(L.ev2, s));
     TM_CUDA(tmb::launch_rescore(L.cand.as<Candidate>(), ncand, g.tp.as<TemplParam>(), g.q.as<float>(),
-                                g.order.as<int>(), ctx->raw.as<float>(), w0, L.dist.as<float>(), s));
+                                g.order.as<int>(), ctx->raw.as<float>(), pv, mean, w0, L.dist.as<float>(),
+                                L.akeys.as<uint32_t>(), L.counters.as<uint32_t>() + 6, s)); // (the keys come later)
     if (ncand > 0)
-        count_launch(L);
+        count_launch(L, 2);
     if (L.profile)
         TM_CUDA(cudaEventRecord(L.ev3, s));
     unsigned long long *keys[2] = {L.akeys.as<unsigned long long>(), L.akeys.as<unsigned long long>() + cn};
@@ -505,7 +506,7 @@ void execute_group(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
     }
 
     std::vector<uint8_t> flags; // fetched only when some kNN bound is unbounded
-    rescore_and_answer(ctx, L, g, ncand, w0, res, [&](int, std::vector<Hit> &degenerate) {
+    rescore_and_answer(ctx, L, g, ncand, tmb::PrefixView{}, ls.mean.as<float>(), w0, res, [&](int, std::vector<Hit> &degenerate) {
         if (flags.empty())
         {
             flags.resize(W);
@@ -715,7 +716,8 @@ void execute_group_mixed(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
     }
     std::vector<uint16_t> run;
     std::vector<float> raw;
-    rescore_and_answer(ctx, L, g, ncand, w0, res, [&](int t, std::vector<Hit> &degenerate) {
+    const tmb::PrefixView pv{ctx->prefix.as<double2>(), ctx->ptot.as<double2>(), ctx->pcen.as<double>()};
+    rescore_and_answer(ctx, L, g, ncand, pv, nullptr, w0, res, [&](int t, std::vector<Hit> &degenerate) {
         if (run.empty())
         {
             run.resize(W);

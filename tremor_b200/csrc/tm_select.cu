@@ -307,20 +307,233 @@ template <bool MIXED> __global__ void __launch_bounds__(B_THREADS) k_passb(const
     }
 }
 
-// Exact (reference-arithmetic) distance of every candidate.
-__global__ void k_rescore(const Candidate *__restrict__ cand, uint32_t count, const TemplParam *__restrict__ tp,
-                          const float *__restrict__ q, const int *__restrict__ order, const float *__restrict__ raw,
-                          uint64_t w0, float *__restrict__ dist)
+// ---- exact (reference-arithmetic) distance of every candidate -------------------------
+//
+// The reference's window mean and std are floats rounded from FP64 sums taken sample by
+// sample. Their rounding is almost always certain without those chains: with S the true sum,
+// a chain of m additions is within m u sum |x| of S (u = 2^-53), and the chain of squared
+// differences within (m + 4) u of its value plus m (mean error)^2; whatever FP64 estimate of
+// mean and variance is at hand, with its own error bound, gives an interval that holds the
+// reference's FP64 value, and when both ends round to the same float that is the reference's
+// float. certain_stats decides so; the estimate comes from the prefix sums where the group has
+// them, else from 16 lanes' sums. A candidate it cannot decide (about one in 10^4; every one
+// near a level step or a loud stretch) goes to a list that k_rescore_serial takes one thread
+// per candidate, with the chains themselves.
+//
+// k_rescore gives a candidate 16 lanes (replica_distance16): loads are 64 bytes wide instead
+// of one sample per lane and window, and the chains 16 times shorter. Measured with its serial part (before: one
+// thread per candidate running both chains, 32 cache lines per load, never less than one
+// candidate's latency): 17000 candidates of 8192 samples 0.24 ms (0.63), 68000 of 16384 1.03
+// (1.56), 0.7 M of 4096 1.64 (2.73; without prefix sums 2.5-3.0, 3.3), 3.4 M of 256-8192 8.2
+// (10.3-12.9). Bound by L1: 8 bytes of sample and template per candidate and sample.
+__device__ __forceinline__ bool certain_stats(double mean, double mean_err, double var, double var_rel, int m, float &mean_f,
+                                              float &std_f)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    constexpr double u = 1.1102230246251565e-16;
+    const double md = (double)m;
+    // the chain's sum over m, and the division's rounding
+    const double chain = (md + 2.0) * u * 1.01 * sqrt(fma(mean, mean, var)) + 2.0 * u * fabs(mean);
+    const double em = (mean_err + chain) * 1.01;
+    mean_f = __double2float_rn(mean - em);
+    if (!(var > 1e-20 && var < 1e36 && var_rel < 1e-3) || mean_f != __double2float_rn(mean + em))
+        return false;
+    const double es = (0.5 * var_rel + (md + 8.0) * u + chain * chain / var) * 1.01;
+    const double sd = sqrt(var);
+    std_f = __double2float_rn(sd - sd * es);
+    return std_f == __double2float_rn(sd + sd * es);
+}
+
+// Statistics of window [g, g + m) from the prefix sums (prefix_stats_tail's quantities, kept in
+// FP64): false when their bound does not apply or does not decide.
+__device__ __forceinline__ bool prefix_exact_stats(const PrefixView &pv, uint64_t g, int m, double inv_m, float &mean_f,
+                                                   float &std_f)
+{
+    const double2 qa = pv.Q[g], qb = pv.Q[g + (uint64_t)m];
+    const uint64_t e = g + (uint64_t)m, b1 = g >> kPrefixBlockLog;
+    PrefixSums ps;
+    if (e >> kPrefixBlockLog == b1)
+        ps = prefix_sums_one_block(qa, qb, (float)(g - (b1 << kPrefixBlockLog)), (float)(e - (b1 << kPrefixBlockLog)),
+                                   (float)qa.y);
+    else
+        ps = prefix_sums_two_blocks(pv, qa, qb, g, m);
+    const double c = pv.C[b1], mu = ps.s1 * inv_m, var = fma(-mu, mu, ps.s2 * inv_m);
+    // e_var as prefix_stats_tail bounds it; the additional roundings of mu, c + mu and var here
+    const double e1 = (double)ps.e_s1 * inv_m, e2 = (double)ps.e_s2 * inv_m;
+    const double e_var = e2 + 2.0 * fabs(mu) * e1 + e1 * e1 + 16.0 * kEps64 * (fabs(var) + 2.0 * mu * mu);
+    return certain_stats(c + mu, e1 + 4.0 * kEps64 * (fabs(mu) + fabs(c)), var, e_var / var * 1.01, m, mean_f, std_f);
+}
+
+// The same from the sums of x - a and (x - a)^2 over the window by 16 lanes, a near the mean (the
+// per-length statistics' float; conversions to FP64, 16 per clock and SM, bound this: one each).
+__device__ __forceinline__ bool sums_exact_stats(const float *__restrict__ x, int m, double a, int lane, unsigned half,
+                                                 float &mean_f, float &std_f)
+{
+    double s1 = 0.0, s2 = 0.0, t1 = 0.0, t2 = 0.0;
+    int i = lane;
+    for (; i + 16 < m; i += 32)
+    {
+        const double c = (double)clean32(x[i]) - a, d = (double)clean32(x[i + 16]) - a;
+        s1 += c;
+        t1 += d;
+        s2 = fma(c, c, s2);
+        t2 = fma(d, d, t2);
+    }
+    if (i < m)
+    {
+        const double c = (double)clean32(x[i]) - a;
+        s1 += c;
+        s2 = fma(c, c, s2);
+    }
+    s1 += t1;
+    s2 += t2;
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1)
+    {
+        s1 += __shfl_xor_sync(half, s1, off);
+        s2 += __shfl_xor_sync(half, s2, off);
+    }
+    // additions in any order: within m u of the sum of magnitudes, at most sqrt(m s2); each term's
+    // own roundings and the divisions' within the margins
+    const double md = (double)m, u = kEps64, del = s1 / md, ms = s2 / md, var = fma(-del, del, ms);
+    const double em = (md + 8.0) * u * 1.01 * sqrt(ms) + 2.0 * u * fabs(a + del);
+    const double ev = (md + 8.0) * u * 1.01 * ms + 2.0 * fabs(del) * em + em * em + 4.0 * u * del * del;
+    return certain_stats(a + del, em, var, ev / var * 1.01, m, mean_f, std_f);
+}
+
+constexpr int R_THREADS = 256;
+
+// PREFIX: statistics from the prefix sums (windows of at most kPrefixBlock samples), else from
+// the samples. todo: the
+// undecided candidates' indices, their number in *todo_count.
+template <bool PREFIX>
+__global__ void __launch_bounds__(R_THREADS) k_rescore(const Candidate *__restrict__ cand, uint32_t count,
+                                                       const TemplParam *__restrict__ tp, const float *__restrict__ q,
+                                                       const int *__restrict__ order, const float *__restrict__ raw,
+                                                       const PrefixView pv, const float *__restrict__ mean, uint64_t w0,
+                                                       float *__restrict__ dist, uint32_t *__restrict__ todo,
+                                                       uint32_t *__restrict__ todo_count)
+{
+    const uint32_t i = blockIdx.x * (R_THREADS / 16) + (threadIdx.x >> 4);
     if (i >= count)
-        return;
+        return; // a whole half warp
+    const int lane = threadIdx.x & 15;
+    const unsigned half = 0xffffu << (threadIdx.x & 16);
     const Candidate c = cand[i];
-    const TemplParam p = tp[c.templ];
+    const TemplParam &p = tp[c.templ];
     const uint64_t g = w0 + c.window;
+    const int m = p.m;
     float mean_f, std_f;
-    exact_stats(raw, g, p.m, mean_f, std_f);
-    dist[i] = replica_distance(q + p.q_offset, order + p.order_offset, raw, g, p.m, mean_f, std_f);
+    if (!(PREFIX ? prefix_exact_stats(pv, g, m, p.inv_m, mean_f, std_f)
+                 : sums_exact_stats(raw + g, m, (double)mean[c.window], lane, half, mean_f, std_f)))
+    {
+        if (lane == 0)
+            todo[atomicAdd(todo_count, 1u)] = i;
+        return;
+    }
+    const float d = replica_distance16(q + p.q_offset, order + p.order_offset, raw, g, m, mean_f, std_f, lane, half);
+    if (lane == 0)
+        dist[i] = d;
+}
+
+// The undecided candidates: four warps per SM quarter, each taking up to 16 at a time. It stages
+// 1024 samples in shared memory as doubles, split evenly between its candidates, by coalesced
+// loads one stage ahead; then lane c runs candidate c's chain over its share. (One thread per
+// candidate loading for itself costs 32 cache lines per load, and converting in the chain is
+// bound by the conversions, 16 per clock and SM: 8 windows of 8192 samples took 940 us.)
+constexpr int S_WARPS = 4, S_CANDS = 16, S_LOADS = 32; // 32 S_LOADS samples per stage
+
+__global__ void __launch_bounds__(S_WARPS * 32) k_rescore_serial(const Candidate *__restrict__ cand,
+                                                                const TemplParam *__restrict__ tp, const float *__restrict__ q,
+                                                                const int *__restrict__ order, const float *__restrict__ raw,
+                                                                uint64_t w0, float *__restrict__ dist,
+                                                                const uint32_t *__restrict__ todo,
+                                                                const uint32_t *__restrict__ todo_count)
+{
+    __shared__ double tile[S_WARPS][32 * S_LOADS + S_CANDS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t count = *todo_count, warps = gridDim.x * S_WARPS;
+    const uint32_t per = min((count + warps - 1) / warps, (uint32_t)S_CANDS);
+    // samples of a candidate per stage: 64 for 16 candidates .. 1024 for one
+    const int slog = 10 - (per > 1 ? 32 - __clz(per - 1) : 0), stage = 1 << slog;
+    for (uint32_t n0 = (blockIdx.x * S_WARPS + warp) * per; n0 < count; n0 += warps * per)
+    {
+        const int nc = (int)min(per, count - n0);
+        // lane c: candidate n0 + c
+        uint32_t idx = 0, row = 0;
+        uint64_t g = 0;
+        int m = 0;
+        if (lane < nc)
+        {
+            idx = todo[n0 + lane];
+            const Candidate c = cand[idx];
+            row = c.templ;
+            m = tp[row].m;
+            g = w0 + c.window;
+        }
+        const int longest = (int)__reduce_max_sync(0xffffffffu, (uint32_t)m);
+        // each(v): the lane's samples in order, missing ones as 0
+        auto chain = [&](auto each) {
+            float next[S_LOADS];
+            auto load = [&](int s) {
+#pragma unroll
+                for (int k = 0; k < S_LOADS; k++)
+                {
+                    const int c = 32 * k >> slog, at = s + (32 * k & (stage - 1)) + lane;
+                    const uint64_t gc = __shfl_sync(0xffffffffu, g, c);
+                    next[k] = at < __shfl_sync(0xffffffffu, m, c) ? clean32(raw[gc + (uint64_t)at]) : 0.0f;
+                }
+            };
+            load(0);
+            for (int s = 0; s < longest; s += stage)
+            {
+                __syncwarp(); // the last stage has been read
+#pragma unroll
+                for (int k = 0; k < S_LOADS; k++)
+                    tile[warp][(32 * k >> slog) * (stage + 1) + (32 * k & (stage - 1)) + lane] = (double)next[k];
+                __syncwarp();
+                if (s + stage < longest)
+                    load(s + stage);
+                const double *v = tile[warp] + (lane & ((32 * S_LOADS >> slog) - 1)) * (stage + 1);
+                const int n = min(stage, m - s); // none for lanes without a candidate
+                int k = 0;
+                for (; k + 32 <= n; k += 32)
+                {
+#pragma unroll
+                    for (int i = 0; i < 32; i++)
+                        each(v[k + i]);
+                }
+                for (; k < n; k++)
+                    each(v[k]);
+            }
+        };
+        // exact_stats' operations
+        double sum = 0.0, squares = 0.0;
+        chain([&](double v) { sum = __dadd_rn(sum, v); });
+        const double md = (double)max(m, 1), mean = __ddiv_rn(sum, md);
+        chain([&](double v) {
+            const double c = __dsub_rn(v, mean);
+            squares = __fma_rn(c, c, squares);
+        });
+        const double sd = __dsqrt_rn(__ddiv_rn(squares, md));
+        const float mean_f = __double2float_rn(mean), std_f = sd <= 1e-12 ? 0.0f : __double2float_rn(sd);
+        for (int c = 0; c < nc; c += 2) // the distances, one per half warp
+        {
+            const int src = c + (lane >> 4);
+            const uint32_t r = __shfl_sync(0xffffffffu, row, src);
+            const uint64_t gc = __shfl_sync(0xffffffffu, g, src);
+            const float mc = __shfl_sync(0xffffffffu, mean_f, src), sc = __shfl_sync(0xffffffffu, std_f, src);
+            const uint32_t at = __shfl_sync(0xffffffffu, idx, src);
+            if (src < nc)
+            {
+                const TemplParam &p = tp[r];
+                const float d = replica_distance16(q + p.q_offset, order + p.order_offset, raw, gc, p.m, mc, sc, lane & 15,
+                                                   0xffffu << (lane & 16));
+                if ((lane & 15) == 0)
+                    dist[at] = d;
+            }
+            __syncwarp();
+        }
+    }
 }
 
 // ---- launchers --------------------------------------------------------------------
@@ -373,11 +586,24 @@ cudaError_t launch_passb(const uint2 *list, const uint32_t *counters, uint32_t c
     return cudaGetLastError();
 }
 
+// pv: the prefix sums, when the group's windows have them (Q not null); else mean: the
+// windows' means, near enough to centre their sums. todo: scratch of `count` indices;
+// todo_count: its counter, zeroed here.
 cudaError_t launch_rescore(const Candidate *cand, uint32_t count, const TemplParam *tp, const float *q,
-                           const int *order, const float *raw, uint64_t w0, float *dist, cudaStream_t s)
+                           const int *order, const float *raw, const PrefixView &pv, const float *mean, uint64_t w0, float *dist,
+                           uint32_t *todo, uint32_t *todo_count, cudaStream_t s)
 {
-    if (count > 0)
-        k_rescore<<<(count + 127) / 128, 128, 0, s>>>(cand, count, tp, q, order, raw, w0, dist);
+    if (count == 0)
+        return cudaSuccess;
+    if (const cudaError_t e = cudaMemsetAsync(todo_count, 0, sizeof(uint32_t), s); e != cudaSuccess)
+        return e;
+    const unsigned grid = (count - 1) / (R_THREADS / 16) + 1;
+    if (pv.Q != nullptr)
+        k_rescore<true><<<grid, R_THREADS, 0, s>>>(cand, count, tp, q, order, raw, pv, mean, w0, dist, todo, todo_count);
+    else
+        k_rescore<false><<<grid, R_THREADS, 0, s>>>(cand, count, tp, q, order, raw, pv, mean, w0, dist, todo, todo_count);
+    const unsigned serial = std::min((count - 1) / S_WARPS + 1, 148u * 4u); // how many are undecided the device knows
+    k_rescore_serial<<<serial, S_WARPS * 32, 0, s>>>(cand, tp, q, order, raw, w0, dist, todo, todo_count);
     return cudaGetLastError();
 }
 
