@@ -316,9 +316,9 @@ __global__ void __launch_bounds__(N / 16) k_fft_forward(const float *__restrict_
 // the windows' statistics), the FP64 pipe 35 and 28 %, issue 40 %; templates of distinct lengths
 // also compute their windows' statistics (issue 49 %). Per template and 2^25 samples, in ms
 // (before: FP64 passes of radix 16, 16, 16, 2 with block-wide barriers, steps of 8192 for up to
-// 8192 samples, longer pieces above): m = 1024 0.169 (0.49), 2048 0.170 (0.49), 4096 0.204
-// (0.49), 8192 0.320 (0.49), 16384 0.43 (0.62); with distinct lengths 1000 0.249, 2000 0.274,
-// 4096 0.307 (0.71), 8192 0.432 (0.71), 16000 0.63 (1.07). 32 points per thread and two exchanges
+// 8192 samples, longer pieces above): m = 1024 0.166 (0.49), 2048 0.166 (0.49), 4096 0.196
+// (0.49), 8192 0.306 (0.49), 16384 0.42 (0.62); with distinct lengths 1000 0.244, 2000 0.272,
+// 4096 0.301 (0.71), 8192 0.424 (0.71), 16000 0.63 (1.07). 32 points per thread and two exchanges
 // (radix 16, 16, 16; 8 warps per SM) took 0.177 at m = 2048 and 0.409 at distinct 4096, also
 // with the epilogue on warps of its own: too few warps to hide the latencies.
 template <int N> struct FftShape
@@ -329,7 +329,9 @@ template <int N> struct FftShape
     static constexpr int Ex = 8 * Group;         // doubles of one exchange plane
     static constexpr int Pitch = fft_pitch(N);   // entries of a spectrum
     static constexpr int Dot = N / 4 + 4;        // floats of that transform's outputs (the pad: see the epilogue)
-    // the twiddle tables: the packing's roots, then those of the two last radix-8 passes
+    // the twiddle tables: the packing's roots, then those of the two last radix-8 passes, even
+    // entries before odd ones: a thread takes an even one and the next, and a quarter warp's 16-byte
+    // loads fall in distinct banks (side by side, two to a bank, 1 to 2.5 % of the kernel's time)
     static constexpr int TabB = T + 1, TabC = TabB + 4 * (N == 4096 ? 8 : 16), Tabs = TabC + N / 64;
     static constexpr size_t Smem =
         2 * sizeof(double) * Ex + 8 * sizeof(float) * Dot + sizeof(double2) * Tabs + 2 * sizeof(FftRow);
@@ -730,9 +732,10 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
         read_pairs();
         {
             const int k = (2 * s) & (Ns2 - 1);
-            const double2 *w = tab + C::TabB + k;
+            const double2 *w = tab + C::TabB + k / 2; // of k, then of k + 1
             radix8(A, w[0], w[Ns2], w[2 * Ns2], w[3 * Ns2]);
-            radix8(B, w[1], w[Ns2 + 1], w[2 * Ns2 + 1], w[3 * Ns2 + 1]);
+            w += Ns2 / 2;
+            radix8(B, w[0], w[Ns2], w[2 * Ns2], w[3 * Ns2]);
             group_sync<N>(g);
             const int b = 9 * (2 * s - k) + k;
 #pragma unroll
@@ -746,13 +749,13 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
         group_sync<N>(g);
         read_pairs();
         {
-            const double2 *w = tab + C::TabC + 2 * s;
+            const double2 *w = tab + C::TabC + s; // of 2 s, then of 2 s + 1
             {
                 const double2 w1 = w[0], w2 = csqr(w1);
                 radix8(A, w1, w2, csqr(w2), mul_w8(w1));
             }
             {
-                const double2 w1 = w[1], w2 = csqr(w1);
+                const double2 w1 = w[C::GT], w2 = csqr(w1);
                 radix8(B, w1, w2, csqr(w2), mul_w8(w1));
             }
             // outputs n1 = 2 s + (Q / 8) r and the next of transform g: correlation outputs 16 n1 + 2 g (+ 1)
@@ -1000,13 +1003,14 @@ template <int N> static void corr_tables(double2 *tab)
         tab[i] = root_of(i, 2 * N);
     for (int k = 0; k < Ns; k++)
     {
-        tab[C::TabB + k] = root_of(k, 8 * Ns);
-        tab[C::TabB + Ns + k] = root_of(2 * k, 8 * Ns);
-        tab[C::TabB + 2 * Ns + k] = root_of(4 * k, 8 * Ns);
-        tab[C::TabB + 3 * Ns + k] = root_of(k + Ns, 8 * Ns);
+        double2 *w = tab + C::TabB + (k & 1) * (Ns / 2) + k / 2;
+        w[0] = root_of(k, 8 * Ns);
+        w[Ns] = root_of(2 * k, 8 * Ns);
+        w[2 * Ns] = root_of(4 * k, 8 * Ns);
+        w[3 * Ns] = root_of(k + Ns, 8 * Ns);
     }
     for (int b = 0; b < N / 64; b++)
-        tab[C::TabC + b] = root_of(b, N / 8);
+        tab[C::TabC + (b & 1) * C::GT + b / 2] = root_of(b, N / 8);
 }
 
 void fft_roots(double2 *host)

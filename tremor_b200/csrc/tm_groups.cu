@@ -417,9 +417,9 @@ double tensor_cost_sorted(const tm_ctx *ctx, const int *m, size_t n)
 // Modelled milliseconds of the FFT branch per template of length m per 2^25 samples; shared: a
 // template of the same length precedes it, whose window statistics it takes. The branch's time
 // depends on the length through the pieces' step alone, and within a class little on it; the
-// factors are the classes' times over that of distinct lengths at 4096 (0.304 ms) or 16000
-// (0.63 ms): 0.245, 0.273, 0.304, 0.428 distinct at 1000, 2000, 4096, 8192; 0.167, 0.167,
-// 0.201, 0.315 shared, and 0.43 shared at 16384.
+// factors are the classes' times over that of distinct lengths at 4096 (0.301 ms) or 16000
+// (0.63 ms): 0.244, 0.272, 0.301, 0.424 distinct at 1000, 2000, 4096, 8192; 0.166, 0.166,
+// 0.196, 0.306 shared, and 0.42 shared at 16384.
 double fft_time(const tm_ctx *ctx, int m, bool shared)
 {
     static const double distinct[tmb::kFftClasses] = {0.81, 0.90, 1.0, 1.41};
