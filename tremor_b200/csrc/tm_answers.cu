@@ -17,7 +17,7 @@
 //   radix sort 2       by the new key; the sort is stable, so equal distances stay in
 //                      position order: (distance, position) order within a kNN run
 //   k_answer_segments  each template's run [start, end), its windows and distances
-//   k_select_knn       one warp per kNN template: the greedy exclusion selection over
+//   k_select_knn       one block per kNN template: the greedy exclusion selection over
 //                      its run (finite distances only), up to k answers
 // The sorts are CUB's device radix sort from the CUDA toolkit, over 32 + ceil(log2 T)
 // (+1) key bits. Within a template no window appears twice: every (template, window)
@@ -31,7 +31,7 @@
 namespace tmb {
 
 constexpr int kAnswerThreads = 256;
-constexpr int kSelectWarps = 4;
+constexpr int kSelectThreads = 256;
 
 __device__ __forceinline__ void warp_slot(bool keep, uint32_t *counter, uint32_t &slot)
 {
@@ -121,72 +121,142 @@ __global__ void __launch_bounds__(kAnswerThreads)
         end[t] = i + 1;
 }
 
-// Greedy exclusion selection of one kNN template per warp over its run in (distance,
+// Greedy exclusion selection of one kNN template per block over its run in (distance,
 // position) order: a candidate is kept when no kept window lies closer than merge
 // (|gap| < merge), until k are kept (ZnormSearch.hpp:170-189). Only finite distances
 // take part; the run's FLT_MAX entries, at its end, are left to the host, which needs
-// them only when the reference's queue would not have filled. Lanes take 32 candidates
-// at a time; the survivors of the kept-set check are accepted in lane order, each one
-// removing the later survivors within merge of it. out_n[slot] = answers kept.
-__global__ void __launch_bounds__(kSelectWarps * 32)
-    k_select_knn(const int *__restrict__ slots, int nk, const TemplParam *__restrict__ tp,
-                 const uint32_t *__restrict__ start, const uint32_t *__restrict__ end,
-                 const uint32_t *__restrict__ window, const float *__restrict__ dist, int kcap,
-                 uint32_t *__restrict__ out_n, uint32_t *__restrict__ out_win, float *__restrict__ out_dist)
+// them only when the reference's queue would not have filled. out_n[slot] = answers kept.
+//
+// A run is long when its nearest windows crowd around few events (tens of thousands of
+// candidates for 100 answers), and almost all of it falls to the check against the kept
+// windows: the block takes one candidate per thread, with the next ones on their way from
+// memory, and only the survivors, in order, go to one warp, which accepts them in turn,
+// each one removing the later ones within merge of it. Bound by the chain of chunks, one
+// after another, of the longest run: 3.4 million candidates of 96 templates in 0.41 ms,
+// where a warp per template, 32 candidates at a time, took 4.8.
+__global__ void __launch_bounds__(kSelectThreads)
+    k_select_knn(const int *__restrict__ slots, const TemplParam *__restrict__ tp, const uint32_t *__restrict__ start,
+                 const uint32_t *__restrict__ end, const uint32_t *__restrict__ window,
+                 const float *__restrict__ dist, int kcap, uint32_t *__restrict__ out_n,
+                 uint32_t *__restrict__ out_win, float *__restrict__ out_dist)
 {
-    extern __shared__ uint32_t kept_win[]; // kSelectWarps x kcap
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int slot = blockIdx.x * kSelectWarps + warp;
-    if (slot >= nk)
-        return; // whole warp
+    extern __shared__ uint4 kept_smem[]; // the kept windows: kcap, rounded up to fours
+    __shared__ uint32_t left_win[kSelectThreads], warp_left[kSelectThreads / 32];
+    __shared__ float left_dist[kSelectThreads];
+    __shared__ int kept_count;
+    uint32_t *kw = reinterpret_cast<uint32_t *>(kept_smem);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, slot = blockIdx.x;
     const int t = slots[slot];
     const int k = min(tp[t].k, kcap);
     const uint32_t merge = (uint32_t)max(tp[t].merge, 0);
     const uint32_t a = start[t], b = end[t];
-    uint32_t *kw = kept_win + warp * kcap;
     uint32_t *ow = out_win + (size_t)slot * kcap;
     float *od = out_dist + (size_t)slot * kcap;
     int n = 0;
-    for (uint32_t base = a; base < b && n < k; base += 32)
+    uint32_t w = 0u;
+    float d = kFltMax;
+    if (a + tid < b)
     {
-        const uint32_t i = base + lane;
-        const bool valid = i < b;
-        const uint32_t w = valid ? window[i] : 0u;
-        const float d = valid ? dist[i] : 0.0f;
-        bool pass = valid && d < kFltMax;
-        if (merge > 0 && pass)
-            for (int j = 0; j < n; j++)
-            {
-                const uint32_t kj = kw[j];
-                if ((w > kj ? w - kj : kj - w) < merge)
-                {
-                    pass = false;
-                    break;
-                }
-            }
-        const bool last = __any_sync(0xffffffffu, valid && !(d < kFltMax));
-        unsigned pb = __ballot_sync(0xffffffffu, pass);
-        while (pb != 0u && n < k)
+        w = window[a + tid];
+        d = dist[a + tid];
+    }
+    for (uint32_t base = a; base < b && n < k; base += kSelectThreads)
+    {
+        const uint32_t cw = w, next = base + kSelectThreads + tid;
+        const float cd = d;
+        w = 0u;
+        d = kFltMax;
+        if (next < b)
         {
-            const int leader = __ffs(pb) - 1;
-            const uint32_t lw = __shfl_sync(0xffffffffu, w, leader);
-            const float ld = __shfl_sync(0xffffffffu, d, leader);
-            if (lane == 0)
-            {
-                kw[n] = lw;
-                ow[n] = lw;
-                od[n] = ld;
-            }
-            n++;
-            if (lane == leader || (pass && (w > lw ? w - lw : lw - w) < merge))
-                pass = false;
-            pb = __ballot_sync(0xffffffffu, pass);
+            w = window[next];
+            d = dist[next];
         }
-        __syncwarp();
-        if (last)
+        bool pass = cd < kFltMax; // false past the run's end too
+        const bool last = !pass;
+        if (merge > 0 && pass)
+        {
+            int j = 0;
+            for (; j + 4 <= n && pass; j += 4)
+            {
+                const uint4 q = kept_smem[j / 4];
+                pass = __usad(cw, q.x, 0u) >= merge && __usad(cw, q.y, 0u) >= merge && __usad(cw, q.z, 0u) >= merge &&
+                       __usad(cw, q.w, 0u) >= merge;
+            }
+            for (; j < n && pass; j++)
+                pass = __usad(cw, kw[j], 0u) >= merge;
+        }
+        // the survivors, in order
+        const unsigned ballot = __ballot_sync(0xffffffffu, pass);
+        if (lane == 0)
+            warp_left[warp] = (uint32_t)__popc(ballot);
+        const bool stop = __syncthreads_or(last);
+        uint32_t pos = (uint32_t)__popc(ballot & ((1u << lane) - 1u)), total = 0;
+#pragma unroll
+        for (int i = 0; i < kSelectThreads / 32; i++)
+        {
+            const uint32_t c = warp_left[i];
+            pos += i < warp ? c : 0u;
+            total += c;
+        }
+        if (total > 0) // the same in every thread
+        {
+            if (pass)
+            {
+                left_win[pos] = cw;
+                left_dist[pos] = cd;
+            }
+            __syncthreads();
+            if (warp == 0)
+            {
+                const int n0 = n;
+                for (uint32_t i0 = 0; i0 < total && n < k; i0 += 32)
+                {
+                    const bool valid = i0 + lane < total;
+                    const uint32_t lw = valid ? left_win[i0 + lane] : 0u;
+                    const float ld = valid ? left_dist[i0 + lane] : 0.0f;
+                    bool open = valid;
+                    for (int j = n0; j < n && merge > 0; j++) // kept since the check
+                        open = open && __usad(lw, kw[j], 0u) >= merge;
+                    unsigned ob = __ballot_sync(0xffffffffu, open);
+                    if (merge == 0)
+                    {
+                        const int at = n + __popc(ob & ((1u << lane) - 1u));
+                        if (open && at < k)
+                        {
+                            ow[at] = lw;
+                            od[at] = ld;
+                        }
+                        n = min(k, n + __popc(ob));
+                        continue;
+                    }
+                    while (ob != 0u && n < k)
+                    {
+                        const int leader = __ffs(ob) - 1;
+                        const uint32_t aw = __shfl_sync(0xffffffffu, lw, leader);
+                        if (lane == leader)
+                        {
+                            kw[n] = lw;
+                            ow[n] = lw;
+                            od[n] = ld;
+                        }
+                        n++;
+                        open = open && lane != leader && __usad(lw, aw, 0u) >= merge;
+                        ob = __ballot_sync(0xffffffffu, open);
+                    }
+                    __syncwarp();
+                }
+                if (lane == 0)
+                    kept_count = n;
+            }
+            __syncthreads();
+            n = kept_count;
+        }
+        else
+            __syncthreads(); // warp_left is written again
+        if (stop)
             break;
     }
-    if (lane == 0)
+    if (tid == 0)
         out_n[slot] = (uint32_t)n;
 }
 
@@ -264,9 +334,8 @@ cudaError_t launch_select_knn(const int *slots, int nk, const TemplParam *tp, co
                               uint32_t *out_n, uint32_t *out_win, float *out_dist, cudaStream_t s)
 {
     if (nk > 0)
-        k_select_knn<<<(nk + kSelectWarps - 1) / kSelectWarps, kSelectWarps * 32,
-                       sizeof(uint32_t) * kSelectWarps * kcap, s>>>(slots, nk, tp, start, end, window, dist, kcap,
-                                                                    out_n, out_win, out_dist);
+        k_select_knn<<<nk, kSelectThreads, sizeof(uint4) * ((kcap + 3) / 4), s>>>(slots, tp, start, end, window, dist,
+                                                                                  kcap, out_n, out_win, out_dist);
     return cudaGetLastError();
 }
 

@@ -118,7 +118,7 @@ std::shared_ptr<PinnedBlock> acquire_block(Lane &L, size_t need)
     return pool.back();
 }
 
-// Largest k whose selection runs on the device (k_select_knn keeps k windows per warp in
+// Largest k whose selection runs on the device (k_select_knn keeps k windows per block in
 // shared memory); groups with a larger k select on the host.
 constexpr int kMaxDeviceK = 1024;
 
