@@ -265,7 +265,7 @@ struct Lane
     HostBuf h_split, h_q, h_order, h_slots, h_counters;
     uint32_t cand_cap = 1u << 22, list_cap = 1u << 20;
     // FFT branch: the template spectra of a launch
-    DevBuf fft_Y, fft_stats; // (fft_stats: the correlation kernel's per-block statistics cache)
+    DevBuf fft_Y, fft_stats, fft_cuts; // (fft_stats: the correlation kernel's per-block statistics cache)
     // instrumentation
     bool profile = false;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr, ev3 = nullptr, ev4 = nullptr;
@@ -350,8 +350,8 @@ struct tm_ctx
     std::mutex fft_mu;
     int sms = 148;
     // model: the FFT branch's ms per template per 2^25 samples, for templates of 4096 samples and
-    // of 16384, of distinct lengths (B200 defaults; tm_autotune measures both); fft_time
-    // scales them to other lengths and to equal ones
+    // of 16384, that evaluate all their windows (B200 defaults; tm_autotune measures both);
+    // fft_time scales them to other lengths and to templates that need not
     double fft_ms = 0.307;
     double fft_long_ms = 0.63;
     // the context's own memory pool for per-batch buffers (DevBuf::reserve_on); it keeps
@@ -473,7 +473,8 @@ void prepare_group_mixed(tm_ctx *ctx, Lane &L, const std::vector<int> &idx_in, c
 void prepare_fft(tm_ctx *ctx, Lane &L, GroupPlan &g);
 int plan_col_tile(const tm_ctx *ctx, const tm_request *reqs, const std::vector<int> &idx, double *cost = nullptr);
 double tile_time(const tm_ctx *ctx, bool mixed, int v, double k);
-double fft_time(const tm_ctx *ctx, int m, bool shared);
+double fft_time(const tm_ctx *ctx, int m, int longer, bool skips);
+uint32_t fft_stage_end(uint32_t p0, uint32_t pieces, int rows, int cls, int sms);
 void create_batch(tm_ctx *ctx, Lane &L, const tm_request *requests, int count, tm_batch &b, bool serving = false);
 
 // tm_serve.cu

@@ -1,6 +1,8 @@
 // The FFT branch's constants, launch arguments and launchers (tm_fftk.cu).
 #pragma once
 
+#include <cmath>
+
 #include "tm_internal.cuh"
 #include "tm_prefix.cuh"
 
@@ -39,14 +41,24 @@ struct FftRow
 {
     double inv_m;
     double sum[kFftMaxParts - 1]; // the sums of its parts after the first
-    float s1, c_lin, a3, thr;
+    float s1, c_lin, a3, thr; // thr: infinite for kNN
     float4 c0;
     float qs, s1_max;
     int row; // its row in tp
     int m, mode;
     uint32_t wcount;
-    int pad[2];
+    float e_norm; // fft_e_norm
+    float inv_a3; // 1 / (1 - a3), rounded up
 };
+
+// An FFT dot product's error: norms of the template and of the piece's samples times this; the
+// largest norm of a template of length m is qs / sqrt(m). 1 % is left for FP32 rounding.
+constexpr double kFftKappa = 10.0 * 16.0 * 111.0 * 1.1102230246251565e-16;
+inline float fft_e_norm(float qs, int m, int cls)
+{
+    const double sm = sqrt((double)m);
+    return (float)(1.01 * kFftKappa * (double)qs / sm * (2.0 * sm + sqrt(2.0 * fft_class(cls).n)));
+}
 
 struct FftArgs
 {
@@ -70,6 +82,8 @@ struct FftArgs
     Candidate *cand;
     uint32_t *cand_count, cand_cap;
     float *dbg_d, *dbg_e; // diagnostics: d and e of every window, [t][W]; null in searches
+    int prune;            // some template has a cut: no window with d - e above it is wanted
+    const float *cuts;    // the cuts of rows' templates; null: their thr
     float4 *stats;        // per block, the folded statistics of a piece's windows (a lane's scratch, kFftStats)
 };
 
@@ -86,6 +100,10 @@ cudaError_t launch_fft_pieces(const float *clean, uint64_t n, const double *cent
                               double2 *X, double *shifts, double *norms, cudaStream_t s);
 cudaError_t launch_fft_templates(const float *q, const TemplParam *tp, const FftRow *rows, int nrows, int cls, int parts,
                                  const double2 *roots, double2 *Y, cudaStream_t s);
+// Cuts of the templates of rows from the minima of the first nb_seen buckets (tm_select.cu): a
+// threshold, a kNN bound or infinity. sup: nk x nb_seen keys of scratch, where super is set.
+cudaError_t launch_fft_cuts(const FftRow *rows, int nrows, const uint32_t *bmin_u, uint32_t *sup, uint32_t nb, uint32_t nb_seen,
+                            int blog, const TemplParam *tp, const int *slots, int nk, bool super, float *cuts, cudaStream_t s);
 cudaError_t launch_fft_corr(FftArgs a, int cls, const double2 *roots, int sms, cudaStream_t s);
 
 } // namespace tmb

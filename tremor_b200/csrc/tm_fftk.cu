@@ -57,7 +57,6 @@ namespace tmb {
 // and the twiddle tables (R1 then R2).
 template <int N> constexpr int kFBuf = N + N / 16 + 16;
 template <int N> constexpr size_t kFSmem = sizeof(double2) * (size_t)(kFBuf<N> + kFftRoots);
-constexpr double kFftKappa = 10.0 * 16.0 * 111.0 * 1.1102230246251565e-16;
 
 __device__ __forceinline__ int pidx(int i) { return i + (i >> 4); }
 
@@ -311,16 +310,29 @@ __global__ void __launch_bounds__(N / 16) k_fft_forward(const float *__restrict_
 // twiddles are folded into the butterflies, a + w b by four FMAs and a - w b = 2 a - (a + w b)
 // by two.
 //
-// What bounds it (16 templates or more of one length): the load/store unit's data pipe, 73 %
-// busy with N = 4096 and 60 % with 8192 (three exchanges of 16 bytes a point, the spectra and
-// the windows' statistics), the FP64 pipe 35 and 28 %, issue 40 %; templates of distinct lengths
-// also compute their windows' statistics (issue 49 %). Per template and 2^25 samples, in ms
-// (before: FP64 passes of radix 16, 16, 16, 2 with block-wide barriers, steps of 8192 for up to
-// 8192 samples, longer pieces above): m = 1024 0.166 (0.49), 2048 0.166 (0.49), 4096 0.196
-// (0.49), 8192 0.306 (0.49), 16384 0.42 (0.62); with distinct lengths 1000 0.244, 2000 0.272,
-// 4096 0.301 (0.71), 8192 0.424 (0.71), 16000 0.63 (1.07). 32 points per thread and two exchanges
-// (radix 16, 16, 16; 8 warps per SM) took 0.177 at m = 2048 and 0.409 at distinct 4096, also
-// with the epilogue on warps of its own: too few warps to hide the latencies.
+// Skipped windows. Once a template has a cut (its threshold; a kNN bound from the first pieces),
+// almost no window can be an answer, and a chunk of 128 windows needs its statistics only where
+// some dot product exceeds what 1 / sd of that chunk allows. The bounds of 1 / sd and of the mean
+// come from the last template of the piece that evaluated every window, if at most 10 % shorter:
+// items of a piece go from the shortest template to the longest (chunk_limit has the argument).
+// The others read neither prefix sums nor kept statistics.
+//
+// What bounds it: the load/store unit's data pipe, about 70 % busy (three exchanges of 16 bytes a
+// point, the spectra, the outputs), the FP64 pipe 35 %, and the two barriers of an item; an item
+// that evaluates all its windows also reads 34 bytes of prefix sums and runs per window (or 12
+// bytes of a shared length's kept statistics) and issues 70 instructions for it. Per template
+// and 2^25 samples, in ms, skipping / kept statistics / all its own (FP64 passes of radix 16, 16,
+// 16, 2 with block-wide barriers, steps of 8192 for up to 8192 samples, longer pieces above and
+// no skipping took 0.49 with kept statistics and 0.71 without, 0.62 and 1.07 above 8192): m =
+// 1024 0.128 / 0.169 / 0.25, 2048 0.149 / 0.167 / 0.278, 4096 0.167 / 0.203 / 0.31, 8192 0.248 /
+// 0.315 / 0.43, 16000 0.38 / 0.42 / 0.63. 32 points per thread and two exchanges (radix 16, 16, 16; 8
+// warps per SM) took 0.177 at m = 2048 and 0.409 with distinct lengths at 4096 before windows
+// were skipped, also with the epilogue on warps of its own: too few warps to hide the latencies.
+struct FftItem // what an item needs of its piece, and its row's cut
+{
+    double shift[kFftMaxParts], norm[kFftMaxParts];
+    float cut, pad[3];
+};
 template <int N> struct FftShape
 {
     static constexpr int T = N / 16;             // threads
@@ -333,13 +345,14 @@ template <int N> struct FftShape
     // entries before odd ones: a thread takes an even one and the next, and a quarter warp's 16-byte
     // loads fall in distinct banks (side by side, two to a bank, 1 to 2.5 % of the kernel's time)
     static constexpr int TabB = T + 1, TabC = TabB + 4 * (N == 4096 ? 8 : 16), Tabs = TabC + N / 64;
-    static constexpr size_t Smem =
-        2 * sizeof(double) * Ex + 8 * sizeof(float) * Dot + sizeof(double2) * Tabs + 2 * sizeof(FftRow);
+    static constexpr int Chunks = N == 4096 ? 56 : 96; // 128-window chunks of the longest step
+    static constexpr size_t Smem = 2 * sizeof(double) * Ex + 8 * sizeof(float) * Dot + sizeof(double2) * Tabs +
+                                   2 * sizeof(FftRow) + 2 * sizeof(FftItem) + sizeof(float4) * Chunks;
 };
 static_assert(FftShape<8192>::Smem <= 227 * 1024, "shared memory of k_fft_corr");
 static_assert(2 * (FftShape<4096>::Smem + 1024) <= 228 * 1024, "two blocks of k_fft_corr<4096> per SM");
 static_assert(FftShape<8192>::Tabs + FftShape<4096>::Tabs == kFftAllRoots - kFftRoots, "twiddle tables");
-static_assert(sizeof(FftRow) % 16 == 0 && sizeof(FftRow) / 4 <= 32, "one warp copies a row");
+static_assert(sizeof(FftRow) % 16 == 0 && sizeof(FftRow) / 16 <= 8 && sizeof(FftItem) % 16 == 0, "one warp copies them");
 
 // (a, b) -> (a + w b, a - w b), and with i w in place of w
 __device__ __forceinline__ void bfly(double2 &a, double2 &b, double2 w)
@@ -481,6 +494,57 @@ __device__ __forceinline__ void fold_window(float mu, float iv, float rel_sd, fl
          stats_error(ws, m, qs, s1) + 2.0f * e_dot * iv * 1.01f;
 }
 
+// The terms of ew = k0 + kr |r| + kq (mu / sd)^2 + (ki + s1m kb + km |mu|) / sd, the fast path's
+// statistics, that an item's windows share; kb is of the window's prefix block.
+struct FoldItem
+{
+    float k0, kr, kq, km, ki, s1m, e_dot, shift;
+};
+__device__ __forceinline__ FoldItem fold_item(const FftRow &P, const FftItem &I, int parts)
+{
+    FoldItem f;
+    f.s1m = 2.5f * P.s1_max;
+    f.kr = P.c0.x;
+    f.kq = P.c0.z;
+    f.km = P.c0.w + f.s1m * 1.3e-7f;
+    f.k0 = P.c0.x + P.c0.y + 1.25f * (4.0f * (float)P.m + 2.0f * P.qs) * kFastRelSd;
+    float norm = (float)I.norm[0], moved = 0.0f; // moved: the rounding of the other parts' shift corrections
+    for (int i = 1; i < parts; i++)
+    {
+        norm += (float)I.norm[i];
+        moved += fabsf((float)(I.shift[i] - I.shift[0]));
+    }
+    f.e_dot = fmaf(P.e_norm, norm, (float)(8.1 * kEps64) * P.qs * moved);
+    f.shift = (float)I.shift[0];
+    f.ki = P.c0.w * fabsf(f.shift) + 2.02f * f.e_dot;
+    return f;
+}
+
+// The dot product below which no window of a chunk has d - e <= cut, from the chunk's bounds b
+// at a length m0 <= m: the largest 1 / sd and |mu - shift| / sd of its windows, kb and 1 / m0. For the
+// windows of m samples that begin at the same places the sum of squared deviations is no
+// smaller (it splits into that of the first m0 samples and two terms >= 0), so 1 / sd is at
+// most g = sqrt(m / m0) times larger; and the means differ by at most h sd, h = sqrt((m - m0) /
+// m0): with D between the means of the first m0 and of the other samples, m var >= (m0 (m - m0)
+// / m) D^2, and mu moves by D (m - m0) / m. d - e > cut where d > (cut + ew) / (1 - a3) for every
+// window, and d = c_lin - 2 (dot / sd - s1 (mu - shift) / sd). 1e-5 of c_lin is left for the
+// FP32 rounding of all of this. A NaN or a value <= 0: no dot product is below it.
+__device__ __forceinline__ float sqrt_approx(float x)
+{
+    float y;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float chunk_limit(const FftRow &P, float4 b, float cut, const FoldItem &f)
+{
+    const float q = (float)P.m * b.w;
+    const float g = sqrt_approx(q), h = sqrt_approx(fmaxf(q - 1.0f, 0.0f) + 1e-6f);
+    const float iv = b.x * g, r = fmaf(b.y, g, h), r0 = fmaf(fabsf(f.shift), iv, r);
+    const float ew = f.k0 + f.kr * r + f.kq * r0 * r0 + f.km * r0 + fmaf(f.s1m, b.z, f.ki) * iv;
+    const float cross = 0.5f * (P.c_lin * (1.0f - 2e-5f) - (fmaxf(cut, 0.0f) + ew) * P.inv_a3) - r * fabsf(P.s1);
+    return __fdividef(cross, iv); // below 0, NaN or infinite where no window is searched: any will do
+}
+
 // Statistics by the full bound (two prefix blocks, or ill-conditioned): false when they are
 // not trusted.
 __device__ __forceinline__ bool window_stats_full(const PrefixView &pv, double2 qa, double2 qb, uint64_t g, int m,
@@ -539,6 +603,18 @@ __device__ __forceinline__ void bucket_min(const FftArgs &a, int row, uint32_t b
     }
 }
 
+// A copy from global to shared memory in the background (16, 8 or 4 bytes), and the wait for
+// all of this thread's.
+template <int BYTES> __device__ __forceinline__ void copy_async(void *dst, const void *src)
+{
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    if (BYTES == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(BYTES) : "memory");
+}
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Two adjacent bins of a spectrum (32 bytes), X[k] and its partner X[N - k] (spectrum_slot). A
 // block reads them once per item, so they are not kept in L1 (4 % of the kernel's time).
 __device__ __forceinline__ void load_pair(const double2 *p, double2 &x, double2 &xn)
@@ -552,7 +628,8 @@ __device__ __forceinline__ void load_pair(const double2 *p, double2 &x, double2 
 // length in its slice of a global scratch (L2-resident).
 //
 // Per item: product, packing and pass 1; the eight transforms, whose outputs go to shared
-// memory as floats; the epilogue over the item's windows, 128 per warp at a time. A warp goes
+// memory as floats; the epilogue over the item's windows (those it cannot skip), 128 per warp at a
+// time. A warp goes
 // on to the next item's product while others are in the epilogue.
 template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096 ? 2 : 1) k_fft_corr(const FftArgs a)
 {
@@ -563,19 +640,31 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
     float *dots = reinterpret_cast<float *>(csm + 2 * C::Ex);
     double2 *tab = reinterpret_cast<double2 *>(dots + 8 * C::Dot);
     FftRow *srow = reinterpret_cast<FftRow *>(tab + C::Tabs); // this item's row and the next one's
+    FftItem *sitem = reinterpret_cast<FftItem *>(srow + 2);
+    float4 *bounds = reinterpret_cast<float4 *>(sitem + 2); // of the chunks of 128 windows (chunk_limit)
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const uint64_t total = (uint64_t)a.p_count * (uint32_t)a.nrows;
     const uint64_t item0 = total * blockIdx.x / gridDim.x;
     const uint32_t items = (uint32_t)(total * (blockIdx.x + 1) / gridDim.x - item0);
     uint32_t pi = (uint32_t)(item0 / (uint32_t)a.nrows);
-    int ti = (int)(item0 % (uint32_t)a.nrows), cached_m = -1;
-    auto load_row = [&](int slot, int i) { // by the first threads of warp 0
-        if (t < (int)(sizeof(FftRow) / 4))
-            reinterpret_cast<uint32_t *>(&srow[slot])[t] = reinterpret_cast<const uint32_t *>(a.rows + i)[t];
+    int ti = a.nrows - 1 - (int)(item0 % (uint32_t)a.nrows); // the shortest template first
+    int cached_m = -1, bound_m = -1;                         // lengths of the kept statistics and chunk bounds
+    auto fetch = [&](int slot, int i, uint32_t p) { // by warp 0, in the background
+        const int parts = PARTS ? (int)min((uint32_t)a.parts, a.pieces - p) : 1;
+        if (t < (int)(sizeof(FftRow) / 16))
+            copy_async<16>(reinterpret_cast<char *>(&srow[slot]) + 16 * t, reinterpret_cast<const char *>(a.rows + i) + 16 * t);
+        else if (t == 8 && a.cuts != nullptr)
+            copy_async<4>(&sitem[slot].cut, a.cuts + i);
+        else if (t >= 16 && t < 16 + parts)
+            copy_async<8>(&sitem[slot].shift[t - 16], a.shifts + p + (t - 16));
+        else if (t >= 24 && t < 24 + parts)
+            copy_async<8>(&sitem[slot].norm[t - 24], a.norms + p + (t - 24));
     };
     for (int i = t; i < C::Tabs; i += T)
         tab[i] = a.tabs[i];
-    load_row(0, ti);
+    if (warp == 0 && items > 0)
+        fetch(0, ti, a.p_first + pi);
+    copies_wait();
     __syncthreads();
     float4 *cache = a.stats + (size_t)blockIdx.x * (3 * (L / 4));
     const int g = t / C::GT, s = t % C::GT; // this thread's transform of N / 8 points and its place there
@@ -583,6 +672,7 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
     for (uint32_t item = 0; item < items; item++)
     {
         const FftRow &P = srow[item & 1];
+        const FftItem &I = sitem[item & 1];
         const uint32_t p = a.p_first + pi;
         const int m = P.m, base = (PARTS ? (int)a.step : m) - 1;
         const uint64_t piece_w = (uint64_t)p * a.step;
@@ -591,7 +681,7 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
         double add = 0.0;
         if (PARTS)
             for (int i = 1; i < parts; i++)
-                add = fma(a.shifts[p + i] - a.shifts[p], P.sum[i - 1], add);
+                add = fma(I.shift[i] - I.shift[0], P.sum[i - 1], add);
 
         // ---- product, real-transform packing: C[k] for this thread's bins ----
         double2 A[8], B[8];
@@ -682,7 +772,8 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
             }
         }
         __syncthreads();
-        load_row((item + 1) & 1, ti + 1 < a.nrows ? ti + 1 : 0); // the last item's epilogue is over: its slot is free
+        if (warp == 0 && item + 1 < items) // the last item's epilogue is over: its slot is free
+            fetch((item + 1) & 1, ti > 0 ? ti - 1 : a.nrows - 1, ti > 0 ? p : p + 1);
 
         // ---- transform g: radix 16 (N = 8192) or 8 (N = 4096) with Ns = 1, then 8 and 8 ----
         constexpr int Ns2 = N == 4096 ? 8 : 16, R8 = Q / 8 + Q / 64; // R8: elements Q / 8 apart, padded
@@ -769,6 +860,17 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
                           : make_float4((float)x.x, (float)x.y, (float)y.x, (float)y.y);
             }
         }
+        // ---- may the item skip chunks of its windows? chunk i of this warp where all its dots are below
+        // the limit of lane i (computed while the block gathers) ----
+        constexpr int kWarps = T / 32, MaxChunks = (C::Chunks + kWarps - 1) / kWarps;
+        const int chunks = (int)a.step / 128, per = chunks / kWarps; // a multiple of the warps
+        const bool knn = P.mode == TM_MODE_KNN;
+        const float cut = a.cuts != nullptr ? I.cut : P.thr;
+        const bool skip = bound_m > 0 && bound_m <= m && 10 * m <= 11 * bound_m && cut < inf_f();
+        float limit = -1.0f;
+        if (skip && lane < per)
+            limit = chunk_limit(P, bounds[warp + kWarps * lane], cut, fold_item(P, I, parts));
+        copies_wait();
         __syncthreads();
 
         // ---- epilogue: window o of the piece is output i = o + base; a lane's windows are 128 c +
@@ -776,7 +878,6 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
         // warp's 32 consecutive outputs in distinct banks but for a few. What a chunk needs from
         // global memory is loaded while the one before is evaluated ----
         const int64_t rel = (int64_t)piece_w - (int64_t)a.w0; // window o of the piece is rel + o of the range
-        const bool knn = P.mode == TM_MODE_KNN;
         const float s1 = P.s1, c_lin = P.c_lin, a3 = P.a3, thr = P.thr;
         const int i0 = base + lane;
         const float *dl = dots + ((i0 >> 1) & 7) * C::Dot + 2 * (i0 >> 4) + (i0 & 1);
@@ -829,44 +930,50 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
                 emit_strided(mask, lane, (uint32_t)P.row, (uint32_t)(first + lane), a.cand, a.cand_count, a.cand_cap);
             }
         };
-        constexpr int kWarps = T / 32;
-        const int chunks = (int)a.step / 128; // a multiple of the warps
-        int c = warp;
-        if (m == cached_m)
+        uint32_t todo = (1u << per) - 1u; // this warp's chunks warp + kWarps i
+        if (skip)
+        {
+#pragma unroll
+            for (int i = 0; i < MaxChunks; i++)
+                { // past the last chunk: within shared memory, and no bit of todo
+                    const float *x = dl + 16 * (warp + kWarps * i);
+                    const float most = fmaxf(fmaxf(fmaxf(x[0], x[4]), fmaxf(x[8], x[12])), 0.0f);
+                    const float l = __shfl_sync(0xffffffffu, limit, i);
+                    if (__all_sync(0xffffffffu, most < l))
+                        todo &= ~(1u << i);
+                }
+        }
+        int c = warp + kWarps * (__ffs(todo) - 1);
+        auto next_chunk = [&]() { // after c, or c again at the end
+            todo &= todo - 1;
+            return todo != 0u ? warp + kWarps * (__ffs(todo) - 1) : c;
+        };
+        if (todo == 0u)
+        {
+        }
+        else if (m == cached_m)
         {
             const float4 *cc = cache + lane;
             float4 x = cc[32 * c], y = cc[L / 4 + 32 * c], z = cc[L / 2 + 32 * c];
-            for (; c < chunks; c += kWarps)
+            while (todo != 0u)
             {
                 const float iv[4] = {x.x, x.y, x.z, x.w}, ms[4] = {y.x, y.y, y.z, y.w}, ew[4] = {z.x, z.y, z.z, z.w};
-                const int n = c + kWarps < chunks ? c + kWarps : c;
+                const int n = next_chunk();
                 x = cc[32 * n];
                 y = cc[L / 4 + 32 * n];
                 z = cc[L / 2 + 32 * n];
                 evaluate(c, iv, ms, ew);
+                c = n;
             }
         }
         else
         {
             // the next item's template has the same length and meets the same piece
-            const bool keep = item + 1 < items && ti + 1 < a.nrows && srow[(item + 1) & 1].m == m;
-            const float shift = (float)a.shifts[p];
-            const float fm = (float)m, s1m = 2.5f * P.s1_max;
-            // ew = k0 + kr |r| + kq (mu / sd)^2 + (ki + km |mu|) / sd for the fast path's statistics
-            const float kr = P.c0.x, kq = P.c0.z, km = P.c0.w + s1m * 1.3e-7f;
-            const float k0 = P.c0.x + P.c0.y + 1.25f * (4.0f * fm + 2.0f * P.qs) * kFastRelSd;
-            float e_dot;
-            {
-                const double sm = sqrt((double)m), qn = (double)P.qs / sm; // ||q||_2 (the largest of this length)
-                double e = 0.0;
-                for (int i = 0; i < parts; i++)
-                    e += a.norms[p + i];
-                e *= kFftKappa * qn * (2.0 * sm + sqrt((double)L));
-                for (int i = 1; i < parts; i++) // the rounding of the other parts' shift corrections
-                    e += 8.0 * kEps64 * fabs(a.shifts[p + i] - a.shifts[p]) * qn * sm;
-                e_dot = (float)(e * 1.01);
-            }
-            const float ki = P.c0.w * fabsf(shift) + 2.02f * e_dot;
+            const bool keep = !skip && item + 1 < items && ti > 0 && srow[(item + 1) & 1].m == m;
+            const bool record = !skip && a.prune != 0 && item + 1 < items && ti > 0;
+            const FoldItem F = fold_item(P, I, parts);
+            const float shift = F.shift;
+            const float s1m = F.s1m, k0 = F.k0, kr = F.kr, kq = F.kq, km = F.km;
             // the piece's windows in the template's range; loads for windows outside take the
             // nearest one inside (an empty range takes the piece's first sample, which exists)
             const int64_t left = (int64_t)P.wcount - rel;
@@ -908,9 +1015,9 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
                 }
             };
             uint64_t b0 = ~0ull; // the prefix block whose constants follow
-            float cen = 0.0f, kib = 0.0f, va = 0.0f, vb = 0.0f;
+            float cen = 0.0f, kb = 0.0f, kib = 0.0f, va = 0.0f, vb = 0.0f;
             load(c);
-            for (; c < chunks; c += kWarps)
+            while (todo != 0u)
             {
                 const int f = 128 * c, o = f + lane;
                 // the block of the warp's first window; almost always that of every window's samples too
@@ -923,7 +1030,8 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
                     b0 = b;
                     cen = (float)a.pv.C[b];
                     const BlockBounds bb = block_bounds(a.pv.T[b].y);
-                    kib = ki + s1m * (bb.b * fim + 1.9e-7f * fabsf(cen));
+                    kb = bb.b * fim + 1.9e-7f * fabsf(cen);
+                    kib = F.ki + s1m * kb;
                     va = bb.a * fim * (1.00001f / 0.9e-7f);
                     vb = 2.0f * bb.b * fim * (1.00001f / 0.9e-7f);
                 }
@@ -945,6 +1053,7 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
                     ew[j] = srch ? e : __int_as_float(0x7fc00000);
                     slow |= (srch && (!ok || be != b) ? 1u : 0u) << j;
                 }
+                float iv_max = 0.0f, r_max = 0.0f; // the bounds of the lane's windows with full statistics
                 // two prefix blocks, or ill-conditioned: the full bound, one window at a time
                 for (; slow != 0u; slow &= slow - 1)
                 {
@@ -954,7 +1063,10 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
                     const float v = ok ? st.y : 0.0f;
                     float x = 0.0f, e = inf_f();
                     if (ok)
-                        fold_window(st.x, v, st.z, st.w, P.c0, P.qs, P.s1_max, m, shift, e_dot, x, e);
+                        fold_window(st.x, v, st.z, st.w, P.c0, P.qs, P.s1_max, m, shift, F.e_dot, x, e);
+                    const float v_most = ok && st.z < 0.1f ? v * (1.0f + 2.0f * st.z) : inf_f();
+                    iv_max = fmaxf(iv_max, v_most);
+                    r_max = fmaxf(r_max, (fabsf(x) + st.w) * v_most);
 #pragma unroll
                     for (int j = 0; j < 4; j++)
                         if (j == jj)
@@ -964,7 +1076,25 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
                             ew[j] = e;
                         }
                 }
-                load(c + kWarps < chunks ? c + kWarps : c);
+                if (record)
+                {
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                    {
+                        iv_max = fmaxf(iv_max, iv[j]);
+                        r_max = fmaxf(r_max, fabsf(ms[j] * iv[j]));
+                        // none for a constant run: a longer template's window may leave it
+                        if (rn[j] >= (uint32_t)m && rn[j] != 65535u)
+                            iv_max = inf_f();
+                    }
+                    // as whole numbers: not negative, and a NaN above all
+                    const uint32_t mi = __reduce_max_sync(0xffffffffu, __float_as_uint(iv_max));
+                    const uint32_t mr = __reduce_max_sync(0xffffffffu, __float_as_uint(r_max));
+                    if (lane == 0)
+                        bounds[c] = make_float4(__uint_as_float(mi), __uint_as_float(mr), kb, fim);
+                }
+                const int n = next_chunk();
+                load(n);
                 if (keep)
                 {
                     float4 *cc = cache + 32 * c + lane;
@@ -973,14 +1103,20 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
                     cc[L / 2] = make_float4(ew[0], ew[1], ew[2], ew[3]);
                 }
                 evaluate(c, iv, ms, ew);
+                c = n;
             }
+            __syncwarp(); // the warp's bounds are read by its lanes
         }
-        cached_m = m;
-        if (++ti == a.nrows)
+        if (!skip)
         {
-            ti = 0;
+            cached_m = m;
+            bound_m = a.prune != 0 ? m : -1;
+        }
+        if (--ti < 0)
+        {
+            ti = a.nrows - 1;
             pi++;
-            cached_m = -1; // the cache holds the last piece's statistics
+            cached_m = bound_m = -1; // they hold the last piece's statistics
         }
     }
 }

@@ -295,7 +295,7 @@ void prepare_fft(tm_ctx *ctx, Lane &L, GroupPlan &g)
         r.s1 = p.s1;
         r.c_lin = p.c_lin;
         r.a3 = p.a3;
-        r.thr = p.thr_ed;
+        r.thr = p.mode == TM_MODE_KNN ? HUGE_VALF : p.thr_ed;
         r.c0 = make_float4(p.a1_main, p.a2, p.a5, p.a6);
         r.qs = p.qs;
         r.s1_max = std::fabs(p.s1);
@@ -320,6 +320,11 @@ void prepare_fft(tm_ctx *ctx, Lane &L, GroupPlan &g)
             g.fft_rows[i].qs = g.fft_rows[i - 1].qs;
             g.fft_rows[i].s1_max = g.fft_rows[i - 1].s1_max;
         }
+    for (tmb::FftRow &r : g.fft_rows)
+    {
+        r.e_norm = tmb::fft_e_norm(r.qs, r.m, tmb::fft_class_of(r.m));
+        r.inv_a3 = r.a3 < 0.5f ? (1.0f / (1.0f - r.a3)) * 1.000001f : HUGE_VALF;
+    }
     if (g.fft_rows.empty())
         return;
     const size_t bytes = sizeof(tmb::FftRow) * g.fft_rows.size();
@@ -414,20 +419,30 @@ double tensor_cost_sorted(const tm_ctx *ctx, const int *m, size_t n)
     return best;
 }
 
-// Modelled milliseconds of the FFT branch per template of length m per 2^25 samples; shared: a
-// template of the same length precedes it, whose window statistics it takes. The branch's time
-// depends on the length through the pieces' step alone, and within a class little on it; the
-// factors are the classes' times over that of distinct lengths at 4096 (0.301 ms) or 16000
-// (0.63 ms): 0.244, 0.272, 0.301, 0.424 distinct at 1000, 2000, 4096, 8192; 0.166, 0.166,
-// 0.196, 0.306 shared, and 0.42 shared at 16384.
-double fft_time(const tm_ctx *ctx, int m, bool shared)
+// Modelled milliseconds of the FFT branch per template of length m per 2^25 samples. longer: the
+// next longer template's length in the group, m where a template shares its length (0: none);
+// skips: the template has a cut, so that it can skip windows by a neighbour's bounds
+// (tm_fftk.cu), which reach 10 % in length. The time depends on the length through the pieces'
+// step alone, and within a class little on it; the factors are the classes' times over that of
+// a template that evaluates all its windows at 4096 (0.307 ms) or 16000 (0.63 ms): 0.247, 0.275,
+// 0.307, 0.43 ms at 1000, 2000, 4096, 8192; 0.167, 0.167, 0.200, 0.315 with the statistics of
+// the template before it of the same length, 0.42 at 16384; 0.128, 0.149, 0.167, 0.248 where
+// almost all are skipped, 0.38 at 16000.
+double fft_time(const tm_ctx *ctx, int m, int longer, bool skips)
 {
-    static const double distinct[tmb::kFftClasses] = {0.81, 0.90, 1.0, 1.41};
+    static const double all[tmb::kFftClasses] = {0.81, 0.90, 1.0, 1.41};
     static const double same[tmb::kFftClasses] = {0.55, 0.55, 0.66, 1.04};
+    static const double skip[tmb::kFftClasses] = {0.42, 0.49, 0.55, 0.81};
     const int cls = tmb::fft_class_of(m);
-    if (tmb::fft_parts(m, cls) > 1)
-        return ctx->fft_long_ms * (shared ? 0.69 : 1.0);
-    return ctx->fft_ms * (shared ? same[cls] : distinct[cls]);
+    const bool parts = tmb::fft_parts(m, cls) > 1;
+    const double unit = parts ? ctx->fft_long_ms : ctx->fft_ms, every = unit * (parts ? 1.0 : all[cls]);
+    if (longer < m)
+        return every;
+    if (!skips)
+        return longer == m ? unit * (parts ? 0.69 : same[cls]) : every;
+    // one template in so many, a tenth of the length apart, evaluates all its windows and sets bounds
+    const double sets = std::min(1.0, std::log(static_cast<double>(longer) / m) / std::log(1.1));
+    return sets * every + (1.0 - sets) * unit * (parts ? 0.61 : skip[cls]);
 }
 
 // Device memory that the FFT branch's resident arrays for these lengths would still take
@@ -473,7 +488,11 @@ size_t plan_fft_split(tm_ctx *ctx, const tm_request *reqs, const std::vector<int
     double best = tensor_cost_sorted(ctx, m.data(), n), fft_cost = 0.0;
     for (size_t f = 1; f <= n; f++)
     {
-        fft_cost += fft_time(ctx, m[f - 1], f > 1 && m[f - 2] == m[f - 1]);
+        const tm_request &r = reqs[sorted_idx[f - 1]];
+        const uint32_t pieces = tmb::fft_pieces(ctx->n, tmb::fft_class_of(r.m));
+        const bool skips = r.mode != TM_MODE_KNN ||
+                           fft_stage_end(0, pieces, static_cast<int>(n), tmb::fft_class_of(r.m), ctx->sms) < pieces;
+        fft_cost += fft_time(ctx, r.m, f > 1 ? m[f - 2] : 0, skips);
         const double c = fft_cost + tensor_cost_sorted(ctx, m.data() + f, n - f);
         if (c < best)
         {

@@ -349,6 +349,15 @@ void rescore_and_answer(tm_ctx *ctx, Lane &L, const GroupPlan &g, uint32_t ncand
         L.phase_ms[5] += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
 }
 
+// Does a merge offset of the group exceed a bucket?
+static bool super_buckets(const GroupPlan &g, int blog)
+{
+    for (int t = 0; t < g.T; t++)
+        if (g.mode[t] == TM_MODE_KNN && g.merge[t] > (1 << blog))
+            return true;
+    return false;
+}
+
 // kNN bound, bucket list and FP32 re-pass after a group's contraction (a: its arguments), then
 // the counters: the group's candidates, whether the contraction gave up waiting. One wait for
 // the device; a list that did not fit is made again, larger.
@@ -358,9 +367,7 @@ static uint32_t collect_candidates(tm_ctx *ctx, Lane &L, const GroupPlan &g, con
     uint32_t *hc = L.h_counters.as<uint32_t>(), *counters = L.counters.as<uint32_t>();
     if (g.nk > 0)
     {
-        bool super = false;
-        for (int t = 0; t < g.T; t++)
-            super = super || (g.mode[t] == TM_MODE_KNN && g.merge[t] > (1 << a.bucket_log));
+        const bool super = super_buckets(g, a.bucket_log);
         if (super)
             L.bmin_s.reserve(sizeof(uint32_t) * static_cast<size_t>(g.nk) * a.nb);
         TM_CUDA(tmb::launch_bucket_select(a.bmin_u, L.bmin_s.as<uint32_t>(), a.nb, a.bucket_log, a.tp, g.slots.as<int>(), g.nk,
@@ -557,6 +564,21 @@ static tm_ctx::FftPieces &ensure_fft(tm_ctx *ctx, Lane &L, int cls)
 // block reads them once per piece.
 constexpr size_t kFftLaunchBins = 192 * 8200;
 
+// Where a launch of kNN templates over the pieces from p0 on ends. A bound from the minima of the
+// first sixteenth of the pieces, then of the first quarter, lets the rest skip almost all of
+// its windows (tm_fftk.cu); where a launch would have fewer than four items per block, the
+// bound would come too late or too dear, and there is one launch.
+uint32_t fft_stage_end(uint32_t p0, uint32_t pieces, int rows, int cls, int sms)
+{
+    const uint64_t blocks = static_cast<uint64_t>(sms) * (tmb::fft_class(cls).n == 4096 ? 2 : 1);
+    const uint64_t least = (4 * blocks + static_cast<uint64_t>(rows) - 1) / static_cast<uint64_t>(rows);
+    const uint64_t first = std::max<uint64_t>((pieces + 15) / 16, least);
+    for (uint64_t end = first; 2 * end <= pieces; end *= 4)
+        if (end > p0)
+            return static_cast<uint32_t>(end);
+    return pieces;
+}
+
 // The FFT branch of a group: per set of rows (prepare_fft), their spectra, then persistent
 // launches over the pieces their windows touch.
 void fft_contract(tm_ctx *ctx, Lane &L, const GroupPlan &g, const tmb::ScanArgs &a)
@@ -580,16 +602,19 @@ void fft_contract(tm_ctx *ctx, Lane &L, const GroupPlan &g, const tmb::ScanArgs 
             TM_CUDA(tmb::launch_fft_templates(g.q.as<float>(), g.tp.as<TemplParam>(), f.rows, nr, set.cls, set.parts,
                                               ctx->fft_roots.as<double2>(), L.fft_Y.as<double2>(), s));
             uint64_t wmax = 0;
+            int knn = 0;
             for (int i = 0; i < nr; i++)
-                wmax = std::max<uint64_t>(wmax, g.fft_rows[static_cast<size_t>(first + i)].wcount);
+            {
+                const tmb::FftRow &r = g.fft_rows[static_cast<size_t>(first + i)];
+                wmax = std::max<uint64_t>(wmax, r.wcount);
+                knn += r.mode == TM_MODE_KNN ? 1 : 0;
+            }
             const uint32_t pa = static_cast<uint32_t>(a.w0 / step);
             const uint32_t pb = std::min<uint32_t>(static_cast<uint32_t>((a.w0 + wmax - 1) / step), X.count - 1);
             f.X = X.X.as<double2>();
             f.shifts = X.shift.as<double>();
             f.norms = X.norm.as<double>();
             f.pieces = X.count;
-            f.p_first = pa;
-            f.p_count = pb >= pa ? pb - pa + 1 : 0;
             f.Y = L.fft_Y.as<double2>();
             f.w0 = a.w0;
             f.W = a.W;
@@ -607,8 +632,31 @@ void fft_contract(tm_ctx *ctx, Lane &L, const GroupPlan &g, const tmb::ScanArgs 
             f.dbg_d = a.dbg_d;
             f.dbg_e = a.dbg_e;
             f.stats = L.fft_stats.as<float4>();
-            TM_CUDA(tmb::launch_fft_corr(f, set.cls, ctx->fft_roots.as<double2>(), ctx->sms, s));
-            count_launch(L, 2);
+            count_launch(L);
+            const uint32_t pieces = pb >= pa ? pb - pa + 1 : 0;
+            for (uint32_t p0 = 0; p0 < pieces;)
+            {
+                const uint32_t p1 = knn > 0 ? fft_stage_end(p0, pieces, nr, set.cls, ctx->sms) : pieces;
+                f.p_first = pa + p0;
+                f.p_count = p1 - p0;
+                f.prune = a.dbg_d == nullptr && nr > 1 && (knn < nr || p0 > 0) ? 1 : 0;
+                TM_CUDA(tmb::launch_fft_corr(f, set.cls, ctx->fft_roots.as<double2>(), ctx->sms, s));
+                count_launch(L);
+                p0 = p1;
+                if (p0 == pieces)
+                    break;
+                const uint64_t seen = static_cast<uint64_t>(pa + p0) * step - a.w0; // windows
+                const uint32_t nb_seen =
+                    static_cast<uint32_t>(std::min<uint64_t>(a.nb, (seen + (1ull << a.bucket_log) - 1) >> a.bucket_log));
+                const bool super = super_buckets(g, a.bucket_log);
+                if (super)
+                    L.bmin_s.reserve(sizeof(uint32_t) * static_cast<size_t>(g.nk) * a.nb);
+                L.fft_cuts.reserve(sizeof(float) * static_cast<size_t>(nr));
+                TM_CUDA(tmb::launch_fft_cuts(f.rows, nr, a.bmin_u, L.bmin_s.as<uint32_t>(), a.nb, nb_seen, a.bucket_log, a.tp,
+                                             g.slots.as<int>(), g.nk, super, L.fft_cuts.as<float>(), s));
+                count_launch(L, super ? 2 : 1);
+                f.cuts = L.fft_cuts.as<float>();
+            }
         }
     }
 }

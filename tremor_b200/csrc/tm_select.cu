@@ -17,8 +17,10 @@
 // pick before it has k answers.
 #include <algorithm>
 
+#include "../../include/tremor_b200.h"
 #include "tm_epilogue.cuh"
 #include "tm_exact.cuh"
+#include "tm_fft.cuh"
 #include "tm_internal.cuh"
 #include "tm_prefix.cuh"
 
@@ -101,42 +103,76 @@ __device__ uint32_t block_select(const uint32_t *__restrict__ keys, uint32_t cou
     return prefix;
 }
 
-// Minima over super-buckets of ceil(merge / bucket) buckets, for the templates whose merge
-// offset exceeds a bucket: sup[slot][i], i < ceil(nb / buckets per super-bucket).
-__global__ void k_super_buckets(const uint32_t *__restrict__ bmin_u, uint32_t nb, int blog, const TemplParam *__restrict__ tp,
-                                const int *__restrict__ knn_slots, uint32_t *__restrict__ sup)
+// Template of a selection's block i: that of a kNN slot, or of a row of the FFT branch.
+__device__ __forceinline__ int select_template(const int *slots, const FftRow *rows, int i)
 {
-    const int t = knn_slots[blockIdx.y], merge = tp[t].merge;
+    return rows != nullptr ? rows[i].row : slots[i];
+}
+// Its place in the scratch of super-buckets.
+__device__ __forceinline__ int select_slot(const int *slots, int nk, const FftRow *rows, int i)
+{
+    if (rows == nullptr)
+        return i;
+    int lo = 0, hi = nk - 1; // the slots' templates ascend
+    while (lo < hi)
+    {
+        const int mid = (lo + hi) / 2;
+        if (slots[mid] < rows[i].row)
+            lo = mid + 1;
+        else
+            hi = mid;
+    }
+    return lo;
+}
+
+// Minima over super-buckets of ceil(merge / bucket) buckets, for the templates whose merge
+// offset exceeds a bucket: sup[slot][i], i < ceil(nb_seen / buckets per super-bucket); nb buckets
+// per template, of which the first nb_seen are looked at.
+__global__ void k_super_buckets(const uint32_t *__restrict__ bmin_u, uint32_t nb, uint32_t nb_seen, int blog,
+                                const TemplParam *__restrict__ tp, const int *__restrict__ knn_slots, int nk,
+                                const FftRow *__restrict__ rows, uint32_t *__restrict__ sup)
+{
+    const int t = select_template(knn_slots, rows, blockIdx.y), merge = tp[t].merge;
     const uint32_t sb = (uint32_t)(((int64_t)merge + (1 << blog) - 1) >> blog);
-    if (sb < 2)
+    if (sb < 2 || tp[t].mode != TM_MODE_KNN)
         return;
     const uint32_t *u = bmin_u + (size_t)t * nb;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < (nb + sb - 1) / sb; i += gridDim.x * blockDim.x)
+    sup += (size_t)select_slot(knn_slots, nk, rows, blockIdx.y) * nb_seen;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < (nb_seen + sb - 1) / sb; i += gridDim.x * blockDim.x)
     {
         uint32_t best = kEmptyKey;
-        for (uint32_t b = i * sb; b < min((i + 1) * sb, nb); b++)
+        for (uint32_t b = i * sb; b < min((i + 1) * sb, nb_seen); b++)
             best = min(best, u[b]);
-        sup[(size_t)blockIdx.y * nb + i] = best;
+        sup[i] = best;
     }
 }
 
-// One block per kNN template slot: tkey[t] = key of the bound T (kEmptyKey: +inf).
+// One block per kNN template slot: tkey[t] = key of the bound T (kEmptyKey: +inf). With rows, one
+// per row of the FFT branch: cuts[row] = its threshold, or the bound from the buckets seen.
 __global__ void __launch_bounds__(1024) k_bucket_select(const uint32_t *__restrict__ bmin_u, const uint32_t *__restrict__ sup,
-                                                        uint32_t nb, int blog, const TemplParam *__restrict__ tp,
-                                                        const int *__restrict__ knn_slots, uint32_t *__restrict__ tkey)
+                                                        uint32_t nb, uint32_t nb_seen, int blog,
+                                                        const TemplParam *__restrict__ tp, const int *__restrict__ knn_slots,
+                                                        int nk, const FftRow *__restrict__ rows, uint32_t *__restrict__ tkey,
+                                                        float *__restrict__ cuts)
 {
-    const int t = knn_slots[blockIdx.x];
+    const int t = select_template(knn_slots, rows, blockIdx.x);
+    if (rows != nullptr && tp[t].mode != TM_MODE_KNN)
+    {
+        if (threadIdx.x == 0)
+            cuts[blockIdx.x] = rows[blockIdx.x].thr;
+        return;
+    }
     const int k = tp[t].k, merge = tp[t].merge;
     const uint32_t *u = bmin_u + (size_t)t * nb;
     uint32_t result;
     if (merge <= 0)
-        result = block_select(u, nb, 1, (uint32_t)k);
+        result = block_select(u, nb_seen, 1, (uint32_t)k);
     else
     {
         const uint32_t sb = (uint32_t)(((int64_t)merge + (1 << blog) - 1) >> blog); // buckets per super-bucket
-        const uint32_t nsb = (nb + sb - 1) / sb;
+        const uint32_t nsb = (nb_seen + sb - 1) / sb;
         if (sb > 1)
-            u = sup + (size_t)blockIdx.x * nb;
+            u = sup + (size_t)select_slot(knn_slots, nk, rows, blockIdx.x) * nb_seen;
         result = kEmptyKey;
         for (uint32_t parity = 0; parity < 2; parity++)
         {
@@ -145,7 +181,12 @@ __global__ void __launch_bounds__(1024) k_bucket_select(const uint32_t *__restri
         }
     }
     if (threadIdx.x == 0)
-        tkey[t] = result;
+    {
+        if (rows != nullptr)
+            cuts[blockIdx.x] = result == kEmptyKey ? inf_f() : key_float(result);
+        else
+            tkey[t] = result;
+    }
 }
 
 // (template slot, bucket) pairs whose minimum of d - E is within the bound. counters: [0]
@@ -542,9 +583,23 @@ __global__ void __launch_bounds__(S_WARPS * 32) k_rescore_serial(const Candidate
 cudaError_t launch_bucket_select(const uint32_t *bmin_u, uint32_t *sup, uint32_t nb, int blog, const TemplParam *tp,
                                  const int *knn_slots, int nk, bool super, uint32_t *tkey, cudaStream_t s)
 {
+    const FftRow *rows = nullptr;
+    float *cuts = nullptr;
     if (super)
-        k_super_buckets<<<dim3(std::min(nb / 256 + 1, 64u), (unsigned)nk), 256, 0, s>>>(bmin_u, nb, blog, tp, knn_slots, sup);
-    k_bucket_select<<<nk, 1024, 0, s>>>(bmin_u, sup, nb, blog, tp, knn_slots, tkey);
+        k_super_buckets<<<dim3(std::min(nb / 256 + 1, 64u), (unsigned)nk), 256, 0, s>>>(bmin_u, nb, nb, blog, tp, knn_slots, nk,
+                                                                                        rows, sup);
+    k_bucket_select<<<nk, 1024, 0, s>>>(bmin_u, sup, nb, nb, blog, tp, knn_slots, nk, rows, tkey, cuts);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_fft_cuts(const FftRow *rows, int nrows, const uint32_t *bmin_u, uint32_t *sup, uint32_t nb, uint32_t nb_seen,
+                            int blog, const TemplParam *tp, const int *slots, int nk, bool super, float *cuts, cudaStream_t s)
+{
+    uint32_t *tkey = nullptr;
+    if (super)
+        k_super_buckets<<<dim3(std::min(nb_seen / 256 + 1, 64u), (unsigned)nrows), 256, 0, s>>>(bmin_u, nb, nb_seen, blog, tp,
+                                                                                                slots, nk, rows, sup);
+    k_bucket_select<<<nrows, 1024, 0, s>>>(bmin_u, sup, nb, nb_seen, blog, tp, slots, nk, rows, tkey, cuts);
     return cudaGetLastError();
 }
 
