@@ -55,7 +55,7 @@ def build(verbose: bool = False, ptxas_info: bool = False) -> Path:
         jobs.append([nvcc, *NVCC_FLAGS, *extra, '-c', str(CSRC / src), '-o', str(OUT / (src + '.o'))])
     for src in CPP_SOURCES:
         # the image exports CXX pointing at a toolchain without libgomp; use the system g++
-        jobs.append(['g++', '-O2', '-std=c++17', '-fPIC', '-ffp-contract=off', '-Wall', '-c', str(CSRC / src),
+        jobs.append(['g++', '-O3', '-std=c++17', '-fPIC', '-ffp-contract=off', '-Wall', '-c', str(CSRC / src),
                      '-o', str(OUT / (src + '.o'))])
     with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 2)) as ex:
         logs = list(ex.map(lambda c: _run(c, verbose), jobs))

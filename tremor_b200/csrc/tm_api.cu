@@ -25,7 +25,7 @@ static void bound_diagnostics_wm(tm_ctx *ctx, int m, const std::vector<int> &idx
     ensure_prefix(ctx, L);
     GroupPlan g;
     uint64_t h2d = 0;
-    prepare_group_mixed(ctx, L, idx, reqs.data(), g, h2d, plan_col_tile(ctx, reqs.data(), idx));
+    prepare_group_mixed(ctx, L, idx, reqs.data(), g, h2d, plan_col_tile(ctx, reqs.data(), idx), false);
     const uint64_t W = g.w_max;
     if (W == 0 || W * static_cast<uint64_t>(count) > (1ull << 31))
         throw Failure{TM_ERR_ARGUMENT, "diagnostics need 0 < windows x templates <= 2^31"};

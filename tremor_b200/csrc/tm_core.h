@@ -469,7 +469,7 @@ int validate_requests(const tm_ctx *ctx, const tm_request *reqs, int count);
 void prepare_group(tm_ctx *ctx, Lane &L, int m, const std::vector<int> &idx, const tm_request *reqs, GroupPlan &g,
                    uint64_t &h2d, int col_tile = 0);
 void prepare_group_mixed(tm_ctx *ctx, Lane &L, const std::vector<int> &idx_in, const tm_request *reqs, GroupPlan &g,
-                         uint64_t &h2d, int col_tile = 0);
+                         uint64_t &h2d, int col_tile, bool fft);
 void prepare_fft(tm_ctx *ctx, Lane &L, GroupPlan &g);
 int plan_col_tile(const tm_ctx *ctx, const tm_request *reqs, const std::vector<int> &idx, double *cost = nullptr);
 double tile_time(const tm_ctx *ctx, bool mixed, int v, double k);

@@ -136,13 +136,16 @@ void prepare_group(tm_ctx *ctx, Lane &L, int m, const std::vector<int> &idx, con
 // in tiles of 128 rows (col_tile 0, k_scan_umma) or col_tile rows (k_scan_wm), any
 // lengths. Padding rows are inert; a tile's K extent is its longest template (shorter rows are
 // zero-padded, which leaves their dot products unchanged). Rows are the template slots of
-// the group: g.index[row] is the request (-1 for padding rows).
+// the group: g.index[row] is the request (-1 for padding rows). A group for the FFT branch
+// (fft; prepare_fft completes it and waits for the copies) has no tiles: one row per template,
+// as long as that needs, and no BF16 halves. Padded like the tiles, 8 templates of 16384 samples
+// took 16 MB of copies and 128 rows of bucket minima.
 void prepare_group_mixed(tm_ctx *ctx, Lane &L, const std::vector<int> &idx_in, const tm_request *reqs, GroupPlan &g,
-                         uint64_t &h2d, int col_tile)
+                         uint64_t &h2d, int col_tile, bool fft)
 {
     std::vector<int> idx = idx_in;
     std::stable_sort(idx.begin(), idx.end(), [&](int a, int b) { return reqs[a].m > reqs[b].m; });
-    const size_t tile_rows = col_tile > 0 ? static_cast<size_t>(col_tile) : 128;
+    const size_t tile_rows = fft ? 1 : col_tile > 0 ? static_cast<size_t>(col_tile) : 128;
     // rows: request per row (-1 = padding)
     std::vector<int> rows;
     std::vector<tmb::TileInfo> tiles;
@@ -172,19 +175,32 @@ void prepare_group_mixed(tm_ctx *ctx, Lane &L, const std::vector<int> &idx_in, c
     g.nblk = std::max(1, g.k_stride / tm_host::kZnormBlock);
     g.umma_constants = true;
     g.index = rows;
-    const int stride = g.k_stride, nblk = g.nblk;
-    const size_t elems = static_cast<size_t>(R) * stride;
+    const int stride = g.k_stride;
+    // where each row's samples and block order begin
+    std::vector<size_t> q_at(static_cast<size_t>(R) + 1, 0), o_at(static_cast<size_t>(R) + 1, 0);
+    for (int t = 0; t < R; t++)
+    {
+        const int len = fft ? (reqs[rows[t]].m + 63) & ~63 : stride;
+        q_at[t + 1] = q_at[t] + static_cast<size_t>(len);
+        o_at[t + 1] = o_at[t] + static_cast<size_t>(std::max(1, len / tm_host::kZnormBlock));
+    }
+    const size_t elems = q_at[R], orders = o_at[R];
     L.h_q.reserve(sizeof(float) * elems);
-    L.h_order.reserve(sizeof(int) * static_cast<size_t>(R) * nblk);
+    L.h_order.reserve(sizeof(int) * orders);
     L.h_slots.reserve(sizeof(int) * R);
-    L.h_split.reserve(2 * sizeof(uint16_t) * elems);
     float *hq = L.h_q.as<float>();
     int *ho = L.h_order.as<int>();
     int *hslots = L.h_slots.as<int>();
-    uint16_t *hh = L.h_split.as<uint16_t>(), *hl = hh + elems;
+    uint16_t *hh = nullptr, *hl = nullptr;
     std::memset(hq, 0, sizeof(float) * elems);
-    std::memset(ho, 0, sizeof(int) * static_cast<size_t>(R) * nblk);
-    std::memset(hh, 0, 2 * sizeof(uint16_t) * elems);
+    std::memset(ho, 0, sizeof(int) * orders);
+    if (!fft)
+    {
+        L.h_split.reserve(2 * sizeof(uint16_t) * elems);
+        hh = L.h_split.as<uint16_t>();
+        hl = hh + elems;
+        std::memset(hh, 0, 2 * sizeof(uint16_t) * elems);
+    }
     g.htp.assign(R, TemplParam{});
     g.mode.assign(R, TM_MODE_THRESHOLD);
     g.k.assign(R, 0);
@@ -214,17 +230,20 @@ void prepare_group_mixed(tm_ctx *ctx, Lane &L, const std::vector<int> &idx_in, c
         const tm_request *r = &reqs[rows[t]];
         const int m = r->m;
         samples += static_cast<uint64_t>(m);
-        float *q = hq + static_cast<size_t>(t) * stride;
+        float *q = hq + q_at[t];
         std::memcpy(q, r->templ, sizeof(float) * m);
         if (!(r->flags & TM_FLAG_ZNORMALIZED))
             tm_host::znormalize(q, m);
-        tm_host::block_order(q, m, ho + static_cast<size_t>(t) * nblk);
+        tm_host::block_order(q, m, ho + o_at[t]);
         double q2 = 0.0, s1 = 0.0;
         for (int i = 0; i < m; i++)
         {
             q2 += static_cast<double>(q[i]) * q[i];
             s1 += q[i];
-            const size_t at = static_cast<size_t>(t) * stride + i;
+        }
+        for (int i = 0; i < m && !fft; i++)
+        {
+            const size_t at = q_at[t] + static_cast<size_t>(i);
             hh[at] = bf16_bits(q[i]);
             hl[at] = bf16_bits(q[i] - bf16_value(hh[at]));
         }
@@ -237,8 +256,8 @@ void prepare_group_mixed(tm_ctx *ctx, Lane &L, const std::vector<int> &idx_in, c
         p.mode = g.mode[t] = r->mode;
         p.k = g.k[t] = r->k;
         p.merge = g.merge[t] = r->merge_offset;
-        p.q_offset = static_cast<int64_t>(t) * stride;
-        p.order_offset = static_cast<int64_t>(t) * nblk;
+        p.q_offset = static_cast<int64_t>(q_at[t]);
+        p.order_offset = static_cast<int64_t>(o_at[t]);
         if (r->mode == TM_MODE_KNN)
             hslots[g.nk++] = t;
         else
@@ -247,24 +266,26 @@ void prepare_group_mixed(tm_ctx *ctx, Lane &L, const std::vector<int> &idx_in, c
     g.tiles = tiles;
     cudaStream_t s = L.stream;
     g.q.reserve_on(sizeof(float) * elems, s, ctx->pool);
-    g.order.reserve_on(sizeof(int) * static_cast<size_t>(R) * nblk, s, ctx->pool);
+    g.order.reserve_on(sizeof(int) * orders, s, ctx->pool);
     g.tp.reserve_on(sizeof(TemplParam) * R, s, ctx->pool);
     g.slots.reserve_on(sizeof(int) * std::max(g.nk, 1), s, ctx->pool);
-    g.q_hi.reserve_on(sizeof(uint16_t) * elems, s, ctx->pool);
-    g.q_lo.reserve_on(sizeof(uint16_t) * elems, s, ctx->pool);
-    g.d_tiles.reserve_on(sizeof(tmb::TileInfo) * tiles.size(), s, ctx->pool);
     TM_CUDA(cudaMemcpyAsync(g.q.p, hq, sizeof(float) * elems, cudaMemcpyHostToDevice, s));
-    TM_CUDA(cudaMemcpyAsync(g.order.p, ho, sizeof(int) * static_cast<size_t>(R) * nblk, cudaMemcpyHostToDevice, s));
+    TM_CUDA(cudaMemcpyAsync(g.order.p, ho, sizeof(int) * orders, cudaMemcpyHostToDevice, s));
     TM_CUDA(cudaMemcpyAsync(g.tp.p, g.htp.data(), sizeof(TemplParam) * R, cudaMemcpyHostToDevice, s));
     if (g.nk > 0)
         TM_CUDA(cudaMemcpyAsync(g.slots.p, hslots, sizeof(int) * g.nk, cudaMemcpyHostToDevice, s));
+    h2d += samples * sizeof(float) + sizeof(int) * orders + sizeof(TemplParam) * R;
+    if (fft)
+        return;
+    g.q_hi.reserve_on(sizeof(uint16_t) * elems, s, ctx->pool);
+    g.q_lo.reserve_on(sizeof(uint16_t) * elems, s, ctx->pool);
+    g.d_tiles.reserve_on(sizeof(tmb::TileInfo) * tiles.size(), s, ctx->pool);
     TM_CUDA(cudaMemcpyAsync(g.q_hi.p, hh, sizeof(uint16_t) * elems, cudaMemcpyHostToDevice, s));
     TM_CUDA(cudaMemcpyAsync(g.q_lo.p, hl, sizeof(uint16_t) * elems, cudaMemcpyHostToDevice, s));
     TM_CUDA(cudaMemcpyAsync(g.d_tiles.p, g.tiles.data(), sizeof(tmb::TileInfo) * tiles.size(), cudaMemcpyHostToDevice,
                             s));
     TM_CUDA(cudaStreamSynchronize(s));
-    h2d += samples * (sizeof(float) + 2 * sizeof(uint16_t)) + sizeof(int) * static_cast<uint64_t>(R) * nblk +
-           sizeof(TemplParam) * R + sizeof(tmb::TileInfo) * tiles.size();
+    h2d += samples * 2 * sizeof(uint16_t) + sizeof(tmb::TileInfo) * tiles.size();
 }
 
 // Makes a prepared mixed-length group one of the FFT branch: its rows with windows, sorted by
@@ -325,11 +346,12 @@ void prepare_fft(tm_ctx *ctx, Lane &L, GroupPlan &g)
         r.e_norm = tmb::fft_e_norm(r.qs, r.m, tmb::fft_class_of(r.m));
         r.inv_a3 = r.a3 < 0.5f ? (1.0f / (1.0f - r.a3)) * 1.000001f : HUGE_VALF;
     }
-    if (g.fft_rows.empty())
-        return;
-    const size_t bytes = sizeof(tmb::FftRow) * g.fft_rows.size();
-    g.d_fft.reserve_on(bytes, L.stream, ctx->pool);
-    TM_CUDA(cudaMemcpyAsync(g.d_fft.p, g.fft_rows.data(), bytes, cudaMemcpyHostToDevice, L.stream));
+    if (!g.fft_rows.empty())
+    {
+        const size_t bytes = sizeof(tmb::FftRow) * g.fft_rows.size();
+        g.d_fft.reserve_on(bytes, L.stream, ctx->pool);
+        TM_CUDA(cudaMemcpyAsync(g.d_fft.p, g.fft_rows.data(), bytes, cudaMemcpyHostToDevice, L.stream));
+    }
     TM_CUDA(cudaStreamSynchronize(L.stream));
 }
 
@@ -573,14 +595,14 @@ void create_batch(tm_ctx *ctx, Lane &L, const tm_request *requests, int count, t
         const int m = requests[idx.front()].m;
         if (specs[gi].kind == 2)
         {
-            prepare_group_mixed(ctx, L, idx, requests, g, b.h2d_bytes, 0);
+            prepare_group_mixed(ctx, L, idx, requests, g, b.h2d_bytes, 0, true);
             prepare_fft(ctx, L, g);
         }
         else if (specs[gi].kind == 0)
             prepare_group(ctx, L, m, idx, requests, g, b.h2d_bytes,
                           tensor && m <= 16384 ? plan_col_tile(ctx, requests, idx) : 0);
         else
-            prepare_group_mixed(ctx, L, idx, requests, g, b.h2d_bytes, plan_col_tile(ctx, requests, idx));
+            prepare_group_mixed(ctx, L, idx, requests, g, b.h2d_bytes, plan_col_tile(ctx, requests, idx), false);
     }
 }
 
