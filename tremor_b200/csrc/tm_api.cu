@@ -650,7 +650,7 @@ int tm_bound_diagnostics(tm_ctx *ctx, const float *queries, int count, int m, fl
             a.qt = ctx->main.fp32_qt.as<float>();
             count_launch(ctx->main); // the template-tile transposition
         }
-        TM_CUDA(use_umma ? tmb::launch_scan_umma(a, s) : tmb::launch_scan_fp32(a, s));
+        TM_CUDA(use_umma ? tmb::launch_scan_umma(a, s) : tmb::launch_scan_fp32(a, ctx->sms, s));
         count_launch(ctx->main);
         TM_CUDA(cudaMemcpyAsync(d, dd.p, pairs * sizeof(float), cudaMemcpyDeviceToHost, s));
         TM_CUDA(cudaMemcpyAsync(e, de.p, pairs * sizeof(float), cudaMemcpyDeviceToHost, s));

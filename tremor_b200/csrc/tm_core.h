@@ -40,7 +40,7 @@ cudaError_t launch_window_stats(const float *clean, const float *raw, uint64_t n
                                 double2 *suf, float *mean, float *inv, uint8_t *flags, cudaStream_t s);
 cudaError_t launch_reference_stats(const float *raw, int m, uint64_t w0, uint64_t count, float *mean, float *stddev,
                                    cudaStream_t s);
-cudaError_t launch_scan_fp32(const ScanArgs &a, cudaStream_t s);
+cudaError_t launch_scan_fp32(const ScanArgs &a, int sms, cudaStream_t s);
 cudaError_t launch_scan_umma(const ScanArgs &a, cudaStream_t s);
 cudaError_t launch_scan_wm(const ScanArgs &a, cudaStream_t s);
 bool umma_supported(int m, int T, uint64_t W);

@@ -12,8 +12,11 @@
 // threshold distance; kNN requests record per 2048-window bucket the smallest d + E
 // and d - E, from which the kNN bound is selected afterwards (tm_select.cu).
 //
-// Tile: 256 windows x 64 templates per CTA, 8 warps; a warp owns 8 templates and a
-// lane 8 consecutive windows (64 FP32 accumulators). K advances in stages of 64
+// Tile: 8 warps per CTA; a warp owns 8 templates and 256 windows, a lane 8 consecutive
+// windows (64 FP32 accumulators). WT warps stand side by side along the templates and 8 / WT along
+// the windows: 64 templates x 256 windows for the full tiles, and 32 x 512, 16 x 1024 or 8 x 2048
+// for what remains of the group, whose padding would cost as much as templates do (70
+// templates, 217 GFLOP: 7.2 ms with 128 rows, 4.3 with 72). K advances in stages of 64
 // samples, three buffers deep with cp.async (one barrier per stage), the tile's shift
 // subtracted as the samples are read into registers. The stage's waveform slice is stored with 4
 // floats of padding after every 32 (xpos), so that the float4 loads of a quarter warp
@@ -24,15 +27,17 @@
 
 namespace tmb {
 
-constexpr int F_WIN = 256, F_TPL = 64, F_THREADS = 256;
+constexpr int F_TPL = 64, F_THREADS = 256;
 // per stage of K samples (64, or 128 when the padded length allows: half the barriers):
-// the waveform slice (F_XS floats, stored with their padding) and the templates' slices
-template <int K> struct FStage
+// the waveform slice (XS floats, stored with their padding) and the templates' slices
+template <int K, int WT> struct FStage
 {
-    static constexpr int XS = F_WIN + K + 16;
+    static constexpr int TPL = 8 * WT, WIN = 256 * (8 / WT); // templates and windows of a tile
+    static constexpr int XS = WIN + K + 16;
     static constexpr int XS_PAD = XS + ((XS + 31) >> 5) * 4;
 };
 
+static_assert(FStage<128, 1>::WIN + 16 + 63 <= kStagePad, "the last tile's samples");
 __device__ __forceinline__ int xpos(int i) { return i + ((i >> 5) << 2); }
 
 __device__ __forceinline__ void cp_async4(void *smem, const void *gmem)
@@ -68,35 +73,38 @@ template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.as
 // that stage st - 1 used, so one barrier per stage both publishes stage st and retires
 // stage st - 1.
 constexpr int F_BUFS = 3;
-template <int K> constexpr size_t f_smem()
+template <int K, int WT> constexpr size_t f_smem()
 {
-    return sizeof(float) * (size_t)F_BUFS * (FStage<K>::XS_PAD + F_TPL * K);
+    return sizeof(float) * (size_t)F_BUFS * (FStage<K, WT>::XS_PAD + FStage<K, WT>::TPL * K);
 }
 
-template <int F_K>
-__global__ void __launch_bounds__(F_THREADS, 2) k_scan_fp32(ScanArgs a)
+// t0: the first template of the grid's tiles, a multiple of 64.
+template <int F_K, int WT>
+__global__ void __launch_bounds__(F_THREADS, 2) k_scan_fp32(ScanArgs a, int t0)
 {
-    constexpr int F_XS = FStage<F_K>::XS, F_XS_PAD = FStage<F_K>::XS_PAD;
+    constexpr int F_XS = FStage<F_K, WT>::XS, F_XS_PAD = FStage<F_K, WT>::XS_PAD;
+    constexpr int TPL = FStage<F_K, WT>::TPL, WIN = FStage<F_K, WT>::WIN;
     extern __shared__ __align__(16) float fsm[];
     float(*xs)[F_XS_PAD] = reinterpret_cast<float(*)[F_XS_PAD]>(fsm);
-    float(*qs)[F_K][F_TPL] = reinterpret_cast<float(*)[F_K][F_TPL]>(fsm + F_BUFS * F_XS_PAD);
-    __shared__ TemplParam tps[F_TPL];
+    float(*qs)[F_K][TPL] = reinterpret_cast<float(*)[F_K][TPL]>(fsm + F_BUFS * F_XS_PAD);
+    __shared__ TemplParam tps[TPL];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t tile_j = blockIdx.x * F_WIN;
-    const int tile_t = blockIdx.y * F_TPL;
-    if (tid < F_TPL)
+    const int wt = warp % WT;
+    const uint32_t tile_j = blockIdx.x * WIN, warp_j = tile_j + 256 * (warp / WT);
+    const int tile_t = t0 + blockIdx.y * TPL;
+    const bool active = warp_j < a.W && tile_t + 8 * wt < a.T; // this warp has windows and templates
+    if (tid < TPL)
         tps[tid] = a.tp[tile_t + tid];
-    const uint32_t jmid = min(tile_j + F_WIN / 2, a.W - 1);
-    const float shift = a.mean[jmid];
-    const float *xg = a.x + a.w0 + tile_j;
-    const float *qg = a.qt + (size_t)tile_t * a.m_pad; // the tile's templates, [k][64]
+    const float shift = a.mean[min(warp_j + 128, a.W - 1)]; // of the warp's windows
+    const float *xg = a.x + a.w0 + tile_j; // read up to the padding of the record
+    const float *qg = a.qt + (size_t)(tile_t / F_TPL) * F_TPL * a.m_pad + tile_t % F_TPL; // [k][64] per 64 templates
 
     auto load_stage = [&](int buf, int k0) {
         for (int i = tid; i < F_XS; i += F_THREADS)
             cp_async4(&xs[buf][xpos(i)], xg + k0 + i);
-        for (int i = tid; i < F_TPL * F_K / 4; i += F_THREADS)
-            cp_async16(&qs[buf][0][0] + i * 4, qg + (size_t)k0 * F_TPL + i * 4);
+        for (int i = tid; i < TPL * F_K / 4; i += F_THREADS)
+            cp_async16(&qs[buf][0][0] + i * 4, qg + (size_t)(k0 + i / (TPL / 4)) * F_TPL + 4 * (i % (TPL / 4)));
         cp_commit();
     };
 
@@ -122,8 +130,10 @@ __global__ void __launch_bounds__(F_THREADS, 2) k_scan_fp32(ScanArgs a)
         __syncthreads(); // stage st visible to all; every warp is done with stage st - 1
         if (st + 2 < stages)
             load_stage((st + 2) % F_BUFS, (st + 2) * F_K);
-        const float *xw = &xs[cur][0];
-        const float *qw = &qs[cur][0][8 * warp];
+        const float *xw = &xs[cur][xpos(256 * (warp / WT))];
+        const float *qw = &qs[cur][0][8 * wt];
+        if (!active)
+            continue;
 #pragma unroll 4
         for (int kk = 0; kk < F_K; kk += 4)
         {
@@ -141,8 +151,8 @@ __global__ void __launch_bounds__(F_THREADS, 2) k_scan_fp32(ScanArgs a)
 #pragma unroll
             for (int i = 0; i < 4; i++)
             {
-                const float4 qa = *reinterpret_cast<const float4 *>(qw + (kk + i) * F_TPL);
-                const float4 qb = *reinterpret_cast<const float4 *>(qw + (kk + i) * F_TPL + 4);
+                const float4 qa = *reinterpret_cast<const float4 *>(qw + (kk + i) * TPL);
+                const float4 qb = *reinterpret_cast<const float4 *>(qw + (kk + i) * TPL + 4);
                 const uint64_t q2[4] = {f2pack(qa.x, qa.y), f2pack(qa.z, qa.w), f2pack(qb.x, qb.y),
                                         f2pack(qb.z, qb.w)};
 #pragma unroll
@@ -164,7 +174,9 @@ __global__ void __launch_bounds__(F_THREADS, 2) k_scan_fp32(ScanArgs a)
             f2unpack(acc2[w][p2], acc[w][2 * p2], acc[w][2 * p2 + 1]);
 
     // ---- fused epilogue ----
-    const uint32_t j0 = tile_j + 8 * lane;
+    if (!active)
+        return;
+    const uint32_t j0 = warp_j + 8 * lane;
     float mu[8], iv[8];
 #pragma unroll
     for (int w = 0; w < 8; w++)
@@ -173,11 +185,11 @@ __global__ void __launch_bounds__(F_THREADS, 2) k_scan_fp32(ScanArgs a)
         mu[w] = j < a.W ? a.mean[j] : 0.0f;
         iv[w] = j < a.W ? a.inv[j] : 0.0f;
     }
-    const uint32_t bucket = tile_j >> a.bucket_log;
+    const uint32_t bucket = warp_j >> a.bucket_log;
 #pragma unroll
     for (int tt = 0; tt < 8; tt++)
     {
-        const int tl = 8 * warp + tt;
+        const int tl = 8 * wt + tt;
         const TemplParam &p = tps[tl];
         const int t = tile_t + tl;
         if (t >= a.T)
@@ -244,22 +256,43 @@ __global__ void k_template_tiles(const float *__restrict__ q, int m_pad, float *
     }
 }
 
-cudaError_t launch_scan_fp32(const ScanArgs &a, cudaStream_t s)
+template <int K, int WT> static cudaError_t launch_tiles(const ScanArgs &a, int t0, int tiles, cudaStream_t s)
 {
-    dim3 grid((a.W + F_WIN - 1) / F_WIN, (a.T + F_TPL - 1) / F_TPL);
-    // m_pad is a multiple of 64, so of 32
-    k_template_tiles<<<dim3((unsigned)(a.m_pad / 32), grid.y), 256, 0, s>>>(a.q, a.m_pad, a.qt);
-    if (a.m_pad % 128 == 0)
-    {
-        cudaFuncSetAttribute(k_scan_fp32<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f_smem<128>());
-        k_scan_fp32<128><<<grid, F_THREADS, f_smem<128>(), s>>>(a);
-    }
-    else
-    {
-        cudaFuncSetAttribute(k_scan_fp32<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f_smem<64>());
-        k_scan_fp32<64><<<grid, F_THREADS, f_smem<64>(), s>>>(a);
-    }
+    auto *kernel = k_scan_fp32<K, WT>;
+    const cudaError_t e =
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f_smem<K, WT>());
+    if (e != cudaSuccess)
+        return e;
+    constexpr unsigned win = FStage<K, WT>::WIN;
+    kernel<<<dim3((a.W + win - 1) / win, (unsigned)tiles), F_THREADS, f_smem<K, WT>(), s>>>(a, t0);
     return cudaGetLastError();
+}
+
+template <int K> static cudaError_t launch_k(const ScanArgs &a, int sms, cudaStream_t s)
+{
+    // full tiles, then what remains in the narrowest tile that holds it, unless its longer windows
+    // leave multiprocessors without a block (the idle warps of a wider one only load)
+    const int full = a.T / F_TPL, left = a.T % F_TPL;
+    cudaError_t e = cudaSuccess;
+    if (full > 0)
+        e = launch_tiles<K, 8>(a, 0, full, s);
+    if (left == 0 || e != cudaSuccess)
+        return e;
+    const auto fits = [&](int wt) { return left <= 8 * wt && (uint64_t)a.W > (uint64_t)(2048 / wt) * (sms - 1); };
+    if (fits(1))
+        return launch_tiles<K, 1>(a, full * F_TPL, 1, s);
+    if (fits(2))
+        return launch_tiles<K, 2>(a, full * F_TPL, 1, s);
+    if (fits(4))
+        return launch_tiles<K, 4>(a, full * F_TPL, 1, s);
+    return launch_tiles<K, 8>(a, full * F_TPL, 1, s);
+}
+
+cudaError_t launch_scan_fp32(const ScanArgs &a, int sms, cudaStream_t s)
+{
+    // m_pad is a multiple of 64, so of 32
+    k_template_tiles<<<dim3((unsigned)(a.m_pad / 32), (unsigned)((a.T + F_TPL - 1) / F_TPL)), 256, 0, s>>>(a.q, a.m_pad, a.qt);
+    return a.m_pad % 128 == 0 ? launch_k<128>(a, sms, s) : launch_k<64>(a, sms, s);
 }
 
 } // namespace tmb

@@ -486,7 +486,7 @@ void execute_group(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
         {
             L.fp32_qt.reserve(sizeof(float) * static_cast<size_t>(g.T_pad) * g.m_pad);
             a.qt = L.fp32_qt.as<float>();
-            TM_CUDA(tmb::launch_scan_fp32(a, s));
+            TM_CUDA(tmb::launch_scan_fp32(a, ctx->sms, s));
             count_launch(L); // the template-tile transposition
         }
         count_launch(L);
