@@ -92,7 +92,7 @@ struct FftArgs
 constexpr int kFftStats = 3 * (16384 / 4);
 
 constexpr int kFftRoots = 384; // entries of the forward kernel's twiddle tables; the correlation kernels' follow
-constexpr int kFftAllRoots = kFftRoots + (513 + 64 + 128) + (257 + 32 + 64);
+constexpr int kFftAllRoots = kFftRoots + (513 + 16 + 128) + (257 + 8 + 64);
 
 uint32_t fft_pieces(uint64_t n, int cls);
 void fft_roots(double2 *host); // kFftAllRoots entries

@@ -315,19 +315,23 @@ __global__ void __launch_bounds__(N / 16) k_fft_forward(const float *__restrict_
 // some dot product exceeds what 1 / sd of that chunk allows. The bounds of 1 / sd and of the mean
 // come from the last template of the piece that evaluated every window, if at most 10 % shorter:
 // items of a piece go from the shortest template to the longest (chunk_limit has the argument).
-// The others read neither prefix sums nor kept statistics.
+// Each thread compares the outputs that it holds in registers; where none of the block's is
+// above its limit, the item ends there: no float outputs in shared memory, no prefix sums.
 //
-// What bounds it: the load/store unit's data pipe, about 70 % busy (three exchanges of 16 bytes a
-// point, the spectra, the outputs), the FP64 pipe 35 %, and the two barriers of an item; an item
-// that evaluates all its windows also reads 34 bytes of prefix sums and runs per window (or 12
-// bytes of a shared length's kept statistics) and issues 70 instructions for it. Per template
-// and 2^25 samples, in ms, skipping / kept statistics / all its own (FP64 passes of radix 16, 16,
-// 16, 2 with block-wide barriers, steps of 8192 for up to 8192 samples, longer pieces above and
-// no skipping took 0.49 with kept statistics and 0.71 without, 0.62 and 1.07 above 8192): m =
-// 1024 0.128 / 0.169 / 0.25, 2048 0.149 / 0.167 / 0.278, 4096 0.167 / 0.203 / 0.31, 8192 0.248 /
-// 0.315 / 0.43, 16000 0.38 / 0.42 / 0.63. 32 points per thread and two exchanges (radix 16, 16, 16; 8
-// warps per SM) took 0.177 at m = 2048 and 0.409 with distinct lengths at 4096 before windows
-// were skipped, also with the epilogue on warps of its own: too few warps to hide the latencies.
+// What bounds it: the load/store unit's data pipe (50 to 70 % busy: three exchanges of 16 bytes a
+// point and the spectra), the FP64 pipe 40 %, and with N = 8192 one block per multiprocessor,
+// whose phases hardly overlap; an item that evaluates all its windows also reads 34 bytes of
+// prefix sums and runs per window (or 12 bytes of a shared length's kept statistics) and issues
+// 70 instructions for it. Per template and 2^25 samples, in ms, skipping / kept statistics / all
+// its own (FP64 passes of radix 16, 16, 16, 2 with block-wide barriers, steps of 8192 for up to
+// 8192 samples, longer pieces above and no skipping took 0.49 with kept statistics and 0.71
+// without, 0.62 and 1.07 above 8192): m = 1024 0.113 / 0.171 / 0.25, 2048 0.131 / 0.168 / 0.28,
+// 4096 0.154 / 0.208 / 0.32, 8192 0.230 / 0.326 / 0.44, 16000 0.36 / 0.43 / 0.64. With the outputs
+// compared after they went through shared memory, and four roots per radix-8 pass loaded instead
+// of one: 0.128, 0.149, 0.167, 0.248 and 0.38. 32 points per thread and two exchanges (radix 16,
+// 16, 16; 8 warps per multiprocessor) took 0.177 at m = 2048 and 0.409 with distinct lengths at
+// 4096 before windows were skipped, also with the epilogue on warps of its own: too few warps to
+// hide the latencies.
 struct FftItem // what an item needs of its piece, and its row's cut
 {
     double shift[kFftMaxParts], norm[kFftMaxParts];
@@ -344,10 +348,11 @@ template <int N> struct FftShape
     // the twiddle tables: the packing's roots, then those of the two last radix-8 passes, even
     // entries before odd ones: a thread takes an even one and the next, and a quarter warp's 16-byte
     // loads fall in distinct banks (side by side, two to a bank, 1 to 2.5 % of the kernel's time)
-    static constexpr int TabB = T + 1, TabC = TabB + 4 * (N == 4096 ? 8 : 16), Tabs = TabC + N / 64;
+    static constexpr int TabB = T + 1, TabC = TabB + (N == 4096 ? 8 : 16), Tabs = TabC + N / 64;
     static constexpr int Chunks = N == 4096 ? 56 : 96; // 128-window chunks of the longest step
     static constexpr size_t Smem = 2 * sizeof(double) * Ex + 8 * sizeof(float) * Dot + sizeof(double2) * Tabs +
-                                   2 * sizeof(FftRow) + 2 * sizeof(FftItem) + sizeof(float4) * Chunks;
+                                   2 * sizeof(FftRow) + 2 * sizeof(FftItem) + sizeof(float4) * Chunks +
+                                   sizeof(int) * (N / 64 + 2 * (N / 2048));
 };
 static_assert(FftShape<8192>::Smem <= 227 * 1024, "shared memory of k_fft_corr");
 static_assert(2 * (FftShape<4096>::Smem + 1024) <= 228 * 1024, "two blocks of k_fft_corr<4096> per SM");
@@ -535,6 +540,7 @@ __device__ __forceinline__ float sqrt_approx(float x)
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+__device__ __forceinline__ float max_nan(float a, float b) { return a > b || a != a ? a : b; } // NaN if one is
 __device__ __forceinline__ float chunk_limit(const FftRow &P, float4 b, float cut, const FoldItem &f)
 {
     const float q = (float)P.m * b.w;
@@ -642,6 +648,8 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
     FftRow *srow = reinterpret_cast<FftRow *>(tab + C::Tabs); // this item's row and the next one's
     FftItem *sitem = reinterpret_cast<FftItem *>(srow + 2);
     float4 *bounds = reinterpret_cast<float4 *>(sitem + 2); // of the chunks of 128 windows (chunk_limit)
+    int *limits = reinterpret_cast<int *>(bounds + C::Chunks);         // of the 128 outputs from 128 k on
+    uint32_t *above = reinterpret_cast<uint32_t *>(limits + N / 64);   // those with an output above, a bit each: two items
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const uint64_t total = (uint64_t)a.p_count * (uint32_t)a.nrows;
     const uint64_t item0 = total * blockIdx.x / gridDim.x;
@@ -682,6 +690,27 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
         if (PARTS)
             for (int i = 1; i < parts; i++)
                 add = fma(I.shift[i] - I.shift[0], P.sum[i - 1], add);
+
+        // ---- may the item skip chunks of its windows? limits of the outputs 128 k to 128 k + 127, whose
+        // windows lie in two chunks, as the high words of doubles ----
+        const int chunks = (int)a.step / 128; // a multiple of the warps
+        const float cut = a.cuts != nullptr ? I.cut : P.thr;
+        const bool skip = bound_m > 0 && bound_m <= m && 10 * m <= 11 * bound_m && cut < inf_f();
+        if (skip && t < N / 64)
+        {
+            const int c = t - ((base + 127) >> 7);
+            float4 b = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            for (int i = c; i <= c + 1; i++)
+                if (i >= 0 && i < chunks)
+                {
+                    const float4 x = bounds[i];
+                    b = make_float4(max_nan(b.x, x.x), max_nan(b.y, x.y), fmaxf(b.z, x.z), x.w);
+                }
+            const float limit = chunk_limit(P, b, cut, fold_item(P, I, parts));
+            limits[t] = c + 1 < 0 || c >= chunks ? 0x7fffffff : limit > 0.0f ? __double2hiint((double)limit) : (int)0x80000000;
+            if (t < N / 2048)
+                above[(item & 1) * (N / 2048) + t] = 0u;
+        }
 
         // ---- product, real-transform packing: C[k] for this thread's bins ----
         double2 A[8], B[8];
@@ -824,9 +853,14 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
         {
             const int k = (2 * s) & (Ns2 - 1);
             const double2 *w = tab + C::TabB + k / 2; // of k, then of k + 1
-            radix8(A, w[0], w[Ns2], w[2 * Ns2], w[3 * Ns2]);
-            w += Ns2 / 2;
-            radix8(B, w[0], w[Ns2], w[2 * Ns2], w[3 * Ns2]);
+            {
+                const double2 w1 = w[0], w2 = csqr(w1);
+                radix8(A, w1, w2, csqr(w2), mul_w8(w1));
+            }
+            {
+                const double2 w1 = w[Ns2 / 2], w2 = csqr(w1);
+                radix8(B, w1, w2, csqr(w2), mul_w8(w1));
+            }
             group_sync<N>(g);
             const int b = 9 * (2 * s - k) + k;
 #pragma unroll
@@ -849,34 +883,57 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
                 const double2 w1 = w[C::GT], w2 = csqr(w1);
                 radix8(B, w1, w2, csqr(w2), mul_w8(w1));
             }
-            // outputs n1 = 2 s + (Q / 8) r and the next of transform g: correlation outputs 16 n1 + 2 g (+ 1)
+        }
+        // outputs n1 = 2 s + (Q / 8) r and the next of transform g: correlation outputs 16 n1 + 2 g (+ 1)
+        if (PARTS)
+        {
+#pragma unroll
+            for (int r = 0; r < 8; r++)
+            {
+                A[r] = make_double2(A[r].x + add, A[r].y + add);
+                B[r] = make_double2(B[r].x + add, B[r].y + add);
+            }
+        }
+        copies_wait();
+        bool any = true; // has a chunk to be evaluated?
+        if (skip)
+        {
+            const int *limit = limits + (s >> 2);
+            uint32_t high = 0;
+#pragma unroll
+            for (int r = 0; r < 8; r++)
+            {
+                const double2 x = A[out8(r)], y = B[out8(r)];
+                const int most = max(max(__double2hiint(x.x), __double2hiint(x.y)), max(__double2hiint(y.x), __double2hiint(y.y)));
+                high |= (most >= limit[(Q / 64) * r] ? 1u : 0u) << r;
+            }
+            any = __syncthreads_or(high != 0u) != 0;
+            uint32_t *mine = above + (item & 1) * (N / 2048);
+            for (; high != 0u; high &= high - 1)
+            {
+                const int k = (s >> 2) + (Q / 64) * (__ffs(high) - 1);
+                atomicOr(&mine[k >> 5], 1u << (k & 31));
+            }
+        }
+        if (any)
+        {
             float *d = dots + g * C::Dot + 4 * s;
 #pragma unroll
             for (int r = 0; r < 8; r++)
             {
                 const double2 x = A[out8(r)], y = B[out8(r)];
-                *reinterpret_cast<float4 *>(d + (Q / 4) * r) =
-                    PARTS ? make_float4((float)(x.x + add), (float)(x.y + add), (float)(y.x + add), (float)(y.y + add))
-                          : make_float4((float)x.x, (float)x.y, (float)y.x, (float)y.y);
+                *reinterpret_cast<float4 *>(d + (Q / 4) * r) = make_float4((float)x.x, (float)x.y, (float)y.x, (float)y.y);
             }
+            __syncthreads();
         }
-        // ---- may the item skip chunks of its windows? chunk i of this warp where all its dots are below
-        // the limit of lane i (computed while the block gathers) ----
-        constexpr int kWarps = T / 32, MaxChunks = (C::Chunks + kWarps - 1) / kWarps;
-        const int chunks = (int)a.step / 128, per = chunks / kWarps; // a multiple of the warps
-        const bool knn = P.mode == TM_MODE_KNN;
-        const float cut = a.cuts != nullptr ? I.cut : P.thr;
-        const bool skip = bound_m > 0 && bound_m <= m && 10 * m <= 11 * bound_m && cut < inf_f();
-        float limit = -1.0f;
-        if (skip && lane < per)
-            limit = chunk_limit(P, bounds[warp + kWarps * lane], cut, fold_item(P, I, parts));
-        copies_wait();
-        __syncthreads();
 
         // ---- epilogue: window o of the piece is output i = o + base; a lane's windows are 128 c +
         // 32 j + lane, j < 4. Output i = 16 n1 + 2 g + h is at dots[g Dot + 2 n1 + h]: the pad puts a
         // warp's 32 consecutive outputs in distinct banks but for a few. What a chunk needs from
         // global memory is loaded while the one before is evaluated ----
+        constexpr int kWarps = T / 32;
+        const int per = chunks / kWarps;
+        const bool knn = P.mode == TM_MODE_KNN;
         const int64_t rel = (int64_t)piece_w - (int64_t)a.w0; // window o of the piece is rel + o of the range
         const float s1 = P.s1, c_lin = P.c_lin, a3 = P.a3, thr = P.thr;
         const int i0 = base + lane;
@@ -930,19 +987,16 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
                 emit_strided(mask, lane, (uint32_t)P.row, (uint32_t)(first + lane), a.cand, a.cand_count, a.cand_cap);
             }
         };
-        uint32_t todo = (1u << per) - 1u; // this warp's chunks warp + kWarps i
-        if (skip)
-        {
-#pragma unroll
-            for (int i = 0; i < MaxChunks; i++)
-                { // past the last chunk: within shared memory, and no bit of todo
-                    const float *x = dl + 16 * (warp + kWarps * i);
-                    const float most = fmaxf(fmaxf(fmaxf(x[0], x[4]), fmaxf(x[8], x[12])), 0.0f);
-                    const float l = __shfl_sync(0xffffffffu, limit, i);
-                    if (__all_sync(0xffffffffu, most < l))
-                        todo &= ~(1u << i);
-                }
-        }
+        uint32_t todo = any ? (1u << per) - 1u : 0u; // this warp's chunks warp + kWarps i
+        if (skip && any)
+            for (int i = 0; i < per; i++)
+            {
+                // its outputs are among 128 and the next (none past the last)
+                const int k = (128 * (warp + kWarps * i) + base) >> 7, n = min(k + 1, N / 64 - 1);
+                const uint32_t *set = above + (item & 1) * (N / 2048);
+                if (((set[k >> 5] >> (k & 31) | set[n >> 5] >> (n & 31)) & 1u) == 0u)
+                    todo &= ~(1u << i);
+            }
         int c = warp + kWarps * (__ffs(todo) - 1);
         auto next_chunk = [&]() { // after c, or c again at the end
             todo &= todo - 1;
@@ -1105,7 +1159,8 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
                 evaluate(c, iv, ms, ew);
                 c = n;
             }
-            __syncwarp(); // the warp's bounds are read by its lanes
+            if (record)
+                __syncthreads(); // the bounds are read by other warps
         }
         if (!skip)
         {
@@ -1123,8 +1178,8 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
 
 // The twiddle tables, in extended precision rounded to double: the forward kernel's R1[a] =
 // e^{2 pi i a / 32768} (a < 128) and R2[b] = e^{2 pi i 128 b / 32768} (b < 256), then the
-// correlation kernel's: e^{2 pi i t / L} (t <= 512); w, w^2, w^4 and w e^{2 pi i / 8}, 16 each,
-// of w = e^{2 pi i k / 128} (k < 16); e^{2 pi i b / 1024} (b < 128).
+// correlation kernel's, for N = 8192: e^{2 pi i t / L} (t <= 512), e^{2 pi i k / 128} (k < 16) and
+// e^{2 pi i b / 1024} (b < 128).
 static double2 root_of(long double num, long double den)
 {
     const long double a = 6.283185307179586476925286766559005768L * num / den;
@@ -1139,11 +1194,7 @@ template <int N> static void corr_tables(double2 *tab)
         tab[i] = root_of(i, 2 * N);
     for (int k = 0; k < Ns; k++)
     {
-        double2 *w = tab + C::TabB + (k & 1) * (Ns / 2) + k / 2;
-        w[0] = root_of(k, 8 * Ns);
-        w[Ns] = root_of(2 * k, 8 * Ns);
-        w[2 * Ns] = root_of(4 * k, 8 * Ns);
-        w[3 * Ns] = root_of(k + Ns, 8 * Ns);
+        tab[C::TabB + (k & 1) * (Ns / 2) + k / 2] = root_of(k, 8 * Ns);
     }
     for (int b = 0; b < N / 64; b++)
         tab[C::TabC + (b & 1) * C::GT + b / 2] = root_of(b, N / 8);

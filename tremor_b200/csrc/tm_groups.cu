@@ -448,13 +448,13 @@ double tensor_cost_sorted(const tm_ctx *ctx, const int *m, size_t n)
 // step alone, and within a class little on it; the factors are the classes' times over that of
 // a template that evaluates all its windows at 4096 (0.307 ms) or 16000 (0.63 ms): 0.247, 0.275,
 // 0.307, 0.43 ms at 1000, 2000, 4096, 8192; 0.167, 0.167, 0.200, 0.315 with the statistics of
-// the template before it of the same length, 0.42 at 16384; 0.128, 0.149, 0.167, 0.248 where
-// almost all are skipped, 0.38 at 16000.
+// the template before it of the same length, 0.42 at 16384; 0.113, 0.131, 0.154, 0.230 where
+// almost all are skipped, 0.36 at 16000.
 double fft_time(const tm_ctx *ctx, int m, int longer, bool skips)
 {
     static const double all[tmb::kFftClasses] = {0.81, 0.90, 1.0, 1.41};
     static const double same[tmb::kFftClasses] = {0.55, 0.55, 0.66, 1.04};
-    static const double skip[tmb::kFftClasses] = {0.42, 0.49, 0.55, 0.81};
+    static const double skip[tmb::kFftClasses] = {0.37, 0.43, 0.50, 0.75};
     const int cls = tmb::fft_class_of(m);
     const bool parts = tmb::fft_parts(m, cls) > 1;
     const double unit = parts ? ctx->fft_long_ms : ctx->fft_ms, every = unit * (parts ? 1.0 : all[cls]);
@@ -464,7 +464,7 @@ double fft_time(const tm_ctx *ctx, int m, int longer, bool skips)
         return longer == m ? unit * (parts ? 0.69 : same[cls]) : every;
     // one template in so many, a tenth of the length apart, evaluates all its windows and sets bounds
     const double sets = std::min(1.0, std::log(static_cast<double>(longer) / m) / std::log(1.1));
-    return sets * every + (1.0 - sets) * unit * (parts ? 0.61 : skip[cls]);
+    return sets * every + (1.0 - sets) * unit * (parts ? 0.58 : skip[cls]);
 }
 
 // Device memory that the FFT branch's resident arrays for these lengths would still take
