@@ -116,9 +116,9 @@ int tm_set_tiles(tm_ctx *ctx, int tiles);
  * 2^25 windows, [group kind: one length, several][shape: rows, columns 128, 64, 32]
  * [K: 256, 1024, 4096, 16384], 32 doubles in that order, then the FFT branch's
  * milliseconds per template per 2^25 samples for templates of up to 8192 samples and for
- * longer ones (measured with lengths of up to 4096 and 16384, too far apart to share anything;
- * the planner scales them to other lengths and to templates that share their windows'
- * statistics or skip windows). tm_autotune measures it on this device (a few seconds, its own
+ * longer ones (measured with distinct lengths near 4096 and 16384, every window evaluated; the
+ * planner scales them to other lengths and to templates that share their windows' statistics
+ * or skip windows). tm_autotune measures it on this device (a few seconds, its own
  * synthetic record), stores it in the context and copies it to ms (up to capacity values); returns 34
  * or an error. tm_set_tile_model installs a saved one (count 34; 33 keeps the long-template
  * FFT figure, 32 both). No counterpart in the reference. */

@@ -1,6 +1,6 @@
 """The FFT branch's chunks of windows that a template's cut lets it skip: answers equal the oracle's
-with thresholds and with kNN bounds known from the first part of the record, over lengths that
-share a chunk's bounds and lengths too far apart to, and over records whose deviation jumps, that
+with thresholds and with kNN bounds known from the first part of the record, over lengths at, above
+and below those that the chunks' bounds are kept at, and over records whose deviation jumps, that
 stand constant, miss samples, carry an offset or cross a prefix block."""
 import numpy as np
 import pytest
@@ -38,11 +38,13 @@ def _check(x, reqs, answers):
 
 
 @pytest.mark.parametrize('kind', ['plain', 'jumps', 'constant', 'offset'])
-@pytest.mark.parametrize('lengths', [[300, 301, 329, 330, 331, 400, 400, 440, 441], [2049, 2049, 2050, 2254, 2255],
-                                     [4097, 4000, 3700, 64], [8192, 8193, 9000]])
+@pytest.mark.parametrize('lengths', [[300, 301, 329, 330, 331, 400, 400, 440, 441] * 2 + [3, 16, 17, 21],
+                                     [2049, 2049, 1500, 1254, 1255] * 4, [4097, 4000, 3700, 2050] * 4,
+                                     [8192, 8000, 4098] * 3 + [8193, 9000, 16384] * 3])
 def test_thresholds(kind, lengths):
+    """Enough pieces and templates of each class for windows to be skipped."""
     rng = np.random.default_rng(sum(lengths))
-    x = _record(kind, 150_000, rng)
+    x = _record(kind, 170_000, rng)
     reqs = []
     for i, m in enumerate(lengths):
         p = int(rng.integers(0, len(x) - m))
@@ -50,7 +52,12 @@ def test_thresholds(kind, lengths):
         reqs.append(tb.Request(t.astype(np.float32), tb.MODE_THRESHOLD, correlation=(0.9, 0.6, 0.3)[i % 3]))
     with tb.Context(x) as ctx:
         ctx.set_tiles(tb.TILES_FFT)
-        _check(x, reqs, ctx.scan_batch(reqs))
+        answers = ctx.scan_batch(reqs)
+        ctx.set_tiles(tb.TILES_ROWS)
+        rows = ctx.scan_batch(reqs)
+    for i, ((p, d), (pr, dr)) in enumerate(zip(answers, rows)):
+        assert np.array_equal(p, pr) and np.array_equal(d.view(np.uint32), dr.view(np.uint32)), i
+    _check(x, reqs[-4:], answers[-4:])
 
 
 @pytest.mark.parametrize('kind', ['plain', 'jumps', 'constant', 'offset'])

@@ -268,10 +268,11 @@ int tm_autotune(tm_ctx *ctx, double *ms, int capacity)
                     table[mixed][v][ki] = per * (33554432.0 / windows);
                 }
             }
-        // the FFT branch, 8 templates each, more than 10 % apart in length, so that each
-        // evaluates all its windows with statistics of its own (the time does not depend on the
-        // length within either kind): templates of up to 4096 samples and of up to 16384
+        // the FFT branch, 8 templates of distinct lengths each, which evaluate all their windows
+        // with statistics of their own (the time does not depend on the length within either
+        // kind): templates of up to 8192 samples (4089-4096 here) and longer ones (16377-16384)
         tc->tiles = TM_TILES_FFT;
+        tc->fft_skip = false;
         double fft_per[2];
         for (int kind = 0; kind < 2; kind++)
         {
@@ -279,7 +280,7 @@ int tm_autotune(tm_ctx *ctx, double *ms, int capacity)
             std::vector<tm_request> fr(8);
             for (int t = 0; t < 8; t++)
             {
-                const int m = static_cast<int>((kind == 0 ? 4096.0 : 16384.0) / std::pow(1.1008, t));
+                const int m = (kind == 0 ? 4096 : 16384) - t;
                 ft[t].resize(static_cast<size_t>(m));
                 for (int i = 0; i < m; i++)
                     ft[t][i] = std::sin(0.003f * static_cast<float>(i) * (1.0f + 0.01f * t) +

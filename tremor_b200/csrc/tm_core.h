@@ -347,6 +347,8 @@ struct tm_ctx
         bool ready = false;
     } fft[tmb::kFftClasses];
     tmh::DevBuf fft_roots;
+    tmh::DevBuf fft_bounds[tmb::kFftBases]; // the chunks' bounds, by base length, built on first use
+    bool fft_skip = true;                   // off while tm_autotune measures templates that evaluate every window
     std::mutex fft_mu;
     int sms = 148;
     // model: the FFT branch's ms per template per 2^25 samples, for templates of 4096 samples and
@@ -473,7 +475,7 @@ void prepare_group_mixed(tm_ctx *ctx, Lane &L, const std::vector<int> &idx_in, c
 void prepare_fft(tm_ctx *ctx, Lane &L, GroupPlan &g);
 int plan_col_tile(const tm_ctx *ctx, const tm_request *reqs, const std::vector<int> &idx, double *cost = nullptr);
 double tile_time(const tm_ctx *ctx, bool mixed, int v, double k);
-double fft_time(const tm_ctx *ctx, int m, int longer, bool skips);
+double fft_time(const tm_ctx *ctx, int m, bool shared, bool skips);
 uint32_t fft_stage_end(uint32_t p0, uint32_t pieces, int rows, int cls, int sms);
 void create_batch(tm_ctx *ctx, Lane &L, const tm_request *requests, int count, tm_batch &b, bool serving = false);
 

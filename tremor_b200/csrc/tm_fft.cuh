@@ -35,6 +35,27 @@ inline int fft_parts(int m, int cls)
     return m <= single ? 1 : (m + step - 1) / step;
 }
 
+// Lengths that the bounds of the record's chunks of 128 windows are kept at (k_chunk_bounds): a
+// template takes those of the largest of them that it reaches, at most a tenth shorter.
+constexpr int kFftBases = 100;
+__host__ __device__ constexpr int fft_base_next(int m) { return m + 1 > m * 11 / 10 ? m + 1 : m * 11 / 10; }
+inline int fft_base(int m) // its index
+{
+    int i = 0;
+    for (int b = 1; fft_base_next(b) <= m; b = fft_base_next(b))
+        i++;
+    return i;
+}
+inline int fft_base_length(int index)
+{
+    int b = 1;
+    for (int i = 0; i < index; i++)
+        b = fft_base_next(b);
+    return b;
+}
+// Chunks of a record, those of its last pieces' windows past the end included.
+inline size_t fft_chunks(uint64_t n) { return (size_t)((n + 16384) / 128); }
+
 // One template of a correlation launch. The bound coefficients (a1_main, a2, a5, a6), qs and
 // |s1| are the largest of the launch's templates of its length.
 struct FftRow
@@ -49,6 +70,8 @@ struct FftRow
     uint32_t wcount;
     float e_norm; // fft_e_norm
     float inv_a3; // 1 / (1 - a3), rounded up
+    int base;     // fft_base(m)
+    int pad[3];
 };
 
 // An FFT dot product's error: norms of the template and of the piece's samples times this; the
@@ -84,6 +107,7 @@ struct FftArgs
     float *dbg_d, *dbg_e; // diagnostics: d and e of every window, [t][W]; null in searches
     int prune;            // some template has a cut: no window with d - e above it is wanted
     const float *cuts;    // the cuts of rows' templates; null: their thr
+    const float4 *bounds[kFftBases]; // with prune, the chunks' bounds at the rows' bases
     float4 *stats;        // per block, the folded statistics of a piece's windows (a lane's scratch, kFftStats)
 };
 
@@ -104,6 +128,7 @@ cudaError_t launch_fft_templates(const float *q, const TemplParam *tp, const Fft
 // threshold, a kNN bound or infinity. sup: nk x nb_seen keys of scratch, where super is set.
 cudaError_t launch_fft_cuts(const FftRow *rows, int nrows, const uint32_t *bmin_u, uint32_t *sup, uint32_t nb, uint32_t nb_seen,
                             int blog, const TemplParam *tp, const int *slots, int nk, bool super, float *cuts, cudaStream_t s);
+cudaError_t launch_chunk_bounds(const PrefixView &pv, const uint16_t *run, uint64_t n, int m, float4 *bounds, cudaStream_t s);
 cudaError_t launch_fft_corr(FftArgs a, int cls, const double2 *roots, int sms, cudaStream_t s);
 
 } // namespace tmb

@@ -313,10 +313,10 @@ __global__ void __launch_bounds__(N / 16) k_fft_forward(const float *__restrict_
 // Skipped windows. Once a template has a cut (its threshold; a kNN bound from the first pieces),
 // almost no window can be an answer, and a chunk of 128 windows needs its statistics only where
 // some dot product exceeds what 1 / sd of that chunk allows. The bounds of 1 / sd and of the mean
-// come from the last template of the piece that evaluated every window, if at most 10 % shorter:
-// items of a piece go from the shortest template to the longest (chunk_limit has the argument).
-// Each thread compares the outputs that it holds in registers; where none of the block's is
-// above its limit, the item ends there: no float outputs in shared memory, no prefix sums.
+// are kept for the record, at lengths a tenth apart (k_chunk_bounds); those at the next
+// shorter length bound them at the template's (chunk_limit has the argument). Each thread
+// compares the outputs that it holds in registers; where none of the block's is above its limit,
+// the item ends there: no float outputs in shared memory, no prefix sums.
 //
 // What bounds it: the load/store unit's data pipe (50 to 70 % busy: three exchanges of 16 bytes a
 // point and the spectra), the FP64 pipe 40 %, and with N = 8192 one block per multiprocessor,
@@ -325,10 +325,12 @@ __global__ void __launch_bounds__(N / 16) k_fft_forward(const float *__restrict_
 // 70 instructions for it. Per template and 2^25 samples, in ms, skipping / kept statistics / all
 // its own (FP64 passes of radix 16, 16, 16, 2 with block-wide barriers, steps of 8192 for up to
 // 8192 samples, longer pieces above and no skipping took 0.49 with kept statistics and 0.71
-// without, 0.62 and 1.07 above 8192): m = 1024 0.113 / 0.171 / 0.25, 2048 0.131 / 0.168 / 0.28,
-// 4096 0.154 / 0.208 / 0.32, 8192 0.230 / 0.326 / 0.44, 16000 0.36 / 0.43 / 0.64. With the outputs
+// without, 0.62 and 1.07 above 8192): m = 1024 0.109 / 0.171 / 0.25, 2048 0.127 / 0.169 / 0.28,
+// 4096 0.153 / 0.214 / 0.32, 8192 0.231 / 0.331 / 0.44, 16000 0.33 / 0.44 / 0.63. With the outputs
 // compared after they went through shared memory, and four roots per radix-8 pass loaded instead
-// of one: 0.128, 0.149, 0.167, 0.248 and 0.38. 32 points per thread and two exchanges (radix 16,
+// of one, skipping took 0.128, 0.149, 0.167, 0.248 and 0.38; with the chunks' bounds from the last
+// template of the piece that evaluated every window, if at most a tenth shorter, one item in
+// ten to one in two evaluated them all. 32 points per thread and two exchanges (radix 16,
 // 16, 16; 8 warps per multiprocessor) took 0.177 at m = 2048 and 0.409 with distinct lengths at
 // 4096 before windows were skipped, also with the epilogue on warps of its own: too few warps to
 // hide the latencies.
@@ -351,7 +353,7 @@ template <int N> struct FftShape
     static constexpr int TabB = T + 1, TabC = TabB + (N == 4096 ? 8 : 16), Tabs = TabC + N / 64;
     static constexpr int Chunks = N == 4096 ? 56 : 96; // 128-window chunks of the longest step
     static constexpr size_t Smem = 2 * sizeof(double) * Ex + 8 * sizeof(float) * Dot + sizeof(double2) * Tabs +
-                                   2 * sizeof(FftRow) + 2 * sizeof(FftItem) + sizeof(float4) * Chunks +
+                                   3 * sizeof(FftRow) + 2 * sizeof(FftItem) + sizeof(float4) * Chunks +
                                    sizeof(int) * (N / 64 + 2 * (N / 2048));
 };
 static_assert(FftShape<8192>::Smem <= 227 * 1024, "shared memory of k_fft_corr");
@@ -525,15 +527,15 @@ __device__ __forceinline__ FoldItem fold_item(const FftRow &P, const FftItem &I,
     return f;
 }
 
-// The dot product below which no window of a chunk has d - e <= cut, from the chunk's bounds b
-// at a length m0 <= m: the largest 1 / sd and |mu - shift| / sd of its windows, kb and 1 / m0. For the
-// windows of m samples that begin at the same places the sum of squared deviations is no
-// smaller (it splits into that of the first m0 samples and two terms >= 0), so 1 / sd is at
-// most g = sqrt(m / m0) times larger; and the means differ by at most h sd, h = sqrt((m - m0) /
-// m0): with D between the means of the first m0 and of the other samples, m var >= (m0 (m - m0)
-// / m) D^2, and mu moves by D (m - m0) / m. d - e > cut where d > (cut + ew) / (1 - a3) for every
-// window, and d = c_lin - 2 (dot / sd - s1 (mu - shift) / sd). 1e-5 of c_lin is left for the
-// FP32 rounding of all of this. A NaN or a value <= 0: no dot product is below it.
+// The dot product below which no window has d - e <= cut, among windows whose 1 / sd is at most
+// iv at a length m0 <= m, |mu - shift| / sd at most r and |mu| / sd at most r0. For the windows
+// of m samples that begin at the same places the sum of squared deviations is no smaller (it
+// splits into that of the first m0 samples and two terms >= 0), so 1 / sd is at most g = sqrt(m /
+// m0) times larger; and the means differ by at most h sd, h = sqrt((m - m0) / m0): with D between
+// the means of the first m0 and of the other samples, m var >= (m0 (m - m0) / m) D^2, and mu moves
+// by D (m - m0) / m. d - e > cut where d > (cut + ew) / (1 - a3) for every window, and d = c_lin - 2
+// (dot / sd - s1 (mu - shift) / sd). 1e-5 of c_lin is left for the FP32 rounding of all of this. A
+// NaN or a value <= 0: no dot product is below it.
 __device__ __forceinline__ float sqrt_approx(float x)
 {
     float y;
@@ -541,14 +543,55 @@ __device__ __forceinline__ float sqrt_approx(float x)
     return y;
 }
 __device__ __forceinline__ float max_nan(float a, float b) { return a > b || a != a ? a : b; } // NaN if one is
-__device__ __forceinline__ float chunk_limit(const FftRow &P, float4 b, float cut, const FoldItem &f)
+__device__ __forceinline__ float chunk_limit(const FftRow &P, float iv, float r, float r0, float inv_m0, float cut,
+                                             const FoldItem &f)
 {
-    const float q = (float)P.m * b.w;
+    const float q = (float)P.m * inv_m0;
     const float g = sqrt_approx(q), h = sqrt_approx(fmaxf(q - 1.0f, 0.0f) + 1e-6f);
-    const float iv = b.x * g, r = fmaf(b.y, g, h), r0 = fmaf(fabsf(f.shift), iv, r);
-    const float ew = f.k0 + f.kr * r + f.kq * r0 * r0 + f.km * r0 + fmaf(f.s1m, b.z, f.ki) * iv;
+    iv *= g;
+    r = fmaf(r, g, h);
+    r0 = fmaf(r0, g, h);
+    const float ew = f.k0 + f.kr * r + f.kq * r0 * r0 + f.km * r0 + f.ki * iv;
     const float cross = 0.5f * (P.c_lin * (1.0f - 2e-5f) - (fmaxf(cut, 0.0f) + ew) * P.inv_a3) - r * fabsf(P.s1);
     return __fdividef(cross, iv); // below 0, NaN or infinite where no window is searched: any will do
+}
+
+// The bounds of each chunk of 128 windows of m samples, a warp per chunk: the largest 1 / sd and |mu
+// - c| / sd, c the centre of the first window's prefix block, then c and 1 / m. Infinite where the
+// statistics of a window are not trusted, or it is part of a constant run, which a longer
+// template's window may leave. Bound by the loads of the prefix sums, and read only once per
+// record and length: 0.14 ms per 2^25 samples.
+__global__ void __launch_bounds__(256) k_chunk_bounds(PrefixView pv, const uint16_t *__restrict__ run, uint64_t n, int m,
+                                                      double inv_m, uint32_t chunks, float4 *__restrict__ bounds)
+{
+    const int lane = threadIdx.x & 31;
+    const uint32_t c = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (c >= chunks)
+        return; // whole warp
+    const uint64_t first = 128ull * c;
+    const float centre = first < n ? (float)pv.C[first >> kPrefixBlockLog] : 0.0f;
+    float iv_max = 0.0f, r_max = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+    {
+        const uint64_t w = first + 32 * j + lane;
+        if (w + (uint64_t)m > n)
+            continue;
+        const uint32_t rn = run[w];
+        if (rn == 65535u)
+            continue; // no window of any length is searched here
+        WindowStats ws;
+        const bool ok = rn < (uint32_t)m && window_prefix_stats(pv, pv.Q[w], pv.Q[w + m], w, m, inv_m, ws) == 0;
+        const float iv = ok ? ws.iv * (1.0f + 2.0f * ws.rel_sd) : inf_f();
+        iv_max = fmaxf(iv_max, iv);
+        if (ok)
+            r_max = fmaxf(r_max, (fabsf(ws.mu - centre) + ws.e_mu + 2e-7f * (fabsf(ws.mu) + fabsf(centre))) * iv);
+    }
+    // as whole numbers: not negative, and a NaN above all
+    const uint32_t mi = __reduce_max_sync(0xffffffffu, __float_as_uint(iv_max));
+    const uint32_t mr = __reduce_max_sync(0xffffffffu, __float_as_uint(r_max));
+    if (lane == 0)
+        bounds[c] = make_float4(__uint_as_float(mi), __uint_as_float(mr), centre, (float)inv_m * 1.000001f);
 }
 
 // Statistics by the full bound (two prefix blocks, or ill-conditioned): false when they are
@@ -645,41 +688,57 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
     double *re = csm, *im = csm + C::Ex;
     float *dots = reinterpret_cast<float *>(csm + 2 * C::Ex);
     double2 *tab = reinterpret_cast<double2 *>(dots + 8 * C::Dot);
-    FftRow *srow = reinterpret_cast<FftRow *>(tab + C::Tabs); // this item's row and the next one's
-    FftItem *sitem = reinterpret_cast<FftItem *>(srow + 2);
-    float4 *bounds = reinterpret_cast<float4 *>(sitem + 2); // of the chunks of 128 windows (chunk_limit)
-    int *limits = reinterpret_cast<int *>(bounds + C::Chunks);         // of the 128 outputs from 128 k on
-    uint32_t *above = reinterpret_cast<uint32_t *>(limits + N / 64);   // those with an output above, a bit each: two items
+    FftRow *srow = reinterpret_cast<FftRow *>(tab + C::Tabs); // the rows of this item and the next two
+    FftItem *sitem = reinterpret_cast<FftItem *>(srow + 3);   // of this item and the next
+    float4 *bounds = reinterpret_cast<float4 *>(sitem + 2);   // the next item's chunks (this item's until pass 1)
+    int *limits = reinterpret_cast<int *>(bounds + C::Chunks); // of the 128 outputs from 128 k on
+    uint32_t *above = reinterpret_cast<uint32_t *>(limits + N / 64); // those with an output above, a bit each: two items
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const uint64_t total = (uint64_t)a.p_count * (uint32_t)a.nrows;
     const uint64_t item0 = total * blockIdx.x / gridDim.x;
     const uint32_t items = (uint32_t)(total * (blockIdx.x + 1) / gridDim.x - item0);
     uint32_t pi = (uint32_t)(item0 / (uint32_t)a.nrows);
-    int ti = a.nrows - 1 - (int)(item0 % (uint32_t)a.nrows); // the shortest template first
-    int cached_m = -1, bound_m = -1;                         // lengths of the kept statistics and chunk bounds
-    auto fetch = [&](int slot, int i, uint32_t p) { // by warp 0, in the background
-        const int parts = PARTS ? (int)min((uint32_t)a.parts, a.pieces - p) : 1;
+    int ti = (int)(item0 % (uint32_t)a.nrows), cached_m = -1;
+    // by warp 0, in the background: an item's row, and, once that is here, what else it needs
+    auto fetch_row = [&](uint32_t item, int i) {
         if (t < (int)(sizeof(FftRow) / 16))
-            copy_async<16>(reinterpret_cast<char *>(&srow[slot]) + 16 * t, reinterpret_cast<const char *>(a.rows + i) + 16 * t);
-        else if (t == 8 && a.cuts != nullptr)
-            copy_async<4>(&sitem[slot].cut, a.cuts + i);
-        else if (t >= 16 && t < 16 + parts)
-            copy_async<8>(&sitem[slot].shift[t - 16], a.shifts + p + (t - 16));
-        else if (t >= 24 && t < 24 + parts)
-            copy_async<8>(&sitem[slot].norm[t - 24], a.norms + p + (t - 24));
+            copy_async<16>(reinterpret_cast<char *>(&srow[item % 3]) + 16 * t, reinterpret_cast<const char *>(a.rows + i) + 16 * t);
     };
+    auto fetch_item = [&](uint32_t item, int i, uint32_t p) {
+        const int parts = PARTS ? (int)min((uint32_t)a.parts, a.pieces - p) : 1;
+        FftItem &I = sitem[item & 1];
+        if (t == 8 && a.cuts != nullptr)
+            copy_async<4>(&I.cut, a.cuts + i);
+        else if (t >= 16 && t < 16 + parts)
+            copy_async<8>(&I.shift[t - 16], a.shifts + p + (t - 16));
+        else if (t >= 24 && t < 24 + parts)
+            copy_async<8>(&I.norm[t - 24], a.norms + p + (t - 24));
+        if (a.prune != 0)
+        {
+            const float4 *b = a.bounds[srow[item % 3].base] + (size_t)p * (a.step / 128);
+            for (int c = t; c < (int)a.step / 128; c += 32)
+                copy_async<16>(bounds + c, b + c);
+        }
+    };
+    auto after = [&](int i) { return i + 1 < a.nrows ? i + 1 : 0; };
     for (int i = t; i < C::Tabs; i += T)
         tab[i] = a.tabs[i];
-    if (warp == 0 && items > 0)
-        fetch(0, ti, a.p_first + pi);
-    copies_wait();
+    if (warp == 0)
+    {
+        fetch_row(0, ti);
+        fetch_row(1, after(ti));
+        copies_wait();
+        __syncwarp();
+        fetch_item(0, ti, a.p_first + pi);
+        copies_wait();
+    }
     __syncthreads();
     float4 *cache = a.stats + (size_t)blockIdx.x * (3 * (L / 4));
     const int g = t / C::GT, s = t % C::GT; // this thread's transform of N / 8 points and its place there
     double *gre = re + g * C::Group, *gim = im + g * C::Group;
     for (uint32_t item = 0; item < items; item++)
     {
-        const FftRow &P = srow[item & 1];
+        const FftRow &P = srow[item % 3];
         const FftItem &I = sitem[item & 1];
         const uint32_t p = a.p_first + pi;
         const int m = P.m, base = (PARTS ? (int)a.step : m) - 1;
@@ -695,18 +754,21 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
         // windows lie in two chunks, as the high words of doubles ----
         const int chunks = (int)a.step / 128; // a multiple of the warps
         const float cut = a.cuts != nullptr ? I.cut : P.thr;
-        const bool skip = bound_m > 0 && bound_m <= m && 10 * m <= 11 * bound_m && cut < inf_f();
+        const bool skip = a.prune != 0 && cut < inf_f();
         if (skip && t < N / 64)
         {
             const int c = t - ((base + 127) >> 7);
-            float4 b = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            for (int i = c; i <= c + 1; i++)
-                if (i >= 0 && i < chunks)
-                {
-                    const float4 x = bounds[i];
-                    b = make_float4(max_nan(b.x, x.x), max_nan(b.y, x.y), fmaxf(b.z, x.z), x.w);
-                }
-            const float limit = chunk_limit(P, b, cut, fold_item(P, I, parts));
+            const float shift = (float)I.shift[0];
+            float iv = 0.0f, r = 0.0f, r0 = 0.0f, inv_m0 = 1.0f;
+            for (int i = max(c, 0); i <= min(c + 1, chunks - 1); i++)
+            {
+                const float4 x = bounds[i];
+                iv = max_nan(iv, x.x);
+                r = max_nan(r, fmaf(fabsf(x.z - shift), x.x, x.y));
+                r0 = max_nan(r0, fmaf(fabsf(x.z), x.x, x.y));
+                inv_m0 = x.w;
+            }
+            const float limit = chunk_limit(P, iv, r, r0, inv_m0, cut, fold_item(P, I, parts));
             limits[t] = c + 1 < 0 || c >= chunks ? 0x7fffffff : limit > 0.0f ? __double2hiint((double)limit) : (int)0x80000000;
             if (t < N / 2048)
                 above[(item & 1) * (N / 2048) + t] = 0u;
@@ -801,8 +863,12 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
             }
         }
         __syncthreads();
-        if (warp == 0 && item + 1 < items) // the last item's epilogue is over: its slot is free
-            fetch((item + 1) & 1, ti > 0 ? ti - 1 : a.nrows - 1, ti > 0 ? p : p + 1);
+        if (warp == 0 && item + 1 < items) // the last item's epilogue is over: its slots are free
+        {
+            const int next = after(ti);
+            fetch_item(item + 1, next, next > 0 ? p : p + 1);
+            fetch_row(item + 2, after(next));
+        }
 
         // ---- transform g: radix 16 (N = 8192) or 8 (N = 4096) with Ns = 1, then 8 and 8 ----
         constexpr int Ns2 = N == 4096 ? 8 : 16, R8 = Q / 8 + Q / 64; // R8: elements Q / 8 apart, padded
@@ -1023,8 +1089,7 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
         else
         {
             // the next item's template has the same length and meets the same piece
-            const bool keep = !skip && item + 1 < items && ti > 0 && srow[(item + 1) & 1].m == m;
-            const bool record = !skip && a.prune != 0 && item + 1 < items && ti > 0;
+            const bool keep = !skip && item + 1 < items && ti + 1 < a.nrows && srow[(item + 1) % 3].m == m;
             const FoldItem F = fold_item(P, I, parts);
             const float shift = F.shift;
             const float s1m = F.s1m, k0 = F.k0, kr = F.kr, kq = F.kq, km = F.km;
@@ -1069,7 +1134,7 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
                 }
             };
             uint64_t b0 = ~0ull; // the prefix block whose constants follow
-            float cen = 0.0f, kb = 0.0f, kib = 0.0f, va = 0.0f, vb = 0.0f;
+            float cen = 0.0f, kib = 0.0f, va = 0.0f, vb = 0.0f;
             load(c);
             while (todo != 0u)
             {
@@ -1084,8 +1149,7 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
                     b0 = b;
                     cen = (float)a.pv.C[b];
                     const BlockBounds bb = block_bounds(a.pv.T[b].y);
-                    kb = bb.b * fim + 1.9e-7f * fabsf(cen);
-                    kib = F.ki + s1m * kb;
+                    kib = F.ki + s1m * (bb.b * fim + 1.9e-7f * fabsf(cen));
                     va = bb.a * fim * (1.00001f / 0.9e-7f);
                     vb = 2.0f * bb.b * fim * (1.00001f / 0.9e-7f);
                 }
@@ -1107,7 +1171,6 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
                     ew[j] = srch ? e : __int_as_float(0x7fc00000);
                     slow |= (srch && (!ok || be != b) ? 1u : 0u) << j;
                 }
-                float iv_max = 0.0f, r_max = 0.0f; // the bounds of the lane's windows with full statistics
                 // two prefix blocks, or ill-conditioned: the full bound, one window at a time
                 for (; slow != 0u; slow &= slow - 1)
                 {
@@ -1118,9 +1181,6 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
                     float x = 0.0f, e = inf_f();
                     if (ok)
                         fold_window(st.x, v, st.z, st.w, P.c0, P.qs, P.s1_max, m, shift, F.e_dot, x, e);
-                    const float v_most = ok && st.z < 0.1f ? v * (1.0f + 2.0f * st.z) : inf_f();
-                    iv_max = fmaxf(iv_max, v_most);
-                    r_max = fmaxf(r_max, (fabsf(x) + st.w) * v_most);
 #pragma unroll
                     for (int j = 0; j < 4; j++)
                         if (j == jj)
@@ -1129,23 +1189,6 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
                             ms[j] = x;
                             ew[j] = e;
                         }
-                }
-                if (record)
-                {
-#pragma unroll
-                    for (int j = 0; j < 4; j++)
-                    {
-                        iv_max = fmaxf(iv_max, iv[j]);
-                        r_max = fmaxf(r_max, fabsf(ms[j] * iv[j]));
-                        // none for a constant run: a longer template's window may leave it
-                        if (rn[j] >= (uint32_t)m && rn[j] != 65535u)
-                            iv_max = inf_f();
-                    }
-                    // as whole numbers: not negative, and a NaN above all
-                    const uint32_t mi = __reduce_max_sync(0xffffffffu, __float_as_uint(iv_max));
-                    const uint32_t mr = __reduce_max_sync(0xffffffffu, __float_as_uint(r_max));
-                    if (lane == 0)
-                        bounds[c] = make_float4(__uint_as_float(mi), __uint_as_float(mr), kb, fim);
                 }
                 const int n = next_chunk();
                 load(n);
@@ -1159,19 +1202,14 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
                 evaluate(c, iv, ms, ew);
                 c = n;
             }
-            if (record)
-                __syncthreads(); // the bounds are read by other warps
         }
         if (!skip)
-        {
             cached_m = m;
-            bound_m = a.prune != 0 ? m : -1;
-        }
-        if (--ti < 0)
+        if (++ti == a.nrows)
         {
-            ti = a.nrows - 1;
+            ti = 0;
             pi++;
-            cached_m = bound_m = -1; // they hold the last piece's statistics
+            cached_m = -1; // the cache holds the last piece's statistics
         }
     }
 }
@@ -1260,6 +1298,13 @@ template <int N, bool PARTS> static cudaError_t launch_corr(FftArgs a, int sms, 
     const uint64_t most = (uint64_t)sms * (N == 4096 ? 2 : 1);
     if (items > 0)
         kernel<<<(unsigned)std::min(items, most), N / 16, smem, s>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_chunk_bounds(const PrefixView &pv, const uint16_t *run, uint64_t n, int m, float4 *bounds, cudaStream_t s)
+{
+    const uint32_t chunks = (uint32_t)fft_chunks(n);
+    k_chunk_bounds<<<(chunks + 7) / 8, 256, 0, s>>>(pv, run, n, m, 1.0 / m, chunks, bounds);
     return cudaGetLastError();
 }
 

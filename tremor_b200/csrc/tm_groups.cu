@@ -324,6 +324,7 @@ void prepare_fft(tm_ctx *ctx, Lane &L, GroupPlan &g)
         r.m = p.m;
         r.mode = p.mode;
         r.wcount = p.wcount;
+        r.base = tmb::fft_base(p.m);
         if (g.fft_rows.empty() || g.fft_rows[run].m != p.m)
             run = g.fft_rows.size();
         g.fft_rows.push_back(r);
@@ -441,30 +442,22 @@ double tensor_cost_sorted(const tm_ctx *ctx, const int *m, size_t n)
     return best;
 }
 
-// Modelled milliseconds of the FFT branch per template of length m per 2^25 samples. longer: the
-// next longer template's length in the group, m where a template shares its length (0: none);
-// skips: the template has a cut, so that it can skip windows by a neighbour's bounds
-// (tm_fftk.cu), which reach 10 % in length. The time depends on the length through the pieces'
-// step alone, and within a class little on it; the factors are the classes' times over that of
-// a template that evaluates all its windows at 4096 (0.307 ms) or 16000 (0.63 ms): 0.247, 0.275,
-// 0.307, 0.43 ms at 1000, 2000, 4096, 8192; 0.167, 0.167, 0.200, 0.315 with the statistics of
-// the template before it of the same length, 0.42 at 16384; 0.113, 0.131, 0.154, 0.230 where
-// almost all are skipped, 0.36 at 16000.
-double fft_time(const tm_ctx *ctx, int m, int longer, bool skips)
+// Modelled milliseconds of the FFT branch per template of length m per 2^25 samples. shared: a
+// template of the same length precedes it, whose window statistics it takes; skips: it has a
+// cut, so that it need not evaluate most windows (tm_fftk.cu). The time depends on the length
+// through the pieces' step alone, and within a class little on it; the factors are the classes'
+// times over that of a template that evaluates all its windows at 4096 (0.307 ms) or 16000
+// (0.63 ms): 0.247, 0.275, 0.307, 0.43 ms at 1000, 2000, 4096, 8192; shared 0.171, 0.168, 0.208,
+// 0.326, and 0.43 at 16384; skipping 0.109, 0.127, 0.153, 0.231, and 0.33 at 16000.
+double fft_time(const tm_ctx *ctx, int m, bool shared, bool skips)
 {
     static const double all[tmb::kFftClasses] = {0.81, 0.90, 1.0, 1.41};
     static const double same[tmb::kFftClasses] = {0.55, 0.55, 0.66, 1.04};
-    static const double skip[tmb::kFftClasses] = {0.37, 0.43, 0.50, 0.75};
+    static const double skip[tmb::kFftClasses] = {0.36, 0.42, 0.50, 0.75};
     const int cls = tmb::fft_class_of(m);
-    const bool parts = tmb::fft_parts(m, cls) > 1;
-    const double unit = parts ? ctx->fft_long_ms : ctx->fft_ms, every = unit * (parts ? 1.0 : all[cls]);
-    if (longer < m)
-        return every;
-    if (!skips)
-        return longer == m ? unit * (parts ? 0.69 : same[cls]) : every;
-    // one template in so many, a tenth of the length apart, evaluates all its windows and sets bounds
-    const double sets = std::min(1.0, std::log(static_cast<double>(longer) / m) / std::log(1.1));
-    return sets * every + (1.0 - sets) * unit * (parts ? 0.58 : skip[cls]);
+    if (tmb::fft_parts(m, cls) > 1)
+        return ctx->fft_long_ms * (skips ? 0.53 : shared ? 0.69 : 1.0);
+    return ctx->fft_ms * (skips ? skip[cls] : shared ? same[cls] : all[cls]);
 }
 
 // Device memory that the FFT branch's resident arrays for these lengths would still take
@@ -514,7 +507,7 @@ size_t plan_fft_split(tm_ctx *ctx, const tm_request *reqs, const std::vector<int
         const uint32_t pieces = tmb::fft_pieces(ctx->n, tmb::fft_class_of(r.m));
         const bool skips = r.mode != TM_MODE_KNN ||
                            fft_stage_end(0, pieces, static_cast<int>(n), tmb::fft_class_of(r.m), ctx->sms) < pieces;
-        fft_cost += fft_time(ctx, r.m, f > 1 ? m[f - 2] : 0, skips);
+        fft_cost += fft_time(ctx, r.m, f > 1 && m[f - 2] == r.m, skips);
         const double c = fft_cost + tensor_cost_sorted(ctx, m.data() + f, n - f);
         if (c < best)
         {

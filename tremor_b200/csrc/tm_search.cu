@@ -560,6 +560,50 @@ static tm_ctx::FftPieces &ensure_fft(tm_ctx *ctx, Lane &L, int cls)
     return f;
 }
 
+// The chunks' bounds at the bases of rows [first, first + count), in table; false where the memory
+// for one is not to be had, or it would take a hundredth of what is free: the windows are
+// then all evaluated.
+static bool ensure_bounds(tm_ctx *ctx, Lane &L, const GroupPlan &g, int first, int count, const float4 **table)
+{
+    std::lock_guard<std::mutex> lk(ctx->fft_mu);
+    std::vector<int> fresh;
+    size_t free_b = 0, total_b = 0;
+    try
+    {
+        for (int i = first; i < first + count; i++)
+        {
+            const int base = g.fft_rows[static_cast<size_t>(i)].base;
+            if (ctx->fft_bounds[base].p == nullptr)
+            {
+                const size_t need = sizeof(float4) * tmb::fft_chunks(ctx->n);
+                TM_CUDA(cudaMemGetInfo(&free_b, &total_b));
+                if (need > free_b / 100)
+                    throw Failure{TM_ERR_NO_MEMORY, "bounds of the record's chunks"};
+                ctx->fft_bounds[base].reserve(need);
+                fresh.push_back(base);
+                const tmb::PrefixView pv{ctx->prefix.as<double2>(), ctx->ptot.as<double2>(), ctx->pcen.as<double>()};
+                TM_CUDA(tmb::launch_chunk_bounds(pv, ctx->run.as<uint16_t>(), ctx->n, tmb::fft_base_length(base),
+                                                 ctx->fft_bounds[base].as<float4>(), L.stream));
+                count_launch(L);
+            }
+            table[base] = ctx->fft_bounds[base].as<float4>();
+        }
+        if (!fresh.empty())
+            TM_CUDA(cudaStreamSynchronize(L.stream)); // other lanes' streams read them
+    }
+    catch (const Failure &f)
+    {
+        cudaGetLastError();
+        cudaStreamSynchronize(L.stream);
+        for (const int base : fresh)
+            ctx->fft_bounds[base].release();
+        if (f.code != TM_ERR_NO_MEMORY)
+            throw;
+        return false;
+    }
+    return true;
+}
+
 // Spectrum entries of one correlation launch's templates: 25 MB, well within L2, where every
 // block reads them once per piece.
 constexpr size_t kFftLaunchBins = 192 * 8200;
@@ -634,12 +678,16 @@ void fft_contract(tm_ctx *ctx, Lane &L, const GroupPlan &g, const tmb::ScanArgs 
             f.stats = L.fft_stats.as<float4>();
             count_launch(L);
             const uint32_t pieces = pb >= pa ? pb - pa + 1 : 0;
+            // fewer items than multiprocessors: bounds and cuts would cost more than they save
+            const bool cuts = ctx->fft_skip && a.dbg_d == nullptr &&
+                              static_cast<uint64_t>(pieces) * nr >= static_cast<uint64_t>(ctx->sms) &&
+                              ensure_bounds(ctx, L, g, first, nr, f.bounds);
             for (uint32_t p0 = 0; p0 < pieces;)
             {
-                const uint32_t p1 = knn > 0 ? fft_stage_end(p0, pieces, nr, set.cls, ctx->sms) : pieces;
+                const uint32_t p1 = knn > 0 && cuts ? fft_stage_end(p0, pieces, nr, set.cls, ctx->sms) : pieces;
                 f.p_first = pa + p0;
                 f.p_count = p1 - p0;
-                f.prune = a.dbg_d == nullptr && nr > 1 && (knn < nr || p0 > 0) ? 1 : 0;
+                f.prune = cuts && (knn < nr || p0 > 0) ? 1 : 0;
                 TM_CUDA(tmb::launch_fft_corr(f, set.cls, ctx->fft_roots.as<double2>(), ctx->sms, s));
                 count_launch(L);
                 p0 = p1;

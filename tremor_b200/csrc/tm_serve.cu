@@ -65,12 +65,12 @@ static uint64_t serve_bytes(const tm_ctx *ctx, const tm_request &r)
 }
 
 // Modelled device milliseconds of a request: the cheaper of the FFT branch (a constant per
-// template, by kind, beside one of 3 % more samples) and its share of a full 128-row tile of mixed lengths at its own K, from
+// template, by kind) and its share of a full 128-row tile of mixed lengths at its own K, from
 // the planner's model (ms per 2^25 windows), scaled to the record's windows.
 static double serve_cost(const tm_ctx *ctx, const tm_request &r)
 {
     const double scale = static_cast<double>(ctx->n - static_cast<uint64_t>(r.m) + 1) / 33554432.0;
-    const double fft = fft_time(ctx, r.m, r.m + r.m / 32, true);
+    const double fft = fft_time(ctx, r.m, false, true);
     const double row = tile_time(ctx, true, 0, static_cast<double>((r.m + 63) & ~63)) / 128.0;
     return std::min(fft, row) * scale;
 }
