@@ -7,7 +7,7 @@
 // selection over the candidates in (ED^2, position) order (ZnormSearch.hpp:170-189).
 // Here both happen on the device, so the host receives finished runs:
 //   k_answer_keys      keeps the candidates that can be answers (threshold templates:
-//                      exact ED^2 <= threshold; kNN templates: all of them) as
+//                      exact ED^2 <= threshold; kNN templates: all that are not excluded) as
 //                      (template << 32 | window, ED^2) pairs
 //   radix sort 1       by that key: template-major, position order within a template
 //   k_answer_rekey     (only when the group has kNN templates) kNN entries get the key
@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(kAnswerThreads)
         c = cand[i];
         d = dist[i];
         knn = tp[c.templ].mode == TM_MODE_KNN;
-        keep = knn || d <= tp[c.templ].thr_ed;
+        keep = knn ? d != kExcluded : d <= tp[c.templ].thr_ed;
     }
     uint32_t slot, unused;
     warp_slot(keep, kept, slot);

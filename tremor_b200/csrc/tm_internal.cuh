@@ -27,6 +27,16 @@ inline uint32_t bucket_count(uint64_t windows, int log)
 {
     return (uint32_t)(((windows + (1ull << log) - 1) >> log) + 3) & ~3u;
 }
+// Distance given to a kNN candidate that is excluded without one (k_rescore): no candidate has it.
+constexpr float kExcluded = -1.0f;
+// What excludes kNN candidates: the buckets' minima of d - E, the certain minima that k_passb left
+// where those of d + E were, the bounds. nb = 0: nothing does (or the buckets are too large).
+struct Exclusion
+{
+    const uint32_t *bmin_l, *certain, *tkey;
+    uint32_t nb;
+};
+constexpr uint32_t kNoWindow = 0xffffffffu;
 constexpr int kStagePad = 16384 + 512; // zero samples after the waveform (template padding)
 
 // per-window flags (one byte per window and length)

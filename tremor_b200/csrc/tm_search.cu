@@ -231,11 +231,20 @@ void add_span(Lane &L, int phase, cudaEvent_t a, cudaEvent_t b)
     L.phase_ms[phase] += ms;
 }
 
+// What k_passb left for the re-scoring of a group's kNN candidates; nothing where the buckets are
+// larger than the re-pass's 256 windows.
+static tmb::Exclusion exclusion(const Lane &L, const GroupPlan &g, uint32_t nb, int blog)
+{
+    if (g.nk == 0 || blog != 8)
+        return tmb::Exclusion{};
+    return tmb::Exclusion{L.bmin_l.as<uint32_t>(), L.bmin_u.as<uint32_t>(), L.tkey.as<uint32_t>(), nb};
+}
+
 // Exact re-scoring of a group's ncand candidates (pv: prefix sums of mixed groups, mean: window means of the others), answer order and kNN selection on the
 // device, one copy to a pinned block that the result keeps, canonical answers.
 template <class Degenerate>
 void rescore_and_answer(tm_ctx *ctx, Lane &L, const GroupPlan &g, uint32_t ncand, const tmb::PrefixView &pv,
-                        const float *mean, uint64_t w0, tm_result &res, Degenerate degenerate_windows)
+                        const float *mean, uint64_t w0, const tmb::Exclusion &ex, tm_result &res, Degenerate degenerate_windows)
 {
     cudaStream_t s = L.stream;
     const int T = g.T, nk = g.nk;
@@ -258,7 +267,7 @@ void rescore_and_answer(tm_ctx *ctx, Lane &L, const GroupPlan &g, uint32_t ncand
         TM_CUDA(cudaEventRecord(L.ev2, s));
     TM_CUDA(tmb::launch_rescore(L.cand.as<Candidate>(), ncand, g.tp.as<TemplParam>(), g.q.as<float>(),
                                 g.order.as<int>(), ctx->raw.as<float>(), pv, mean, w0, L.dist.as<float>(),
-                                L.akeys.as<uint32_t>(), L.counters.as<uint32_t>() + 6, s)); // (the keys come later)
+                                L.akeys.as<uint32_t>(), L.counters.as<uint32_t>() + 6, ex, s)); // (the keys come later)
     if (ncand > 0)
         count_launch(L, 2);
     if (L.profile)
@@ -513,7 +522,7 @@ void execute_group(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
     }
 
     std::vector<uint8_t> flags; // fetched only when some kNN bound is unbounded
-    rescore_and_answer(ctx, L, g, ncand, tmb::PrefixView{}, ls.mean.as<float>(), w0, res, [&](int, std::vector<Hit> &degenerate) {
+    rescore_and_answer(ctx, L, g, ncand, tmb::PrefixView{}, ls.mean.as<float>(), w0, exclusion(L, g, nb, blog), res, [&](int, std::vector<Hit> &degenerate) {
         if (flags.empty())
         {
             flags.resize(W);
@@ -813,7 +822,7 @@ void execute_group_mixed(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
     std::vector<uint16_t> run;
     std::vector<float> raw;
     const tmb::PrefixView pv{ctx->prefix.as<double2>(), ctx->ptot.as<double2>(), ctx->pcen.as<double>()};
-    rescore_and_answer(ctx, L, g, ncand, pv, nullptr, w0, res, [&](int t, std::vector<Hit> &degenerate) {
+    rescore_and_answer(ctx, L, g, ncand, pv, nullptr, w0, exclusion(L, g, nb, blog), res, [&](int t, std::vector<Hit> &degenerate) {
         if (run.empty())
         {
             run.resize(W);

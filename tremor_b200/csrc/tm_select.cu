@@ -245,10 +245,21 @@ struct PassB
     const uint16_t *run;
     Candidate *cand;
     uint32_t *cand_count, cand_cap;
+    uint32_t nb;
+    const uint32_t *bmin_l;
+    uint32_t *certain; // the certain minima (below), over the minima of d + E; null: none
 };
 
+// Certain minima. The window v of a 256-window bucket with the smallest d + E is certain to be kept
+// before any window within its template's merge offset when all of those have d - E above it:
+// the bucket's own by the re-pass, the others by their buckets' minima of d - E (those that no
+// list holds are above the bound). Then those windows are in no answer, whatever their
+// exact distances: k_rescore leaves them out (8 templates of 16384, k = 10, merge 8192: 1.03 ->
+// 0.48 ms for the re-scoring, most of it the undecided candidates' chains).
 template <bool MIXED> __global__ void __launch_bounds__(B_THREADS) k_passb(const PassB a)
 {
+    __shared__ uint32_t s_least;
+    __shared__ uint32_t s_where;
     __shared__ __align__(16) float xs[B_XS + ((B_XS + 31) >> 5) * 4];
     __shared__ __align__(16) float qs[B_KC];
     __shared__ float part[B_THREADS / 32][B_WIN];
@@ -264,7 +275,11 @@ template <bool MIXED> __global__ void __launch_bounds__(B_THREADS) k_passb(const
         const uint32_t windows = MIXED ? p.wcount : a.W;
         const uint32_t jb = (item.y << a.bucket_log) + (((uint32_t)unit & ((1u << ulog) - 1u)) << 8);
         if (jb >= windows)
+        {
+            if (a.certain != nullptr && tid == 0)
+                a.certain[(size_t)t * a.nb + item.y] = kNoWindow;
             continue; // past the template's range (uniform)
+        }
         const uint32_t jm = min(jb + B_WIN / 2, windows - 1);
         const float shift = MIXED ? a.x[a.w0 + jm] : a.mean[jm];
         const float *xg = a.x + a.w0 + jb;
@@ -314,18 +329,24 @@ template <bool MIXED> __global__ void __launch_bounds__(B_THREADS) k_passb(const
         const uint32_t tk = a.tkey[t], j = jb + tid;
         const float T = tk == kEmptyKey ? inf_f() : key_float(tk);
         bool hit = false;
+        float lower = inf_f(), upper = inf_f(); // windows that are not searched
         if (MIXED)
         {
             if (j < windows && a.raw[a.w0 + j] != kMissing && a.run[a.w0 + j] < m)
             {
                 WindowStats ws;
                 if (window_prefix_stats(a.pv, a.pv.Q[a.w0 + j], a.pv.Q[a.w0 + j + m], a.w0 + j, m, p.inv_m, ws) != 0)
+                {
                     hit = true; // statistics not trustworthy: always re-scored
+                    lower = -inf_f();
+                }
                 else
                 {
                     float d, e;
                     fast_distance_mixed(p, p.a1_fp32, dot, ws.mu, ws.iv, shift, stats_error(ws, m, p.qs, p.s1), d, e);
-                    hit = d - e <= T;
+                    lower = d - e;
+                    upper = d + e;
+                    hit = lower <= T;
                 }
             }
         }
@@ -333,7 +354,37 @@ template <bool MIXED> __global__ void __launch_bounds__(B_THREADS) k_passb(const
         {
             float d, e;
             fast_distance(p, p.a1_fp32, dot, a.mean[j], a.inv[j], shift, d, e);
-            hit = d - e <= T;
+            lower = d - e;
+            upper = d + e;
+            hit = lower <= T;
+        }
+        if (a.certain != nullptr && p.merge > 0) // uniform
+        {
+            if (tid == 0)
+                s_least = kEmptyKey;
+            __syncthreads();
+            const uint32_t key = upper < inf_f() ? float_key(upper) : kEmptyKey;
+            const uint32_t least_w = __reduce_min_sync(0xffffffffu, key);
+            if (lane == 0)
+                atomicMin(&s_least, least_w);
+            __syncthreads();
+            const uint32_t least = s_least;
+            if (key == least)
+                s_where = j; // one of them; where two are that low, there is no certain one
+            const int near = __syncthreads_count(!(lower > key_float(least))); // a NaN is not above
+            int bad = least == kEmptyKey || least > tk || near != 1 ? 1 : 0;
+            const uint32_t v = s_where;
+            if (bad == 0)
+            {
+                const uint32_t far = (uint32_t)p.merge - 1u;
+                const uint32_t b0 = (v > far ? v - far : 0u) >> 8;
+                const uint32_t b1 = min((uint32_t)(((uint64_t)v + far) >> 8), a.nb - 1);
+                for (uint32_t b = b0 + tid; b <= b1; b += B_THREADS)
+                    bad |= b != item.y && a.bmin_l[(size_t)t * a.nb + b] <= least ? 1 : 0;
+            }
+            bad = __syncthreads_or(bad);
+            if (tid == 0)
+                a.certain[(size_t)t * a.nb + item.y] = bad != 0 ? kNoWindow : v;
         }
         const unsigned ballot = __ballot_sync(0xffffffffu, hit);
         if (ballot != 0u)
@@ -441,6 +492,27 @@ __device__ __forceinline__ bool sums_exact_stats(const float *__restrict__ x, in
     return certain_stats(a + del, em, var, ev / var * 1.01, m, mean_f, std_f);
 }
 
+// Is window w within the merge offset of a certain minimum of a listed bucket (k_passb)? The 16
+// lanes look at the buckets up to 16384 windows away: larger merge offsets exclude less than they
+// could.
+__device__ __forceinline__ bool excluded_window(const Exclusion &x, uint32_t t, uint32_t w, int merge, int lane, unsigned half)
+{
+    const uint32_t far = (uint32_t)min(merge, 16384) - 1u, bound = x.tkey[t];
+    const uint32_t b0 = (w > far ? w - far : 0u) >> 8, b1 = min((uint32_t)(((uint64_t)w + far) >> 8), x.nb - 1);
+    const uint32_t *l = x.bmin_l + (size_t)t * x.nb, *c = x.certain + (size_t)t * x.nb;
+    bool out = false;
+    for (uint32_t b = b0 + lane; b <= b1; b += 16)
+    {
+        const uint32_t key = l[b];
+        if (key != kEmptyKey && key <= bound) // listed
+        {
+            const uint32_t v = c[b];
+            out = out || (v != kNoWindow && v != w && __usad(v, w, 0u) <= far);
+        }
+    }
+    return __any_sync(half, out);
+}
+
 constexpr int R_THREADS = 256;
 
 // PREFIX: statistics from the prefix sums (windows of at most kPrefixBlock samples), else from
@@ -452,7 +524,7 @@ __global__ void __launch_bounds__(R_THREADS) k_rescore(const Candidate *__restri
                                                        const int *__restrict__ order, const float *__restrict__ raw,
                                                        const PrefixView pv, const float *__restrict__ mean, uint64_t w0,
                                                        float *__restrict__ dist, uint32_t *__restrict__ todo,
-                                                       uint32_t *__restrict__ todo_count)
+                                                       uint32_t *__restrict__ todo_count, const Exclusion ex)
 {
     const uint32_t i = blockIdx.x * (R_THREADS / 16) + (threadIdx.x >> 4);
     if (i >= count)
@@ -463,6 +535,12 @@ __global__ void __launch_bounds__(R_THREADS) k_rescore(const Candidate *__restri
     const TemplParam &p = tp[c.templ];
     const uint64_t g = w0 + c.window;
     const int m = p.m;
+    if (ex.nb > 0 && p.mode == TM_MODE_KNN && p.merge > 0 && excluded_window(ex, c.templ, c.window, p.merge, lane, half))
+    {
+        if (lane == 0)
+            dist[i] = kExcluded;
+        return;
+    }
     float mean_f, std_f;
     if (!(PREFIX ? prefix_exact_stats(pv, g, m, p.inv_m, mean_f, std_f)
                  : sums_exact_stats(raw + g, m, (double)mean[c.window], lane, half, mean_f, std_f)))
@@ -633,6 +711,9 @@ cudaError_t launch_passb(const uint2 *list, const uint32_t *counters, uint32_t c
     a.cand = c.cand;
     a.cand_count = c.cand_count;
     a.cand_cap = c.cand_cap;
+    a.nb = c.nb;
+    a.bmin_l = c.bmin_l;
+    a.certain = c.bucket_log == 8 ? c.bmin_u : nullptr; // the bound has been selected
     const unsigned grid = 8u * (unsigned)sms; // resident blocks; the list's length is known on the device only
     if (mixed)
         k_passb<true><<<grid, B_THREADS, 0, s>>>(a);
@@ -646,7 +727,7 @@ cudaError_t launch_passb(const uint2 *list, const uint32_t *counters, uint32_t c
 // todo_count: its counter, zeroed here.
 cudaError_t launch_rescore(const Candidate *cand, uint32_t count, const TemplParam *tp, const float *q,
                            const int *order, const float *raw, const PrefixView &pv, const float *mean, uint64_t w0, float *dist,
-                           uint32_t *todo, uint32_t *todo_count, cudaStream_t s)
+                           uint32_t *todo, uint32_t *todo_count, const Exclusion &ex, cudaStream_t s)
 {
     if (count == 0)
         return cudaSuccess;
@@ -654,9 +735,9 @@ cudaError_t launch_rescore(const Candidate *cand, uint32_t count, const TemplPar
         return e;
     const unsigned grid = (count - 1) / (R_THREADS / 16) + 1;
     if (pv.Q != nullptr)
-        k_rescore<true><<<grid, R_THREADS, 0, s>>>(cand, count, tp, q, order, raw, pv, mean, w0, dist, todo, todo_count);
+        k_rescore<true><<<grid, R_THREADS, 0, s>>>(cand, count, tp, q, order, raw, pv, mean, w0, dist, todo, todo_count, ex);
     else
-        k_rescore<false><<<grid, R_THREADS, 0, s>>>(cand, count, tp, q, order, raw, pv, mean, w0, dist, todo, todo_count);
+        k_rescore<false><<<grid, R_THREADS, 0, s>>>(cand, count, tp, q, order, raw, pv, mean, w0, dist, todo, todo_count, ex);
     const unsigned serial = std::min((count - 1) / S_WARPS + 1, 148u * 4u); // how many are undecided the device knows
     k_rescore_serial<<<serial, S_WARPS * 32, 0, s>>>(cand, tp, q, order, raw, w0, dist, todo, todo_count);
     return cudaGetLastError();
