@@ -17,6 +17,8 @@
 //   radix sort 2       by the new key; the sort is stable, so equal distances stay in
 //                      position order: (distance, position) order within a kNN run
 //   k_answer_segments  each template's run [start, end), its windows and distances
+// Few answers (launch_answer_runs has the rule) take k_answer_runs in place of the sorts, the rekeying
+// and the segments: one block per template gathers its entries and sorts them in shared memory.
 //   k_select_knn       one block per kNN template: the greedy exclusion selection over
 //                      its run (finite distances only), up to k answers
 // The sorts are CUB's device radix sort from the CUDA toolkit, over 32 + ceil(log2 T)
@@ -31,7 +33,7 @@
 namespace tmb {
 
 constexpr int kAnswerThreads = 256;
-constexpr int kSelectThreads = 256;
+constexpr int kSelectThreads = 256, kRunThreads = 512;
 
 __device__ __forceinline__ void warp_slot(bool keep, uint32_t *counter, uint32_t &slot)
 {
@@ -48,11 +50,11 @@ __device__ __forceinline__ void warp_slot(bool keep, uint32_t *counter, uint32_t
     slot = base + (uint32_t)__popc(ballot & ((1u << lane) - 1u));
 }
 
-// kept[0]: answers kept, kept[1]: of which belong to kNN templates.
+// kept[0]: answers kept, kept[1]: of which belong to kNN templates; tcount: by template (or null).
 __global__ void __launch_bounds__(kAnswerThreads)
     k_answer_keys(const Candidate *__restrict__ cand, const float *__restrict__ dist, uint32_t count,
                   const TemplParam *__restrict__ tp, unsigned long long *__restrict__ keys, float *__restrict__ vals,
-                  uint32_t *__restrict__ kept)
+                  uint32_t *__restrict__ kept, uint32_t *__restrict__ tcount)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     bool keep = false, knn = false;
@@ -68,6 +70,12 @@ __global__ void __launch_bounds__(kAnswerThreads)
     uint32_t slot, unused;
     warp_slot(keep, kept, slot);
     warp_slot(keep && knn, kept + 1, unused);
+    if (tcount != nullptr)
+    {
+        const uint32_t same = __match_any_sync(0xffffffffu, keep ? c.templ : 0xffffffffu);
+        if (keep && (int)(threadIdx.x & 31) == __ffs(same) - 1)
+            atomicAdd(&tcount[c.templ], (uint32_t)__popc(same));
+    }
     if (keep)
     {
         keys[slot] = ((unsigned long long)c.templ << 32) | (unsigned long long)c.window;
@@ -119,6 +127,78 @@ __global__ void __launch_bounds__(kAnswerThreads)
         start[t] = i;
     if (i + 1 == count || ((uint32_t)(keys[i + 1] >> 32) & tmask) != t)
         end[t] = i + 1;
+}
+
+// The run of template blockIdx.x: its entries among all that are kept, in (distance, position) order
+// for kNN, by position for a threshold, after the runs of the templates before it, thresholds
+// first. Bound by latency, of the walk over the answers and of the 66 to 78 steps of the bitonic
+// sort: 3300 answers of 16 templates in 15 us, where two radix sorts of five passes, of one
+// block each, and what lay between took 110.
+__global__ void __launch_bounds__(kRunThreads)
+    k_answer_runs(const unsigned long long *__restrict__ keys, const float *__restrict__ vals, uint32_t kept,
+                  const TemplParam *__restrict__ tp, int T, const uint32_t *__restrict__ tcount, uint32_t *__restrict__ start,
+                  uint32_t *__restrict__ end, uint32_t *__restrict__ window, float *__restrict__ dist)
+{
+    extern __shared__ unsigned long long run[];
+    __shared__ uint32_t offset, filled;
+    const int t = blockIdx.x, tid = threadIdx.x;
+    const bool knn = tp[t].mode == TM_MODE_KNN;
+    const uint32_t n = tcount[t];
+    if (tid == 0)
+        offset = filled = 0u;
+    __syncthreads();
+    uint32_t before = 0;
+    for (int i = tid; i < T; i += kRunThreads)
+    {
+        const bool other = tp[i].mode == TM_MODE_KNN;
+        if (other == knn ? i < t : knn)
+            before += tcount[i];
+    }
+    before = __reduce_add_sync(0xffffffffu, before);
+    if ((tid & 31) == 0 && before > 0)
+        atomicAdd(&offset, before);
+    for (uint32_t i = tid; i < kept && n > 0; i += kRunThreads)
+    {
+        const unsigned long long key = keys[i];
+        if ((int)(key >> 32) == t)
+        {
+            const unsigned long long w = (uint32_t)key, d = float_key(vals[i]);
+            run[atomicAdd(&filled, 1u)] = knn ? d << 32 | w : w << 32 | d;
+        }
+    }
+    uint32_t size = 2;
+    while (size < n)
+        size *= 2;
+    for (uint32_t i = n + tid; i < size; i += kRunThreads)
+        run[i] = ~0ull;
+    __syncthreads();
+    for (uint32_t k = 2; k <= size && n > 1; k *= 2)
+        for (uint32_t j = k / 2; j > 0; j /= 2)
+        {
+            for (uint32_t p = tid; p < size / 2; p += kRunThreads)
+            {
+                const uint32_t i = 2 * p - (p & (j - 1)), o = i + j; // bit j of i is clear
+                const unsigned long long a = run[i], b = run[o];
+                if ((a > b) == ((i & k) == 0u))
+                {
+                    run[i] = b;
+                    run[o] = a;
+                }
+            }
+            __syncthreads();
+        }
+    const uint32_t at = offset;
+    for (uint32_t i = tid; i < n; i += kRunThreads)
+    {
+        const uint32_t hi = (uint32_t)(run[i] >> 32), lo = (uint32_t)run[i];
+        window[at + i] = knn ? lo : hi;
+        dist[at + i] = key_float(knn ? hi : lo);
+    }
+    if (tid == 0)
+    {
+        start[t] = n > 0 ? at : 0u;
+        end[t] = n > 0 ? at + n : 0u;
+    }
 }
 
 // Greedy exclusion selection of one kNN template per block over its run in (distance,
@@ -270,11 +350,34 @@ int answer_template_bits(int T)
 }
 
 cudaError_t launch_answer_keys(const Candidate *cand, const float *dist, uint32_t count, const TemplParam *tp,
-                               unsigned long long *keys, float *vals, uint32_t *kept, cudaStream_t s)
+                               unsigned long long *keys, float *vals, uint32_t *kept, uint32_t *tcount, cudaStream_t s)
 {
     if (count > 0)
         k_answer_keys<<<(count + kAnswerThreads - 1) / kAnswerThreads, kAnswerThreads, 0, s>>>(cand, dist, count, tp,
-                                                                                              keys, vals, kept);
+                                                                                              keys, vals, kept, tcount);
+    return cudaGetLastError();
+}
+
+// When few answers are few: at most 4096 of one template, which fit in shared memory (45 us; 58 by
+// radix for thresholds, twice that for kNN), and at most 32768 in all, since each template's block
+// walks over all of them (50000 took 62 us, by radix 66), 2^24 looks by all blocks.
+constexpr uint32_t kRunMost = 4096, kRunAnswers = 32768;
+constexpr uint64_t kRunLooks = 1ull << 24;
+bool answer_runs_apply(uint32_t count, int T, uint32_t most)
+{
+    return most <= kRunMost && count <= kRunAnswers && (uint64_t)count * (uint64_t)T <= kRunLooks;
+}
+
+cudaError_t launch_answer_runs(const unsigned long long *keys, const float *vals, uint32_t count, uint32_t most,
+                               const TemplParam *tp, int T, const uint32_t *tcount, uint32_t *start, uint32_t *end,
+                               uint32_t *window, float *dist, cudaStream_t s)
+{
+    uint32_t size = 2;
+    while (size < most)
+        size *= 2;
+    if (T > 0)
+        k_answer_runs<<<T, kRunThreads, sizeof(unsigned long long) * size, s>>>(keys, vals, count, tp, T, tcount, start, end,
+                                                                               window, dist);
     return cudaGetLastError();
 }
 

@@ -60,7 +60,11 @@ cudaError_t launch_prefix_sums(const float *clean, uint64_t n, const double *cen
                                double2 *block_totals, double2 *Q, cudaStream_t s);
 cudaError_t launch_runs(const float *clean, const float *raw, uint64_t n, uint16_t *run, uint32_t *first, cudaStream_t s);
 cudaError_t launch_answer_keys(const Candidate *cand, const float *dist, uint32_t count, const TemplParam *tp,
-                               unsigned long long *keys, float *vals, uint32_t *kept, cudaStream_t s);
+                               unsigned long long *keys, float *vals, uint32_t *kept, uint32_t *tcount, cudaStream_t s);
+bool answer_runs_apply(uint32_t count, int T, uint32_t most);
+cudaError_t launch_answer_runs(const unsigned long long *keys, const float *vals, uint32_t count, uint32_t most,
+                               const TemplParam *tp, int T, const uint32_t *tcount, uint32_t *start, uint32_t *end,
+                               uint32_t *window, float *dist, cudaStream_t s);
 size_t answer_sort_scratch(uint32_t count, int T);
 cudaError_t launch_answer_order(unsigned long long *const keys[2], float *const vals32[2],
                                 unsigned long long *const vals64[2], uint32_t count, uint32_t knn_count,

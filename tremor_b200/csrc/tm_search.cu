@@ -259,10 +259,14 @@ void rescore_and_answer(tm_ctx *ctx, Lane &L, const GroupPlan &g, uint32_t ncand
     L.avals.reserve(2 * sizeof(float) * cn);
     if (nk > 0)
         L.avals64.reserve(2 * sizeof(unsigned long long) * cn);
-    L.segs.reserve(sizeof(uint32_t) * (2 * static_cast<size_t>(std::max(T, 1)) +
+    L.segs.reserve(sizeof(uint32_t) * (3 * static_cast<size_t>(std::max(T, 1)) +
                                           (device_knn ? static_cast<size_t>(nk) * (1 + 2 * kcap) : 0)));
-    uint32_t *hc = L.h_counters.as<uint32_t>();
     uint32_t *d_kept = L.counters.as<uint32_t>() + 3;
+    uint32_t *d_start = L.segs.as<uint32_t>(), *d_end = d_start + T, *d_tcount = d_end + T;
+    // answers by template, to choose how they are sorted; not counted where there are too many anyway
+    const bool counted = ncand <= (1u << 20);
+    L.h_counters.reserve(sizeof(uint32_t) * (8 + static_cast<size_t>(T)));
+    uint32_t *hc = L.h_counters.as<uint32_t>();
     if (L.profile)
         TM_CUDA(cudaEventRecord(L.ev2, s));
     TM_CUDA(tmb::launch_rescore(L.cand.as<Candidate>(), ncand, g.tp.as<TemplParam>(), g.q.as<float>(),
@@ -277,25 +281,38 @@ void rescore_and_answer(tm_ctx *ctx, Lane &L, const GroupPlan &g, uint32_t ncand
     unsigned long long *vals64[2] = {L.avals64.as<unsigned long long>(),
                                      L.avals64.as<unsigned long long>() + (nk > 0 ? cn : 0)};
     TM_CUDA(cudaMemsetAsync(d_kept, 0, 2 * sizeof(uint32_t), s));
+    if (counted)
+        TM_CUDA(cudaMemsetAsync(d_tcount, 0, sizeof(uint32_t) * T, s));
     TM_CUDA(tmb::launch_answer_keys(L.cand.as<Candidate>(), L.dist.as<float>(), ncand, g.tp.as<TemplParam>(),
-                                    keys[0], vals32[0], d_kept, s));
+                                    keys[0], vals32[0], d_kept, counted ? d_tcount : nullptr, s));
     TM_CUDA(cudaMemcpyAsync(hc + 3, d_kept, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    if (counted)
+        TM_CUDA(cudaMemcpyAsync(hc + 8, d_tcount, sizeof(uint32_t) * T, cudaMemcpyDeviceToHost, s));
     TM_CUDA(cudaStreamSynchronize(s));
     if (ncand > 0)
         count_launch(L);
     const uint32_t kept = hc[3], knn_kept = hc[4], thr_kept = kept - knn_kept;
-    const size_t scratch = tmb::answer_sort_scratch(kept, T);
-    L.sort_tmp.reserve(scratch);
-    uint32_t *d_start = L.segs.as<uint32_t>(), *d_end = d_start + T;
-    uint32_t *d_knn_n = d_end + T, *d_knn_win = d_knn_n + nk;
+    uint32_t *d_knn_n = d_tcount + T, *d_knn_win = d_knn_n + nk;
     float *d_knn_dist = reinterpret_cast<float *>(d_knn_win + static_cast<size_t>(nk) * kcap);
     uint32_t *d_win = reinterpret_cast<uint32_t *>(L.cand.p); // the candidates are consumed: reuse
     float *d_dist = L.dist.as<float>();                       // likewise the re-scored distances
-    TM_CUDA(cudaMemsetAsync(d_start, 0, 2 * sizeof(uint32_t) * T, s));
-    TM_CUDA(tmb::launch_answer_order(keys, vals32, vals64, kept, knn_kept, g.tp.as<TemplParam>(), T, L.sort_tmp.p,
-                                     scratch, d_start, d_end, d_win, d_dist, s));
-    if (kept > 0)
-        count_launch(L, knn_kept > 0 ? 4 : 2); // each radix sort counted as one launch
+    const uint32_t most = counted && T > 0 ? *std::max_element(hc + 8, hc + 8 + T) : 0;
+    if (counted && tmb::answer_runs_apply(kept, T, most))
+    {
+        TM_CUDA(tmb::launch_answer_runs(keys[0], vals32[0], kept, most, g.tp.as<TemplParam>(), T, d_tcount, d_start, d_end,
+                                        d_win, d_dist, s));
+        count_launch(L);
+    }
+    else
+    {
+        const size_t scratch = tmb::answer_sort_scratch(kept, T);
+        L.sort_tmp.reserve(scratch);
+        TM_CUDA(cudaMemsetAsync(d_start, 0, 2 * sizeof(uint32_t) * T, s));
+        TM_CUDA(tmb::launch_answer_order(keys, vals32, vals64, kept, knn_kept, g.tp.as<TemplParam>(), T, L.sort_tmp.p,
+                                         scratch, d_start, d_end, d_win, d_dist, s));
+        if (kept > 0)
+            count_launch(L, knn_kept > 0 ? 4 : 2); // each radix sort counted as one launch
+    }
     if (device_knn)
     {
         TM_CUDA(tmb::launch_select_knn(g.slots.as<int>(), nk, g.tp.as<TemplParam>(), d_start, d_end, d_win, d_dist,
