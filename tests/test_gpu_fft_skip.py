@@ -84,3 +84,20 @@ def test_bounds_from_the_first_pieces(kind):
     for i, ((p, d), (pr, dr)) in enumerate(zip(answers, rows)):
         assert np.array_equal(p, pr) and np.array_equal(d.view(np.uint32), dr.view(np.uint32)), i
     _check(x, reqs[:4], answers[:4])
+
+
+def test_contexts_give_the_bounds_back():
+    """Twelve contexts, each with the bounds of some 40 lengths (10 MB of them), leave no more memory
+    taken than one of them does."""
+    import torch
+    rng = np.random.default_rng(9)
+    x = _record('plain', 1 << 21, rng)
+    reqs = [tb.Request(rng.normal(size=int(64 * 1.1 ** i)).astype(np.float32), tb.MODE_THRESHOLD, correlation=0.9)
+            for i in range(40)]
+    free = []
+    for _ in range(12):
+        with tb.Context(x) as ctx:
+            ctx.set_tiles(tb.TILES_FFT)
+            ctx.scan_batch(reqs)
+        free.append(torch.cuda.mem_get_info()[0])
+    assert free[0] - free[-1] < 10 * (1 << 20)

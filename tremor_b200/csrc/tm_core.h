@@ -293,7 +293,7 @@ struct Lane
         if (stream)
             cudaStreamSynchronize(stream);
         for (DevBuf *b : {&tkey, &bmin_u, &bmin_l, &bmin_s, &list, &counters, &cand, &dist, &fp32_qt, &akeys, &avals, &avals64, &sort_tmp,
-                          &segs, &fft_Y, &fft_stats})
+                          &segs, &fft_Y, &fft_stats, &fft_cuts})
             b->release();
         for (HostBuf *b : {&h_split, &h_q, &h_order, &h_slots, &h_counters})
             b->release();

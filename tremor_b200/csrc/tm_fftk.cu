@@ -12,8 +12,9 @@
 // length allows (fft_class_of): L = 8192 and S = 7168 or 6144 for templates of up to 1025 or
 // 2049 samples, L = 16384 and S = 12288 up to 4097 samples and 8192 above. Two blocks of the
 // shorter pieces share an SM and overlap; at 2049 samples and above the shorter pieces' wasted
-// outputs cost more than that gains (m = 4096: 0.259 ms per template and 2^25 samples with L =
-// 8192, 0.224 with 16384; m = 1024: 0.181 against 0.212). A template longer than 8192 samples
+// outputs cost more than that gains (an item takes 3.44 us per SM with L = 8192 and 8.3 with
+// 16384, windows skipped: m = 4096 0.19 ms per template and 2^25 samples with L = 8192, 0.153
+// with 16384; m = 1024 0.109 against 0.123). A template longer than 8192 samples
 // is cut in two parts whose products are added before the one inverse transform (part 1 meets
 // the next piece, whose start is 8192 samples later):
 //     V[k] = X_p[k] Y_0[k] + X_{p+1}[k] Y_1[k],

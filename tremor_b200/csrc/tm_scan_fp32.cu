@@ -9,7 +9,7 @@
 // tm_epilogue.cuh), so the
 // epilogue can decide, without the reference arithmetic, which windows are certainly
 // out of an answer set: threshold requests emit every window with d - E <= the
-// threshold distance; kNN requests record per 2048-window bucket the smallest d + E
+// threshold distance; kNN requests record per bucket (256 windows or more) the smallest d + E
 // and d - E, from which the kNN bound is selected afterwards (tm_select.cu).
 //
 // Tile: 8 warps per CTA; a warp owns 8 templates and 256 windows, a lane 8 consecutive

@@ -587,7 +587,7 @@ static tm_ctx::FftPieces &ensure_fft(tm_ctx *ctx, Lane &L, int cls)
 }
 
 // The chunks' bounds at the bases of rows [first, first + count), in table; false where the memory
-// for one is not to be had, or it would take a hundredth of what is free: the windows are
+// for one is not to be had, or it would take a 400th of what is free: the windows are
 // then all evaluated.
 static bool ensure_bounds(tm_ctx *ctx, Lane &L, const GroupPlan &g, int first, int count, const float4 **table)
 {
@@ -603,7 +603,7 @@ static bool ensure_bounds(tm_ctx *ctx, Lane &L, const GroupPlan &g, int first, i
             {
                 const size_t need = sizeof(float4) * tmb::fft_chunks(ctx->n);
                 TM_CUDA(cudaMemGetInfo(&free_b, &total_b));
-                if (need > free_b / 100)
+                if (need > free_b / 400)
                     throw Failure{TM_ERR_NO_MEMORY, "bounds of the record's chunks"};
                 ctx->fft_bounds[base].reserve(need);
                 fresh.push_back(base);
