@@ -49,7 +49,8 @@ cudaError_t launch_bucket_select(const uint32_t *bmin_u, uint32_t *sup, uint32_t
 cudaError_t launch_list_buckets(const uint32_t *bmin_l, uint32_t nb, const int *knn_slots, int nk,
                                 const uint32_t *tkey, uint2 *list, uint32_t *counters, uint32_t cap, cudaStream_t s);
 cudaError_t launch_passb(const uint2 *list, const uint32_t *counters, uint32_t cap, const ScanArgs &c, const uint32_t *tkey,
-                         bool mixed, int sms, cudaStream_t s);
+                         bool mixed, const int *knn_slots, int nk, float *lower, uint32_t *bins, float *tight, int sms,
+                         cudaStream_t s);
 cudaError_t launch_rescore(const Candidate *cand, uint32_t count, const TemplParam *tp, const float *q,
                            const int *order, const float *raw, const PrefixView &pv, const float *mean, uint64_t w0, float *dist,
                            uint32_t *todo, uint32_t *todo_count, const Exclusion &ex, cudaStream_t s);
@@ -269,7 +270,7 @@ struct Lane
     HostBuf h_split, h_q, h_order, h_slots, h_counters;
     uint32_t cand_cap = 1u << 22, list_cap = 1u << 20;
     // FFT branch: the template spectra of a launch
-    DevBuf fft_Y, fft_stats, fft_cuts; // (fft_stats: the correlation kernel's per-block statistics cache)
+    DevBuf fft_Y, fft_stats, fft_cuts, lower, bins, tight; // (fft_stats: the correlation kernel's per-block statistics cache)
     // instrumentation
     bool profile = false;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr, ev3 = nullptr, ev4 = nullptr;
@@ -293,7 +294,7 @@ struct Lane
         if (stream)
             cudaStreamSynchronize(stream);
         for (DevBuf *b : {&tkey, &bmin_u, &bmin_l, &bmin_s, &list, &counters, &cand, &dist, &fp32_qt, &akeys, &avals, &avals64, &sort_tmp,
-                          &segs, &fft_Y, &fft_stats, &fft_cuts})
+                          &segs, &fft_Y, &fft_stats, &fft_cuts, &lower, &bins, &tight})
             b->release();
         for (HostBuf *b : {&h_split, &h_q, &h_order, &h_slots, &h_counters})
             b->release();

@@ -29,13 +29,17 @@ inline uint32_t bucket_count(uint64_t windows, int log)
 }
 // Distance given to a kNN candidate that is excluded without one (k_rescore): no candidate has it.
 constexpr float kExcluded = -1.0f;
-// What excludes kNN candidates: the buckets' minima of d - E, the certain minima that k_passb left
-// where those of d + E were, the bounds. nb = 0: nothing does (or the buckets are too large).
+// What excludes kNN candidates. With a merge offset: the buckets' minima of d - E, the certain minima
+// that k_passb left where those of d + E were, the bounds; nb = 0: nothing does (or the buckets are
+// too large). Without: the candidates' d - E and the templates' tight bounds (k_tight_bound), or
+// null.
 struct Exclusion
 {
     const uint32_t *bmin_l, *certain, *tkey;
     uint32_t nb;
+    const float *lower, *tight;
 };
+constexpr int kTightBins = 256; // counts of a template's d + E between 0 and its bound
 constexpr uint32_t kNoWindow = 0xffffffffu;
 constexpr int kStagePad = 16384 + 512; // zero samples after the waveform (template padding)
 

@@ -231,13 +231,28 @@ void add_span(Lane &L, int phase, cudaEvent_t a, cudaEvent_t b)
     L.phase_ms[phase] += ms;
 }
 
-// What k_passb left for the re-scoring of a group's kNN candidates; nothing where the buckets are
-// larger than the re-pass's 256 windows.
+// Has the group kNN templates without a merge offset?
+static bool tight_bounds(const GroupPlan &g)
+{
+    for (int t = 0; t < g.T; t++)
+        if (g.mode[t] == TM_MODE_KNN && g.merge[t] <= 0)
+            return true;
+    return false;
+}
+
+// What k_passb left for the re-scoring of a group's kNN candidates; no certain minima where the
+// buckets are larger than the re-pass's 256 windows.
 static tmb::Exclusion exclusion(const Lane &L, const GroupPlan &g, uint32_t nb, int blog)
 {
-    if (g.nk == 0 || blog != 8)
-        return tmb::Exclusion{};
-    return tmb::Exclusion{L.bmin_l.as<uint32_t>(), L.bmin_u.as<uint32_t>(), L.tkey.as<uint32_t>(), nb};
+    tmb::Exclusion ex{};
+    if (g.nk > 0 && blog == 8)
+        ex = tmb::Exclusion{L.bmin_l.as<uint32_t>(), L.bmin_u.as<uint32_t>(), L.tkey.as<uint32_t>(), nb};
+    if (tight_bounds(g))
+    {
+        ex.lower = L.lower.as<float>();
+        ex.tight = L.tight.as<float>();
+    }
+    return ex;
 }
 
 // Exact re-scoring of a group's ncand candidates (pv: prefix sums of mixed groups, mean: window means of the others), answer order and kNN selection on the
@@ -407,8 +422,17 @@ static uint32_t collect_candidates(tm_ctx *ctx, Lane &L, const GroupPlan &g, con
             L.list.reserve(sizeof(uint2) * static_cast<size_t>(L.list_cap));
             TM_CUDA(tmb::launch_list_buckets(a.bmin_l, a.nb, g.slots.as<int>(), g.nk, L.tkey.as<uint32_t>(), L.list.as<uint2>(),
                                              counters, L.list_cap, s));
-            TM_CUDA(tmb::launch_passb(L.list.as<uint2>(), counters, L.list_cap, a, L.tkey.as<uint32_t>(), mixed, ctx->sms, s));
-            count_launch(L, 2);
+            const bool tight = tight_bounds(g);
+            if (tight)
+            {
+                L.lower.reserve(sizeof(float) * static_cast<size_t>(L.cand_cap));
+                L.bins.reserve(sizeof(uint32_t) * tmb::kTightBins * static_cast<size_t>(g.T));
+                L.tight.reserve(sizeof(float) * static_cast<size_t>(g.T));
+            }
+            TM_CUDA(tmb::launch_passb(L.list.as<uint2>(), counters, L.list_cap, a, L.tkey.as<uint32_t>(), mixed,
+                                      g.slots.as<int>(), g.nk, tight ? L.lower.as<float>() : nullptr,
+                                      tight ? L.bins.as<uint32_t>() : nullptr, L.tight.as<float>(), ctx->sms, s));
+            count_launch(L, tight ? 3 : 2);
         }
         if (L.profile)
             TM_CUDA(cudaEventRecord(L.ev2, s));

@@ -248,6 +248,8 @@ struct PassB
     uint32_t nb;
     const uint32_t *bmin_l;
     uint32_t *certain; // the certain minima (below), over the minima of d + E; null: none
+    float *lower;      // for templates without a merge offset, each candidate's d - E,
+    uint32_t *bins;    //   and counts of d + E (k_tight_bound); null: none has no offset
 };
 
 // Certain minima. The window v of a 256-window bucket with the smallest d + E is certain to be kept
@@ -386,6 +388,9 @@ template <bool MIXED> __global__ void __launch_bounds__(B_THREADS) k_passb(const
             if (tid == 0)
                 a.certain[(size_t)t * a.nb + item.y] = bad != 0 ? kNoWindow : v;
         }
+        if (a.bins != nullptr && p.merge <= 0 && upper <= T && T < inf_f() && T > 0.0f)
+            atomicAdd(&a.bins[(size_t)t * kTightBins + min((int)(fmaxf(upper, 0.0f) * ((float)kTightBins / T)), kTightBins - 1)],
+                      1u);
         const unsigned ballot = __ballot_sync(0xffffffffu, hit);
         if (ballot != 0u)
         {
@@ -394,9 +399,47 @@ template <bool MIXED> __global__ void __launch_bounds__(B_THREADS) k_passb(const
                 base = atomicAdd(a.cand_count, (uint32_t)__popc(ballot));
             base = __shfl_sync(0xffffffffu, base, 0) + (uint32_t)__popc(ballot & ((1u << lane) - 1u));
             if (hit && base < a.cand_cap)
+            {
                 a.cand[base] = Candidate{t, j};
+                if (a.lower != nullptr)
+                    a.lower[base] = lower;
+            }
         }
     }
+}
+
+// Without a merge offset the answers are the k nearest windows, wherever they lie: those of a few
+// events often fill the k that the bound took from as many buckets. tight[t]: a bound that at
+// least k windows of the re-pass have d + E below, from their counts (infinite where there are
+// fewer): no window with d - E above it can be an answer. 128 templates of 4096, k = 100, 2^25
+// samples, 0.7 M candidates: 2.9 -> 0.26 ms for the re-scoring, 0.35 -> 0.07 for the sort.
+__global__ void __launch_bounds__(kTightBins) k_tight_bound(const uint32_t *__restrict__ bins, const TemplParam *__restrict__ tp,
+                                                            const int *__restrict__ knn_slots,
+                                                            const uint32_t *__restrict__ tkey, float *__restrict__ tight)
+{
+    __shared__ uint32_t sums[kTightBins / 32];
+    const int t = knn_slots[blockIdx.x], tid = threadIdx.x, lane = tid & 31;
+    const uint32_t tk = tkey[t];
+    if (tid == 0)
+        tight[t] = inf_f();
+    if (tk == kEmptyKey || tp[t].merge > 0)
+        return; // whole block
+    const uint32_t k = (uint32_t)tp[t].k, mine = bins[(size_t)t * kTightBins + tid];
+    uint32_t incl = mine;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1)
+    {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off)
+            incl += v;
+    }
+    if (lane == 31)
+        sums[tid >> 5] = incl;
+    __syncthreads();
+    for (int w = 0; w < tid >> 5; w++)
+        incl += sums[w];
+    if (incl >= k && incl - mine < k) // one thread at most
+        tight[t] = key_float(tk) * (float)(tid + 1) / (float)kTightBins * (1.0f + 1e-6f);
 }
 
 // ---- exact (reference-arithmetic) distance of every candidate -------------------------
@@ -536,6 +579,12 @@ __global__ void __launch_bounds__(R_THREADS) k_rescore(const Candidate *__restri
     const uint64_t g = w0 + c.window;
     const int m = p.m;
     if (ex.nb > 0 && p.mode == TM_MODE_KNN && p.merge > 0 && excluded_window(ex, c.templ, c.window, p.merge, lane, half))
+    {
+        if (lane == 0)
+            dist[i] = kExcluded;
+        return;
+    }
+    if (ex.tight != nullptr && p.mode == TM_MODE_KNN && p.merge <= 0 && ex.lower[i] > ex.tight[c.templ])
     {
         if (lane == 0)
             dist[i] = kExcluded;
@@ -690,9 +739,15 @@ cudaError_t launch_list_buckets(const uint32_t *bmin_l, uint32_t nb, const int *
 }
 
 cudaError_t launch_passb(const uint2 *list, const uint32_t *counters, uint32_t cap, const ScanArgs &c, const uint32_t *tkey,
-                         bool mixed, int sms, cudaStream_t s)
+                         bool mixed, const int *knn_slots, int nk, float *lower, uint32_t *bins, float *tight, int sms,
+                         cudaStream_t s)
 {
     PassB a{};
+    if (bins != nullptr)
+        if (const cudaError_t e = cudaMemsetAsync(bins, 0, sizeof(uint32_t) * kTightBins * (size_t)c.T, s); e != cudaSuccess)
+            return e;
+    a.lower = lower;
+    a.bins = bins;
     a.list = list;
     a.counters = counters;
     a.cap = cap;
@@ -719,6 +774,8 @@ cudaError_t launch_passb(const uint2 *list, const uint32_t *counters, uint32_t c
         k_passb<true><<<grid, B_THREADS, 0, s>>>(a);
     else
         k_passb<false><<<grid, B_THREADS, 0, s>>>(a);
+    if (bins != nullptr)
+        k_tight_bound<<<nk, kTightBins, 0, s>>>(bins, c.tp, knn_slots, tkey, tight);
     return cudaGetLastError();
 }
 
