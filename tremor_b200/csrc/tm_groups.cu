@@ -505,8 +505,10 @@ size_t plan_fft_split(tm_ctx *ctx, const tm_request *reqs, const std::vector<int
     {
         const tm_request &r = reqs[sorted_idx[f - 1]];
         const uint32_t pieces = tmb::fft_pieces(ctx->n, tmb::fft_class_of(r.m));
-        const bool skips = r.mode != TM_MODE_KNN ||
-                           fft_stage_end(0, pieces, static_cast<int>(n), tmb::fft_class_of(r.m), ctx->sms) < pieces;
+        // as fft_contract decides, were all templates of this one's class
+        const bool skips = static_cast<uint64_t>(pieces) * n >= static_cast<uint64_t>(ctx->sms) &&
+                           (r.mode != TM_MODE_KNN ||
+                            fft_stage_end(0, pieces, static_cast<int>(n), tmb::fft_class_of(r.m), ctx->sms) < pieces);
         fft_cost += fft_time(ctx, r.m, f > 1 && m[f - 2] == r.m, skips);
         const double c = fft_cost + tensor_cost_sorted(ctx, m.data() + f, n - f);
         if (c < best)
