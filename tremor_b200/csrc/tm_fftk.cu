@@ -1163,7 +1163,8 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
                     const double var = fma(-mu_c, mu_c, (qb[j].y - qa[j].y) * inv_m);
                     const float fvar = (float)var, fmu = (float)mu_c;
                     const float mu = fmu + cen;
-                    const bool ok = fvar > fmaxf(fmaf(vb, fabsf(fmu), va), fmaxf(1e-6f * fmu * fmu, 2e-22f)) && fvar < 1e36f;
+                    // vb is NaN where the block's squares pass FLT_MAX: a comparison of its own, false then
+                    const bool ok = fvar >= fmaf(vb, fabsf(fmu), va) && fvar > fmaxf(1e-6f * fmu * fmu, 2e-22f) && fvar < 1e36f;
                     const bool srch = o + 32 * j >= o_lo && o + 32 * j < o_hi && rn[j] < (uint32_t)m;
                     const float v = rsqrtf(fvar), x = mu - shift, r0 = mu * v;
                     const float e = fmaf(kr, fabsf(x * v), k0) + fmaf(kq * r0, r0, fmaf(km, fabsf(mu), kib) * v);
