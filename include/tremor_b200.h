@@ -53,7 +53,8 @@ extern "C" {
 #define TM_ERR_TOO_LARGE (-8) /* input larger than the fixed scratch of tm_window_stats_noalloc */
 
 /* TREMOR_MISSING_VALUE (ZnormSearch.hpp:21): a missing sample counts as 0; a window
- * whose first sample is missing is not searched. */
+ * whose first sample is missing is not searched. A window with a sample that is not finite
+ * is in no answer: its distance is NaN. */
 #define TM_MISSING_VALUE (-100000.0f)
 
 /* query modes, as Tremor::setModeKNN / setModeThreshold (Tremor.hpp:152-153) */

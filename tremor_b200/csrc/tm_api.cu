@@ -146,8 +146,20 @@ int tm_ctx_create(const float *raw, uint64_t n, int device, tm_ctx **out)
         ctx->clean.reserve(sizeof(float) * total);
         TM_CUDA(cudaMemsetAsync(ctx->raw.p, 0, sizeof(float) * total, ctx->main.stream));
         TM_CUDA(cudaMemcpyAsync(ctx->raw.p, raw, sizeof(float) * n, cudaMemcpyHostToDevice, ctx->main.stream));
-        TM_CUDA(tmb::launch_clean(ctx->raw.as<float>(), ctx->clean.as<float>(), n, total, ctx->main.stream));
+        ctx->main.counters.reserve(8 * sizeof(uint32_t));
+        uint32_t *d_odd = ctx->main.counters.as<uint32_t>(), odd = 0;
+        TM_CUDA(cudaMemsetAsync(d_odd, 0, sizeof(uint32_t), ctx->main.stream));
+        TM_CUDA(tmb::launch_clean(ctx->raw.as<float>(), ctx->clean.as<float>(), n, total, d_odd, ctx->main.stream));
+        TM_CUDA(cudaMemcpyAsync(&odd, d_odd, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->main.stream));
         TM_CUDA(cudaStreamSynchronize(ctx->main.stream));
+        if (odd != 0)
+        {
+            ctx->odd.reserve(sizeof(uint32_t) * n);
+            ctx->suf.reserve(sizeof(uint32_t) * tmb::odd_chunks(n)); // scratch
+            TM_CUDA(tmb::launch_odd_next(ctx->raw.as<float>(), n, ctx->suf.as<uint32_t>(), ctx->odd.as<uint32_t>(),
+                                         ctx->main.stream));
+            TM_CUDA(cudaStreamSynchronize(ctx->main.stream));
+        }
     });
     if (rc != TM_OK)
     {
@@ -171,7 +183,7 @@ int tm_ctx_destroy(tm_ctx *ctx)
         kv.second->inv.release();
         kv.second->flags.release();
     }
-    for (DevBuf *b : {&ctx->prefix, &ctx->ptot, &ctx->pcen, &ctx->run, &ctx->raw, &ctx->clean, &ctx->suf,
+    for (DevBuf *b : {&ctx->prefix, &ctx->ptot, &ctx->pcen, &ctx->run, &ctx->raw, &ctx->clean, &ctx->odd, &ctx->suf,
                       &ctx->fft_roots})
         b->release();
     for (tm_ctx::FftPieces &f : ctx->fft)

@@ -35,9 +35,13 @@
 
 
 namespace tmb {
-cudaError_t launch_clean(const float *raw, float *clean, uint64_t n, uint64_t n_total, cudaStream_t s);
-cudaError_t launch_window_stats(const float *clean, const float *raw, uint64_t n, int m, uint64_t w0, uint64_t W,
-                                double2 *suf, float *mean, float *inv, uint8_t *flags, cudaStream_t s);
+cudaError_t launch_clean(const float *raw, float *clean, uint64_t n, uint64_t n_total, uint32_t *odd, cudaStream_t s);
+uint32_t odd_chunks(uint64_t n);
+cudaError_t launch_odd_next(const float *raw, uint64_t n, uint32_t *first, uint32_t *next, cudaStream_t s);
+cudaError_t launch_odd_buckets(uint32_t *bmin_u, uint32_t nb, int blog, const TemplParam *tp, const int *knn_slots, int nk,
+                               const uint32_t *odd, uint64_t w0, uint32_t W, cudaStream_t s);
+cudaError_t launch_window_stats(const float *clean, const float *raw, const uint32_t *odd, uint64_t n, int m, uint64_t w0,
+                                uint64_t W, double2 *suf, float *mean, float *inv, uint8_t *flags, cudaStream_t s);
 cudaError_t launch_reference_stats(const float *raw, int m, uint64_t w0, uint64_t count, float *mean, float *stddev,
                                    cudaStream_t s);
 cudaError_t launch_scan_fp32(const ScanArgs &a, int sms, cudaStream_t s);
@@ -321,6 +325,7 @@ struct tm_ctx
     int device = 0;
     uint64_t n = 0;
     tmh::DevBuf raw, clean;
+    tmh::DevBuf odd; // distances to the next sample that is not finite; empty where all are
     uint64_t range_first = 0, range_count = UINT64_MAX;
     int kernel = TM_KERNEL_AUTO;
     int tiles = TM_TILES_AUTO;

@@ -36,6 +36,7 @@ struct ScanArgs
     const double2 *PT;     //   their block totals
     const double *PC;      //   and block centres
     const uint16_t *run;   // constant-run lengths
+    const uint32_t *odd;   // distances to the next sample that is not finite; null where all are
     const TileInfo *tiles; // mixed lengths: per tile, its K blocks
     int k_stride;          // row stride of the template arrays
     uint64_t n;            // samples of the waveform (P has n + 1 entries)

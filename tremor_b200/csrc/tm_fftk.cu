@@ -1012,7 +1012,8 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
             for (int j = 0; j < 4; j++)
             {
                 const float cross = (dl[16 * c + 4 * j] - ms[j] * s1) * iv[j];
-                d[j] = c_lin - 2.0f * cross;
+                // at most FLT_MAX, not NaN: d - e is -inf where ew is inf, whatever the dot product
+                d[j] = fminf(c_lin - 2.0f * cross, kFltMax);
                 const float e = ew[j] + a3 * fmaxf(d[j], 0.0f);
                 lo[j] = d[j] - e;
                 lmin = fminf(lmin, lo[j]);

@@ -41,10 +41,11 @@ struct Exclusion
 };
 constexpr int kTightBins = 256; // counts of a template's d + E between 0 and its bound
 constexpr uint32_t kNoWindow = 0xffffffffu;
+constexpr uint32_t kNoOdd = 0xffffffffu; // no sample that is not finite follows (launch_odd_next)
 constexpr int kStagePad = 16384 + 512; // zero samples after the waveform (template padding)
 
 // per-window flags (one byte per window and length)
-constexpr uint8_t kFlagMissingStart = 1; // first sample missing: not searched
+constexpr uint8_t kFlagNotSearched = 1;  // first sample missing, or a sample that is not finite
 constexpr uint8_t kFlagDegenerate = 2;   // reference std <= 1e-12: distance FLT_MAX
 constexpr uint8_t kFlagNeedsExact = 4;   // prefix-sum statistics not trusted: two-pass fix-up
 constexpr uint8_t kFlagExact = 8;        // statistics are the reference's two-pass values

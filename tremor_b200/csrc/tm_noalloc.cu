@@ -78,7 +78,7 @@ __device__ __forceinline__ void finish(const float *__restrict__ raw, uint64_t j
     {
         mean[j] = 0.0f;
         stddev[j] = 0.0f;
-        flags[j] = kFlagMissingStart;
+        flags[j] = kFlagNotSearched;
         return;
     }
     const double mu = s / (double)m;

@@ -44,7 +44,7 @@ LengthStats &ensure_length(tm_ctx *ctx, Lane &L, int m)
         ls->flags.reserve(W + 64);
         const uint64_t a_count = (w0 + W - 1) / m - w0 / m + 1;
         ctx->suf.reserve(a_count * static_cast<uint64_t>(m) * sizeof(double2));
-        TM_CUDA(tmb::launch_window_stats(ctx->clean.as<float>(), ctx->raw.as<float>(), ctx->n, m, w0, W,
+        TM_CUDA(tmb::launch_window_stats(ctx->clean.as<float>(), ctx->raw.as<float>(), ctx->odd.as<uint32_t>(), ctx->n, m, w0, W,
                                         ctx->suf.as<double2>(), ls->mean.as<float>(), ls->inv.as<float>(),
                                         ls->flags.as<uint8_t>(), L.stream));
         count_launch(L, 3);
@@ -399,6 +399,16 @@ static bool super_buckets(const GroupPlan &g, int blog)
     return false;
 }
 
+// The contraction kernels of several lengths see samples that are not finite as 0: minima that may be
+// those of windows with such a sample must not bound the answers.
+static void forget_odd_buckets(Lane &L, const GroupPlan &g, const tmb::ScanArgs &a)
+{
+    if (a.odd == nullptr || g.nk == 0)
+        return;
+    TM_CUDA(tmb::launch_odd_buckets(a.bmin_u, a.nb, a.bucket_log, a.tp, g.slots.as<int>(), g.nk, a.odd, a.w0, a.W, L.stream));
+    count_launch(L);
+}
+
 // kNN bound, bucket list and FP32 re-pass after a group's contraction (a: its arguments), then
 // the counters: the group's candidates, whether the contraction gave up waiting. One wait for
 // the device; a list that did not fit is made again, larger.
@@ -411,6 +421,7 @@ static uint32_t collect_candidates(tm_ctx *ctx, Lane &L, const GroupPlan &g, con
         const bool super = super_buckets(g, a.bucket_log);
         if (super)
             L.bmin_s.reserve(sizeof(uint32_t) * static_cast<size_t>(g.nk) * a.nb);
+        forget_odd_buckets(L, g, a);
         TM_CUDA(tmb::launch_bucket_select(a.bmin_u, L.bmin_s.as<uint32_t>(), a.nb, a.bucket_log, a.tp, g.slots.as<int>(), g.nk,
                                           super, L.tkey.as<uint32_t>(), s));
         count_launch(L, super ? 2 : 1);
@@ -570,7 +581,7 @@ void execute_group(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
             TM_CUDA(cudaMemcpy(flags.data(), ls.flags.p, W, cudaMemcpyDeviceToHost));
         }
         for (uint64_t j = 0; j < W; j++)
-            if ((flags[j] & tmb::kFlagDegenerate) && !(flags[j] & tmb::kFlagMissingStart))
+            if ((flags[j] & tmb::kFlagDegenerate) && !(flags[j] & tmb::kFlagNotSearched))
                 degenerate.push_back(Hit{w0 + j, FLT_MAX});
     });
 }
@@ -751,6 +762,7 @@ void fft_contract(tm_ctx *ctx, Lane &L, const GroupPlan &g, const tmb::ScanArgs 
                 if (super)
                     L.bmin_s.reserve(sizeof(uint32_t) * static_cast<size_t>(g.nk) * a.nb);
                 L.fft_cuts.reserve(sizeof(float) * static_cast<size_t>(nr));
+                forget_odd_buckets(L, g, a);
                 TM_CUDA(tmb::launch_fft_cuts(f.rows, nr, a.bmin_u, L.bmin_s.as<uint32_t>(), a.nb, nb_seen, a.bucket_log, a.tp,
                                              g.slots.as<int>(), g.nk, super, L.fft_cuts.as<float>(), s));
                 count_launch(L, super ? 2 : 1);
@@ -829,6 +841,7 @@ void execute_group_mixed(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
         a.PT = ctx->ptot.as<double2>();
         a.PC = ctx->pcen.as<double>();
         a.run = ctx->run.as<uint16_t>();
+        a.odd = ctx->odd.as<uint32_t>();
         a.tiles = g.d_tiles.as<tmb::TileInfo>();
         a.k_stride = g.k_stride;
         a.n = ctx->n;
@@ -863,6 +876,7 @@ void execute_group_mixed(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
     }
     std::vector<uint16_t> run;
     std::vector<float> raw;
+    std::vector<uint32_t> odd; // stays empty where all samples are finite
     const tmb::PrefixView pv{ctx->prefix.as<double2>(), ctx->ptot.as<double2>(), ctx->pcen.as<double>()};
     rescore_and_answer(ctx, L, g, ncand, pv, nullptr, w0, exclusion(L, g, nb, blog), res, [&](int t, std::vector<Hit> &degenerate) {
         if (run.empty())
@@ -871,10 +885,15 @@ void execute_group_mixed(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
             raw.resize(W);
             TM_CUDA(cudaMemcpy(run.data(), ctx->run.as<uint16_t>() + w0, W * sizeof(uint16_t), cudaMemcpyDeviceToHost));
             TM_CUDA(cudaMemcpy(raw.data(), ctx->raw.as<float>() + w0, W * sizeof(float), cudaMemcpyDeviceToHost));
+            if (ctx->odd.p != nullptr)
+            {
+                odd.resize(W);
+                TM_CUDA(cudaMemcpy(odd.data(), ctx->odd.as<uint32_t>() + w0, W * sizeof(uint32_t), cudaMemcpyDeviceToHost));
+            }
         }
         const TemplParam &p = g.htp[t];
         for (uint64_t j = 0; j < p.wcount; j++)
-            if (run[j] >= p.m && raw[j] != TM_MISSING_VALUE)
+            if (run[j] >= p.m && raw[j] != TM_MISSING_VALUE && (odd.empty() || odd[j] >= static_cast<uint32_t>(p.m)))
                 degenerate.push_back(Hit{w0 + j, FLT_MAX});
     });
 }

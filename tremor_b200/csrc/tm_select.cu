@@ -189,6 +189,23 @@ __global__ void __launch_bounds__(1024) k_bucket_select(const uint32_t *__restri
     }
 }
 
+// The minima of d + E of buckets with a window that has a sample that is not finite (odd:
+// launch_odd_next) are taken out: one such window may have given them.
+__global__ void k_odd_buckets(uint32_t *__restrict__ bmin_u, uint32_t nb, int blog, const TemplParam *__restrict__ tp,
+                              const int *__restrict__ knn_slots, int nk, const uint32_t *__restrict__ odd, uint64_t w0,
+                              uint32_t W)
+{
+    const uint32_t used = (W - 1 >> blog) + 1; // the rest of a row is padding
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < (uint64_t)nk * used;
+         i += (uint64_t)gridDim.x * blockDim.x)
+    {
+        const int t = knn_slots[i / used];
+        const uint32_t b = (uint32_t)(i % used);
+        if (odd[w0 + ((uint64_t)b << blog)] < (uint32_t)tp[t].m + (1u << blog) - 1u)
+            bmin_u[(size_t)t * nb + b] = kEmptyKey;
+    }
+}
+
 // (template slot, bucket) pairs whose minimum of d - E is within the bound. counters: [0]
 // candidates so far, kept in [5] for a list that has to be made again; [1] the list's length.
 __global__ void k_list_buckets(const uint32_t *__restrict__ bmin_l, uint32_t nb, const int *__restrict__ knn_slots,
@@ -243,6 +260,7 @@ struct PassB
     const float *raw;        // several lengths: statistics from the prefix sums
     PrefixView pv;
     const uint16_t *run;
+    const uint32_t *odd; // several lengths, a record with samples that are not finite; else null
     Candidate *cand;
     uint32_t *cand_count, cand_cap;
     uint32_t nb;
@@ -334,7 +352,8 @@ template <bool MIXED> __global__ void __launch_bounds__(B_THREADS) k_passb(const
         float lower = inf_f(), upper = inf_f(); // windows that are not searched
         if (MIXED)
         {
-            if (j < windows && a.raw[a.w0 + j] != kMissing && a.run[a.w0 + j] < m)
+            if (j < windows && a.raw[a.w0 + j] != kMissing && a.run[a.w0 + j] < m &&
+                (a.odd == nullptr || a.odd[a.w0 + j] >= (uint32_t)m))
             {
                 WindowStats ws;
                 if (window_prefix_stats(a.pv, a.pv.Q[a.w0 + j], a.pv.Q[a.w0 + j + m], a.w0 + j, m, p.inv_m, ws) != 0)
@@ -730,6 +749,13 @@ cudaError_t launch_fft_cuts(const FftRow *rows, int nrows, const uint32_t *bmin_
     return cudaGetLastError();
 }
 
+cudaError_t launch_odd_buckets(uint32_t *bmin_u, uint32_t nb, int blog, const TemplParam *tp, const int *knn_slots, int nk,
+                               const uint32_t *odd, uint64_t w0, uint32_t W, cudaStream_t s)
+{
+    k_odd_buckets<<<1184, 256, 0, s>>>(bmin_u, nb, blog, tp, knn_slots, nk, odd, w0, W);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_list_buckets(const uint32_t *bmin_l, uint32_t nb, const int *knn_slots, int nk,
                                 const uint32_t *tkey, uint2 *list, uint32_t *counters, uint32_t cap, cudaStream_t s)
 {
@@ -763,6 +789,7 @@ cudaError_t launch_passb(const uint2 *list, const uint32_t *counters, uint32_t c
     a.raw = c.raw;
     a.pv = PrefixView{c.P, c.PT, c.PC};
     a.run = c.run;
+    a.odd = c.odd;
     a.cand = c.cand;
     a.cand_count = c.cand_count;
     a.cand_cap = c.cand_cap;

@@ -20,14 +20,105 @@
 
 namespace tmb {
 
-__global__ void k_clean(const float *__restrict__ raw, float *__restrict__ clean, uint64_t n, uint64_t n_total)
+// The record as the contractions and sums read it: 0 for missing samples, and for those that are not
+// finite, of which one would make every sum, transform and tile that it enters not finite too.
+// *odd is set where there is one of the latter.
+__global__ void k_clean(const float *__restrict__ raw, float *__restrict__ clean, uint64_t n, uint64_t n_total,
+                        uint32_t *__restrict__ odd)
 {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n_total;
          i += (uint64_t)gridDim.x * blockDim.x)
     {
         float v = i < n ? raw[i] : 0.0f;
+        if (!isfinite(v))
+        {
+            v = 0.0f;
+            *odd = 1u;
+        }
         clean[i] = v == kMissing ? 0.0f : v;
     }
+}
+
+// Only for a record with samples that are not finite: next[i], the distance from sample i to the
+// first of them at or after it (kNoOdd: none). A window whose next[start] is below its length has
+// one. The reference's distance of such a window is NaN, so that it is in no answer. Pass 1 finds
+// each chunk's first, pass 2 a sample's next in its chunk, else the first of the chunks after.
+constexpr int O_THREADS = 1024, O_PER = 8, O_CHUNK = O_THREADS * O_PER;
+
+__device__ __forceinline__ uint32_t odd_first(const float *__restrict__ raw, uint64_t n, uint64_t base)
+{
+    for (int k = 0; k < O_PER; k++)
+        if (base + k < n && !isfinite(raw[base + k]))
+            return (uint32_t)k;
+    return kNoOdd;
+}
+
+__global__ void __launch_bounds__(O_THREADS) k_odd_first(const float *__restrict__ raw, uint64_t n, uint32_t *__restrict__ first)
+{
+    __shared__ uint32_t best;
+    if (threadIdx.x == 0)
+        best = kNoOdd;
+    __syncthreads();
+    const uint32_t off = threadIdx.x * O_PER, f = odd_first(raw, n, (uint64_t)blockIdx.x * O_CHUNK + off);
+    if (f != kNoOdd)
+        atomicMin(&best, off + f);
+    __syncthreads();
+    if (threadIdx.x == 0)
+        first[blockIdx.x] = best;
+}
+
+__global__ void __launch_bounds__(O_THREADS) k_odd_next(const float *__restrict__ raw, uint64_t n,
+                                                        const uint32_t *__restrict__ first, uint32_t chunks,
+                                                        uint32_t *__restrict__ next)
+{
+    __shared__ uint32_t from[O_THREADS]; // the first at or after thread t's samples, in the chunk
+    __shared__ unsigned long long after; // the first of the chunks after
+    const int t = threadIdx.x;
+    const uint32_t off = t * O_PER;
+    const uint64_t base = (uint64_t)blockIdx.x * O_CHUNK + off;
+    const uint32_t mine = odd_first(raw, n, base);
+    from[t] = mine == kNoOdd ? kNoOdd : off + mine;
+    if (t == 0)
+        after = ~0ull;
+    __syncthreads();
+    for (int d = 1; d < O_THREADS; d <<= 1)
+    {
+        const uint32_t v = t + d < O_THREADS ? from[t + d] : kNoOdd;
+        __syncthreads();
+        from[t] = min(from[t], v);
+        __syncthreads();
+    }
+    for (uint32_t c0 = blockIdx.x + 1; c0 < chunks; c0 += O_THREADS)
+    {
+        const uint32_t c = c0 + t, f = c < chunks ? first[c] : kNoOdd;
+        if (f != kNoOdd)
+            atomicMin(&after, (unsigned long long)c * O_CHUNK + f);
+        if (__syncthreads_or(f != kNoOdd))
+            break;
+    }
+    __syncthreads();
+    const uint32_t later = t + 1 < O_THREADS ? from[t + 1] : kNoOdd;
+    unsigned long long at = later != kNoOdd ? (unsigned long long)blockIdx.x * O_CHUNK + later : after;
+    for (int k = O_PER - 1; k >= 0; k--)
+        if (base + k < n)
+        {
+            if (!isfinite(raw[base + k]))
+                at = base + k;
+            next[base + k] = at == ~0ull ? kNoOdd : (uint32_t)min(at - (base + k), (unsigned long long)kNoOdd - 1);
+        }
+}
+
+// Windows with a sample that is not finite are not searched; their means stay those of the clean
+// record, which may serve as a tile's shift.
+__global__ void k_odd_windows(const uint32_t *__restrict__ next, int m, uint64_t w0, uint64_t W, float *__restrict__ inv,
+                              uint8_t *__restrict__ flags)
+{
+    for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < W; r += (uint64_t)gridDim.x * blockDim.x)
+        if (next[w0 + r] < (uint32_t)m)
+        {
+            inv[r] = 0.0f;
+            flags[r] = kFlagNotSearched;
+        }
 }
 
 // One warp per segment [a*m, (a+1)*m) ∩ [0, n): suffix sums of (x, x^2) in FP64.
@@ -77,7 +168,7 @@ __device__ __forceinline__ void finalize_window(uint64_t j, uint64_t w0, int m, 
     {
         mean[r] = 0.0f;
         inv[r] = 0.0f;
-        flags[r] = kFlagMissingStart;
+        flags[r] = kFlagNotSearched;
         return;
     }
     const double mu = s / (double)m;
@@ -196,15 +287,27 @@ __global__ void k_reference_stats(const float *__restrict__ raw, int m, uint64_t
 
 // ---- launchers --------------------------------------------------------------------
 
-cudaError_t launch_clean(const float *raw, float *clean, uint64_t n, uint64_t n_total, cudaStream_t s)
+// odd: zeroed before; set where a sample is not finite.
+cudaError_t launch_clean(const float *raw, float *clean, uint64_t n, uint64_t n_total, uint32_t *odd, cudaStream_t s)
 {
-    k_clean<<<1184, 256, 0, s>>>(raw, clean, n, n_total);
+    k_clean<<<1184, 256, 0, s>>>(raw, clean, n, n_total, odd);
     return cudaGetLastError();
 }
 
-// suf must hold (a_count * m) double2.
-cudaError_t launch_window_stats(const float *clean, const float *raw, uint64_t n, int m, uint64_t w0, uint64_t W,
-                                double2 *suf, float *mean, float *inv, uint8_t *flags, cudaStream_t s)
+uint32_t odd_chunks(uint64_t n) { return (uint32_t)((n + O_CHUNK - 1) / O_CHUNK); }
+
+// next: n entries; first: scratch of odd_chunks(n).
+cudaError_t launch_odd_next(const float *raw, uint64_t n, uint32_t *first, uint32_t *next, cudaStream_t s)
+{
+    const uint32_t chunks = odd_chunks(n);
+    k_odd_first<<<chunks, O_THREADS, 0, s>>>(raw, n, first);
+    k_odd_next<<<chunks, O_THREADS, 0, s>>>(raw, n, first, chunks, next);
+    return cudaGetLastError();
+}
+
+// suf must hold (a_count * m) double2. odd: launch_odd_next's distances, or null.
+cudaError_t launch_window_stats(const float *clean, const float *raw, const uint32_t *odd, uint64_t n, int m, uint64_t w0,
+                                uint64_t W, double2 *suf, float *mean, float *inv, uint8_t *flags, cudaStream_t s)
 {
     const uint64_t a_lo = w0 / (uint64_t)m;
     const uint64_t a_hi = (w0 + W - 1) / (uint64_t)m;
@@ -215,6 +318,8 @@ cudaError_t launch_window_stats(const float *clean, const float *raw, uint64_t n
     const double r2max = 5e-7 / ((double)m * 1.1102230246251565e-16);
     k_window_stats<<<(unsigned)blocks, threads, 0, s>>>(clean, raw, suf, n, m, a_lo, a_count, w0, W, mean, inv, flags,
                                                         r2max);
+    if (odd != nullptr)
+        k_odd_windows<<<1184, 256, 0, s>>>(odd, m, w0, W, inv, flags);
     k_exact_stats<<<1184, 256, 0, s>>>(raw, m, w0, W, mean, inv, flags);
     return cudaGetLastError();
 }
