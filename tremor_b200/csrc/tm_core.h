@@ -408,6 +408,13 @@ template <class F> inline int guarded(tm_ctx *ctx, F body)
     }
 }
 
+// Windows of a length in the context's range.
+inline uint64_t windows_in_range(const tm_ctx *ctx, int m)
+{
+    const uint64_t total = ctx->n - static_cast<uint64_t>(m) + 1, w0 = ctx->range_first;
+    return w0 >= total ? 0 : std::min<uint64_t>(ctx->range_count, total - w0);
+}
+
 inline void count_launch(Lane &L, int k = 1) { L.all_launches += k; }
 
 // One group of same-length requests of a batch, prepared on the host and resident on
@@ -420,6 +427,7 @@ struct GroupPlan
     std::vector<int> index; // request index of each slot
     std::vector<int> mode, k, merge;
     std::vector<float> thr; // threshold distance per slot
+    std::vector<char> inert; // templates that are not finite, padding on the device
     std::vector<TemplParam> htp;
     DevBuf q, order, tp, slots, q_hi, q_lo;
     int t_rows = 0;

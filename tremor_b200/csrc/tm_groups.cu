@@ -29,6 +29,18 @@ void fill_param(TemplParam &p, int m, double q2, double s1, double gamma_main, d
 double gamma_fp32(int m) { return 1.01 * static_cast<double>((m + 63) & ~63) * kU; }
 double gamma_bf16(int m) { return 1.2e-5 + (3.0 * ((m + 63) & ~63) / 16.0 + 16.0) * 2.384185791015625e-07; }
 
+// A z-normalised template with a value that is not finite has a finite distance to no window, and on
+// the device it is 0, with the constants of padding: the kernels bound a window's error for all
+// templates of a tile or length at once. finish_answers has what is left of its answer.
+static bool make_inert(GroupPlan &g, int t, float *q, TemplParam &p)
+{
+    std::fill(q, q + p.m, 0.0f);
+    fill_param(p, p.m, 0.0, 0.0, 0.0, 0.0);
+    p.mode = TM_MODE_THRESHOLD;
+    p.thr_ed = g.thr[t] = -FLT_MAX;
+    return g.inert[t] = true;
+}
+
 // Host preparation of one group (bit-identical template z-normalisation and block
 // order, epilogue constants) and its upload.
 void prepare_group(tm_ctx *ctx, Lane &L, int m, const std::vector<int> &idx, const tm_request *reqs, GroupPlan &g,
@@ -59,6 +71,7 @@ void prepare_group(tm_ctx *ctx, Lane &L, int m, const std::vector<int> &idx, con
     g.merge.assign(T, 0);
     g.thr.assign(T, 0.0f);
     g.a1_umma.assign(T, 0.0f);
+    g.inert.assign(T, 0);
     g.nk = 0;
     for (int t = 0; t < T; t++)
     {
@@ -83,7 +96,9 @@ void prepare_group(tm_ctx *ctx, Lane &L, int m, const std::vector<int> &idx, con
         p.merge = g.merge[t] = r->merge_offset;
         p.q_offset = static_cast<int64_t>(t) * m_pad;
         p.order_offset = static_cast<int64_t>(t) * nblk;
-        if (r->mode == TM_MODE_KNN)
+        if (!std::isfinite(q2) && make_inert(g, t, q, p))
+            g.a1_umma[t] = 0.0f;
+        else if (r->mode == TM_MODE_KNN)
             hslots[g.nk++] = t;
         else
             p.thr_ed = g.thr[t] = tm_host::cc_to_ed(r->correlation, m);
@@ -207,13 +222,9 @@ void prepare_group_mixed(tm_ctx *ctx, Lane &L, const std::vector<int> &idx_in, c
     g.merge.assign(R, 0);
     g.thr.assign(R, -FLT_MAX);
     g.a1_umma.assign(R, 0.0f);
+    g.inert.assign(R, 0);
     g.nk = 0;
     g.w_max = 0;
-    const uint64_t w0 = ctx->range_first;
-    auto wcount_of = [&](int m) {
-        const uint64_t total = ctx->n - static_cast<uint64_t>(m) + 1;
-        return static_cast<uint32_t>(w0 >= total ? 0 : std::min<uint64_t>(ctx->range_count, total - w0));
-    };
     uint64_t samples = 0;
     for (int t = 0; t < R; t++)
     {
@@ -241,27 +252,32 @@ void prepare_group_mixed(tm_ctx *ctx, Lane &L, const std::vector<int> &idx_in, c
             q2 += static_cast<double>(q[i]) * q[i];
             s1 += q[i];
         }
-        for (int i = 0; i < m && !fft; i++)
-        {
-            const size_t at = q_at[t] + static_cast<size_t>(i);
-            hh[at] = bf16_bits(q[i]);
-            hl[at] = bf16_bits(q[i] - bf16_value(hh[at]));
-        }
         fill_param(p, m, q2, s1, gamma_bf16(m), gamma_fp32(m));
         g.a1_umma[t] = p.a1_main;
         p.inv_m = 1.0 / static_cast<double>(m);
         p.qs = static_cast<float>(std::sqrt(q2 * m));
-        p.wcount = wcount_of(m);
+        p.wcount = static_cast<uint32_t>(windows_in_range(ctx, m));
         g.w_max = std::max(g.w_max, p.wcount);
         p.mode = g.mode[t] = r->mode;
         p.k = g.k[t] = r->k;
         p.merge = g.merge[t] = r->merge_offset;
         p.q_offset = static_cast<int64_t>(q_at[t]);
         p.order_offset = static_cast<int64_t>(o_at[t]);
-        if (r->mode == TM_MODE_KNN)
+        if (!std::isfinite(q2) && make_inert(g, t, q, p))
+        {
+            g.a1_umma[t] = p.qs = 0.0f;
+            p.wcount = 0;
+        }
+        else if (r->mode == TM_MODE_KNN)
             hslots[g.nk++] = t;
         else
             p.thr_ed = g.thr[t] = tm_host::cc_to_ed(r->correlation, m);
+        for (int i = 0; i < m && !fft; i++)
+        {
+            const size_t at = q_at[t] + static_cast<size_t>(i);
+            hh[at] = bf16_bits(q[i]);
+            hl[at] = bf16_bits(q[i] - bf16_value(hh[at]));
+        }
     }
     g.tiles = tiles;
     cudaStream_t s = L.stream;

@@ -153,7 +153,8 @@ void finish_answers(Lane &L, const GroupPlan &g, const AnswerView &v, uint64_t w
     for (int t = 0; t < g.T; t++)
     {
         const bool knn = g.mode[t] == TM_MODE_KNN;
-        slot += knn ? 1 : 0;
+        const bool inert = g.inert[t] != 0; // has no run and no slot: only constant windows can be answers
+        slot += knn && !inert ? 1 : 0;
         if (g.index[t] < 0)
             continue; // padding row of a mixed-length tile
         Answer &out = res.answers[g.index[t]];
@@ -184,8 +185,8 @@ void finish_answers(Lane &L, const GroupPlan &g, const AnswerView &v, uint64_t w
             continue;
         }
         std::vector<Hit> kept;
-        const bool unbounded = v.tkey[t] == tmb::kEmptyKey;
-        if (v.device_knn && (static_cast<int>(v.knn_n[slot]) >= g.k[t] || !unbounded))
+        const bool unbounded = inert || v.tkey[t] == tmb::kEmptyKey;
+        if (v.device_knn && !inert && (static_cast<int>(v.knn_n[slot]) >= g.k[t] || !unbounded))
         {
             const size_t at = static_cast<size_t>(slot) * v.kcap;
             for (uint32_t i = 0; i < v.knn_n[slot]; i++)
@@ -892,7 +893,8 @@ void execute_group_mixed(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
             }
         }
         const TemplParam &p = g.htp[t];
-        for (uint64_t j = 0; j < p.wcount; j++)
+        const uint64_t windows = windows_in_range(ctx, p.m);
+        for (uint64_t j = 0; j < windows; j++)
             if (run[j] >= p.m && raw[j] != TM_MISSING_VALUE && (odd.empty() || odd[j] >= static_cast<uint32_t>(p.m)))
                 degenerate.push_back(Hit{w0 + j, FLT_MAX});
     });
