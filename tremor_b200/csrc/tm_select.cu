@@ -127,23 +127,26 @@ __device__ __forceinline__ int select_slot(const int *slots, int nk, const FftRo
 
 // Minima over super-buckets of ceil(merge / bucket) buckets, for the templates whose merge
 // offset exceeds a bucket: sup[slot][i], i < ceil(nb_seen / buckets per super-bucket); nb buckets
-// per template, of which the first nb_seen are looked at.
+// per template, of which the first nb_seen are looked at. count: the rows, or the nk slots.
 __global__ void k_super_buckets(const uint32_t *__restrict__ bmin_u, uint32_t nb, uint32_t nb_seen, int blog,
                                 const TemplParam *__restrict__ tp, const int *__restrict__ knn_slots, int nk,
-                                const FftRow *__restrict__ rows, uint32_t *__restrict__ sup)
+                                const FftRow *__restrict__ rows, int count, uint32_t *__restrict__ sup)
 {
-    const int t = select_template(knn_slots, rows, blockIdx.y), merge = tp[t].merge;
-    const uint32_t sb = (uint32_t)(((int64_t)merge + (1 << blog) - 1) >> blog);
-    if (sb < 2 || tp[t].mode != TM_MODE_KNN)
-        return;
-    const uint32_t *u = bmin_u + (size_t)t * nb;
-    sup += (size_t)select_slot(knn_slots, nk, rows, blockIdx.y) * nb_seen;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < (nb_seen + sb - 1) / sb; i += gridDim.x * blockDim.x)
+    for (int r = blockIdx.y; r < count; r += gridDim.y)
     {
-        uint32_t best = kEmptyKey;
-        for (uint32_t b = i * sb; b < min((i + 1) * sb, nb_seen); b++)
-            best = min(best, u[b]);
-        sup[i] = best;
+        const int t = select_template(knn_slots, rows, r), merge = tp[t].merge;
+        const uint32_t sb = (uint32_t)(((int64_t)merge + (1 << blog) - 1) >> blog);
+        if (sb < 2 || tp[t].mode != TM_MODE_KNN)
+            continue;
+        const uint32_t *u = bmin_u + (size_t)t * nb;
+        uint32_t *s = sup + (size_t)select_slot(knn_slots, nk, rows, r) * nb_seen;
+        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < (nb_seen + sb - 1) / sb; i += gridDim.x * blockDim.x)
+        {
+            uint32_t best = kEmptyKey;
+            for (uint32_t b = i * sb; b < min((i + 1) * sb, nb_seen); b++)
+                best = min(best, u[b]);
+            s[i] = best;
+        }
     }
 }
 
@@ -208,27 +211,30 @@ __global__ void k_odd_buckets(uint32_t *__restrict__ bmin_u, uint32_t nb, int bl
 
 // (template slot, bucket) pairs whose minimum of d - E is within the bound. counters: [0]
 // candidates so far, kept in [5] for a list that has to be made again; [1] the list's length.
-__global__ void k_list_buckets(const uint32_t *__restrict__ bmin_l, uint32_t nb, const int *__restrict__ knn_slots,
+__global__ void k_list_buckets(const uint32_t *__restrict__ bmin_l, uint32_t nb, const int *__restrict__ knn_slots, int nk,
                                const uint32_t *__restrict__ tkey, uint2 *__restrict__ list, uint32_t *__restrict__ counters,
                                uint32_t cap)
 {
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
         counters[5] = counters[0];
-    const int t = knn_slots[blockIdx.y];
-    const uint32_t bound = tkey[t];
-    const uint4 *row = reinterpret_cast<const uint4 *>(bmin_l + (size_t)t * nb); // nb is a multiple of 4
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nb / 4; i += gridDim.x * blockDim.x)
+    for (int s = blockIdx.y; s < nk; s += gridDim.y)
     {
-        const uint4 v = row[i];
-        const uint32_t l[4] = {v.x, v.y, v.z, v.w};
+        const int t = knn_slots[s];
+        const uint32_t bound = tkey[t];
+        const uint4 *row = reinterpret_cast<const uint4 *>(bmin_l + (size_t)t * nb); // nb is a multiple of 4
+        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nb / 4; i += gridDim.x * blockDim.x)
+        {
+            const uint4 v = row[i];
+            const uint32_t l[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int k = 0; k < 4; k++)
-            if (l[k] != kEmptyKey && l[k] <= bound)
-            {
-                const uint32_t at = atomicAdd(&counters[1], 1u);
-                if (at < cap)
-                    list[at] = make_uint2((uint32_t)t, 4 * i + k);
-            }
+            for (int k = 0; k < 4; k++)
+                if (l[k] != kEmptyKey && l[k] <= bound)
+                {
+                    const uint32_t at = atomicAdd(&counters[1], 1u);
+                    if (at < cap)
+                        list[at] = make_uint2((uint32_t)t, 4 * i + k);
+                }
+        }
     }
 }
 
@@ -725,6 +731,9 @@ __global__ void __launch_bounds__(S_WARPS * 32) k_rescore_serial(const Candidate
 
 // ---- launchers --------------------------------------------------------------------
 
+// Templates side by side in a grid, whose y extent is limited; the kernels take the rest in turn.
+static unsigned grid_rows(int count) { return (unsigned)std::min(count, 32768); }
+
 // sup: scratch of nk x nb keys (used by templates whose merge offset exceeds a bucket).
 cudaError_t launch_bucket_select(const uint32_t *bmin_u, uint32_t *sup, uint32_t nb, int blog, const TemplParam *tp,
                                  const int *knn_slots, int nk, bool super, uint32_t *tkey, cudaStream_t s)
@@ -732,8 +741,8 @@ cudaError_t launch_bucket_select(const uint32_t *bmin_u, uint32_t *sup, uint32_t
     const FftRow *rows = nullptr;
     float *cuts = nullptr;
     if (super)
-        k_super_buckets<<<dim3(std::min(nb / 256 + 1, 64u), (unsigned)nk), 256, 0, s>>>(bmin_u, nb, nb, blog, tp, knn_slots, nk,
-                                                                                        rows, sup);
+        k_super_buckets<<<dim3(std::min(nb / 256 + 1, 64u), grid_rows(nk)), 256, 0, s>>>(bmin_u, nb, nb, blog, tp, knn_slots, nk,
+                                                                                         rows, nk, sup);
     k_bucket_select<<<nk, 1024, 0, s>>>(bmin_u, sup, nb, nb, blog, tp, knn_slots, nk, rows, tkey, cuts);
     return cudaGetLastError();
 }
@@ -743,8 +752,8 @@ cudaError_t launch_fft_cuts(const FftRow *rows, int nrows, const uint32_t *bmin_
 {
     uint32_t *tkey = nullptr;
     if (super)
-        k_super_buckets<<<dim3(std::min(nb_seen / 256 + 1, 64u), (unsigned)nrows), 256, 0, s>>>(bmin_u, nb, nb_seen, blog, tp,
-                                                                                                slots, nk, rows, sup);
+        k_super_buckets<<<dim3(std::min(nb_seen / 256 + 1, 64u), grid_rows(nrows)), 256, 0, s>>>(bmin_u, nb, nb_seen, blog, tp,
+                                                                                                 slots, nk, rows, nrows, sup);
     k_bucket_select<<<nrows, 1024, 0, s>>>(bmin_u, sup, nb, nb_seen, blog, tp, slots, nk, rows, tkey, cuts);
     return cudaGetLastError();
 }
@@ -759,8 +768,8 @@ cudaError_t launch_odd_buckets(uint32_t *bmin_u, uint32_t nb, int blog, const Te
 cudaError_t launch_list_buckets(const uint32_t *bmin_l, uint32_t nb, const int *knn_slots, int nk,
                                 const uint32_t *tkey, uint2 *list, uint32_t *counters, uint32_t cap, cudaStream_t s)
 {
-    k_list_buckets<<<dim3(std::min(nb / 1024 + 1, 64u), (unsigned)nk), 256, 0, s>>>(bmin_l, nb, knn_slots, tkey, list, counters,
-                                                                                   cap);
+    k_list_buckets<<<dim3(std::min(nb / 1024 + 1, 64u), grid_rows(nk)), 256, 0, s>>>(bmin_l, nb, knn_slots, nk, tkey, list,
+                                                                                    counters, cap);
     return cudaGetLastError();
 }
 
