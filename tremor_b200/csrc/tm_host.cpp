@@ -11,11 +11,15 @@
 
 namespace tm_host {
 
-// A second copy of a function for processors with FMA, chosen when the library is
+// A second copy of a function for x86 processors with FMA, chosen when the library is
 // loaded: std::fma is a call otherwise. The results are the same. Normalising and ordering a
 // template took 11 ns per sample with the calls and one chain of a block's energy at a time,
 // 2.9 so.
+#if defined(__x86_64__)
 #define TM_WITH_FMA __attribute__((target_clones("fma", "default")))
+#else // other hosts have fused multiply-adds throughout
+#define TM_WITH_FMA
+#endif
 
 float cc_to_ed(float cc, int m) { return 2.0f * static_cast<float>(m) * (1.0f - cc); } // ZnormSearch.hpp:23-26
 
