@@ -23,7 +23,9 @@ static void bound_diagnostics_wm(tm_ctx *ctx, int m, const std::vector<int> &idx
     cudaStream_t s = L.stream;
     const int count = static_cast<int>(idx.size());
     ensure_prefix(ctx, L);
-    GroupPlan g;
+    tm_batch one; // gives its group's buffers back
+    one.groups.resize(1);
+    GroupPlan &g = one.groups[0];
     uint64_t h2d = 0;
     prepare_group_mixed(ctx, L, idx, reqs.data(), g, h2d, plan_col_tile(ctx, reqs.data(), idx), false);
     const uint64_t W = g.w_max;
@@ -33,7 +35,7 @@ static void bound_diagnostics_wm(tm_ctx *ctx, int m, const std::vector<int> &idx
         g.htp[t].thr_ed = -FLT_MAX; // emit nothing
     TM_CUDA(cudaMemcpyAsync(g.tp.p, g.htp.data(), sizeof(TemplParam) * g.T, cudaMemcpyHostToDevice, s));
     const size_t pairs = W * static_cast<size_t>(count);
-    DevBuf dd, de, dc, dx, todo;
+    ScopedBuf dd, de, dc, dx, todo;
     dd.reserve(pairs * sizeof(float));
     de.reserve(pairs * sizeof(float));
     L.counters.reserve(8 * sizeof(uint32_t));
@@ -106,7 +108,6 @@ static void bound_diagnostics_wm(tm_ctx *ctx, int m, const std::vector<int> &idx
     uint32_t err = 0;
     TM_CUDA(cudaMemcpyAsync(&err, L.counters.as<uint32_t>() + 2, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     TM_CUDA(cudaStreamSynchronize(s));
-    g.release();
     if (err != 0)
         throw Failure{TM_ERR_TIMEOUT, "contraction kernel gave up waiting"};
 }
@@ -379,7 +380,7 @@ int tm_window_stats(tm_ctx *ctx, int m, uint64_t first, uint64_t count, float *m
         return TM_OK;
     return guarded(ctx, [&] {
         TM_CUDA(cudaSetDevice(ctx->device));
-        DevBuf dm, ds;
+        ScopedBuf dm, ds;
         dm.reserve(count * sizeof(float));
         ds.reserve(count * sizeof(float));
         TM_CUDA(tmb::launch_reference_stats(ctx->raw.as<float>(), m, first, count, dm.as<float>(), ds.as<float>(),
@@ -388,8 +389,6 @@ int tm_window_stats(tm_ctx *ctx, int m, uint64_t first, uint64_t count, float *m
         TM_CUDA(cudaMemcpyAsync(mean, dm.p, count * sizeof(float), cudaMemcpyDeviceToHost, ctx->main.stream));
         TM_CUDA(cudaMemcpyAsync(stddev, ds.p, count * sizeof(float), cudaMemcpyDeviceToHost, ctx->main.stream));
         TM_CUDA(cudaStreamSynchronize(ctx->main.stream));
-        dm.release();
-        ds.release();
     });
 }
 
@@ -614,7 +613,9 @@ int tm_bound_diagnostics(tm_ctx *ctx, const float *queries, int count, int m, fl
             bound_diagnostics_wm(ctx, m, idx, reqs, d, e, exact);
             return;
         }
-        GroupPlan g;
+        tm_batch one; // gives its group's buffers back
+        one.groups.resize(1);
+        GroupPlan &g = one.groups[0];
         uint64_t h2d = 0;
         prepare_group(ctx, ctx->main, m, idx, reqs.data(), g, h2d);
         LengthStats &ls = ensure_length(ctx, ctx->main, m);
@@ -631,7 +632,7 @@ int tm_bound_diagnostics(tm_ctx *ctx, const float *queries, int count, int m, fl
         cudaStream_t s = ctx->main.stream;
         TM_CUDA(cudaMemcpyAsync(g.tp.p, g.htp.data(), sizeof(TemplParam) * g.T_pad, cudaMemcpyHostToDevice, s));
         const size_t pairs = W * static_cast<size_t>(count);
-        DevBuf dd, de, dc;
+        ScopedBuf dd, de, dc, dx, todo;
         dd.reserve(pairs * sizeof(float));
         de.reserve(pairs * sizeof(float));
         ctx->main.counters.reserve(8 * sizeof(uint32_t));
@@ -676,7 +677,6 @@ int tm_bound_diagnostics(tm_ctx *ctx, const float *queries, int count, int m, fl
                 for (uint64_t j = 0; j < W; j++)
                     all[static_cast<size_t>(t) * W + j] = Candidate{static_cast<uint32_t>(t), static_cast<uint32_t>(j)};
             dc.reserve(pairs * sizeof(Candidate));
-            DevBuf dx, todo;
             dx.reserve(pairs * sizeof(float));
             todo.reserve(pairs * sizeof(uint32_t));
             TM_CUDA(cudaMemcpyAsync(dc.p, all.data(), pairs * sizeof(Candidate), cudaMemcpyHostToDevice, s));
@@ -686,16 +686,10 @@ int tm_bound_diagnostics(tm_ctx *ctx, const float *queries, int count, int m, fl
             count_launch(ctx->main);
             TM_CUDA(cudaMemcpyAsync(exact, dx.p, pairs * sizeof(float), cudaMemcpyDeviceToHost, s));
             TM_CUDA(cudaStreamSynchronize(s));
-            dx.release();
-            todo.release();
         }
         uint32_t err = 0;
         TM_CUDA(cudaMemcpyAsync(&err, ctx->main.counters.as<uint32_t>() + 2, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
         TM_CUDA(cudaStreamSynchronize(s));
-        dd.release();
-        de.release();
-        dc.release();
-        g.release();
         if (err != 0)
             throw Failure{TM_ERR_TIMEOUT, "contraction kernel gave up waiting"};
     });

@@ -153,6 +153,15 @@ struct DevBuf
     }
 };
 
+// A device buffer of one call, given back where that ends, by a failure too.
+struct ScopedBuf : DevBuf
+{
+    ScopedBuf() = default;
+    ScopedBuf(const ScopedBuf &) = delete;
+    ScopedBuf &operator=(const ScopedBuf &) = delete;
+    ~ScopedBuf() { release(); }
+};
+
 // Grow-only pinned host buffer.
 struct HostBuf
 {

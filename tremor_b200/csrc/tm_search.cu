@@ -73,7 +73,7 @@ void ensure_prefix(tm_ctx *ctx, Lane &L)
     ctx->pcen.reserve(sizeof(double) * (blocks + 1));
     TM_CUDA(cudaMemsetAsync(ctx->ptot.p, 0, sizeof(double2) * (blocks + 1), s));
     ctx->run.reserve(sizeof(uint16_t) * n);
-    DevBuf totals, run_first;
+    ScopedBuf totals, run_first;
     totals.reserve(sizeof(double2) * chunks);
     run_first.reserve(sizeof(uint32_t) * chunks);
     // centres: the mean of each block, from uncentred chunk sums
@@ -99,8 +99,6 @@ void ensure_prefix(tm_ctx *ctx, Lane &L)
                              run_first.as<uint32_t>(), s));
     TM_CUDA(cudaStreamSynchronize(s));
     count_launch(L, 4 + 2);
-    totals.release();
-    run_first.release();
     ctx->prefix_ready = true;
 }
 
