@@ -1,0 +1,55 @@
+"""Searches with little device memory left: what does not fit is done in less, with the same answers."""
+import numpy as np
+import pytest
+
+import tremor_b200 as tb
+
+pytestmark = pytest.mark.gpu
+
+
+class _Taken:
+    """All but `left` bytes of the device's free memory."""
+
+    def __init__(self, left):
+        import torch
+        torch.cuda.synchronize()
+        self.hold = [torch.empty(max(0, torch.cuda.mem_get_info()[0] - left), dtype=torch.uint8, device='cuda')]
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
+        import torch
+        self.hold.clear()
+        torch.cuda.empty_cache()
+
+
+def _record(n):
+    from tremor_b200 import synth
+    rng = np.random.default_rng(n)
+    return synth.ar2_waveform(n, rng), rng
+
+
+def _same(got, want):
+    for i, ((p0, d0), (p1, d1)) in enumerate(zip(got, want)):
+        assert np.array_equal(p0, p1) and np.array_equal(d0.view(np.uint32), d1.view(np.uint32)), i
+
+
+@pytest.mark.parametrize('tiles', [tb.TILES_AUTO, tb.TILES_FFT])
+def test_spectra_of_fewer_classes(tiles):
+    """2^24 samples: the prefix sums take 302 MB, spectra of the four classes 154, 180, 179 and 268 MB: with
+    room for 0.8 of 900 MB the longest pieces serve every template."""
+    x, rng = _record(1 << 24)
+    reqs = [tb.Request(rng.normal(size=m).astype(np.float32), tb.MODE_KNN, k=3, merge_offset=m // 2)
+            for m in (700, 1900, 3900, 8000, 12000)]
+    with tb.Context(x) as ctx:
+        ctx.set_tiles(tiles)
+        want = ctx.scan_batch(reqs)
+    with tb.Context(x) as ctx:
+        ctx.set_tiles(tiles)
+        ctx.profile_enable(True)
+        with _Taken(900 << 20):
+            got = ctx.scan_batch(reqs)
+        assert ctx.profile_read()[0] == 'fft'
+        _same(got, want)
+        _same(ctx.scan_batch(reqs), want)  # with memory again, and one class resident

@@ -78,7 +78,7 @@ static void bound_diagnostics_wm(tm_ctx *ctx, int m, const std::vector<int> &idx
     a.col_tile = g.col_tile;
     if (ctx->tiles == TM_TILES_FFT)
     {
-        prepare_fft(ctx, L, g);
+        prepare_fft(ctx, L, g, FftClasses());
         fft_contract(ctx, L, g, a);
     }
     else

@@ -499,10 +499,16 @@ void prepare_group(tm_ctx *ctx, Lane &L, int m, const std::vector<int> &idx, con
                    uint64_t &h2d, int col_tile = 0);
 void prepare_group_mixed(tm_ctx *ctx, Lane &L, const std::vector<int> &idx_in, const tm_request *reqs, GroupPlan &g,
                          uint64_t &h2d, int col_tile, bool fft);
-void prepare_fft(tm_ctx *ctx, Lane &L, GroupPlan &g);
+// Class of pieces that takes the templates of each (fft_class_of), itself or a longer one.
+struct FftClasses
+{
+    int use[tmb::kFftClasses] = {0, 1, 2, 3};
+    int of(int m) const { return use[tmb::fft_class_of(m)]; }
+};
+void prepare_fft(tm_ctx *ctx, Lane &L, GroupPlan &g, const FftClasses &classes);
 int plan_col_tile(const tm_ctx *ctx, const tm_request *reqs, const std::vector<int> &idx, double *cost = nullptr);
 double tile_time(const tm_ctx *ctx, bool mixed, int v, double k);
-double fft_time(const tm_ctx *ctx, int m, bool shared, bool skips);
+double fft_time(const tm_ctx *ctx, int m, int cls, bool shared, bool skips);
 uint32_t fft_stage_end(uint32_t p0, uint32_t pieces, int rows, int cls, int sms);
 void create_batch(tm_ctx *ctx, Lane &L, const tm_request *requests, int count, tm_batch &b, bool serving = false);
 

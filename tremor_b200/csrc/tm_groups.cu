@@ -307,7 +307,7 @@ void prepare_group_mixed(tm_ctx *ctx, Lane &L, const std::vector<int> &idx_in, c
 // Makes a prepared mixed-length group one of the FFT branch: its rows with windows, sorted by
 // length as they are, in sets of one class and number of parts, and what the correlation
 // kernel needs per row.
-void prepare_fft(tm_ctx *ctx, Lane &L, GroupPlan &g)
+void prepare_fft(tm_ctx *ctx, Lane &L, GroupPlan &g, const FftClasses &classes)
 {
     g.fft = true;
     g.fft_sets.clear();
@@ -319,7 +319,7 @@ void prepare_fft(tm_ctx *ctx, Lane &L, GroupPlan &g)
         const TemplParam &p = g.htp[static_cast<size_t>(t)];
         if (g.index[t] < 0 || p.wcount == 0)
             continue;
-        const int cls = tmb::fft_class_of(p.m), parts = tmb::fft_parts(p.m, cls);
+        const int cls = classes.of(p.m), parts = tmb::fft_parts(p.m, cls);
         const int step = static_cast<int>(tmb::fft_class(cls).step);
         if (g.fft_sets.empty() || g.fft_sets.back().cls != cls || g.fft_sets.back().parts != parts)
             g.fft_sets.push_back(GroupPlan::FftSet{cls, parts, static_cast<int>(g.fft_rows.size()), 0});
@@ -360,7 +360,7 @@ void prepare_fft(tm_ctx *ctx, Lane &L, GroupPlan &g)
         }
     for (tmb::FftRow &r : g.fft_rows)
     {
-        r.e_norm = tmb::fft_e_norm(r.qs, r.m, tmb::fft_class_of(r.m));
+        r.e_norm = tmb::fft_e_norm(r.qs, r.m, classes.of(r.m));
         r.inv_a3 = r.a3 < 0.5f ? (1.0f / (1.0f - r.a3)) * 1.000001f : HUGE_VALF;
     }
     if (!g.fft_rows.empty())
@@ -458,74 +458,86 @@ double tensor_cost_sorted(const tm_ctx *ctx, const int *m, size_t n)
     return best;
 }
 
-// Modelled milliseconds of the FFT branch per template of length m per 2^25 samples. shared: a
+// Modelled milliseconds of the FFT branch per template of length m, in pieces of class cls, per 2^25
+// samples. shared: a
 // template of the same length precedes it, whose window statistics it takes; skips: it has a
 // cut, so that it need not evaluate most windows (tm_fftk.cu). The time depends on the length
 // through the pieces' step alone, and within a class little on it; the factors are the classes'
 // times over that of a template that evaluates all its windows at 4096 (0.307 ms) or 16000
 // (0.63 ms): 0.247, 0.275, 0.307, 0.43 ms at 1000, 2000, 4096, 8192; shared 0.171, 0.168, 0.208,
 // 0.326, and 0.43 at 16384; skipping 0.109, 0.127, 0.153, 0.231, and 0.33 at 16000.
-double fft_time(const tm_ctx *ctx, int m, bool shared, bool skips)
+double fft_time(const tm_ctx *ctx, int m, int cls, bool shared, bool skips)
 {
     static const double all[tmb::kFftClasses] = {0.81, 0.90, 1.0, 1.41};
     static const double same[tmb::kFftClasses] = {0.55, 0.55, 0.66, 1.04};
     static const double skip[tmb::kFftClasses] = {0.36, 0.42, 0.50, 0.75};
-    const int cls = tmb::fft_class_of(m);
     if (tmb::fft_parts(m, cls) > 1)
         return ctx->fft_long_ms * (skips ? 0.53 : shared ? 0.69 : 1.0);
     return ctx->fft_ms * (skips ? skip[cls] : shared ? same[cls] : all[cls]);
 }
 
-// Device memory that the FFT branch's resident arrays for these lengths would still take
-// (prefix sums, runs, the classes' spectra).
-static size_t fft_missing_bytes(tm_ctx *ctx, const std::vector<int> &m)
+// Classes for templates of these lengths: each its own (9 to 16 bytes of spectra per sample and class,
+// and the prefix sums) where what is not resident yet takes at most 0.8 of the free memory; else
+// those that are not resident share a longer one, resident or the longest of them, whose pieces
+// serve every shorter template. False where that is too much as well.
+static bool fft_classes(tm_ctx *ctx, const std::vector<int> &m, FftClasses &classes)
 {
     std::lock_guard<std::mutex> lk(ctx->fft_mu);
-    size_t need = ctx->prefix_ready ? 0 : 18 * static_cast<size_t>(ctx->n);
-    bool counted[tmb::kFftClasses] = {};
+    bool wanted[tmb::kFftClasses] = {};
     for (int len : m)
-    {
-        const int cls = tmb::fft_class_of(len);
-        if (!ctx->fft[cls].ready && !counted[cls])
-            need += sizeof(double2) * static_cast<size_t>(tmb::fft_pieces(ctx->n, cls)) *
-                    tmb::fft_pitch(tmb::fft_class(cls).n);
-        counted[cls] = true;
-    }
-    return need;
+        wanted[tmb::fft_class_of(len)] = true;
+    const auto missing = [&](const FftClasses &c) {
+        size_t need = ctx->prefix_ready ? 0 : 18 * static_cast<size_t>(ctx->n);
+        bool counted[tmb::kFftClasses] = {};
+        for (int i = 0; i < tmb::kFftClasses; i++)
+        {
+            const int cls = c.use[i];
+            if (wanted[i] && !ctx->fft[cls].ready && !counted[cls])
+                need += sizeof(double2) * static_cast<size_t>(tmb::fft_pieces(ctx->n, cls)) *
+                        tmb::fft_pitch(tmb::fft_class(cls).n);
+            counted[cls] = counted[cls] || wanted[i];
+        }
+        return need;
+    };
+    classes = FftClasses();
+    const size_t need = missing(classes);
+    if (need == 0)
+        return true;
+    size_t free_b = 0, total_b = 0;
+    TM_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    const size_t room = free_b / 10 * 8;
+    if (need <= room)
+        return true;
+    FftClasses fewer;
+    int shared = -1; // from the longest down
+    for (int i = tmb::kFftClasses - 1; i >= 0; i--)
+        if (ctx->fft[i].ready)
+            shared = i;
+        else if (wanted[i])
+            shared = fewer.use[i] = shared < 0 ? i : shared;
+    if (missing(fewer) > room)
+        return false;
+    classes = fewer;
+    return true;
 }
 
-// How many of a group's templates (ordered longest first) go to the FFT branch: all of
-// them when it is forced (TM_TILES_FFT); under TM_TILES_AUTO with the automatic kernel,
-// the f minimising the FFT's time of f templates + the tensor cost of the other
-// templates: the longest templates set a tile's K extent, so moving a few of them to the
-// FFT (whose cost does not grow with the length) can shorten every tile they would have
-// padded. Lengths up to 16384 (the FFT pieces' step); otherwise none.
-size_t plan_fft_split(tm_ctx *ctx, const tm_request *reqs, const std::vector<int> &sorted_idx)
+// The f of the least modelled time (plan_fft_split), pieces by these classes; m: the lengths.
+static size_t cheapest_split(const tm_ctx *ctx, const tm_request *reqs, const std::vector<int> &sorted_idx,
+                             const std::vector<int> &m, const FftClasses &classes)
 {
-    const size_t n = sorted_idx.size();
-    if (n == 0 || ctx->kernel == TM_KERNEL_FP32 || !tmb::umma_supported(0, 0, 0))
-        return 0;
-    for (int i : sorted_idx)
-        if (reqs[i].m > tmb::kFftMaxM)
-            return 0;
-    if (ctx->tiles == TM_TILES_FFT)
-        return n;
-    if (ctx->tiles != TM_TILES_AUTO || ctx->kernel != TM_KERNEL_AUTO)
-        return 0;
-    std::vector<int> m(n);
-    for (size_t i = 0; i < n; i++)
-        m[i] = reqs[sorted_idx[i]].m;
+    const size_t n = m.size();
     size_t best_f = 0;
     double best = tensor_cost_sorted(ctx, m.data(), n), fft_cost = 0.0;
     for (size_t f = 1; f <= n; f++)
     {
         const tm_request &r = reqs[sorted_idx[f - 1]];
-        const uint32_t pieces = tmb::fft_pieces(ctx->n, tmb::fft_class_of(r.m));
+        const int cls = classes.of(r.m);
+        const uint32_t pieces = tmb::fft_pieces(ctx->n, cls);
         // as fft_contract decides, were all templates of this one's class
         const bool skips = static_cast<uint64_t>(pieces) * n >= static_cast<uint64_t>(ctx->sms) &&
                            (r.mode != TM_MODE_KNN ||
-                            fft_stage_end(0, pieces, static_cast<int>(n), tmb::fft_class_of(r.m), ctx->sms) < pieces);
-        fft_cost += fft_time(ctx, r.m, f > 1 && m[f - 2] == r.m, skips);
+                            fft_stage_end(0, pieces, static_cast<int>(n), cls, ctx->sms) < pieces);
+        fft_cost += fft_time(ctx, r.m, cls, f > 1 && m[f - 2] == r.m, skips);
         const double c = fft_cost + tensor_cost_sorted(ctx, m.data() + f, n - f);
         if (c < best)
         {
@@ -533,16 +545,46 @@ size_t plan_fft_split(tm_ctx *ctx, const tm_request *reqs, const std::vector<int
             best_f = f;
         }
     }
-    // a record too large for the branch's arrays beside its other ones is left to the tiles
-    if (best_f > 0)
-        if (const size_t need = fft_missing_bytes(ctx, std::vector<int>(m.begin(), m.begin() + best_f)); need > 0)
-        {
-            size_t free_b = 0, total_b = 0;
-            TM_CUDA(cudaMemGetInfo(&free_b, &total_b));
-            if (need > free_b / 10 * 8)
-                return 0;
-        }
     return best_f;
+}
+
+// How many of a group's templates (ordered longest first) go to the FFT branch: all of
+// them when it is forced (TM_TILES_FFT); under TM_TILES_AUTO with the automatic kernel,
+// the f minimising the FFT's time of f templates + the tensor cost of the other
+// templates: the longest templates set a tile's K extent, so moving a few of them to the
+// FFT (whose cost does not grow with the length) can shorten every tile they would have
+// padded. Lengths up to 16384 (kFftMaxM); otherwise none. classes: those of their pieces.
+size_t plan_fft_split(tm_ctx *ctx, const tm_request *reqs, const std::vector<int> &sorted_idx, FftClasses &classes)
+{
+    const size_t n = sorted_idx.size();
+    if (n == 0 || ctx->kernel == TM_KERNEL_FP32 || !tmb::umma_supported(0, 0, 0))
+        return 0;
+    for (int i : sorted_idx)
+        if (reqs[i].m > tmb::kFftMaxM)
+            return 0;
+    std::vector<int> m(n);
+    for (size_t i = 0; i < n; i++)
+        m[i] = reqs[sorted_idx[i]].m;
+    if (ctx->tiles == TM_TILES_FFT)
+    {
+        fft_classes(ctx, m, classes);
+        return n;
+    }
+    if (ctx->tiles != TM_TILES_AUTO || ctx->kernel != TM_KERNEL_AUTO)
+        return 0;
+    // pieces of other classes where memory is short, at another time; a record too large for the
+    // branch's arrays beside its other ones is left to the tiles
+    size_t f = 0;
+    for (int attempt = 0; attempt < 3; attempt++)
+    {
+        const FftClasses priced = classes;
+        f = cheapest_split(ctx, reqs, sorted_idx, m, priced);
+        if (f == 0 || !fft_classes(ctx, std::vector<int>(m.begin(), m.begin() + f), classes))
+            return 0;
+        if (std::equal(priced.use, priced.use + tmb::kFftClasses, classes.use))
+            break;
+    }
+    return f;
 }
 
 // Groups of a batch. Lengths with a full 128-template tile (or any length, on the FP32
@@ -581,14 +623,16 @@ void create_batch(tm_ctx *ctx, Lane &L, const tm_request *requests, int count, t
     {
         std::vector<int> idx;
         int kind; // 0: one length, per-length statistics; 1: prefix statistics, tiles; 2: FFT branch
+        FftClasses classes{};
     };
     std::vector<Spec> specs;
     for (std::vector<int> &list : lists)
     {
         std::stable_sort(list.begin(), list.end(), [&](int a, int c) { return requests[a].m > requests[c].m; });
-        const size_t f = tensor ? plan_fft_split(ctx, requests, list) : 0;
+        FftClasses classes;
+        const size_t f = tensor ? plan_fft_split(ctx, requests, list, classes) : 0;
         if (f > 0)
-            specs.push_back(Spec{std::vector<int>(list.begin(), list.begin() + f), 2});
+            specs.push_back(Spec{std::vector<int>(list.begin(), list.begin() + f), 2, classes});
         if (f < list.size())
         {
             std::vector<int> part(list.begin() + f, list.end());
@@ -607,7 +651,7 @@ void create_batch(tm_ctx *ctx, Lane &L, const tm_request *requests, int count, t
         if (specs[gi].kind == 2)
         {
             prepare_group_mixed(ctx, L, idx, requests, g, b.h2d_bytes, 0, true);
-            prepare_fft(ctx, L, g);
+            prepare_fft(ctx, L, g, specs[gi].classes);
         }
         else if (specs[gi].kind == 0)
             prepare_group(ctx, L, m, idx, requests, g, b.h2d_bytes,

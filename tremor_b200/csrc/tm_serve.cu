@@ -70,7 +70,7 @@ static uint64_t serve_bytes(const tm_ctx *ctx, const tm_request &r)
 static double serve_cost(const tm_ctx *ctx, const tm_request &r)
 {
     const double scale = static_cast<double>(ctx->n - static_cast<uint64_t>(r.m) + 1) / 33554432.0;
-    const double fft = fft_time(ctx, r.m, false, true);
+    const double fft = fft_time(ctx, r.m, tmb::fft_class_of(r.m), false, true);
     const double row = tile_time(ctx, true, 0, static_cast<double>((r.m + 63) & ~63)) / 128.0;
     return std::min(fft, row) * scale;
 }
