@@ -53,3 +53,28 @@ def test_spectra_of_fewer_classes(tiles):
         assert ctx.profile_read()[0] == 'fft'
         _same(got, want)
         _same(ctx.scan_batch(reqs), want)  # with memory again, and one class resident
+
+
+def test_chunk_bounds_stay_small():
+    """The bounds of 2^22 samples' chunks, 0.5 MB for each of some ninety lengths, with 300 MB free: no more
+    of them are kept than take a tenth of that, and the answers are those of all windows evaluated."""
+    import torch
+    x, rng = _record(1 << 22)
+    lengths = [20]
+    while lengths[-1] < 15_000:
+        lengths.append(int(lengths[-1] * 1.08) + 1)
+    batches = [[tb.Request(rng.normal(size=m).astype(np.float32), tb.MODE_THRESHOLD, correlation=0.3 + 8 / m ** 0.5)
+                for m in lengths[i::9]] for i in range(9)]
+    with tb.Context(x) as ctx:
+        ctx.set_tiles(tb.TILES_ROWS)
+        want = [ctx.scan_batch(b) for b in batches]
+    with tb.Context(x) as ctx:
+        ctx.set_tiles(tb.TILES_FFT)
+        _same(ctx.scan_batch(batches[0]), want[0])  # its other buffers are there now
+        with _Taken(300 << 20):
+            before = torch.cuda.mem_get_info()[0]
+            for b, w in zip(batches, want):
+                _same(ctx.scan_batch(b), w)
+            assert before - torch.cuda.mem_get_info()[0] < 36 << 20
+        for b, w in zip(batches, want):
+            _same(ctx.scan_batch(b), w)

@@ -190,8 +190,8 @@ int tm_ctx_destroy(tm_ctx *ctx)
     for (tm_ctx::FftPieces &f : ctx->fft)
         for (DevBuf *b : {&f.X, &f.shift, &f.norm})
             b->release();
-    for (DevBuf &b : ctx->fft_bounds)
-        b.release();
+    for (tm_ctx::FftBounds &b : ctx->fft_bounds)
+        b.buf.reset();
     // buffers of batches that outlive the context return to the pool when those batches
     // are destroyed; the driver releases the pool's memory once none is outstanding
     if (ctx->pool)

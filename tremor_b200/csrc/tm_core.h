@@ -282,6 +282,8 @@ struct Lane
     std::vector<std::shared_ptr<PinnedBlock>> pool;
     HostBuf h_split, h_q, h_order, h_slots, h_counters;
     uint32_t cand_cap = 1u << 22, list_cap = 1u << 20;
+    std::vector<std::shared_ptr<ScopedBuf>> bounds; // the chunks' bounds that the search in flight reads
+    bool no_bounds = false;                         // it goes without: memory ran out
     // FFT branch: the template spectra of a launch
     DevBuf fft_Y, fft_stats, fft_cuts, lower, bins, tight; // (fft_stats: the correlation kernel's per-block statistics cache)
     // instrumentation
@@ -311,6 +313,7 @@ struct Lane
             b->release();
         for (HostBuf *b : {&h_split, &h_q, &h_order, &h_slots, &h_counters})
             b->release();
+        bounds.clear();
         pool.clear(); // blocks still held by results are freed with the last of them
         for (cudaEvent_t *e : {&ev0, &ev1, &ev2, &ev3, &ev4})
             if (*e)
@@ -366,7 +369,13 @@ struct tm_ctx
         bool ready = false;
     } fft[tmb::kFftClasses];
     tmh::DevBuf fft_roots;
-    tmh::DevBuf fft_bounds[tmb::kFftBases]; // the chunks' bounds, by base length, built on first use
+    // the chunks' bounds by base length, built on first use; a search holds those that it reads
+    struct FftBounds
+    {
+        std::shared_ptr<tmh::ScopedBuf> buf;
+        uint64_t last_use = 0;
+    } fft_bounds[tmb::kFftBases];
+    uint64_t fft_bounds_clock = 0;
     bool fft_skip = true;                   // off while tm_autotune measures templates that evaluate every window
     std::mutex fft_mu;
     int sms = 148;

@@ -621,47 +621,93 @@ static tm_ctx::FftPieces &ensure_fft(tm_ctx *ctx, Lane &L, int cls)
 }
 
 // The chunks' bounds at the bases of rows [first, first + count), in table; false where the memory
-// for one is not to be had, or it would take a 400th of what is free: the windows are
-// then all evaluated.
+// for them is not to be had: the windows are then all evaluated. All that are kept take at most a
+// tenth of the memory that is free without them; those used longest ago go first.
 static bool ensure_bounds(tm_ctx *ctx, Lane &L, const GroupPlan &g, int first, int count, const float4 **table)
 {
+    if (L.no_bounds)
+        return false;
     std::lock_guard<std::mutex> lk(ctx->fft_mu);
+    const size_t each = sizeof(float4) * tmb::fft_chunks(ctx->n);
+    bool wanted[tmb::kFftBases] = {};
+    size_t asked = 0, resident = 0;
     std::vector<int> fresh;
-    size_t free_b = 0, total_b = 0;
-    try
+    for (int i = first; i < first + count; i++)
     {
-        for (int i = first; i < first + count; i++)
+        const int base = g.fft_rows[static_cast<size_t>(i)].base;
+        if (wanted[base])
+            continue;
+        wanted[base] = true;
+        asked += each;
+        if (!ctx->fft_bounds[base].buf)
+            fresh.push_back(base);
+    }
+    for (const tm_ctx::FftBounds &b : ctx->fft_bounds)
+        resident += b.buf ? each : 0;
+    if (!fresh.empty())
+    {
+        size_t free_b = 0, total_b = 0;
+        TM_CUDA(cudaMemGetInfo(&free_b, &total_b));
+        const size_t budget = (free_b + resident) / 10, more = each * fresh.size();
+        if (asked > budget)
+            return false;
+        while (resident + more > budget)
         {
-            const int base = g.fft_rows[static_cast<size_t>(i)].base;
-            if (ctx->fft_bounds[base].p == nullptr)
+            tm_ctx::FftBounds *oldest = nullptr;
+            for (int base = 0; base < tmb::kFftBases; base++)
+                if (ctx->fft_bounds[base].buf && !wanted[base] &&
+                    (oldest == nullptr || ctx->fft_bounds[base].last_use < oldest->last_use))
+                    oldest = &ctx->fft_bounds[base];
+            oldest->buf.reset(); // there is one: those wanted fit the budget
+            resident -= each;
+        }
+        std::vector<std::shared_ptr<ScopedBuf>> built;
+        try
+        {
+            const tmb::PrefixView pv{ctx->prefix.as<double2>(), ctx->ptot.as<double2>(), ctx->pcen.as<double>()};
+            for (const int base : fresh)
             {
-                const size_t need = sizeof(float4) * tmb::fft_chunks(ctx->n);
-                TM_CUDA(cudaMemGetInfo(&free_b, &total_b));
-                if (need > free_b / 400)
-                    throw Failure{TM_ERR_NO_MEMORY, "bounds of the record's chunks"};
-                ctx->fft_bounds[base].reserve(need);
-                fresh.push_back(base);
-                const tmb::PrefixView pv{ctx->prefix.as<double2>(), ctx->ptot.as<double2>(), ctx->pcen.as<double>()};
+                built.push_back(std::make_shared<ScopedBuf>());
+                built.back()->reserve(each);
                 TM_CUDA(tmb::launch_chunk_bounds(pv, ctx->run.as<uint16_t>(), ctx->n, tmb::fft_base_length(base),
-                                                 ctx->fft_bounds[base].as<float4>(), L.stream));
+                                                 built.back()->as<float4>(), L.stream));
                 count_launch(L);
             }
-            table[base] = ctx->fft_bounds[base].as<float4>();
-        }
-        if (!fresh.empty())
             TM_CUDA(cudaStreamSynchronize(L.stream)); // other lanes' streams read them
+        }
+        catch (const Failure &f)
+        {
+            cudaGetLastError();
+            cudaStreamSynchronize(L.stream);
+            if (f.code != TM_ERR_NO_MEMORY)
+                throw;
+            return false;
+        }
+        for (size_t i = 0; i < fresh.size(); i++)
+            ctx->fft_bounds[fresh[i]].buf = built[i];
     }
-    catch (const Failure &f)
-    {
-        cudaGetLastError();
-        cudaStreamSynchronize(L.stream);
-        for (const int base : fresh)
-            ctx->fft_bounds[base].release();
-        if (f.code != TM_ERR_NO_MEMORY)
-            throw;
-        return false;
-    }
+    ctx->fft_bounds_clock++;
+    for (int base = 0; base < tmb::kFftBases; base++)
+        if (wanted[base])
+        {
+            ctx->fft_bounds[base].last_use = ctx->fft_bounds_clock;
+            L.bounds.push_back(ctx->fft_bounds[base].buf);
+            table[base] = ctx->fft_bounds[base].buf->as<float4>();
+        }
     return true;
+}
+
+// Gives the chunks' bounds back; false where there were none.
+static bool drop_bounds(tm_ctx *ctx)
+{
+    std::lock_guard<std::mutex> lk(ctx->fft_mu);
+    bool any = false;
+    for (tm_ctx::FftBounds &b : ctx->fft_bounds)
+    {
+        any = any || b.buf != nullptr;
+        b.buf.reset();
+    }
+    return any;
 }
 
 // Spectrum entries of one correlation launch's templates: 25 MB, well within L2, where every
@@ -898,7 +944,7 @@ void execute_group_mixed(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
     });
 }
 
-void run_batch(tm_ctx *ctx, Lane &L, tm_batch &b, tm_result &res)
+static void run_groups(tm_ctx *ctx, Lane &L, tm_batch &b, tm_result &res)
 {
     res.answers.assign(static_cast<size_t>(b.count), Answer());
     res.blocks.clear();
@@ -909,6 +955,36 @@ void run_batch(tm_ctx *ctx, Lane &L, tm_batch &b, tm_result &res)
             execute_group_mixed(ctx, L, g, res);
         else
             execute_group(ctx, L, g, res);
+    }
+}
+
+void run_batch(tm_ctx *ctx, Lane &L, tm_batch &b, tm_result &res)
+{
+    struct Held // the bounds that a search reads, let go when it ends
+    {
+        Lane &L;
+        ~Held()
+        {
+            L.bounds.clear();
+            L.no_bounds = false;
+        }
+    } held{L};
+    try
+    {
+        run_groups(ctx, L, b, res);
+    }
+    catch (const Failure &f)
+    {
+        // the chunks' bounds save time, not more: without them where the memory is needed
+        if (f.code != TM_ERR_NO_MEMORY)
+            throw;
+        cudaGetLastError();
+        cudaStreamSynchronize(L.stream);
+        L.bounds.clear();
+        if (!drop_bounds(ctx))
+            throw;
+        L.no_bounds = true;
+        run_groups(ctx, L, b, res);
     }
 }
 
