@@ -78,3 +78,18 @@ def test_chunk_bounds_stay_small():
             assert before - torch.cuda.mem_get_info()[0] < 36 << 20
         for b, w in zip(batches, want):
             _same(ctx.scan_batch(b), w)
+
+
+def test_a_search_after_one_that_ran_out():
+    """The failure of one search is not that of the next on the same thread, nor of a new context."""
+    x, rng = _record(1 << 24)
+    reqs = [tb.Request(rng.normal(size=300).astype(np.float32), tb.MODE_KNN, k=3, merge_offset=100) for _ in range(3)]
+    with tb.Context(x) as ctx:
+        ctx.set_tiles(tb.TILES_FFT)
+        with _Taken(60 << 20):
+            with pytest.raises(tb.TremorError) as e:
+                ctx.scan_batch(reqs)
+        assert e.value.code == -3
+        got = ctx.scan_batch(reqs)
+    with tb.Context(x) as ctx:
+        _same(got, ctx.scan_batch(reqs))

@@ -92,13 +92,21 @@ struct Failure
     std::string what;
 };
 
+// The failure of a call. The thread's last error is cleared: the launches of later calls on this
+// thread ask for it, and would report this one.
+inline Failure failure(cudaError_t e, const char *call)
+{
+    cudaGetLastError();
+    return Failure{e == cudaErrorMemoryAllocation ? TM_ERR_NO_MEMORY : TM_ERR_CUDA,
+                   std::string(call) + ": " + cudaGetErrorString(e)};
+}
+
 #define TM_CUDA(call)                                                                                             \
     do                                                                                                            \
     {                                                                                                             \
-        cudaError_t e_ = (call);                                                                                  \
+        const cudaError_t e_ = (call);                                                                            \
         if (e_ != cudaSuccess)                                                                                    \
-            throw Failure{e_ == cudaErrorMemoryAllocation ? TM_ERR_NO_MEMORY : TM_ERR_CUDA,                      \
-                          std::string(#call) + ": " + cudaGetErrorString(e_)};                                    \
+            throw tmh::failure(e_, #call);                                                                        \
     } while (0)
 
 // Grow-only device buffer.

@@ -677,7 +677,6 @@ static bool ensure_bounds(tm_ctx *ctx, Lane &L, const GroupPlan &g, int first, i
         }
         catch (const Failure &f)
         {
-            cudaGetLastError();
             cudaStreamSynchronize(L.stream);
             if (f.code != TM_ERR_NO_MEMORY)
                 throw;
@@ -978,7 +977,6 @@ void run_batch(tm_ctx *ctx, Lane &L, tm_batch &b, tm_result &res)
         // the chunks' bounds save time, not more: without them where the memory is needed
         if (f.code != TM_ERR_NO_MEMORY)
             throw;
-        cudaGetLastError();
         cudaStreamSynchronize(L.stream);
         L.bounds.clear();
         if (!drop_bounds(ctx))
