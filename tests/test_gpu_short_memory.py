@@ -93,3 +93,17 @@ def test_a_search_after_one_that_ran_out():
         got = ctx.scan_batch(reqs)
     with tb.Context(x) as ctx:
         _same(got, ctx.scan_batch(reqs))
+
+
+def test_larger_buckets():
+    """The minima of 1000 kNN templates over 2^23 windows take 268 MB in buckets of 256 windows, 34 in buckets
+    of 2048: with 150 MB left the larger ones serve."""
+    x, rng = _record(1 << 23)
+    reqs = [tb.Request(rng.normal(size=64).astype(np.float32), tb.MODE_KNN, k=1 + i % 3, merge_offset=(0, 40, 300)[i % 3])
+            for i in range(1000)]
+    with tb.Context(x) as ctx:
+        ctx.set_tiles(tb.TILES_FFT)
+        ctx.scan_batch(reqs[:2])  # the record's own arrays
+        with _Taken(150 << 20):
+            got = ctx.scan_batch(reqs)
+        _same(got, ctx.scan_batch(reqs))

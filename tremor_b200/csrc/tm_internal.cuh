@@ -10,14 +10,15 @@ constexpr float kMissing = -100000.0f; // ZnormSearch.hpp:21
 constexpr float kFltMax = 3.402823466e+38f;
 constexpr int kZnormBlock = 32;      // ZnormSearch.hpp:65
 // Windows per kNN bound bucket: 2^8, or as many (up to 2^11) as keep a group's minima, 8 bytes
-// per template and bucket, within 2 GiB. Small buckets bound the k-th distance more tightly and
+// per template and bucket, within `most` bytes: 2 GiB, or less where memory is short. Small buckets bound the k-th distance more tightly and
 // leave the re-pass fewer windows; each contraction kernel's tile or chunk is at most 2^8
 // windows, so none of them does more work for a smaller bucket.
 constexpr int kBucketLogMin = 8, kBucketLogMax = 11;
-inline int bucket_log(uint64_t templates, uint64_t windows)
+constexpr uint64_t kMinimaBytes = 2ull << 30;
+inline int bucket_log(uint64_t templates, uint64_t windows, uint64_t most = kMinimaBytes)
 {
     int b = kBucketLogMin;
-    while (b < kBucketLogMax && 8 * templates * ((windows >> b) + 4) > (2ull << 30))
+    while (b < kBucketLogMax && 8 * templates * ((windows >> b) + 4) > most)
         b++;
     return b;
 }

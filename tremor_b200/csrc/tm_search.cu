@@ -462,6 +462,23 @@ static uint32_t collect_candidates(tm_ctx *ctx, Lane &L, const GroupPlan &g, con
     throw Failure{TM_ERR_NO_MEMORY, "bucket list overflow"};
 }
 
+// Room for the bucket minima of T templates on W windows, and the buckets' size: they are larger where
+// small ones would take more than a quarter of the memory that is free without them.
+static int reserve_minima(Lane &L, uint64_t T, uint64_t W)
+{
+    const auto bytes = [&](int blog) { return sizeof(uint32_t) * T * tmb::bucket_count(W, blog); };
+    int blog = tmb::bucket_log(T, W);
+    if (bytes(blog) > std::min(L.bmin_u.bytes, L.bmin_l.bytes))
+    {
+        size_t free_b = 0, total_b = 0;
+        TM_CUDA(cudaMemGetInfo(&free_b, &total_b));
+        blog = tmb::bucket_log(T, W, std::min<uint64_t>(tmb::kMinimaBytes, (free_b + L.bmin_u.bytes + L.bmin_l.bytes) / 4));
+    }
+    L.bmin_u.reserve(bytes(blog));
+    L.bmin_l.reserve(bytes(blog));
+    return blog;
+}
+
 // Device pipeline and selection for one prepared group; writes answers[index].
 void execute_group(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
 {
@@ -492,13 +509,8 @@ void execute_group(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
     }
     L.tkey.reserve(sizeof(uint32_t) * T);
 
-    const int blog = tmb::bucket_log(static_cast<uint64_t>(T), W);
+    const int blog = nk > 0 ? reserve_minima(L, static_cast<uint64_t>(T), W) : tmb::bucket_log(static_cast<uint64_t>(T), W);
     const uint32_t nb = tmb::bucket_count(W, blog);
-    if (nk > 0)
-    {
-        L.bmin_u.reserve(sizeof(uint32_t) * static_cast<size_t>(T) * nb);
-        L.bmin_l.reserve(sizeof(uint32_t) * static_cast<size_t>(T) * nb);
-    }
     L.counters.reserve(8 * sizeof(uint32_t));
     L.h_counters.reserve(8 * sizeof(uint32_t));
 
@@ -837,13 +849,8 @@ void execute_group_mixed(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
         throw Failure{TM_ERR_ARGUMENT, "more than 2^32 - 1 windows in one range; split the range"};
     cudaStream_t s = L.stream;
     L.tkey.reserve(sizeof(uint32_t) * T);
-    const int blog = tmb::bucket_log(static_cast<uint64_t>(T), W);
+    const int blog = nk > 0 ? reserve_minima(L, static_cast<uint64_t>(T), W) : tmb::bucket_log(static_cast<uint64_t>(T), W);
     const uint32_t nb = tmb::bucket_count(W, blog);
-    if (nk > 0)
-    {
-        L.bmin_u.reserve(sizeof(uint32_t) * static_cast<size_t>(T) * nb);
-        L.bmin_l.reserve(sizeof(uint32_t) * static_cast<size_t>(T) * nb);
-    }
     L.counters.reserve(8 * sizeof(uint32_t));
     L.h_counters.reserve(8 * sizeof(uint32_t));
     double flops = 0.0;
