@@ -53,15 +53,17 @@ struct Server
 
 // Device bytes a request holds while in flight: its template row (FP32, two BF16 halves,
 // block order) at up to the longest length a batch can have, plus its share of the
-// candidate, sort and answer buffers: kNN about 2k-1 buckets of windows, threshold a
-// fixed fraction of the windows (an estimate: the buffers grow when a batch needs more).
+// candidate, sort and answer buffers: kNN about 2k-1 buckets of windows and its bucket minima,
+// threshold a fixed fraction of the windows (an estimate: the buffers grow when a batch needs
+// more).
 static uint64_t serve_bytes(const tm_ctx *ctx, const tm_request &r)
 {
     const uint64_t W = ctx->n - static_cast<uint64_t>(r.m) + 1;
     const uint64_t row = 10ull * 16384 + sizeof(TemplParam);
     const uint64_t cands = r.mode == TM_MODE_KNN ? std::min<uint64_t>(W, (2ull * r.k) * 512)
                                                  : std::max<uint64_t>(W / 512, 1024);
-    return row + 48ull * cands;
+    const uint64_t minima = r.mode == TM_MODE_KNN ? 8ull * tmb::bucket_count(W, tmb::bucket_log(1, W)) : 0;
+    return row + minima + 48ull * cands;
 }
 
 // Modelled device milliseconds of a request: the cheaper of the FFT branch (a constant per
