@@ -525,7 +525,23 @@ struct FftClasses
 void prepare_fft(tm_ctx *ctx, Lane &L, GroupPlan &g, const FftClasses &classes);
 int plan_col_tile(const tm_ctx *ctx, const tm_request *reqs, const std::vector<int> &idx, double *cost = nullptr);
 double tile_time(const tm_ctx *ctx, bool mixed, int v, double k);
-double fft_time(const tm_ctx *ctx, int m, int cls, bool shared, bool skips);
+double fft_time(const tm_ctx *ctx, int m, int cls, bool shared, bool skips, double evaluated);
+double fft_evaluated(int mode, float correlation, int m);
+// Pieces that the windows of a length touch, the first and their number; which templates skip windows,
+// on this many pieces and rows, where the chunks' bounds fit the memory: thresholds; kNN templates
+// on all pieces but the first part of them, with so many cuts on the way.
+struct FftRange
+{
+    uint32_t first, count;
+};
+FftRange fft_range(const tm_ctx *ctx, int cls, uint64_t windows);
+struct FftSkips
+{
+    bool thresholds = false;
+    double knn_first = 1.0;
+    int cuts = 0;
+};
+FftSkips fft_skips(const tm_ctx *ctx, int cls, uint32_t pieces, int rows);
 uint32_t fft_stage_end(uint32_t p0, uint32_t pieces, int rows, int cls, int sms);
 void create_batch(tm_ctx *ctx, Lane &L, const tm_request *requests, int count, tm_batch &b, bool serving = false);
 

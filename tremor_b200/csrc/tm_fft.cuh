@@ -35,6 +35,10 @@ inline int fft_parts(int m, int cls)
     return m <= single ? 1 : (m + step - 1) / step;
 }
 
+// Templates of one correlation launch: 25 MB of spectra, well within L2, where every block reads them
+// once per piece.
+inline int fft_launch_rows(int cls, int parts) { return 192 * 8200 / (fft_pitch(fft_class(cls).n) * parts); }
+
 // Lengths that the bounds of the record's chunks of 128 windows are kept at (k_chunk_bounds): a
 // template takes those of the largest of them that it reaches, at most a tenth shorter.
 constexpr int kFftBases = 100;

@@ -466,14 +466,29 @@ double tensor_cost_sorted(const tm_ctx *ctx, const int *m, size_t n)
 // times over that of a template that evaluates all its windows at 4096 (0.307 ms) or 16000
 // (0.63 ms): 0.247, 0.275, 0.307, 0.43 ms at 1000, 2000, 4096, 8192; shared 0.171, 0.168, 0.208,
 // 0.326, and 0.43 at 16384; skipping 0.109, 0.127, 0.153, 0.231, and 0.33 at 16000.
-double fft_time(const tm_ctx *ctx, int m, int cls, bool shared, bool skips)
+double fft_time(const tm_ctx *ctx, int m, int cls, bool shared, bool skips, double evaluated)
 {
     static const double all[tmb::kFftClasses] = {0.81, 0.90, 1.0, 1.41};
     static const double same[tmb::kFftClasses] = {0.55, 0.55, 0.66, 1.04};
     static const double skip[tmb::kFftClasses] = {0.36, 0.42, 0.50, 0.75};
     if (tmb::fft_parts(m, cls) > 1)
-        return ctx->fft_long_ms * (skips ? 0.53 : shared ? 0.69 : 1.0);
-    return ctx->fft_ms * (skips ? skip[cls] : shared ? same[cls] : all[cls]);
+        return ctx->fft_long_ms * (skips ? 0.53 + 0.47 * evaluated : shared ? 0.69 : 1.0);
+    return ctx->fft_ms * (skips ? skip[cls] + (all[cls] - skip[cls]) * evaluated : shared ? same[cls] : all[cls]);
+}
+
+// The part of a skipping template's windows that is evaluated all the same, in whole chunks of 128: a
+// kNN bound leaves few; a threshold lets the chunks through where noise reaches it, which depends on
+// c sqrt(m). Time per template and 2^25 samples of AR(2) noise, chirps of 512 samples at c = 0.1 to
+// 0.5 (c sqrt(m) = 2.3 to 11): 0.31, 0.24, 0.17, 0.13, 0.112 ms, with nothing to evaluate 0.111, all
+// 0.25; of 1024 at 0.1 to 0.4: 0.25, 0.155, 0.115, 0.111; white noise 0.17 and 0.111 at 0.1 and 0.2. The
+// row tiles take 0.137 for 1024 samples, which is passed at c sqrt(m) of 7 and 4: the line, where
+// noise is unknown, lies between.
+double fft_evaluated(int mode, float correlation, int m)
+{
+    if (mode == TM_MODE_KNN)
+        return 0.0;
+    const double reach = (7.0 - static_cast<double>(correlation) * std::sqrt(static_cast<double>(m))) / 6.0;
+    return reach > 0.0 ? std::min(reach, 1.0) : 0.0;
 }
 
 // Classes for templates of these lengths: each its own (9 to 16 bytes of spectra per sample and class,
@@ -521,27 +536,78 @@ static bool fft_classes(tm_ctx *ctx, const std::vector<int> &m, FftClasses &clas
     return true;
 }
 
-// The f of the least modelled time (plan_fft_split), pieces by these classes; m: the lengths.
-static size_t cheapest_split(const tm_ctx *ctx, const tm_request *reqs, const std::vector<int> &sorted_idx,
+// Will the chunks' bounds of these lengths fit the memory? (ensure_bounds; asked only where they are
+// many times what a device with little memory left would refuse.)
+static bool bounds_fit(tm_ctx *ctx, const std::vector<int> &m)
+{
+    std::lock_guard<std::mutex> lk(ctx->fft_mu);
+    const size_t each = sizeof(float4) * tmb::fft_chunks(ctx->n);
+    size_t asked = 0, fresh = 0, resident = 0;
+    for (size_t i = 0; i < m.size(); i++)
+        if (i == 0 || tmb::fft_base(m[i]) != tmb::fft_base(m[i - 1])) // by length
+        {
+            asked += each;
+            fresh += ctx->fft_bounds[tmb::fft_base(m[i])].buf ? 0 : each;
+        }
+    if (fresh < (64ull << 20))
+        return true;
+    for (const tm_ctx::FftBounds &b : ctx->fft_bounds)
+        resident += b.buf ? each : 0;
+    size_t free_b = 0, total_b = 0;
+    TM_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    return asked <= (free_b + resident) / 10;
+}
+
+// Milliseconds of a cut on the way through a launch's pieces: the selection, and two launches whose last
+// blocks end alone in place of one (128 templates of 1024 on 400000 windows: 0.30 ms with one cut,
+// 0.19 by the times above; the row tiles take 0.24).
+constexpr double kCutMs = 0.06;
+// And of a second group: a selection, re-pass, re-scoring and copy of its own, a dozen launches and two
+// waits of the host.
+constexpr double kGroupMs = 0.12;
+
+// The f of the least modelled time (plan_fft_split), pieces by these classes; m: the lengths. Which
+// templates skip windows is decided as fft_contract does, per class and number of parts, from the
+// pieces of the window range and the rows of a launch.
+static size_t cheapest_split(tm_ctx *ctx, const tm_request *reqs, const std::vector<int> &sorted_idx,
                              const std::vector<int> &m, const FftClasses &classes)
 {
     const size_t n = m.size();
+    const bool fit = bounds_fit(ctx, m);
     size_t best_f = 0;
-    double best = tensor_cost_sorted(ctx, m.data(), n), fft_cost = 0.0;
+    double best = tensor_cost_sorted(ctx, m.data(), n), done = 0.0; // done: the sets before this one
+    double thr[2] = {}, knn[2] = {}, cuts = 0.0; // this set's, evaluating all and skipping, and its cuts
+    int cls = -1, parts = 0, rows = 0;
+    FftSkips skips;
+    const auto set_cost = [&] {
+        return thr[skips.thresholds ? 1 : 0] + (knn[0] > 0.0 ? skips.knn_first * knn[0] + (1.0 - skips.knn_first) * knn[1] + cuts : 0.0);
+    };
     for (size_t f = 1; f <= n; f++)
     {
         const tm_request &r = reqs[sorted_idx[f - 1]];
-        const int cls = classes.of(r.m);
-        const uint32_t pieces = tmb::fft_pieces(ctx->n, cls);
-        // as fft_contract decides, were all templates of this one's class
-        const bool skips = static_cast<uint64_t>(pieces) * n >= static_cast<uint64_t>(ctx->sms) &&
-                           (r.mode != TM_MODE_KNN ||
-                            fft_stage_end(0, pieces, static_cast<int>(n), cls, ctx->sms) < pieces);
-        fft_cost += fft_time(ctx, r.m, cls, f > 1 && m[f - 2] == r.m, skips);
-        const double c = fft_cost + tensor_cost_sorted(ctx, m.data() + f, n - f);
-        if (c < best)
+        const int c = classes.of(r.m), p = tmb::fft_parts(r.m, c);
+        if (c != cls || p != parts)
         {
-            best = c;
+            done += set_cost();
+            cls = c;
+            parts = p;
+            rows = 0;
+            thr[0] = thr[1] = knn[0] = knn[1] = 0.0;
+        }
+        rows++;
+        const uint64_t windows = windows_in_range(ctx, r.m); // the set's shortest so far has the most
+        if (fit)
+            skips = fft_skips(ctx, cls, fft_range(ctx, cls, windows).count, std::min(rows, tmb::fft_launch_rows(cls, parts)));
+        const double scale = windows > 0 ? 33554432.0 / static_cast<double>(windows) : 0.0;
+        cuts = kCutMs * skips.cuts * scale;
+        double *sum = r.mode == TM_MODE_KNN ? knn : thr;
+        sum[0] += fft_time(ctx, r.m, cls, f > 1 && m[f - 2] == r.m, false, 0.0);
+        sum[1] += fft_time(ctx, r.m, cls, false, true, fft_evaluated(r.mode, r.correlation, r.m));
+        const double cost = done + set_cost() +
+                            (f < n ? tensor_cost_sorted(ctx, m.data() + f, n - f) + kGroupMs * scale : 0.0);
+        if (cost < best)
+        {
+            best = cost;
             best_f = f;
         }
     }

@@ -721,10 +721,6 @@ static bool drop_bounds(tm_ctx *ctx)
     return any;
 }
 
-// Spectrum entries of one correlation launch's templates: 25 MB, well within L2, where every
-// block reads them once per piece.
-constexpr size_t kFftLaunchBins = 192 * 8200;
-
 // Where a launch of kNN templates over the pieces from p0 on ends. A bound from the minima of the
 // first sixteenth of the pieces, then of the first quarter, lets the rest skip almost all of
 // its windows (tm_fftk.cu); where a launch would have fewer than four items per block, the
@@ -741,6 +737,28 @@ uint32_t fft_stage_end(uint32_t p0, uint32_t pieces, int rows, int cls, int sms)
     return pieces;
 }
 
+FftRange fft_range(const tm_ctx *ctx, int cls, uint64_t windows)
+{
+    if (windows == 0)
+        return FftRange{0, 0};
+    const uint64_t step = tmb::fft_class(cls).step, first = ctx->range_first / step;
+    const uint64_t last = std::min<uint64_t>((ctx->range_first + windows - 1) / step, tmb::fft_pieces(ctx->n, cls) - 1);
+    return FftRange{static_cast<uint32_t>(first), static_cast<uint32_t>(last - first + 1)};
+}
+
+FftSkips fft_skips(const tm_ctx *ctx, int cls, uint32_t pieces, int rows)
+{
+    // fewer items than multiprocessors: bounds and cuts would cost more than they save
+    FftSkips skips;
+    if (!ctx->fft_skip || static_cast<uint64_t>(pieces) * static_cast<uint64_t>(rows) < static_cast<uint64_t>(ctx->sms))
+        return skips;
+    skips.thresholds = true;
+    for (uint32_t p = fft_stage_end(0, pieces, rows, cls, ctx->sms); p < pieces; p = fft_stage_end(p, pieces, rows, cls, ctx->sms))
+        if (++skips.cuts == 1)
+            skips.knn_first = static_cast<double>(p) / pieces;
+    return skips;
+}
+
 // The FFT branch of a group: per set of rows (prepare_fft), their spectra, then persistent
 // launches over the pieces their windows touch.
 void fft_contract(tm_ctx *ctx, Lane &L, const GroupPlan &g, const tmb::ScanArgs &a)
@@ -751,7 +769,7 @@ void fft_contract(tm_ctx *ctx, Lane &L, const GroupPlan &g, const tmb::ScanArgs 
         const tm_ctx::FftPieces &X = ensure_fft(ctx, L, set.cls);
         const uint32_t step = tmb::fft_class(set.cls).step;
         const size_t pitch = tmb::fft_pitch(tmb::fft_class(set.cls).n) * static_cast<size_t>(set.parts);
-        const int most = static_cast<int>(kFftLaunchBins / pitch);
+        const int most = tmb::fft_launch_rows(set.cls, set.parts);
         L.fft_Y.reserve(sizeof(double2) * static_cast<size_t>(std::min(most, set.count)) * pitch);
         L.fft_stats.reserve(sizeof(float4) * static_cast<size_t>(ctx->sms) * tmb::kFftStats);
         for (int r0 = 0; r0 < set.count; r0 += most)
@@ -771,8 +789,8 @@ void fft_contract(tm_ctx *ctx, Lane &L, const GroupPlan &g, const tmb::ScanArgs 
                 wmax = std::max<uint64_t>(wmax, r.wcount);
                 knn += r.mode == TM_MODE_KNN ? 1 : 0;
             }
-            const uint32_t pa = static_cast<uint32_t>(a.w0 / step);
-            const uint32_t pb = std::min<uint32_t>(static_cast<uint32_t>((a.w0 + wmax - 1) / step), X.count - 1);
+            const FftRange range = fft_range(ctx, set.cls, wmax);
+            const uint32_t pa = range.first, pieces = range.count;
             f.X = X.X.as<double2>();
             f.shifts = X.shift.as<double>();
             f.norms = X.norm.as<double>();
@@ -795,10 +813,8 @@ void fft_contract(tm_ctx *ctx, Lane &L, const GroupPlan &g, const tmb::ScanArgs 
             f.dbg_e = a.dbg_e;
             f.stats = L.fft_stats.as<float4>();
             count_launch(L);
-            const uint32_t pieces = pb >= pa ? pb - pa + 1 : 0;
-            // fewer items than multiprocessors: bounds and cuts would cost more than they save
-            const bool cuts = ctx->fft_skip && a.dbg_d == nullptr &&
-                              static_cast<uint64_t>(pieces) * nr >= static_cast<uint64_t>(ctx->sms) &&
+            const FftSkips skips = fft_skips(ctx, set.cls, pieces, nr);
+            const bool cuts = (skips.cuts > 0 || (skips.thresholds && knn < nr)) && a.dbg_d == nullptr &&
                               ensure_bounds(ctx, L, g, first, nr, f.bounds);
             for (uint32_t p0 = 0; p0 < pieces;)
             {

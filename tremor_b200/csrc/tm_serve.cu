@@ -66,13 +66,17 @@ static uint64_t serve_bytes(const tm_ctx *ctx, const tm_request &r)
     return row + minima + 48ull * cands;
 }
 
-// Modelled device milliseconds of a request: the cheaper of the FFT branch (a constant per
-// template, by kind) and its share of a full 128-row tile of mixed lengths at its own K, from
-// the planner's model (ms per 2^25 windows), scaled to the record's windows.
+// Modelled device milliseconds of a request: the cheaper of the FFT branch (by class of length,
+// as one that skips windows only where it would in a launch alone) and its share of a full
+// 128-row tile of mixed lengths at its own K, from the planner's model (ms per 2^25 windows),
+// scaled to the record's windows.
 static double serve_cost(const tm_ctx *ctx, const tm_request &r)
 {
     const double scale = static_cast<double>(ctx->n - static_cast<uint64_t>(r.m) + 1) / 33554432.0;
-    const double fft = fft_time(ctx, r.m, tmb::fft_class_of(r.m), false, true);
+    const int cls = tmb::fft_class_of(r.m);
+    const FftSkips skips = fft_skips(ctx, cls, fft_range(ctx, cls, windows_in_range(ctx, r.m)).count, 1);
+    const double first = r.mode == TM_MODE_KNN ? skips.knn_first : fft_evaluated(r.mode, r.correlation, r.m);
+    const double fft = fft_time(ctx, r.m, cls, false, skips.thresholds, first);
     const double row = tile_time(ctx, true, 0, static_cast<double>((r.m + 63) & ~63)) / 128.0;
     return std::min(fft, row) * scale;
 }
