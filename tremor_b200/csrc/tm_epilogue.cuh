@@ -11,7 +11,7 @@ struct ScanArgs
     const float *x;        // clean waveform (missing -> 0), global sample index, zero padded
     const float *q;        // z-normalised templates, T_pad x m_pad, zero padded
     const TemplParam *tp;  // T_pad
-    const float *mean;     // [W] window means
+    const float *mean;     // [W] window means (several lengths, FFT branch: null, or of its one length)
     const float *inv;      // [W] 1 / std; 0 for windows that are not searched
     uint64_t w0;
     uint32_t W;

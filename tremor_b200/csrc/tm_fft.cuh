@@ -103,6 +103,8 @@ struct FftArgs
     PrefixView pv;
     const uint16_t *run;
     const float *raw;
+    const float *mean, *inv; // one length, where the prefix sums lose windows: its own statistics; else null
+    uint32_t *untrusted;     // candidates for want of statistics are counted here
     uint32_t *bmin_u, *bmin_l;
     uint32_t nb;
     int bucket_log;

@@ -502,6 +502,16 @@ __device__ __forceinline__ void fold_window(float mu, float iv, float rel_sd, fl
          stats_error(ws, m, qs, s1) + 2.0f * e_dot * iv * 1.01f;
 }
 
+// The same from the statistics of the one length (fast_distance's bound, its a4 a function of m).
+__device__ __forceinline__ void fold_length_window(float mu, float iv, float4 c0, int m, float shift, float e_dot, float &ms,
+                                                   float &ew)
+{
+    ms = mu - shift;
+    const float r = ms * iv, r0 = mu * iv, a4 = 1.25f * 8.0f * (float)m * (float)m * (float)kEps64;
+    ew = c0.x * (1.0f + fabsf(r)) + c0.y + a4 * (1.0f + 2.0f * r0 * r0) + c0.z * r0 * r0 +
+         c0.w * (fabsf(mu) + fabsf(shift)) * iv + 2.0f * e_dot * iv * 1.01f;
+}
+
 // The terms of ew = k0 + kr |r| + kq (mu / sd)^2 + (ki + s1m kb + km |mu|) / sd, the fast path's
 // statistics, that an item's windows share; kb is of the window's prefix block.
 struct FoldItem
@@ -1048,10 +1058,15 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
             }
             else if (__any_sync(0xffffffffu, lmin <= thr))
             {
-                uint32_t mask = 0;
+                uint32_t mask = 0, lost = 0;
 #pragma unroll
                 for (int j = 0; j < 4; j++)
+                {
                     mask |= (lo[j] <= thr ? 1u : 0u) << j;
+                    lost += lo[j] == -inf_f() ? 1u : 0u;
+                }
+                if (lost > 0)
+                    atomicAdd(a.untrusted, lost);
                 emit_strided(mask, lane, (uint32_t)P.row, (uint32_t)(first + lane), a.cand, a.cand_count, a.cand_cap);
             }
         };
@@ -1180,10 +1195,15 @@ template <int N, bool PARTS> __global__ void __launch_bounds__(N / 16, N == 4096
                     const int jj = __ffs(slow) - 1, w = o + 32 * jj;
                     float4 st;
                     const bool ok = window_stats_full(a.pv, Qp[w], Qp[w + m], piece_w + (uint64_t)w, m, inv_m, st);
-                    const float v = ok ? st.y : 0.0f;
+                    float v = ok ? st.y : 0.0f;
                     float x = 0.0f, e = inf_f();
                     if (ok)
                         fold_window(st.x, v, st.z, st.w, P.c0, P.qs, P.s1_max, m, shift, F.e_dot, x, e);
+                    else if (a.inv != nullptr && a.inv[rel + w] != 0.0f)
+                    {
+                        v = a.inv[rel + w];
+                        fold_length_window(a.mean[rel + w], v, P.c0, m, shift, F.e_dot, x, e);
+                    }
 #pragma unroll
                     for (int j = 0; j < 4; j++)
                         if (j == jj)

@@ -254,7 +254,8 @@ static tmb::Exclusion exclusion(const Lane &L, const GroupPlan &g, uint32_t nb, 
     return ex;
 }
 
-// Exact re-scoring of a group's ncand candidates (pv: prefix sums of mixed groups, mean: window means of the others), answer order and kNN selection on the
+// Exact re-scoring of a group's ncand candidates (pv: prefix sums of mixed groups, mean: window means of the others,
+// and of FFT groups with statistics of their length), answer order and kNN selection on the
 // device, one copy to a pinned block that the result keeps, canonical answers.
 template <class Degenerate>
 void rescore_and_answer(tm_ctx *ctx, Lane &L, const GroupPlan &g, uint32_t ncand, const tmb::PrefixView &pv,
@@ -409,8 +410,8 @@ static void forget_odd_buckets(Lane &L, const GroupPlan &g, const tmb::ScanArgs 
 }
 
 // kNN bound, bucket list and FP32 re-pass after a group's contraction (a: its arguments), then
-// the counters: the group's candidates, whether the contraction gave up waiting. One wait for
-// the device; a list that did not fit is made again, larger.
+// the counters: the group's candidates, whether the contraction gave up waiting, the candidates for
+// want of statistics (in L.h_counters [7]). One wait for the device; a list that did not fit is made again, larger.
 static uint32_t collect_candidates(tm_ctx *ctx, Lane &L, const GroupPlan &g, const tmb::ScanArgs &a, bool mixed)
 {
     cudaStream_t s = L.stream;
@@ -446,7 +447,7 @@ static uint32_t collect_candidates(tm_ctx *ctx, Lane &L, const GroupPlan &g, con
         }
         if (L.profile)
             TM_CUDA(cudaEventRecord(L.ev2, s));
-        TM_CUDA(cudaMemcpyAsync(hc, counters, 3 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+        TM_CUDA(cudaMemcpyAsync(hc, counters, 8 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
         TM_CUDA(cudaStreamSynchronize(s));
         if (L.profile)
             add_span(L, 1, L.ev1, L.ev2);
@@ -523,7 +524,7 @@ void execute_group(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
             TM_CUDA(cudaMemsetAsync(L.bmin_u.p, 0xff, sizeof(uint32_t) * static_cast<size_t>(T) * nb, s));
             TM_CUDA(cudaMemsetAsync(L.bmin_l.p, 0xff, sizeof(uint32_t) * static_cast<size_t>(T) * nb, s));
         }
-        TM_CUDA(cudaMemsetAsync(L.counters.p, 0, 4 * sizeof(uint32_t), s));
+        TM_CUDA(cudaMemsetAsync(L.counters.p, 0, 8 * sizeof(uint32_t), s));
         uint32_t *d_cand_count = L.counters.as<uint32_t>();
 
         tmb::ScanArgs a{};
@@ -802,6 +803,9 @@ void fft_contract(tm_ctx *ctx, Lane &L, const GroupPlan &g, const tmb::ScanArgs 
             f.pv = tmb::PrefixView{a.P, a.PT, a.PC};
             f.run = a.run;
             f.raw = a.raw;
+            f.mean = a.mean;
+            f.inv = a.inv;
+            f.untrusted = a.cand_count + 7;
             f.bmin_u = a.bmin_u;
             f.bmin_l = a.bmin_l;
             f.nb = a.nb;
@@ -869,6 +873,15 @@ void execute_group_mixed(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
     const uint32_t nb = tmb::bucket_count(W, blog);
     L.counters.reserve(8 * sizeof(uint32_t));
     L.h_counters.reserve(8 * sizeof(uint32_t));
+    // The prefix sums lose the windows of a block that is much louder elsewhere: every template of the
+    // group would have all of them re-scored, by their chains. Where a group of one length takes more
+    // time so than the statistics of the length and another contraction, it has these (they stay, for the
+    // next searches): 130 templates of 1500 on 2^17 samples, 4000 of them 10^5 times the rest: 25 ms
+    // with prefix sums alone, 2.3 with both. (The context keeps these statistics for its own lane only.)
+    const bool one_length = g.fft && &L == &ctx->main && g.htp[0].m == g.htp[T - 1].m;
+    LengthStats *ls = one_length && ctx->lengths.count(g.m) > 0 ? &ensure_length(ctx, L, g.m) : nullptr;
+    const double chain_ms = 1.8e-9 * g.m; // of a candidate without statistics
+    const double again_ms = 0.1 + static_cast<double>(W) / 33554432.0 * (1.0 + 0.15 * T);
     double flops = 0.0;
     for (int t = 0; t < T; t++)
         flops += 2.0 * g.htp[t].m * static_cast<double>(g.htp[t].wcount);
@@ -882,7 +895,7 @@ void execute_group_mixed(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
             TM_CUDA(cudaMemsetAsync(L.bmin_u.p, 0xff, sizeof(uint32_t) * static_cast<size_t>(T) * nb, s));
             TM_CUDA(cudaMemsetAsync(L.bmin_l.p, 0xff, sizeof(uint32_t) * static_cast<size_t>(T) * nb, s));
         }
-        TM_CUDA(cudaMemsetAsync(L.counters.p, 0, 4 * sizeof(uint32_t), s));
+        TM_CUDA(cudaMemsetAsync(L.counters.p, 0, 8 * sizeof(uint32_t), s));
         uint32_t *d_cand_count = L.counters.as<uint32_t>();
         tmb::ScanArgs a{};
         a.x = ctx->clean.as<float>();
@@ -907,6 +920,8 @@ void execute_group_mixed(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
         a.P = ctx->prefix.as<double2>();
         a.PT = ctx->ptot.as<double2>();
         a.PC = ctx->pcen.as<double>();
+        a.mean = ls != nullptr ? ls->mean.as<float>() : nullptr;
+        a.inv = ls != nullptr ? ls->inv.as<float>() : nullptr;
         a.run = ctx->run.as<uint16_t>();
         a.odd = ctx->odd.as<uint32_t>();
         a.tiles = g.d_tiles.as<tmb::TileInfo>();
@@ -935,6 +950,12 @@ void execute_group_mixed(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
             L.prof_flops += flops;
         }
         ncand = collect_candidates(ctx, L, g, a, true);
+        if (one_length && ls == nullptr && chain_ms * L.h_counters.as<uint32_t>()[7] > again_ms)
+        {
+            ls = &ensure_length(ctx, L, g.m);
+            attempt--;
+            continue;
+        }
         if (ncand <= L.cand_cap)
             break;
         L.cand_cap = ncand + ncand / 2;
@@ -945,7 +966,7 @@ void execute_group_mixed(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
     std::vector<float> raw;
     std::vector<uint32_t> odd; // stays empty where all samples are finite
     const tmb::PrefixView pv{ctx->prefix.as<double2>(), ctx->ptot.as<double2>(), ctx->pcen.as<double>()};
-    rescore_and_answer(ctx, L, g, ncand, pv, nullptr, w0, exclusion(L, g, nb, blog), res, [&](int t, std::vector<Hit> &degenerate) {
+    rescore_and_answer(ctx, L, g, ncand, pv, ls != nullptr ? ls->mean.as<float>() : nullptr, w0, exclusion(L, g, nb, blog), res, [&](int t, std::vector<Hit> &degenerate) {
         if (run.empty())
         {
             run.resize(W);

@@ -262,13 +262,14 @@ struct PassB
     const uint32_t *tkey;
     uint64_t w0;
     uint32_t W;
-    const float *mean, *inv; // one length: its windows' statistics
+    const float *mean, *inv; // one length: its windows' statistics (FFT branch: null where it has none)
     const float *raw;        // several lengths: statistics from the prefix sums
     PrefixView pv;
     const uint16_t *run;
     const uint32_t *odd; // several lengths, a record with samples that are not finite; else null
     Candidate *cand;
     uint32_t *cand_count, cand_cap;
+    uint32_t *untrusted; // candidates for want of statistics are counted here
     uint32_t nb;
     const uint32_t *bmin_l;
     uint32_t *certain; // the certain minima (below), over the minima of d + E; null: none
@@ -362,7 +363,8 @@ template <bool MIXED> __global__ void __launch_bounds__(B_THREADS) k_passb(const
                 (a.odd == nullptr || a.odd[a.w0 + j] >= (uint32_t)m))
             {
                 WindowStats ws;
-                if (window_prefix_stats(a.pv, a.pv.Q[a.w0 + j], a.pv.Q[a.w0 + j + m], a.w0 + j, m, p.inv_m, ws) != 0)
+                const int code = window_prefix_stats(a.pv, a.pv.Q[a.w0 + j], a.pv.Q[a.w0 + j + m], a.w0 + j, m, p.inv_m, ws);
+                if (code != 0 && (a.inv == nullptr || a.inv[j] == 0.0f))
                 {
                     hit = true; // statistics not trustworthy: always re-scored
                     lower = -inf_f();
@@ -370,7 +372,10 @@ template <bool MIXED> __global__ void __launch_bounds__(B_THREADS) k_passb(const
                 else
                 {
                     float d, e;
-                    fast_distance_mixed(p, p.a1_fp32, dot, ws.mu, ws.iv, shift, stats_error(ws, m, p.qs, p.s1), d, e);
+                    if (code == 0)
+                        fast_distance_mixed(p, p.a1_fp32, dot, ws.mu, ws.iv, shift, stats_error(ws, m, p.qs, p.s1), d, e);
+                    else
+                        fast_distance(p, p.a1_fp32, dot, a.mean[j], a.inv[j], shift, d, e);
                     lower = d - e;
                     upper = d + e;
                     hit = lower <= T;
@@ -417,6 +422,9 @@ template <bool MIXED> __global__ void __launch_bounds__(B_THREADS) k_passb(const
             atomicAdd(&a.bins[(size_t)t * kTightBins + min((int)(fmaxf(upper, 0.0f) * ((float)kTightBins / T)), kTightBins - 1)],
                       1u);
         const unsigned ballot = __ballot_sync(0xffffffffu, hit);
+        const unsigned lost = __ballot_sync(0xffffffffu, hit && lower == -inf_f());
+        if (lost != 0u && lane == 0)
+            atomicAdd(a.untrusted, (uint32_t)__popc(lost));
         if (ballot != 0u)
         {
             uint32_t base = 0;
@@ -583,9 +591,9 @@ __device__ __forceinline__ bool excluded_window(const Exclusion &x, uint32_t t, 
 
 constexpr int R_THREADS = 256;
 
-// PREFIX: statistics from the prefix sums (windows of at most kPrefixBlock samples), else from
-// the samples. todo: the
-// undecided candidates' indices, their number in *todo_count.
+// PREFIX: statistics from the prefix sums (windows of at most kPrefixBlock samples); without them, or
+// where they do not decide, from the samples, if there are means to centre them. todo: the undecided
+// candidates' indices, their number in *todo_count.
 template <bool PREFIX>
 __global__ void __launch_bounds__(R_THREADS) k_rescore(const Candidate *__restrict__ cand, uint32_t count,
                                                        const TemplParam *__restrict__ tp, const float *__restrict__ q,
@@ -616,8 +624,8 @@ __global__ void __launch_bounds__(R_THREADS) k_rescore(const Candidate *__restri
         return;
     }
     float mean_f, std_f;
-    if (!(PREFIX ? prefix_exact_stats(pv, g, m, p.inv_m, mean_f, std_f)
-                 : sums_exact_stats(raw + g, m, (double)mean[c.window], lane, half, mean_f, std_f)))
+    if (!(PREFIX && prefix_exact_stats(pv, g, m, p.inv_m, mean_f, std_f)) &&
+        !(mean != nullptr && sums_exact_stats(raw + g, m, (double)mean[c.window], lane, half, mean_f, std_f)))
     {
         if (lane == 0)
             todo[atomicAdd(todo_count, 1u)] = i;
@@ -802,6 +810,7 @@ cudaError_t launch_passb(const uint2 *list, const uint32_t *counters, uint32_t c
     a.cand = c.cand;
     a.cand_count = c.cand_count;
     a.cand_cap = c.cand_cap;
+    a.untrusted = c.cand_count + 7;
     a.nb = c.nb;
     a.bmin_l = c.bmin_l;
     a.certain = c.bucket_log == 8 ? c.bmin_u : nullptr; // the bound has been selected
@@ -815,8 +824,8 @@ cudaError_t launch_passb(const uint2 *list, const uint32_t *counters, uint32_t c
     return cudaGetLastError();
 }
 
-// pv: the prefix sums, when the group's windows have them (Q not null); else mean: the
-// windows' means, near enough to centre their sums. todo: scratch of `count` indices;
+// pv: the prefix sums, when the group's windows have them (Q not null); mean: the windows' means, near
+// enough to centre their sums, or null; one of the two is there. todo: scratch of `count` indices;
 // todo_count: its counter, zeroed here.
 cudaError_t launch_rescore(const Candidate *cand, uint32_t count, const TemplParam *tp, const float *q,
                            const int *order, const float *raw, const PrefixView &pv, const float *mean, uint64_t w0, float *dist,
