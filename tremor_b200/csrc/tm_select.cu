@@ -591,10 +591,10 @@ __device__ __forceinline__ bool excluded_window(const Exclusion &x, uint32_t t, 
 
 constexpr int R_THREADS = 256;
 
-// PREFIX: statistics from the prefix sums (windows of at most kPrefixBlock samples); without them, or
-// where they do not decide, from the samples, if there are means to centre them. todo: the undecided
+// PREFIX: statistics from the prefix sums (windows of at most kPrefixBlock samples); SUMS: without
+// them, or where they do not decide, from the samples, centred by the means. todo: the undecided
 // candidates' indices, their number in *todo_count.
-template <bool PREFIX>
+template <bool PREFIX, bool SUMS>
 __global__ void __launch_bounds__(R_THREADS) k_rescore(const Candidate *__restrict__ cand, uint32_t count,
                                                        const TemplParam *__restrict__ tp, const float *__restrict__ q,
                                                        const int *__restrict__ order, const float *__restrict__ raw,
@@ -625,7 +625,7 @@ __global__ void __launch_bounds__(R_THREADS) k_rescore(const Candidate *__restri
     }
     float mean_f, std_f;
     if (!(PREFIX && prefix_exact_stats(pv, g, m, p.inv_m, mean_f, std_f)) &&
-        !(mean != nullptr && sums_exact_stats(raw + g, m, (double)mean[c.window], lane, half, mean_f, std_f)))
+        !(SUMS && sums_exact_stats(raw + g, m, (double)mean[c.window], lane, half, mean_f, std_f)))
     {
         if (lane == 0)
             todo[atomicAdd(todo_count, 1u)] = i;
@@ -836,10 +836,8 @@ cudaError_t launch_rescore(const Candidate *cand, uint32_t count, const TemplPar
     if (const cudaError_t e = cudaMemsetAsync(todo_count, 0, sizeof(uint32_t), s); e != cudaSuccess)
         return e;
     const unsigned grid = (count - 1) / (R_THREADS / 16) + 1;
-    if (pv.Q != nullptr)
-        k_rescore<true><<<grid, R_THREADS, 0, s>>>(cand, count, tp, q, order, raw, pv, mean, w0, dist, todo, todo_count, ex);
-    else
-        k_rescore<false><<<grid, R_THREADS, 0, s>>>(cand, count, tp, q, order, raw, pv, mean, w0, dist, todo, todo_count, ex);
+    auto *kernel = pv.Q == nullptr ? k_rescore<false, true> : mean == nullptr ? k_rescore<true, false> : k_rescore<true, true>;
+    kernel<<<grid, R_THREADS, 0, s>>>(cand, count, tp, q, order, raw, pv, mean, w0, dist, todo, todo_count, ex);
     const unsigned serial = std::min((count - 1) / S_WARPS + 1, 148u * 4u); // how many are undecided the device knows
     k_rescore_serial<<<serial, S_WARPS * 32, 0, s>>>(cand, tp, q, order, raw, w0, dist, todo, todo_count);
     return cudaGetLastError();
