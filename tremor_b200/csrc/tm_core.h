@@ -473,6 +473,7 @@ struct GroupPlan
     DevBuf d_fft;
     int k_stride = 0;            // row stride of the template arrays
     uint32_t w_max = 0;          // windows of the shortest template
+    uint64_t range_first = 0, range_count = 0; // the window range that wcount and w_max are of
     std::vector<tmb::TileInfo> tiles; // per tile: K blocks
     DevBuf d_tiles;
     void release()
@@ -522,6 +523,8 @@ struct FftClasses
     int use[tmb::kFftClasses] = {0, 1, 2, 3};
     int of(int m) const { return use[tmb::fft_class_of(m)]; }
 };
+// Brings the windows of a prepared mixed group's templates to the context's range.
+void refresh_range(tm_ctx *ctx, Lane &L, GroupPlan &g);
 void prepare_fft(tm_ctx *ctx, Lane &L, GroupPlan &g, const FftClasses &classes);
 int plan_col_tile(const tm_ctx *ctx, const tm_request *reqs, const std::vector<int> &idx, double *cost = nullptr);
 double tile_time(const tm_ctx *ctx, bool mixed, int v, double k);

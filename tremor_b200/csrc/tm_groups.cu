@@ -223,6 +223,8 @@ void prepare_group_mixed(tm_ctx *ctx, Lane &L, const std::vector<int> &idx_in, c
     g.thr.assign(R, -FLT_MAX);
     g.a1_umma.assign(R, 0.0f);
     g.inert.assign(R, 0);
+    g.range_first = ctx->range_first;
+    g.range_count = ctx->range_count;
     g.nk = 0;
     g.w_max = 0;
     uint64_t samples = 0;
@@ -304,8 +306,8 @@ void prepare_group_mixed(tm_ctx *ctx, Lane &L, const std::vector<int> &idx_in, c
     h2d += samples * 2 * sizeof(uint16_t) + sizeof(tmb::TileInfo) * tiles.size();
 }
 
-// Makes a prepared mixed-length group one of the FFT branch: its rows with windows, sorted by
-// length as they are, in sets of one class and number of parts, and what the correlation
+// Makes a prepared mixed-length group one of the FFT branch: its rows, sorted by length as they
+// are, in sets of one class and number of parts, and what the correlation
 // kernel needs per row.
 void prepare_fft(tm_ctx *ctx, Lane &L, GroupPlan &g, const FftClasses &classes)
 {
@@ -317,7 +319,7 @@ void prepare_fft(tm_ctx *ctx, Lane &L, GroupPlan &g, const FftClasses &classes)
     for (int t = 0; t < g.T; t++)
     {
         const TemplParam &p = g.htp[static_cast<size_t>(t)];
-        if (g.index[t] < 0 || p.wcount == 0)
+        if (g.index[t] < 0 || g.inert[t])
             continue;
         const int cls = classes.of(p.m), parts = tmb::fft_parts(p.m, cls);
         const int step = static_cast<int>(tmb::fft_class(cls).step);
@@ -370,6 +372,32 @@ void prepare_fft(tm_ctx *ctx, Lane &L, GroupPlan &g, const FftClasses &classes)
         TM_CUDA(cudaMemcpyAsync(g.d_fft.p, g.fft_rows.data(), bytes, cudaMemcpyHostToDevice, L.stream));
     }
     TM_CUDA(cudaStreamSynchronize(L.stream));
+}
+
+// A batch is prepared once and run on whatever range the context has then: windows past the record
+// would be read with those of another.
+void refresh_range(tm_ctx *ctx, Lane &L, GroupPlan &g)
+{
+    if (g.range_first == ctx->range_first && g.range_count == ctx->range_count)
+        return;
+    g.w_max = 0;
+    for (int t = 0; t < g.T; t++)
+        if (g.index[t] >= 0)
+        {
+            const uint32_t windows = static_cast<uint32_t>(windows_in_range(ctx, g.htp[t].m));
+            g.w_max = std::max(g.w_max, windows);
+            g.htp[t].wcount = g.inert[t] ? 0 : windows;
+        }
+    TM_CUDA(cudaMemcpyAsync(g.tp.p, g.htp.data(), sizeof(TemplParam) * g.htp.size(), cudaMemcpyHostToDevice, L.stream));
+    if (g.fft && !g.fft_rows.empty())
+    {
+        for (tmb::FftRow &r : g.fft_rows)
+            r.wcount = g.htp[r.row].wcount;
+        TM_CUDA(cudaMemcpyAsync(g.d_fft.p, g.fft_rows.data(), sizeof(tmb::FftRow) * g.fft_rows.size(), cudaMemcpyHostToDevice,
+                                L.stream));
+    }
+    g.range_first = ctx->range_first;
+    g.range_count = ctx->range_count;
 }
 
 // Modelled milliseconds of 128 template rows x 2^25 windows of shape v at K samples:

@@ -854,6 +854,7 @@ void execute_group_mixed(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
     if (ctx->kernel == TM_KERNEL_FP32 && !g.fft)
         throw Failure{TM_ERR_STATE, "batch of several template lengths was prepared for the tensor-core kernel"};
     ensure_prefix(ctx, L);
+    refresh_range(ctx, L, g);
     const int T = g.T, nk = g.nk;
     const uint64_t w0 = ctx->range_first, W = g.w_max;
     if (W == 0)
