@@ -101,7 +101,7 @@ static void bound_diagnostics_wm(tm_ctx *ctx, int m, const std::vector<int> &idx
         TM_CUDA(tmb::launch_rescore(dc.as<Candidate>(), static_cast<uint32_t>(pairs), g.tp.as<TemplParam>(),
                                     g.q.as<float>(), g.order.as<int>(), ctx->raw.as<float>(),
                                     tmb::PrefixView{a.P, a.PT, a.PC}, nullptr, ctx->range_first, dx.as<float>(),
-                                    todo.as<uint32_t>(), L.counters.as<uint32_t>() + 6, tmb::Exclusion{}, s));
+                                    todo.as<uint32_t>(), L.counters.as<uint32_t>() + 6, tmb::Exclusion{}, ctx->sms, s));
         count_launch(L);
         TM_CUDA(cudaMemcpyAsync(exact, dx.p, pairs * sizeof(float), cudaMemcpyDeviceToHost, s));
     }
@@ -284,8 +284,8 @@ int tm_autotune(tm_ctx *ctx, double *ms, int capacity)
                 }
             }
         // the FFT branch, 8 templates of distinct lengths each, which evaluate all their windows
-        // with statistics of their own (the time does not depend on the length within either
-        // kind): templates of up to 8192 samples (4089-4096 here) and longer ones (16377-16384)
+        // with statistics of their own: lengths near 4096 and near 16384, which stand for those up
+        // to 8192 and above, scaled by class (fft_time)
         tc->tiles = TM_TILES_FFT;
         tc->fft_skip = false;
         double fft_per[2];
@@ -682,7 +682,7 @@ int tm_bound_diagnostics(tm_ctx *ctx, const float *queries, int count, int m, fl
             TM_CUDA(cudaMemcpyAsync(dc.p, all.data(), pairs * sizeof(Candidate), cudaMemcpyHostToDevice, s));
             TM_CUDA(tmb::launch_rescore(dc.as<Candidate>(), static_cast<uint32_t>(pairs), g.tp.as<TemplParam>(),
                                         g.q.as<float>(), g.order.as<int>(), ctx->raw.as<float>(), tmb::PrefixView{}, ls.mean.as<float>(), ls.w0,
-                                        dx.as<float>(), todo.as<uint32_t>(), ctx->main.counters.as<uint32_t>() + 6, tmb::Exclusion{}, s));
+                                        dx.as<float>(), todo.as<uint32_t>(), ctx->main.counters.as<uint32_t>() + 6, tmb::Exclusion{}, ctx->sms, s));
             count_launch(ctx->main);
             TM_CUDA(cudaMemcpyAsync(exact, dx.p, pairs * sizeof(float), cudaMemcpyDeviceToHost, s));
             TM_CUDA(cudaStreamSynchronize(s));

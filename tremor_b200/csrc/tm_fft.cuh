@@ -99,10 +99,8 @@ struct FftArgs
     const double2 *tabs;          // twiddle tables of the correlation kernel
     uint64_t w0;                  // window range start (windows are relative to it)
     uint32_t W;
-    uint64_t n;                   // samples of the record
     PrefixView pv;
     const uint16_t *run;
-    const float *raw;
     const float *mean, *inv; // one length, where the prefix sums lose windows: its own statistics; else null
     uint32_t *untrusted;     // candidates for want of statistics are counted here
     uint32_t *bmin_u, *bmin_l;

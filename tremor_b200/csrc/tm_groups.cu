@@ -646,7 +646,7 @@ static size_t cheapest_split(tm_ctx *ctx, const tm_request *reqs, const std::vec
 // them when it is forced (TM_TILES_FFT); under TM_TILES_AUTO with the automatic kernel,
 // the f minimising the FFT's time of f templates + the tensor cost of the other
 // templates: the longest templates set a tile's K extent, so moving a few of them to the
-// FFT (whose cost does not grow with the length) can shorten every tile they would have
+// FFT (whose cost grows little with the length) can shorten every tile they would have
 // padded. Lengths up to 16384 (kFftMaxM); otherwise none. classes: those of their pieces.
 size_t plan_fft_split(tm_ctx *ctx, const tm_request *reqs, const std::vector<int> &sorted_idx, FftClasses &classes)
 {

@@ -286,7 +286,7 @@ void rescore_and_answer(tm_ctx *ctx, Lane &L, const GroupPlan &g, uint32_t ncand
         TM_CUDA(cudaEventRecord(L.ev2, s));
     TM_CUDA(tmb::launch_rescore(L.cand.as<Candidate>(), ncand, g.tp.as<TemplParam>(), g.q.as<float>(),
                                 g.order.as<int>(), ctx->raw.as<float>(), pv, mean, w0, L.dist.as<float>(),
-                                L.akeys.as<uint32_t>(), L.counters.as<uint32_t>() + 6, ex, s)); // (the keys come later)
+                                L.akeys.as<uint32_t>(), L.counters.as<uint32_t>() + 6, ex, ctx->sms, s)); // (the keys come later)
     if (ncand > 0)
         count_launch(L, 2);
     if (L.profile)
@@ -799,10 +799,8 @@ void fft_contract(tm_ctx *ctx, Lane &L, const GroupPlan &g, const tmb::ScanArgs 
             f.Y = L.fft_Y.as<double2>();
             f.w0 = a.w0;
             f.W = a.W;
-            f.n = a.n;
             f.pv = tmb::PrefixView{a.P, a.PT, a.PC};
             f.run = a.run;
-            f.raw = a.raw;
             f.mean = a.mean;
             f.inv = a.inv;
             f.untrusted = a.cand_count + 7;

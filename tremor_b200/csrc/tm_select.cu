@@ -829,7 +829,7 @@ cudaError_t launch_passb(const uint2 *list, const uint32_t *counters, uint32_t c
 // todo_count: its counter, zeroed here.
 cudaError_t launch_rescore(const Candidate *cand, uint32_t count, const TemplParam *tp, const float *q,
                            const int *order, const float *raw, const PrefixView &pv, const float *mean, uint64_t w0, float *dist,
-                           uint32_t *todo, uint32_t *todo_count, const Exclusion &ex, cudaStream_t s)
+                           uint32_t *todo, uint32_t *todo_count, const Exclusion &ex, int sms, cudaStream_t s)
 {
     if (count == 0)
         return cudaSuccess;
@@ -838,7 +838,7 @@ cudaError_t launch_rescore(const Candidate *cand, uint32_t count, const TemplPar
     const unsigned grid = (count - 1) / (R_THREADS / 16) + 1;
     auto *kernel = pv.Q == nullptr ? k_rescore<false, true> : mean == nullptr ? k_rescore<true, false> : k_rescore<true, true>;
     kernel<<<grid, R_THREADS, 0, s>>>(cand, count, tp, q, order, raw, pv, mean, w0, dist, todo, todo_count, ex);
-    const unsigned serial = std::min((count - 1) / S_WARPS + 1, 148u * 4u); // how many are undecided the device knows
+    const unsigned serial = std::min((count - 1) / S_WARPS + 1, 4u * (unsigned)sms); // how many are undecided the device knows
     k_rescore_serial<<<serial, S_WARPS * 32, 0, s>>>(cand, tp, q, order, raw, w0, dist, todo, todo_count);
     return cudaGetLastError();
 }
