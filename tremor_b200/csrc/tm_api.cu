@@ -27,12 +27,15 @@ static void bound_diagnostics_wm(tm_ctx *ctx, int m, const std::vector<int> &idx
     one.groups.resize(1);
     GroupPlan &g = one.groups[0];
     uint64_t h2d = 0;
-    prepare_group_mixed(ctx, L, idx, reqs.data(), g, h2d, plan_col_tile(ctx, reqs.data(), idx), false);
+    const bool fft = ctx->tiles == TM_TILES_FFT;
+    prepare_group_mixed(ctx, L, idx, reqs.data(), g, h2d, fft ? 0 : plan_col_tile(ctx, reqs.data(), idx), fft);
     const uint64_t W = g.w_max;
     if (W == 0 || W * static_cast<uint64_t>(count) > (1ull << 31))
         throw Failure{TM_ERR_ARGUMENT, "diagnostics need 0 < windows x templates <= 2^31"};
     for (int t = 0; t < g.T; t++)
         g.htp[t].thr_ed = -FLT_MAX; // emit nothing
+    if (fft)
+        prepare_fft(ctx, L, g, FftClasses());
     TM_CUDA(cudaMemcpyAsync(g.tp.p, g.htp.data(), sizeof(TemplParam) * g.T, cudaMemcpyHostToDevice, s));
     const size_t pairs = W * static_cast<size_t>(count);
     ScopedBuf dd, de, dc, dx, todo;
@@ -76,11 +79,8 @@ static void bound_diagnostics_wm(tm_ctx *ctx, int m, const std::vector<int> &idx
     a.k_stride = g.k_stride;
     a.n = ctx->n;
     a.col_tile = g.col_tile;
-    if (ctx->tiles == TM_TILES_FFT)
-    {
-        prepare_fft(ctx, L, g, FftClasses());
+    if (fft)
         fft_contract(ctx, L, g, a);
-    }
     else
     {
         TM_CUDA(g.col_tile > 0 ? tmb::launch_scan_wm(a, s) : tmb::launch_scan_umma(a, s));
