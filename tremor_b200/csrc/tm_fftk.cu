@@ -569,8 +569,8 @@ __device__ __forceinline__ float chunk_limit(const FftRow &P, float iv, float r,
 
 // The bounds of each chunk of 128 windows of m samples, a warp per chunk: the largest 1 / sd and |mu
 // - c| / sd, c the centre of the first window's prefix block, then c and 1 / m. Infinite where the
-// statistics of a window are not trusted, or it is part of a constant run, which a longer
-// template's window may leave. Bound by the loads of the prefix sums, and read only once per
+// statistics of a window are not trusted, or it is part of a constant run that a window of the lengths
+// up to the next base may leave. Bound by the loads of the prefix sums, and read only once per
 // record and length: 0.14 ms per 2^25 samples.
 __global__ void __launch_bounds__(256) k_chunk_bounds(PrefixView pv, const uint16_t *__restrict__ run, uint64_t n, int m,
                                                       double inv_m, uint32_t chunks, float4 *__restrict__ bounds)
@@ -589,8 +589,8 @@ __global__ void __launch_bounds__(256) k_chunk_bounds(PrefixView pv, const uint1
         if (w + (uint64_t)m > n)
             continue;
         const uint32_t rn = run[w];
-        if (rn == 65535u)
-            continue; // no window of any length is searched here
+        if (rn + 1u >= (uint32_t)fft_base_next(m))
+            continue; // missing, or constant for every length that takes these bounds: not searched
         WindowStats ws;
         const bool ok = rn < (uint32_t)m && window_prefix_stats(pv, pv.Q[w], pv.Q[w + m], w, m, inv_m, ws) == 0;
         const float iv = ok ? ws.iv * (1.0f + 2.0f * ws.rel_sd) : inf_f();
