@@ -101,7 +101,7 @@ static void bound_diagnostics_wm(tm_ctx *ctx, int m, const std::vector<int> &idx
         TM_CUDA(tmb::launch_rescore(dc.as<Candidate>(), static_cast<uint32_t>(pairs), g.tp.as<TemplParam>(),
                                     g.q.as<float>(), g.order.as<int>(), ctx->raw.as<float>(),
                                     tmb::PrefixView{a.P, a.PT, a.PC}, nullptr, ctx->range_first, dx.as<float>(),
-                                    todo.as<uint32_t>(), L.counters.as<uint32_t>() + 6, tmb::Exclusion{}, ctx->sms, s));
+                                    todo.as<uint32_t>(), L.counters.as<uint32_t>() + 6, tmb::Exclusion{}, m, m, ctx->sms, s));
         count_launch(L);
         TM_CUDA(cudaMemcpyAsync(exact, dx.p, pairs * sizeof(float), cudaMemcpyDeviceToHost, s));
     }
@@ -682,7 +682,7 @@ int tm_bound_diagnostics(tm_ctx *ctx, const float *queries, int count, int m, fl
             TM_CUDA(cudaMemcpyAsync(dc.p, all.data(), pairs * sizeof(Candidate), cudaMemcpyHostToDevice, s));
             TM_CUDA(tmb::launch_rescore(dc.as<Candidate>(), static_cast<uint32_t>(pairs), g.tp.as<TemplParam>(),
                                         g.q.as<float>(), g.order.as<int>(), ctx->raw.as<float>(), tmb::PrefixView{}, ls.mean.as<float>(), ls.w0,
-                                        dx.as<float>(), todo.as<uint32_t>(), ctx->main.counters.as<uint32_t>() + 6, tmb::Exclusion{}, ctx->sms, s));
+                                        dx.as<float>(), todo.as<uint32_t>(), ctx->main.counters.as<uint32_t>() + 6, tmb::Exclusion{}, m, m, ctx->sms, s));
             count_launch(ctx->main);
             TM_CUDA(cudaMemcpyAsync(exact, dx.p, pairs * sizeof(float), cudaMemcpyDeviceToHost, s));
             TM_CUDA(cudaStreamSynchronize(s));

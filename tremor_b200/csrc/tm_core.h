@@ -17,6 +17,7 @@
 #include <thread>
 #include <chrono>
 #include <cfloat>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -57,7 +58,8 @@ cudaError_t launch_passb(const uint2 *list, const uint32_t *counters, uint32_t c
                          cudaStream_t s);
 cudaError_t launch_rescore(const Candidate *cand, uint32_t count, const TemplParam *tp, const float *q,
                            const int *order, const float *raw, const PrefixView &pv, const float *mean, uint64_t w0, float *dist,
-                           uint32_t *todo, uint32_t *todo_count, const Exclusion &ex, int sms, cudaStream_t s);
+                           uint32_t *todo, uint32_t *todo_count, const Exclusion &ex, int shortest, int longest, int sms,
+                           cudaStream_t s);
 uint32_t prefix_chunks(uint64_t n);
 cudaError_t launch_prefix_totals(const float *clean, uint64_t n, const double *centres, double2 *totals,
                                  cudaStream_t s);

@@ -3,7 +3,7 @@
 // reorders), so the results are bit-identical to the reference built with
 // g++ -O2 -mfma (GCC fuses a*b+c in C++ by default):
 //   exact_stats       SkipSequential.cpp:243-259 (= indexing.cpp:128-152)
-//   replica_distance16  l2_dist_znorm_subsequence, ZnormSearch.hpp:103-165, without the
+//   replica_distance  l2_dist_znorm_subsequence, ZnormSearch.hpp:103-165, without the
 //                     early abandon (abandoning never changes the distance of a window
 //                     that ends up in an answer set: partial sums only grow)
 #pragma once
@@ -35,12 +35,58 @@ __device__ __forceinline__ void exact_stats(const float *__restrict__ raw, uint6
 }
 
 // Squared z-normalised ED of the z-normalised template q against window g: 32-sample
-// blocks in `order`, two 8-wide accumulators (acc0 for samples i..i+7, acc1 for i+8..i+15 of
-// each 16-sample step), horizontal sum in hsum256's order (ZnormSearch.hpp:92-97), then
-// the m % 32 tail sequentially. By the 16 lanes of a half warp (`lane` 0..15 of them, `half`
-// their mask): lane l < 8 is acc0[l], lane 8 + l acc1[l], so a step's 16 samples are one
-// coalesced load and every accumulator takes its terms in the reference's order. All lanes
-// return the distance.
+// blocks in `order`, lanes l of two 8-wide accumulators (acc0 for samples i..i+7,
+// acc1 for i+8..i+15 of each 16-sample step), horizontal sum in hsum256's order
+// (ZnormSearch.hpp:92-97), then the m % 32 tail sequentially.
+__device__ __forceinline__ float replica_distance(const float *__restrict__ q, const int *__restrict__ order,
+                                                  const float *__restrict__ raw, uint64_t g, int m, float mean,
+                                                  float stddev)
+{
+    if (stddev <= 1e-12f)
+        return kFltMax;
+    const float *x = raw + g;
+    const float inv = __fdiv_rn(1.0f, stddev);
+    float acc0[8], acc1[8];
+#pragma unroll
+    for (int l = 0; l < 8; l++)
+        acc0[l] = acc1[l] = 0.0f;
+    const int blocks = m / kZnormBlock;
+    for (int b = 0; b < blocks; b++)
+    {
+        const int off = order[b];
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+        {
+            const int i = off + 16 * h;
+#pragma unroll
+            for (int l = 0; l < 8; l++)
+            {
+                const float r0 = clean32(x[i + l]), r1 = clean32(x[i + 8 + l]);
+                const float d0 = __fmaf_rn(-__fsub_rn(r0, mean), inv, q[i + l]);
+                const float d1 = __fmaf_rn(-__fsub_rn(r1, mean), inv, q[i + 8 + l]);
+                acc0[l] = __fmaf_rn(d0, d0, acc0[l]);
+                acc1[l] = __fmaf_rn(d1, d1, acc1[l]);
+            }
+        }
+    }
+    float v[8];
+#pragma unroll
+    for (int l = 0; l < 8; l++)
+        v[l] = __fadd_rn(acc0[l], acc1[l]);
+    const float s0 = __fadd_rn(v[0], v[4]), s1 = __fadd_rn(v[1], v[5]);
+    const float s2 = __fadd_rn(v[2], v[6]), s3 = __fadd_rn(v[3], v[7]);
+    float dist = __fadd_rn(__fadd_rn(s0, s2), __fadd_rn(s1, s3));
+    for (int i = blocks * kZnormBlock; i < m; i++)
+    {
+        const float diff = __fmaf_rn(-__fsub_rn(clean32(x[i]), mean), inv, q[i]);
+        dist = __fmaf_rn(diff, diff, dist);
+    }
+    return dist;
+}
+
+// replica_distance by the 16 lanes of a half warp (`lane` 0..15 of them, `half` their mask):
+// lane l < 8 is acc0[l], lane 8 + l acc1[l], so a step's 16 samples are one coalesced load and
+// every accumulator takes its terms in the same order. All lanes return the distance.
 __device__ __forceinline__ float replica_distance16(const float *__restrict__ q, const int *__restrict__ order,
                                                     const float *__restrict__ raw, uint64_t g, int m, float mean,
                                                     float stddev, int lane, unsigned half)

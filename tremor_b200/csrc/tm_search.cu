@@ -254,8 +254,7 @@ static tmb::Exclusion exclusion(const Lane &L, const GroupPlan &g, uint32_t nb, 
     return ex;
 }
 
-// Exact re-scoring of a group's ncand candidates (pv: prefix sums of mixed groups, mean: window means of the others,
-// and of FFT groups with statistics of their length), answer order and kNN selection on the
+// Exact re-scoring of a group's ncand candidates (pv: prefix sums of mixed groups, mean: window means of the others), answer order and kNN selection on the
 // device, one copy to a pinned block that the result keeps, canonical answers.
 template <class Degenerate>
 void rescore_and_answer(tm_ctx *ctx, Lane &L, const GroupPlan &g, uint32_t ncand, const tmb::PrefixView &pv,
@@ -263,7 +262,10 @@ void rescore_and_answer(tm_ctx *ctx, Lane &L, const GroupPlan &g, uint32_t ncand
 {
     cudaStream_t s = L.stream;
     const int T = g.T, nk = g.nk;
-    int kcap = 1;
+    int kcap = 1, shortest = INT_MAX;
+    for (int t = 0; t < T; t++)
+        if (g.index[t] >= 0)
+            shortest = std::min(shortest, g.htp[t].m);
     for (int t = 0; t < T; t++)
         if (g.mode[t] == TM_MODE_KNN)
             kcap = std::max(kcap, g.k[t]);
@@ -286,7 +288,7 @@ void rescore_and_answer(tm_ctx *ctx, Lane &L, const GroupPlan &g, uint32_t ncand
         TM_CUDA(cudaEventRecord(L.ev2, s));
     TM_CUDA(tmb::launch_rescore(L.cand.as<Candidate>(), ncand, g.tp.as<TemplParam>(), g.q.as<float>(),
                                 g.order.as<int>(), ctx->raw.as<float>(), pv, mean, w0, L.dist.as<float>(),
-                                L.akeys.as<uint32_t>(), L.counters.as<uint32_t>() + 6, ex, ctx->sms, s)); // (the keys come later)
+                                L.akeys.as<uint32_t>(), L.counters.as<uint32_t>() + 6, ex, shortest, g.m, ctx->sms, s)); // (the keys come later)
     if (ncand > 0)
         count_launch(L, 2);
     if (L.profile)
@@ -965,7 +967,7 @@ void execute_group_mixed(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
     std::vector<float> raw;
     std::vector<uint32_t> odd; // stays empty where all samples are finite
     const tmb::PrefixView pv{ctx->prefix.as<double2>(), ctx->ptot.as<double2>(), ctx->pcen.as<double>()};
-    rescore_and_answer(ctx, L, g, ncand, pv, ls != nullptr ? ls->mean.as<float>() : nullptr, w0, exclusion(L, g, nb, blog), res, [&](int t, std::vector<Hit> &degenerate) {
+    rescore_and_answer(ctx, L, g, ncand, pv, nullptr, w0, exclusion(L, g, nb, blog), res, [&](int t, std::vector<Hit> &degenerate) {
         if (run.empty())
         {
             run.resize(W);

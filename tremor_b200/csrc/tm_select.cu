@@ -568,16 +568,16 @@ __device__ __forceinline__ bool sums_exact_stats(const float *__restrict__ x, in
     return certain_stats(a + del, em, var, ev / var * 1.01, m, mean_f, std_f);
 }
 
-// Is window w within the merge offset of a certain minimum of a listed bucket (k_passb)? The 16
-// lanes look at the buckets up to 16384 windows away: larger merge offsets exclude less than they
-// could.
-__device__ __forceinline__ bool excluded_window(const Exclusion &x, uint32_t t, uint32_t w, int merge, int lane, unsigned half)
+// Is window w within the merge offset of a certain minimum of a listed bucket (k_passb)? Lane
+// `lane` of `lanes` looks at its share of the buckets up to 16384 windows away: larger merge offsets
+// exclude less than they could.
+__device__ __forceinline__ bool excluded_window(const Exclusion &x, uint32_t t, uint32_t w, int merge, int lane, int lanes)
 {
     const uint32_t far = (uint32_t)min(merge, 16384) - 1u, bound = x.tkey[t];
     const uint32_t b0 = (w > far ? w - far : 0u) >> 8, b1 = min((uint32_t)(((uint64_t)w + far) >> 8), x.nb - 1);
     const uint32_t *l = x.bmin_l + (size_t)t * x.nb, *c = x.certain + (size_t)t * x.nb;
     bool out = false;
-    for (uint32_t b = b0 + lane; b <= b1; b += 16)
+    for (uint32_t b = b0 + lane; b <= b1; b += lanes)
     {
         const uint32_t key = l[b];
         if (key != kEmptyKey && key <= bound) // listed
@@ -586,21 +586,40 @@ __device__ __forceinline__ bool excluded_window(const Exclusion &x, uint32_t t, 
             out = out || (v != kNoWindow && v != w && __usad(v, w, 0u) <= far);
         }
     }
-    return __any_sync(half, out);
+    return out;
+}
+
+// Up to which length k_rescore_threads takes all candidates, where there are many: T_SHORT samples,
+// T_MIDDLE if the prefix sums leave more than a quarter of those sampled undecided.
+constexpr int T_SAMPLES = 4096, T_SHORT = 192, T_MIDDLE = 1024;
+__device__ __forceinline__ int thread_limit(const uint32_t *sampled)
+{
+    return *sampled > T_SAMPLES / 4 ? T_MIDDLE : T_SHORT;
+}
+
+__global__ void k_rescore_sample(const Candidate *__restrict__ cand, uint32_t count, const TemplParam *__restrict__ tp,
+                                 const PrefixView pv, uint64_t w0, uint32_t *__restrict__ sampled)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x; // < T_SAMPLES
+    const Candidate c = cand[(uint64_t)k * count / T_SAMPLES];
+    const TemplParam &p = tp[c.templ];
+    float mean_f, std_f;
+    if (p.m <= T_MIDDLE && !prefix_exact_stats(pv, w0 + c.window, p.m, p.inv_m, mean_f, std_f))
+        atomicAdd(sampled, 1u);
 }
 
 constexpr int R_THREADS = 256;
 
-// PREFIX: statistics from the prefix sums (windows of at most kPrefixBlock samples); SUMS: without
-// them, or where they do not decide, from the samples, centred by the means. todo: the undecided
-// candidates' indices, their number in *todo_count.
-template <bool PREFIX, bool SUMS>
+// PREFIX: statistics from the prefix sums (windows of at most kPrefixBlock samples), else from
+// the samples, centred by the means. todo: the undecided candidates' indices, their number in
+// *todo_count. What thread_limit leaves to k_rescore_threads is skipped.
+template <bool PREFIX>
 __global__ void __launch_bounds__(R_THREADS) k_rescore(const Candidate *__restrict__ cand, uint32_t count,
                                                        const TemplParam *__restrict__ tp, const float *__restrict__ q,
                                                        const int *__restrict__ order, const float *__restrict__ raw,
                                                        const PrefixView pv, const float *__restrict__ mean, uint64_t w0,
                                                        float *__restrict__ dist, uint32_t *__restrict__ todo,
-                                                       uint32_t *__restrict__ todo_count, const Exclusion ex)
+                                                       uint32_t *__restrict__ todo_count, const Exclusion ex, const uint32_t *__restrict__ sampled)
 {
     const uint32_t i = blockIdx.x * (R_THREADS / 16) + (threadIdx.x >> 4);
     if (i >= count)
@@ -611,7 +630,10 @@ __global__ void __launch_bounds__(R_THREADS) k_rescore(const Candidate *__restri
     const TemplParam &p = tp[c.templ];
     const uint64_t g = w0 + c.window;
     const int m = p.m;
-    if (ex.nb > 0 && p.mode == TM_MODE_KNN && p.merge > 0 && excluded_window(ex, c.templ, c.window, p.merge, lane, half))
+    if (sampled != nullptr && m <= thread_limit(sampled))
+        return;
+    if (ex.nb > 0 && p.mode == TM_MODE_KNN && p.merge > 0 &&
+        __any_sync(half, excluded_window(ex, c.templ, c.window, p.merge, lane, 16)))
     {
         if (lane == 0)
             dist[i] = kExcluded;
@@ -624,8 +646,8 @@ __global__ void __launch_bounds__(R_THREADS) k_rescore(const Candidate *__restri
         return;
     }
     float mean_f, std_f;
-    if (!(PREFIX && prefix_exact_stats(pv, g, m, p.inv_m, mean_f, std_f)) &&
-        !(SUMS && sums_exact_stats(raw + g, m, (double)mean[c.window], lane, half, mean_f, std_f)))
+    if (!(PREFIX ? prefix_exact_stats(pv, g, m, p.inv_m, mean_f, std_f)
+                 : sums_exact_stats(raw + g, m, (double)mean[c.window], lane, half, mean_f, std_f)))
     {
         if (lane == 0)
             todo[atomicAdd(todo_count, 1u)] = i;
@@ -636,7 +658,54 @@ __global__ void __launch_bounds__(R_THREADS) k_rescore(const Candidate *__restri
         dist[i] = d;
 }
 
-// The undecided candidates: four warps per SM quarter, each taking up to 16 at a time. It stages
+// Many candidates of short templates, and many undecided ones (TODO): a thread each, with both chains.
+// Where there are many, neighbours in the list are neighbours in the record, whose loads fall in the
+// same lines, and the chains of one hide behind another's. ns per candidate, by this kernel and by 16
+// lanes (most of them decided; on a record that drifts, half of them not): 100 samples, dense in the
+// record 0.13, 0.31 (0.97), one window in 30 0.25, 0.36; 400 samples 0.49, 0.45 (1.65), 0.75, 0.46;
+// 1500 samples 1.66, 1.03 (1.15).
+constexpr uint32_t T_COUNT = 1u << 16; // this many fill the multiprocessors
+constexpr int T_THREADS = 128;
+
+template <bool TODO>
+__global__ void __launch_bounds__(T_THREADS) k_rescore_threads(const Candidate *__restrict__ cand, uint32_t count,
+                                                               const TemplParam *__restrict__ tp, const float *__restrict__ q,
+                                                               const int *__restrict__ order, const float *__restrict__ raw,
+                                                               uint64_t w0, float *__restrict__ dist,
+                                                               const uint32_t *__restrict__ todo,
+                                                               const uint32_t *__restrict__ todo_count,
+                                                               const uint32_t *__restrict__ sampled, const Exclusion ex)
+{
+    const uint32_t n = TODO ? *todo_count : count;
+    if (TODO && n < T_COUNT)
+        return; // k_rescore_serial's
+    const int limit = TODO ? 0 : thread_limit(sampled);
+    for (uint64_t k = blockIdx.x * (uint64_t)T_THREADS + threadIdx.x; k < n; k += (uint64_t)gridDim.x * T_THREADS)
+    {
+        const uint32_t i = TODO ? todo[k] : (uint32_t)k;
+        const Candidate c = cand[i];
+        const TemplParam &p = tp[c.templ];
+        const int m = p.m;
+        if (!TODO)
+        {
+            if (m > limit)
+                continue;
+            const bool knn = p.mode == TM_MODE_KNN;
+            if ((ex.nb > 0 && knn && p.merge > 0 && excluded_window(ex, c.templ, c.window, p.merge, 0, 1)) ||
+                (ex.tight != nullptr && knn && p.merge <= 0 && ex.lower[i] > ex.tight[c.templ]))
+            {
+                dist[i] = kExcluded;
+                continue;
+            }
+        }
+        const uint64_t g = w0 + c.window;
+        float mean_f, std_f;
+        exact_stats(raw, g, m, mean_f, std_f);
+        dist[i] = replica_distance(q + p.q_offset, order + p.order_offset, raw, g, m, mean_f, std_f);
+    }
+}
+
+// The undecided candidates, where they are few (below `most`): four warps per SM quarter, each taking up to 16 at a time. It stages
 // 1024 samples in shared memory as doubles, split evenly between its candidates, by coalesced
 // loads one stage ahead; then lane c runs candidate c's chain over its share. (One thread per
 // candidate loading for itself costs 32 cache lines per load, and converting in the chain is
@@ -648,11 +717,13 @@ __global__ void __launch_bounds__(S_WARPS * 32) k_rescore_serial(const Candidate
                                                                 const int *__restrict__ order, const float *__restrict__ raw,
                                                                 uint64_t w0, float *__restrict__ dist,
                                                                 const uint32_t *__restrict__ todo,
-                                                                const uint32_t *__restrict__ todo_count)
+                                                                const uint32_t *__restrict__ todo_count, uint32_t most)
 {
     __shared__ double tile[S_WARPS][32 * S_LOADS + S_CANDS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t count = *todo_count, warps = gridDim.x * S_WARPS;
+    if (count >= most)
+        return; // k_rescore_threads'
     const uint32_t per = min((count + warps - 1) / warps, (uint32_t)S_CANDS);
     // samples of a candidate per stage: 64 for 16 candidates .. 1024 for one
     const int slog = 10 - (per > 1 ? 32 - __clz(per - 1) : 0), stage = 1 << slog;
@@ -824,22 +895,40 @@ cudaError_t launch_passb(const uint2 *list, const uint32_t *counters, uint32_t c
     return cudaGetLastError();
 }
 
-// pv: the prefix sums, when the group's windows have them (Q not null); mean: the windows' means, near
-// enough to centre their sums, or null; one of the two is there. todo: scratch of `count` indices;
-// todo_count: its counter, zeroed here.
+// pv: the prefix sums, when the group's windows have them (Q not null); else mean: the
+// windows' means, near enough to centre their sums. shortest, longest: of the templates. todo: scratch
+// of `count` indices; todo_count: its counter and one more, zeroed here.
 cudaError_t launch_rescore(const Candidate *cand, uint32_t count, const TemplParam *tp, const float *q,
                            const int *order, const float *raw, const PrefixView &pv, const float *mean, uint64_t w0, float *dist,
-                           uint32_t *todo, uint32_t *todo_count, const Exclusion &ex, int sms, cudaStream_t s)
+                           uint32_t *todo, uint32_t *todo_count, const Exclusion &ex, int shortest, int longest, int sms,
+                           cudaStream_t s)
 {
     if (count == 0)
         return cudaSuccess;
-    if (const cudaError_t e = cudaMemsetAsync(todo_count, 0, sizeof(uint32_t), s); e != cudaSuccess)
+    if (const cudaError_t e = cudaMemsetAsync(todo_count, 0, 2 * sizeof(uint32_t), s); e != cudaSuccess)
         return e;
+    const bool many = count >= T_COUNT, prefix = pv.Q != nullptr;
+    uint32_t *sampled = many ? todo_count + 1 : nullptr;
+    const unsigned threads = std::min((count - 1) / T_THREADS + 1, 64u * (unsigned)sms);
+    if (many && shortest <= T_MIDDLE)
+    {
+        if (prefix && longest > T_SHORT)
+            k_rescore_sample<<<T_SAMPLES / 256, 256, 0, s>>>(cand, count, tp, pv, w0, sampled);
+        k_rescore_threads<false><<<threads, T_THREADS, 0, s>>>(cand, count, tp, q, order, raw, w0, dist, todo, todo_count, sampled,
+                                                               ex);
+        if (longest <= T_SHORT)
+            return cudaGetLastError();
+    }
     const unsigned grid = (count - 1) / (R_THREADS / 16) + 1;
-    auto *kernel = pv.Q == nullptr ? k_rescore<false, true> : mean == nullptr ? k_rescore<true, false> : k_rescore<true, true>;
-    kernel<<<grid, R_THREADS, 0, s>>>(cand, count, tp, q, order, raw, pv, mean, w0, dist, todo, todo_count, ex);
-    const unsigned serial = std::min((count - 1) / S_WARPS + 1, 4u * (unsigned)sms); // how many are undecided the device knows
-    k_rescore_serial<<<serial, S_WARPS * 32, 0, s>>>(cand, tp, q, order, raw, w0, dist, todo, todo_count);
+    auto *kernel = prefix ? k_rescore<true> : k_rescore<false>;
+    kernel<<<grid, R_THREADS, 0, s>>>(cand, count, tp, q, order, raw, pv, mean, w0, dist, todo, todo_count, ex, sampled);
+    // how many are undecided the device knows
+    if (many)
+        k_rescore_threads<true><<<threads, T_THREADS, 0, s>>>(cand, count, tp, q, order, raw, w0, dist, todo, todo_count, sampled,
+                                                              ex);
+    const unsigned serial = std::min((count - 1) / S_WARPS + 1, 4u * (unsigned)sms);
+    k_rescore_serial<<<serial, S_WARPS * 32, 0, s>>>(cand, tp, q, order, raw, w0, dist, todo, todo_count,
+                                                     many ? T_COUNT : 0xffffffffu);
     return cudaGetLastError();
 }
 
