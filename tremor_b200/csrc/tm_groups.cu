@@ -595,9 +595,9 @@ static bool bounds_fit(tm_ctx *ctx, const std::vector<int> &m)
 // blocks end alone in place of one (128 templates of 1024 on 400000 windows: 0.30 ms with one cut,
 // 0.19 by the times above; the row tiles take 0.24).
 constexpr double kCutMs = 0.06;
-// And of a second group: a selection, re-pass, re-scoring and copy of its own, a dozen launches and two
-// waits of the host.
-constexpr double kGroupMs = 0.12;
+// And of a second group: a re-scoring, sort and copy of its own, a dozen launches and two waits of the
+// host (200 thresholds of 700 on 2^21 samples, in one group and in two).
+constexpr double kGroupMs = 0.07;
 
 // The f of the least modelled time (plan_fft_split), pieces by these classes; m: the lengths. Which
 // templates skip windows is decided as fft_contract does, per class and number of parts, from the
