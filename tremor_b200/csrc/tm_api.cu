@@ -138,9 +138,11 @@ int tm_ctx_create(const float *raw, uint64_t n, int device, tm_ctx **out)
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = device;
-        TM_CUDA(cudaMemPoolCreate(&ctx->pool, &props));
+        ctx->pool = std::make_shared<MemPool>();
+        ctx->pool->device = device;
+        TM_CUDA(cudaMemPoolCreate(&ctx->pool->handle, &props));
         uint64_t keep = 4ull << 30;
-        TM_CUDA(cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep));
+        TM_CUDA(cudaMemPoolSetAttribute(ctx->pool->handle, cudaMemPoolAttrReleaseThreshold, &keep));
         ctx->main.open();
         const uint64_t total = n + tmb::kStagePad;
         ctx->raw.reserve(sizeof(float) * total);
@@ -192,11 +194,7 @@ int tm_ctx_destroy(tm_ctx *ctx)
             b->release();
     for (tm_ctx::FftBounds &b : ctx->fft_bounds)
         b.buf.reset();
-    // buffers of batches that outlive the context return to the pool when those batches
-    // are destroyed; the driver releases the pool's memory once none is outstanding
-    if (ctx->pool)
-        cudaMemPoolDestroy(ctx->pool);
-    delete ctx;
+    delete ctx; // its pool stays until the last batch that outlives it is destroyed (MemPool)
     return TM_OK;
 }
 

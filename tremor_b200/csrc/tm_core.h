@@ -111,12 +111,35 @@ inline Failure failure(cudaError_t e, const char *call)
             throw tmh::failure(e_, #call);                                                                        \
     } while (0)
 
+// A context's memory pool. Every buffer from it holds it, so that it is destroyed after the last one
+// was freed, whether the context or a batch goes first: a pool destroyed with buffers outstanding
+// left the driver in a state in which a later cuCtxSynchronize of the process crashed (580.159).
+struct MemPool
+{
+    cudaMemPool_t handle = nullptr;
+    int device = 0;
+    MemPool() = default;
+    MemPool(const MemPool &) = delete;
+    MemPool &operator=(const MemPool &) = delete;
+    ~MemPool()
+    {
+        if (handle == nullptr)
+            return;
+        int current = 0;
+        cudaGetDevice(&current);
+        cudaSetDevice(device);
+        cudaStreamSynchronize(0); // the last buffers' frees (a context waits for its own streams)
+        cudaMemPoolDestroy(handle);
+        cudaSetDevice(current);
+    }
+};
+
 // Grow-only device buffer.
 struct DevBuf
 {
     void *p = nullptr;
     size_t bytes = 0;
-    bool pooled = false; // from the device's memory pool (reserve_on)
+    std::shared_ptr<MemPool> from; // the memory pool that it is from (reserve_on), if any
     void reserve(size_t need)
     {
         if (need <= bytes)
@@ -131,15 +154,15 @@ struct DevBuf
     // synchronisation and unmapping of cudaFree (tens of milliseconds with a large
     // context), and the next batch's allocation takes it back from there. A buffer that
     // grows is freed after the work already queued on s.
-    void reserve_on(size_t need, cudaStream_t s, cudaMemPool_t pool)
+    void reserve_on(size_t need, cudaStream_t s, const std::shared_ptr<MemPool> &pool)
     {
         if (need <= bytes)
             return;
         drop(s);
         size_t b = std::max<size_t>(need, 256);
-        TM_CUDA(cudaMallocFromPoolAsync(&p, b, pool, s));
+        TM_CUDA(cudaMallocFromPoolAsync(&p, b, pool->handle, s));
         bytes = b;
-        pooled = true;
+        from = pool;
     }
     template <class T> T *as() const { return static_cast<T *>(p); }
     // Callers release only after the work that used the buffer has completed.
@@ -152,14 +175,14 @@ struct DevBuf
     {
         if (p)
         {
-            if (pooled)
+            if (from)
                 cudaFreeAsync(p, s);
             else
                 cudaFree(p);
         }
         p = nullptr;
         bytes = 0;
-        pooled = false;
+        from.reset();
     }
 };
 
@@ -396,7 +419,7 @@ struct tm_ctx
     double fft_long_ms = 0.63;
     // the context's own memory pool for per-batch buffers (DevBuf::reserve_on); it keeps
     // up to 4 GiB of freed memory for the next batch
-    cudaMemPool_t pool = nullptr;
+    std::shared_ptr<tmh::MemPool> pool;
     std::string err;
     tmh::Lane main;                      // the synchronous calls' lane
     // serving engine, while started; replaced only under server_mu, and the serving calls
