@@ -91,4 +91,4 @@ def test_two_parts_skip_windows(mode):
         answers = ctx.scan_batch(reqs)
         ctx.set_tiles(tb.TILES_ROWS)
         _same(answers, ctx.scan_batch(reqs))
-    _check(x, reqs[-2:], answers[-2:])
+    _check(x, reqs[1:2], answers[1:2])

@@ -22,7 +22,7 @@ def _record(n, slope, rng):
 
 @pytest.mark.parametrize('slope', [0.0, 0.05])
 @pytest.mark.parametrize('m,templates,correlation', [(33, 1, 0.9), (192, 2, 0.1), (193, 2, 0.1), (400, 1, 0.9995), (400, 6, 0.7),
-                                                     (1000, 3, 0.9), (1025, 3, 0.6), (16000, 2, 0.9)])
+                                                     (1000, 3, 0.9), (1025, 2, 0.6), (16000, 1, 0.9)])
 def test_thresholds_and_few_answers(m, templates, correlation, slope):
     rng = np.random.default_rng(m + templates)
     x = _record(150_000, slope, rng)
