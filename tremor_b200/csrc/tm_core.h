@@ -225,7 +225,7 @@ struct LengthStats
 {
     int m = 0;
     uint64_t w0 = 0, W = 0;
-    DevBuf mean, inv, flags;
+    ScopedBuf mean, inv, flags;
     uint64_t last_use = 0;
     size_t bytes() const { return mean.bytes + inv.bytes + flags.bytes; }
 };

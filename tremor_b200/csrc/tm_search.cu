@@ -879,7 +879,7 @@ void execute_group_mixed(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
     // time so than the statistics of the length and another contraction, it has these (they stay, for the
     // next searches): 130 templates of 1500 on 2^17 samples, 4000 of them 10^5 times the rest: 25 ms
     // with prefix sums alone, 2.3 with both. (The context keeps these statistics for its own lane only.)
-    const bool one_length = g.fft && &L == &ctx->main && g.htp[0].m == g.htp[T - 1].m;
+    bool one_length = g.fft && &L == &ctx->main && g.htp[0].m == g.htp[T - 1].m;
     LengthStats *ls = one_length && ctx->lengths.count(g.m) > 0 ? &ensure_length(ctx, L, g.m) : nullptr;
     const double chain_ms = 1.8e-9 * g.m; // of a candidate without statistics
     const double again_ms = 0.1 + static_cast<double>(W) / 33554432.0 * (1.0 + 0.15 * T);
@@ -953,9 +953,18 @@ void execute_group_mixed(tm_ctx *ctx, Lane &L, GroupPlan &g, tm_result &res)
         ncand = collect_candidates(ctx, L, g, a, true);
         if (one_length && ls == nullptr && chain_ms * L.h_counters.as<uint32_t>()[7] > again_ms)
         {
-            ls = &ensure_length(ctx, L, g.m);
-            attempt--;
-            continue;
+            try
+            {
+                ls = &ensure_length(ctx, L, g.m);
+                attempt--;
+                continue;
+            }
+            catch (const Failure &f)
+            {
+                if (f.code != TM_ERR_NO_MEMORY)
+                    throw;
+                one_length = false; // as slow as it is, then
+            }
         }
         if (ncand <= L.cand_cap)
             break;
