@@ -25,8 +25,10 @@ static_assert(kPrefixBlock % PX_CHUNK == 0, "chunks tile the prefix blocks");
 
 __device__ __forceinline__ double2 add2(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 
-// Block-wide inclusive scan of one double2 per thread.
-__device__ double2 block_scan(double2 v, double2 *warp_tot)
+// Block-wide scan of one double2 per thread: the sum up to this thread's, and in *before that of the
+// threads before it, by the same additions (the former less the thread's own would carry the rounding
+// of samples that lie after those that it covers).
+__device__ double2 block_scan(double2 v, double2 *warp_tot, double2 *before = nullptr)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
@@ -52,6 +54,13 @@ __device__ double2 block_scan(double2 v, double2 *warp_tot)
         warp_tot[lane] = w; // inclusive warp totals
     }
     __syncthreads();
+    if (before != nullptr)
+    {
+        const double a = __shfl_up_sync(0xffffffffu, v.x, 1), b = __shfl_up_sync(0xffffffffu, v.y, 1);
+        *before = lane > 0 ? make_double2(a, b) : make_double2(0.0, 0.0);
+        if (warp > 0)
+            *before = add2(*before, warp_tot[warp - 1]);
+    }
     if (warp > 0)
         v = add2(v, warp_tot[warp - 1]);
     return v;
@@ -115,9 +124,9 @@ __global__ void __launch_bounds__(PX_THREADS) k_prefix_apply(const float *__rest
     __shared__ double2 warp_tot[32];
     double2 vals[PX_PER_THREAD];
     const uint64_t base = (uint64_t)blockIdx.x * PX_CHUNK + (uint64_t)threadIdx.x * PX_PER_THREAD;
-    const double2 s = chunk_values(clean, n, centres, base, vals);
-    const double2 inc = block_scan(s, warp_tot);
-    double2 run = add2(offsets[blockIdx.x], make_double2(inc.x - s.x, inc.y - s.y));
+    double2 before;
+    block_scan(chunk_values(clean, n, centres, base, vals), warp_tot, &before);
+    double2 run = add2(offsets[blockIdx.x], before);
 #pragma unroll
     for (int k = 0; k < PX_PER_THREAD; k++)
     {
