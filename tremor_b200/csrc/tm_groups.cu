@@ -573,16 +573,21 @@ static bool fft_classes(tm_ctx *ctx, const std::vector<int> &m, FftClasses &clas
 // many times what a device with little memory left would refuse.)
 static bool bounds_fit(tm_ctx *ctx, const std::vector<int> &m)
 {
+    const size_t each = sizeof(float4) * tmb::fft_chunks(ctx->n), little = 64ull << 20;
+    if (each * std::min<size_t>(m.size(), tmb::kFftBases) < little)
+        return true;
     std::lock_guard<std::mutex> lk(ctx->fft_mu);
-    const size_t each = sizeof(float4) * tmb::fft_chunks(ctx->n);
     size_t asked = 0, fresh = 0, resident = 0;
+    int last = -1; // base of the length before
     for (size_t i = 0; i < m.size(); i++)
-        if (i == 0 || tmb::fft_base(m[i]) != tmb::fft_base(m[i - 1])) // by length
+        if (i == 0 || m[i] != m[i - 1])
         {
-            asked += each;
-            fresh += ctx->fft_bounds[tmb::fft_base(m[i])].buf ? 0 : each;
+            const int base = tmb::fft_base(m[i]);
+            asked += base != last ? each : 0;
+            fresh += base != last && !ctx->fft_bounds[base].buf ? each : 0;
+            last = base;
         }
-    if (fresh < (64ull << 20))
+    if (fresh < little)
         return true;
     for (const tm_ctx::FftBounds &b : ctx->fft_bounds)
         resident += b.buf ? each : 0;

@@ -657,10 +657,10 @@ static bool ensure_bounds(tm_ctx *ctx, Lane &L, const GroupPlan &g, int first, i
         if (!ctx->fft_bounds[base].buf)
             fresh.push_back(base);
     }
-    for (const tm_ctx::FftBounds &b : ctx->fft_bounds)
-        resident += b.buf ? each : 0;
     if (!fresh.empty())
     {
+        for (const tm_ctx::FftBounds &b : ctx->fft_bounds)
+            resident += b.buf ? each : 0;
         size_t free_b = 0, total_b = 0;
         TM_CUDA(cudaMemGetInfo(&free_b, &total_b));
         const size_t budget = (free_b + resident) / 10, more = each * fresh.size();

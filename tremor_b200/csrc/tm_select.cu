@@ -422,11 +422,11 @@ template <bool MIXED> __global__ void __launch_bounds__(B_THREADS) k_passb(const
             atomicAdd(&a.bins[(size_t)t * kTightBins + min((int)(fmaxf(upper, 0.0f) * ((float)kTightBins / T)), kTightBins - 1)],
                       1u);
         const unsigned ballot = __ballot_sync(0xffffffffu, hit);
-        const unsigned lost = __ballot_sync(0xffffffffu, hit && lower == -inf_f());
-        if (lost != 0u && lane == 0)
-            atomicAdd(a.untrusted, (uint32_t)__popc(lost));
         if (ballot != 0u)
         {
+            const unsigned lost = MIXED ? __ballot_sync(0xffffffffu, hit && lower == -inf_f()) : 0u;
+            if (lost != 0u && lane == 0)
+                atomicAdd(a.untrusted, (uint32_t)__popc(lost));
             uint32_t base = 0;
             if (lane == 0)
                 base = atomicAdd(a.cand_count, (uint32_t)__popc(ballot));
